@@ -10,7 +10,7 @@ import sys
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
-SRC = ["capi.cu", "fft.cu", "gemm.cu", "ortho.cu", "tc.cu", "serve.cu", "tune.cu", "restart.cu", "vofrho.cu"]
+SRC = ["capi.cu", "fft.cu", "gemm.cu", "fold.cu", "ortho.cu", "tc.cu", "serve.cu", "tune.cu", "restart.cu", "vofrho.cu"]
 HDR = ["cuwaves_internal.cuh", "tc_sm100.cuh", "tc_pipe.cuh"]
 OUT = os.path.join(HERE, "lib", "libcuwaves.so")
 OBJ = os.path.join(HERE, "lib", "obj")

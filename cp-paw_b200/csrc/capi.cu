@@ -26,7 +26,6 @@ int ortho_y_run(Handle* h, const double* s, double* x);
 int ortho_y_general(Handle* h, const double* s1, const double* s2, const double* s3, const int* map, double* x,
                     bool clear_status);
 int smap_run(Handle* h);
-int fold_x_run(Handle* h, const double* x, double2* x1, double2* x2);
 
 namespace {
 
@@ -200,14 +199,16 @@ struct Fric {
 };
 __global__ void k_anneevec(const double* __restrict__ gx, const double* __restrict__ gy,
                            const double* __restrict__ gz, const double* __restrict__ dbucket, int ngl, Fric fm,
-                           double fac1, double fac2, double* __restrict__ anv) {
+                           double fac1, double fac2, double* __restrict__ anv, double* __restrict__ aninv) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= ngl) return;
   const double* F = fm.f;
   const double x = gx[g], y = gy[g], z = gz[g];
   const double svar = F[0] * x * x + F[3] * 2.0 * x * y + F[6] * 2.0 * x * z + F[4] * y * y + F[7] * 2.0 * y * z +
                       F[8] * z * z;
-  anv[g] = fac1 + fac2 * svar * (1.0 + (dbucket ? dbucket[g] : 0.0));
+  const double an = fac1 + fac2 * svar * (1.0 + (dbucket ? dbucket[g] : 0.0));
+  anv[g] = an;
+  aninv[g] = 1.0 / (1.0 + an);
 }
 
 // DEDPROJ = F1 HPROJ + F2 conj(HPROJ) per super wave function (src/paw_waves1.f90:5644-5668)
@@ -269,11 +270,6 @@ __global__ void k_batch_out(const double* __restrict__ scal, const int* __restri
 __global__ void k_add_vec(double* __restrict__ a, const double* __restrict__ b, int n) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) a[i] += b[i];
-}
-
-__global__ void k_copy_psi(const double2* __restrict__ src, double2* __restrict__ dst, size_t n) {
-  for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
-    dst[k] = src[k];
 }
 
 }  // namespace
@@ -353,7 +349,7 @@ static int friction_update(Handle* h) {
   std::memcpy(fm.f, F, sizeof(fm.f));
   k_anneevec<<<ceil_div(h->d.ngl, 256), 256, 0, h->stream>>>(h->g.gx, h->g.gy, h->g.gz,
                                                              h->have_dbucket ? h->g.dbucket : nullptr, h->d.ngl,
-                                                             fm, fac1, fac2, h->g.anv);
+                                                             fm, fac1, fac2, h->g.anv, h->g.aninv);
   CUW_LAUNCH_CHECK("k_anneevec");
   return CUW_OK;
 }
@@ -377,16 +373,17 @@ static int force_dev_run(Handle* h, double* force_dev) {
   CUW_LAUNCH_CHECK("k_dedproj");
   k_force_lambda<<<ceil_div(nb * nb, 256), 256, 0, h->stream>>>(g.rlam0, g.occ, nb, g.wk2);
   CUW_LAUNCH_CHECK("k_force_lambda");
-  CUW_RET(lambda12_run(h, g.wk2, g.lam1c, g.lam2c));
-  CUW_RET(addoproj_run(h, g.hproj, g.oproj, g.lam1c, g.lam2c));
+  CUW_RET(addoproj_run(h, g.hproj, g.oproj, g.wk2));
   CUW_RET(force_gemm(h, g.hproj, force_dev));
   return CUW_OK;
 }
 
 // the part of WAVES$ORTHOGONALIZE after OPSI is formed (src/paw_waves2.f90:242-490)
 static int mark(Handle* h, int phase);
-// (enqueues only: the solve's status is read with the step's results)
-static int ortho_core(Handle* h, int max_iter, double eps) {
+// (enqueues only: the solve's status is read with the step's results).
+// fused: the step's ADDPRO has formed PSIM and OPSI (and left them folded in
+// slots 0 and 1 where it is the folded form)
+static int ortho_core(Handle* h, int max_iter, double eps, bool fused) {
   Device& g = h->g;
   // projections of PSIBAR and OPSI at R(+)
   CUW_RET(mark(h, 1));
@@ -401,21 +398,30 @@ static int ortho_core(Handle* h, int max_iter, double eps) {
     }
   } guard{h->mixed() ? h : nullptr};
   if (h->mixed()) tc_scope(h, true);
-  CUW_RET(proj_compute(h, g.psim, g.proj, g.opsi, g.oproj));
+  if (!h->tc_on() && !(fused && h->sym)) {
+    CUW_RET(fold_psi(h, g.psim, 0));
+    CUW_RET(fold_psi(h, g.opsi, 1));
+  }
+  CUW_RET(proj_compute(h, g.psim, g.proj, g.opsi, g.oproj, true));
   CUW_RET(mark(h, 6));
   // DO*PROJ and DO*OPROJ
   CUW_RET(oproj_compute(h, g.proj, g.hproj));
   CUW_RET(oproj_compute(h, g.oproj, g.pbuf));
-  const size_t mn = (size_t)h->d.nbh * h->d.nbh;
-  double2* pw = g.tmat;
-  double2* oc = g.tmat + 6 * mn;
-  GramPair pc[3] = {{g.proj, g.hproj}, {g.oproj, g.hproj}, {g.oproj, g.pbuf}};
-  CUW_RET(gram_projections(h, pc, 3, oc));
-  GramPair pp[3] = {{g.psim, g.psim}, {g.opsi, g.psim}, {g.opsi, g.opsi}};
-  CUW_RET(gram_planewave(h, pp, 3, pw));
+  if (h->tc_on()) {
+    const size_t mn = (size_t)h->d.nbh * h->d.nbh;
+    double2* pw = g.tmat;
+    double2* oc = g.tmat + 6 * mn;
+    GramPair pc[3] = {{g.proj, g.hproj}, {g.oproj, g.hproj}, {g.oproj, g.pbuf}};
+    CUW_RET(tc_gram(h, pc, 3, false, h->npro, h->d.nbh, (size_t)h->d.nbh, 1, 1.0, oc));
+    GramPair pp[3] = {{g.psim, g.psim}, {g.opsi, g.psim}, {g.opsi, g.opsi}};
+    CUW_RET(tc_gram(h, pp, 3, true, h->d.ngl, h->d.nbh, 1, (size_t)h->ldg, h->gweight, pw));
+    CUW_RET(unravel_run(h, pw, oc, 3, g.mat, g.omat, g.oomat));
+  } else {
+    const FoldPair pp[3] = {{0, 0, g.proj, g.hproj}, {1, 0, g.oproj, g.hproj}, {1, 1, g.oproj, g.pbuf}};
+    CUW_RET(fold_gram(h, pp, 3, g.mat, g.omat, g.oomat));
+  }
   if (h->mixed()) tc_scope(h, false);
   guard.h = nullptr;
-  CUW_RET(unravel_run(h, pw, oc, 3, g.mat, g.omat, g.oomat));
   CUW_RET(mark(h, 7));
   if (h->safeortho) {
     CUW_RET(lambda_init_run(h));
@@ -429,9 +435,14 @@ static int ortho_core(Handle* h, int max_iter, double eps) {
     CUW_RET(ortho_y_general(h, g.mat, g.omat, g.oomat, h->swapstates ? g.smap : nullptr, g.lam, !h->swapstates));
   }
   CUW_RET(mark(h, 8));
-  CUW_RET(lambda12_run(h, g.lam, g.lam1c, g.lam2c));
-  CUW_RET(addopsi_run(h, g.psim, g.opsi, g.lam1c, g.lam2c));
-  CUW_RET(addoproj_run(h, g.proj, g.oproj, g.lam1c, g.lam2c));
+  if (h->tc_on()) {
+    CUW_RET(lambda12_run(h, g.lam, g.lam1c, g.lam2c));
+    CUW_RET(tc_addx(h, true, g.psim, g.opsi, g.lam1c, g.lam2c, h->d.ngl, h->d.nbh, h->d.nbh, 1, (size_t)h->ldg, 1,
+                    (size_t)h->ldg));
+  } else {
+    CUW_RET(fold_addx(h, 1, g.lam, g.psim));
+  }
+  CUW_RET(addoproj_run(h, g.proj, g.oproj, g.lam));
   CUW_RET(store_lambda_run(h));
   h->have_opsi = false;
   return CUW_OK;
@@ -501,7 +512,7 @@ static void free_all(Handle* h) {
                   g.t_nlmn, g.t_isp, g.t_lnofp, g.t_mofp, g.t_lmn0ln, g.t_lox, g.pf, g.xminus[0], g.xminus[1], g.bpre[0],
                   g.bpre[1], g.bsmall, g.jac_a, g.r_plus, g.r_minus, g.r_gx, g.r_gy, g.r_gz, g.r_g2, g.r_ylm,
                   g.r_g0, g.r_v0, g.r_pscore, g.r_vbar, g.r_lmrx, g.qlm, g.r_rhog, g.r_vg, g.r_pot, g.r_vtot,
-                  g.r_grid, g.r_part, g.fpot, g.vqlm, g.r_out, g.prox, g.anv, g.dbucket};
+                  g.r_grid, g.r_part, g.fpot, g.vqlm, g.r_out, g.half, g.prox, g.uf, g.anv, g.aninv, g.dbucket, g.rmpsi};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   h->g = Device();
@@ -593,14 +604,13 @@ extern "C" int cuwaves_create(const cuw_dims* dims, cuw_handle** out) {
     TRYA(g.rlam0, nn * sizeof(double2)); TRYA(g.rlamm, nn * sizeof(double2));
     TRYA(g.igvec, sizeof(int) * 3 * d.ngl); TRYA(g.minusg, sizeof(int) * d.ngl);
     TRYA(g.gx, sizeof(double) * d.ngl); TRYA(g.gy, sizeof(double) * d.ngl); TRYA(g.gz, sizeof(double) * d.ngl);
-    TRYA(g.g2, sizeof(double) * d.ngl); TRYA(g.mpsi, sizeof(double) * d.ngl);
+    TRYA(g.g2, sizeof(double) * d.ngl); TRYA(g.mpsi, sizeof(double) * d.ngl); TRYA(g.rmpsi, sizeof(double) * d.ngl);
     TRYA(g.pro, sizeof(double) * d.ngl * (size_t)nbare); TRYA(g.ylm, sizeof(double) * d.ngl * (size_t)d.lmx);
     TRYA(g.pdesc, sizeof(ProDesc) * std::max(1, h->npro));
     TRYA(g.v, sizeof(double) * h->nr);
     TRYA(g.r0, sizeof(double) * 3 * std::max(1, d.nat)); TRYA(g.rp, sizeof(double) * 3 * std::max(1, d.nat));
     TRYA(g.rm, sizeof(double) * 3 * std::max(1, d.nat)); TRYA(g.force, sizeof(double) * 3 * std::max(1, d.nat));
     TRYA(g.mass, sizeof(double) * std::max(1, d.nat));
-    TRYA(g.eigr, sizeof(double2) * d.ngl * (size_t)std::max(1, d.nat));
     TRYA(g.dh, sizeof(double2) * (size_t)h->lmnxx * h->lmnxx * std::max(1, d.nat));
     TRYA(g.dover, sizeof(double) * (size_t)h->lnxx * h->lnxx * d.nsp);
     TRYA(g.occ, sizeof(double) * d.nb);
@@ -733,6 +743,8 @@ extern "C" int cuwaves_set_gset(cuw_handle* hp, const int* igvec, const int* min
   CUW_TRY(cudaMemcpy(g.pro, pro, sizeof(double) * ngl * (size_t)h->nbarepro, cudaMemcpyHostToDevice));
   CUW_TRY(cudaMemcpy(g.ylm, ylm, sizeof(double) * ngl * (size_t)h->d.lmx, cudaMemcpyHostToDevice));
   CUW_TRY(cudaMemcpy(g.mpsi, mpsi, sizeof(double) * ngl, cudaMemcpyHostToDevice));
+  for (int i = 0; i < ngl; ++i) x[i] = 1.0 / mpsi[i];
+  CUW_TRY(cudaMemcpy(g.rmpsi, x.data(), sizeof(double) * ngl, cudaMemcpyHostToDevice));
   if (bucket) {
     if (!g.bucket) CUW_TRY(cudaMalloc(&g.bucket, sizeof(double) * ngl));
     CUW_TRY(cudaMemcpy(g.bucket, bucket, sizeof(double) * ngl, cudaMemcpyHostToDevice));
@@ -741,6 +753,7 @@ extern "C" int cuwaves_set_gset(cuw_handle* hp, const int* igvec, const int* min
     h->tbucket = false;
   }
   CUW_RET(fft_setup(h, igvec));
+  CUW_RET(fold_setup(h, mg));
   h->have_gset = true;
   return friction_update(h);
 }
@@ -849,6 +862,7 @@ extern "C" int cuwaves_set_cell_friction(cuw_handle* hp, const double* fricmat, 
   Device& g = h->g;
   const size_t nb = sizeof(double) * h->d.ngl;
   if (!g.anv) CUW_TRY(cudaMalloc(&g.anv, nb));
+  if (!g.aninv) CUW_TRY(cudaMalloc(&g.aninv, nb));
   if (dbucket) {
     if (!g.dbucket) CUW_TRY(cudaMalloc(&g.dbucket, nb));
     CUW_TRY(cudaMemcpy(g.dbucket, dbucket, nb, cudaMemcpyHostToDevice));
@@ -1027,7 +1041,7 @@ extern "C" int cuwaves_orthogonalize(cuw_handle* hp, int max_iter, double eps, i
   CUW_RET(oproj_compute(h, h->g.proj, h->g.oproj));
   CUW_RET(eigr_compute(h, h->g.r0));
   CUW_RET(addpro_run(h, ADDPRO_OPSI, nullptr, h->g.oproj));
-  CUW_RET(ortho_core(h, max_iter, eps));
+  CUW_RET(ortho_core(h, max_iter, eps, false));
   int st[2];
   CUW_TRY(cudaMemcpyAsync(st, h->g.ostatus, sizeof(st), cudaMemcpyDeviceToHost, h->stream));
   CUW_TRY(cudaStreamSynchronize(h->stream));
@@ -1078,21 +1092,12 @@ extern "C" int cuwaves_gramschmidt(cuw_handle* hp, int which, const double* r) {
   CUW_RET(eigr_compute(h, rd));
   CUW_RET(proj_compute(h, psi, g.hproj, nullptr, nullptr));
   CUW_RET(oproj_compute(h, g.hproj, g.pbuf));
-  const size_t mn = (size_t)h->d.nbh * h->d.nbh;
-  double2* pw = g.tmat;
-  double2* oc = g.tmat + 6 * mn;
-  GramPair pc[1] = {{g.hproj, g.pbuf}};
-  CUW_RET(gram_projections(h, pc, 1, oc));
-  GramPair pp[1] = {{psi, psi}};
-  CUW_RET(gram_planewave(h, pp, 1, pw));
-  CUW_RET(unravel_run(h, pw, oc, 1, g.mat, nullptr, nullptr));
+  if (!h->sym) CUW_RET(fold_psi(h, psi, 0));  // else proj_compute has folded it
+  const FoldPair pp[1] = {{0, 0, g.hproj, g.pbuf}};
+  CUW_RET(fold_gram(h, pp, 1, g.mat, nullptr, nullptr));
   CUW_RET(ortho_y_run(h, g.mat, g.wk2));
-  CUW_RET(fold_x_run(h, g.wk2, g.lam1c, g.lam2c));
-  // PSIINV = PSI (copy into OPSI), PSI += PSIINV X1 + PSIINV(-) X2
-  size_t n = (size_t)h->ldg * h->d.nbh;
-  k_copy_psi<<<4 * h->nsm, 256, 0, h->stream>>>(psi, g.opsi, n);
-  CUW_LAUNCH_CHECK("k_copy_psi");
-  CUW_RET(addopsi_run(h, psi, g.opsi, g.lam1c, g.lam2c));
+  // PSI += PSI X, from the folded copy
+  CUW_RET(fold_addx(h, 0, g.wk2, psi));
   int st = 0;
   CUW_TRY(cudaMemcpyAsync(&st, g.ostatus, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
   CUW_TRY(cudaStreamSynchronize(h->stream));
@@ -1122,18 +1127,13 @@ extern "C" int cuwaves_overlap_check(cuw_handle* hp, double* mat, double* maxdev
     ~Fp64() { h->fp64_only = old; }
   } fp64{h, h->fp64_only};
   h->fp64_only = true;
-  const int nb = h->d.nb, nbh = h->d.nbh;
-  const size_t mn = (size_t)nbh * nbh;
+  const int nb = h->d.nb;
   CUW_RET(eigr_compute(h, g.r0));
   CUW_RET(proj_compute(h, g.psi0, g.pbuf, nullptr, nullptr));
   CUW_RET(oproj_compute(h, g.pbuf, g.hproj));
-  double2* pw = g.tmat;
-  double2* oc = g.tmat + 2 * mn;
-  GramPair pc[1] = {{g.pbuf, g.hproj}};
-  CUW_RET(gram_projections(h, pc, 1, oc));
-  GramPair pp[1] = {{g.psi0, g.psi0}};
-  CUW_RET(gram_planewave(h, pp, 1, pw));
-  CUW_RET(unravel_run(h, pw, oc, 1, g.wk2, nullptr, nullptr));
+  if (!h->sym) CUW_RET(fold_psi(h, g.psi0, 0));  // else proj_compute has folded it
+  const FoldPair pp[1] = {{0, 0, g.pbuf, g.hproj}};
+  CUW_RET(fold_gram(h, pp, 1, g.wk2, nullptr, nullptr));
   std::vector<double> m((size_t)nb * nb);
   CUW_TRY(cudaMemcpyAsync(m.data(), g.wk2, sizeof(double) * m.size(), cudaMemcpyDeviceToHost, h->stream));
   CUW_TRY(cudaStreamSynchronize(h->stream));
@@ -1215,7 +1215,7 @@ static int step_body(Handle* h, int move_atoms, int max_iter, double eps) {
                                                                        h->delt * h->delt);
     CUW_LAUNCH_CHECK("k_atoms_verlet");
   }
-  CUW_RET(ortho_core(h, max_iter, eps));
+  CUW_RET(ortho_core(h, max_iter, eps, true));
   CUW_RET(mark(h, PH_RED));
   CUW_RET(energy_run(h, RED_WAVEKIN, tmpv, sc + 3));
   CUW_RET(mark(h, PH_MISC));
@@ -1253,7 +1253,7 @@ static bool step_graph(Handle* h, int move_atoms, int max_iter, double eps, int*
     }
   for (Handle::StepGraph& sg : h->graphs) {
     if (std::memcmp(sg.key, key, sizeof(key)) || sg.move != move_atoms || sg.max_iter != max_iter || sg.eps != eps ||
-        sg.rlamm != rlamm)
+        sg.rlamm != rlamm || sg.tabs != h->tabs)
       continue;
     cudaError_t e = cudaGraphLaunch(sg.exec, h->stream);
     if (e != cudaSuccess) {
@@ -1263,6 +1263,7 @@ static bool step_graph(Handle* h, int move_atoms, int max_iter, double eps, int*
     // the host side of the captured step
     std::swap(g.psi0, g.psim);
     h->eigr_src = sg.eigr_after;
+    h->tabs = sg.tabs_after;
     h->have_hpsi = false;
     h->have_opsi = false;
     h->have_rlamm = true;
@@ -1274,6 +1275,7 @@ static bool step_graph(Handle* h, int move_atoms, int max_iter, double eps, int*
   // capture; on any failure restore the host state and run uncaptured
   Device saved = g;
   const double* eigr_saved = h->eigr_src;
+  const int tabs_saved = h->tabs;
   const bool hp = h->have_hpsi, ho = h->have_opsi, hr = h->have_rlamm;
   const long long l0 = h->launches, ep = h->epoch;
   if (cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
@@ -1295,6 +1297,7 @@ static bool step_graph(Handle* h, int move_atoms, int max_iter, double eps, int*
     cudaGetLastError();
     g = saved;
     h->eigr_src = eigr_saved;
+    h->tabs = tabs_saved;
     h->have_hpsi = hp;
     h->have_opsi = ho;
     h->have_rlamm = hr;
@@ -1309,7 +1312,9 @@ static bool step_graph(Handle* h, int move_atoms, int max_iter, double eps, int*
   sg.eps = eps;
   sg.rlamm = rlamm;
   sg.epoch = h->epoch;
+  sg.tabs = tabs_saved;
   sg.eigr_after = h->eigr_src;
+  sg.tabs_after = h->tabs;
   sg.launches = h->launches - l0;
   sg.exec = exec;
   if (h->graphs.size() >= 12) h->drop_graphs();
@@ -1385,10 +1390,11 @@ struct cuw_batch {
   struct Key {
     const void* k[6];
     long long epoch;
-    int rlamm;
+    int rlamm, tabs;
   };
   std::vector<Key> keys;                  // host state of each set the graph was captured for
-  std::vector<const double*> eigr_after;  // EIGR source buffer of each set after a pair of steps
+  // source buffer of the projector tables of each set after a pair of steps, and TAB_*
+  std::vector<std::pair<const double*, int>> eigr_after;
   std::vector<long long> launches;        // kernels per set in the graph
   int move = -1, max_iter = 0;
   double eps = 0.0;
@@ -1409,6 +1415,7 @@ static cuw_batch::Key batch_key(const Handle* h) {
   std::memcpy(k.k, v, sizeof(v));
   k.epoch = h->epoch;
   k.rlamm = h->have_rlamm ? 1 : 0;
+  k.tabs = h->tabs;
   return k;
 }
 
@@ -1417,13 +1424,13 @@ static cuw_batch::Key batch_key(const Handle* h) {
 static int batch_capture(cuw_batch* b, int move, int max_iter, double eps) {
   const int n = (int)b->hs.size();
   std::vector<Device> saved(n);
-  std::vector<const double*> eigr_saved(n);
+  std::vector<std::pair<const double*, int>> eigr_saved(n);
   std::vector<long long> l0(n);
   std::vector<cuw_batch::Key> keys(n);
   for (int i = 0; i < n; ++i) {
     Handle* h = b->hs[i];
     saved[i] = h->g;
-    eigr_saved[i] = h->eigr_src;
+    eigr_saved[i] = {h->eigr_src, h->tabs};
     l0[i] = h->launches;
     keys[i] = batch_key(h);
   }
@@ -1467,7 +1474,8 @@ static int batch_capture(cuw_batch* b, int move, int max_iter, double eps) {
     for (int i = 0; i < n; ++i) {
       Handle* h = b->hs[i];
       h->g = saved[i];
-      h->eigr_src = eigr_saved[i];
+      h->eigr_src = eigr_saved[i].first;
+      h->tabs = eigr_saved[i].second;
       h->launches = l0[i];
       h->err.clear();
     }
@@ -1480,7 +1488,7 @@ static int batch_capture(cuw_batch* b, int move, int max_iter, double eps) {
   b->eigr_after.resize(n);
   b->launches.resize(n);
   for (int i = 0; i < n; ++i) {
-    b->eigr_after[i] = b->hs[i]->eigr_src;
+    b->eigr_after[i] = {b->hs[i]->eigr_src, b->hs[i]->tabs};
     b->launches[i] = b->hs[i]->launches - l0[i];
   }
   b->move = move;
@@ -1549,13 +1557,14 @@ extern "C" int cuwaves_batch_step(cuw_batch* b, int move_atoms, const double* co
   for (int i = 0; i < n && same; ++i) {
     const cuw_batch::Key k = batch_key(b->hs[i]);
     same = std::memcmp(k.k, b->keys[i].k, sizeof(k.k)) == 0 && k.epoch == b->keys[i].epoch &&
-           k.rlamm == b->keys[i].rlamm;
+           k.rlamm == b->keys[i].rlamm && k.tabs == b->keys[i].tabs;
   }
   if (same) {
     CUW_BATCH_TRY(cudaGraphLaunch(b->exec, b->stream));
     for (int i = 0; i < n; ++i) {
       Handle* h = b->hs[i];
-      h->eigr_src = b->eigr_after[i];  // the PSI0/PSIM swaps of two steps cancel
+      h->tabs = b->eigr_after[i].second;
+      h->eigr_src = b->eigr_after[i].first;  // the PSI0/PSIM swaps of two steps cancel
       h->launches += b->launches[i];
       h->graph_replays += 2;
     }
@@ -1724,7 +1733,7 @@ extern "C" int cuwaves_set_option(cuw_handle* hp, int option, double value) {
       if (value != 0.0 && value != 1.0) return h->fail(CUW_ERR_ARG, "CONTRACTION_TILES must be 0 or 1");
       if (!h->mixed() && value == 0.0) return h->fail(CUW_ERR_ARG, "FP64 handles have DMMA tiles only");
       h->dmma_tiles = value != 0.0;
-      return CUW_OK;
+      return h->have_gset ? fold_rooms(h) : CUW_OK;
     case CUW_OPT_SAFEORTHO:
       if (value != 0.0 && value != 1.0) return h->fail(CUW_ERR_ARG, "SAFEORTHO must be 0 or 1");
       h->safeortho = value != 0.0;

@@ -75,6 +75,7 @@ struct Device {
   double *pro = nullptr;         // (NGL, NBAREPRO)
   double *ylm = nullptr;         // (NGL, LMX)
   double *mpsi = nullptr;        // (NGL)
+  double *rmpsi = nullptr;       // (NGL) 1 / MPSI
   double *bucket = nullptr;      // (NGL) or null
   ProDesc *pdesc = nullptr;      // (NPRO)
   // FFT
@@ -94,7 +95,11 @@ struct Device {
   double *mass = nullptr;        // (NAT)
   double2 *eigr = nullptr;       // (NGL, NAT) structure factors of the last position set
   float2 *pf = nullptr;          // (LDG, NPRO) mixed path: PRO(g,p) of the last position set in fp32, 0 for g >= NGL
-  double2 *prox = nullptr;       // (LDG, NPRO) FP64 path: PRO(g,p) of the last position set, 0 for g >= NGL
+  // folded arrays of the FP64 products (fold.cu): the +-G pairs of the sphere,
+  // P(r,p) of the last position set (LDU, NPRO) and two slots of U(r,n) (LDU, NB)
+  int2 *half = nullptr;
+  double *prox = nullptr;
+  double *uf = nullptr;
   double2 *xminus[2] = {nullptr, nullptr};  // (LDG, NBH) mixed path: X(-G) copies of wave-function arrays
   float *bpre[2] = {nullptr, nullptr};       // mixed path: wave-function arrays split into tf32 B tiles
   const double2 *bpre_src[2] = {nullptr, nullptr};  // arrays they hold (valid inside a solve scope)
@@ -113,7 +118,8 @@ struct Device {
   double *maxpart = nullptr;
   int *ostatus = nullptr;        // [0] status, [1] iterations
   int *smap = nullptr;           // (NB) state order of WAVES_ORTHO_Y_C (SAFEORTHO = F, SWAPSTATES = T)
-  double *anv = nullptr, *dbucket = nullptr;  // (NGL) ANNEEVEC and GSET%DBUCKET of the cell friction
+  // (NGL) ANNEEVEC, 1 / (1 + ANNEEVEC) and GSET%DBUCKET of the cell friction
+  double *anv = nullptr, *aninv = nullptr, *dbucket = nullptr;
   double2 *lam1c = nullptr, *lam2c = nullptr;  // (NBH, NBH) folded multipliers
   double2 *tmat = nullptr;       // 12 (NBH, NBH) reduced Gram products
   // scratch for split-K partial sums and band reductions
@@ -148,6 +154,8 @@ struct Handle {
   std::vector<ProDesc> pdesc;
   int npro = 0, nbarepro = 0, lmnxx = 0, lnxx = 0;
   int ldg = 0;                   // leading dimension of wave-function arrays
+  int nh = 0, ldu = 0;           // +-G pairs of the sphere, leading dimension of folded arrays (>= 2 nh)
+  bool sym = false;              // the G set's tables have the parity of real-valued projectors
   double gweight = 0.0;
   double gbas[9] = {0};
   std::vector<int> igvec_h;      // IGVEC(3,NGL) of the G set (restart records)
@@ -187,10 +195,12 @@ struct Handle {
   // reallocation, set-up routines), which retires the graphs.
   struct StepGraph {
     const void* key[6];
+    int tabs = 0;
     int move = 0, max_iter = 0, rlamm = 0;
     double eps = 0.0;
     long long epoch = -1;
-    const double* eigr_after = nullptr;  // EIGR's source buffer after the step
+    const double* eigr_after = nullptr;  // the projector tables' source buffer after the step
+    int tabs_after = 0;
     long long launches = 0;              // kernels in the graph
     cudaGraphExec_t exec = nullptr;
   };
@@ -239,7 +249,10 @@ struct Handle {
   int lyap_max_sweeps = 64;  // sweeps per Lyapunov solve before the fixed point counts as failed
   bool ortho_panel = true;   // ORTHO_X by the panel-staged cluster kernel where it applies (64 < NB <= 128)
   bool tc_scope_open = false;
-  const double* eigr_src = nullptr;  // position buffer (r0, rp or rm) that EIGR (and the fp32 table) was built from
+  // position buffer (r0, rp or rm) that the projector tables were built from,
+  // and which of them (TAB_*) are current for it
+  const double* eigr_src = nullptr;
+  int tabs = 0;
   // potential: density G set size, LMRXX, index of G = 0 (-1: none), and
   // whether cuwaves_cp_step forms V(r) from the density first
   int nglh = 0, lmrxx = 0, ngamma = -1;
@@ -328,9 +341,9 @@ __device__ __forceinline__ double2 pro_value(int g, int ngl, const ProDesc& d, c
 // coefficients of the fused ADDPRO epilogues (see k_addpro)
 struct StepCoef {
   double a1, a2, a3, oscale;
-  // G-dependent friction of a moving cell (ANNEEVEC(G), src/paw_waves1.f90:
-  // 6536-6540) or null; with it the propagation coefficients are formed per G
-  // from fr[g] and dt2 = DELT^2 instead of a1, a2, a3
+  // 1 / (1 + ANNEEVEC(G)) of the G-dependent friction of a moving cell
+  // (src/paw_waves1.f90:6536-6540) or null; with it the propagation coefficients
+  // are formed per G from fr[g] and dt2 = DELT^2 instead of a1, a2, a3
   const double* fr = nullptr;
   double dt2 = 0.0;
 };
@@ -354,16 +367,15 @@ int fft_variants(const Handle* h);
 int vofrho_run(Handle* h, const double* rho_dev);  // POTENTIAL$VOFRHO on the device
 int denmat_run(Handle* h, int lmnxx, double2* denmat, double2* edenmat);
 int eigr_compute(Handle* h, const double* r_dev);
-int proj_compute(Handle* h, const double2* psiA, double2* projA, const double2* psiB, double2* projB);
+int proj_compute(Handle* h, const double2* psiA, double2* projA, const double2* psiB, double2* projB,
+                 bool folded = false);
 int addpro_run(Handle* h, int mode, const double2* hpc, const double2* opc);
 int hproj_compute(Handle* h, const double2* proj, double2* out);
 int oproj_compute(Handle* h, const double2* proj, double2* out);
 int hoproj_compute(Handle* h, const double2* proj, double2* hout, double2* oout);
-int gram_overlaps(Handle* h, double2* projP, double2* projO);
 int ortho_solve(Handle* h, int max_iter, double eps);
 int ortho_result(Handle* h, const int* st, int* iters);
-int addopsi_run(Handle* h, double2* psibar, const double2* opsi, const double2* l1, const double2* l2);
-int addoproj_run(Handle* h, double2* proj, const double2* oproj, const double2* l1, const double2* l2);
+int addoproj_run(Handle* h, double2* proj, const double2* oproj, const double* lam);
 int lambda12_run(Handle* h, const double* lam_real, double2* l1, double2* l2);
 int band_reduce(Handle* h, int what, double* out_host, double* eig_host);
 int force_run(Handle* h, double* force_host);
@@ -374,8 +386,26 @@ struct GramPair {
   const double2* x;
   const double2* y;
 };
-int gram_planewave(Handle* h, const GramPair* pairs, int npair, double2* dst);
-int gram_projections(Handle* h, const GramPair* pairs, int npair, double2* dst);
+// folded FP64 products (fold.cu); slots 0 and 1 hold folded wave-function arrays
+struct FoldPair {
+  int x, y;                // slots
+  const double2 *px, *py;  // projections of x and DO * projections of y
+};
+int fold_setup(Handle* h, const std::vector<int>& minusg);
+int fold_kernels_setup(Handle* h);
+int fold_rooms(Handle* h);
+int fold_room(Handle* h);
+int eigr_room(Handle* h);
+int fold_table_room(Handle* h);
+int fold_table(Handle* h, const double* r_dev);
+int fold_psi(Handle* h, const double2* psi, int slot);
+int fold_proj(Handle* h, double2* proj0, double2* proj1);
+// <x|O|y> of up to three pairs as real NB x NB matrices
+int fold_gram(Handle* h, const FoldPair* pairs, int npair, double* o0, double* o1, double* o2);
+// ADDPRO_FUSED leaves folded PSIM in slot 0 and OPSI in slot 1
+int fold_addpro(Handle* h, int mode, const double2* hpc, const double2* opc, const StepCoef& sc);
+int fold_addx(Handle* h, int slot, const double* lam, double2* out);
+int fold_force(Handle* h, const double2* ded, double* fpart, int* nt);
 int ensure_part(Handle* h, size_t bytes);  // split-K scratch h->g.part of at least `bytes`
 // Raises (never lowers) the dynamic shared-memory limit of kernel fn on the
 // current device.  The limit belongs to the function, so it is shared by all
@@ -397,11 +427,12 @@ int tc_addx(Handle* h, bool xminus, double2* out, const double2* x, const double
             int nn, int nk, size_t sxm, size_t sxk, size_t som, size_t son);
 int tc_force(Handle* h, const double2* ded, double* fpart, int* ntile);
 int propagate_run(Handle* h);
-int opsi_scale_run(Handle* h);
+int opsi_scale(Handle* h, double oscale);
 int switch_lambda_run(Handle* h);
 int gramschmidt_run(Handle* h, double2* psi, const double* r_dev);
 int atoms_verlet_run(Handle* h, const double* mass_dev);
 
+enum { TAB_EIGR = 1, TAB_F32 = 2, TAB_F64 = 4 };
 enum { ADDPRO_HPSI = 0, ADDPRO_OPSI = 1, ADDPRO_FUSED = 2 };
 enum { RED_EKIN = 0, RED_WAVEKIN = 1, RED_EXPECT = 2 };
 

@@ -285,10 +285,6 @@ __device__ __forceinline__ void mma_slice2(Acc& acc, const double2* A, const dou
 struct NoConj {
   __device__ __forceinline__ bool operator()(int) const { return false; }
 };
-struct AllConj {
-  __device__ __forceinline__ bool operator()(int) const { return true; }
-};
-
 template <int MODE, bool AKF, bool BKF, bool CB0, bool CB1, class PA0, class PA1, class PB0, class PB1, class CA0,
           class CA1>
 __device__ __forceinline__ void mainloop2(double2* sm, int kbeg, int kend, PA0 pa0, PA1 pa1, PB0 pb0, PB1 pb1,
@@ -374,35 +370,6 @@ __global__ void k_eigr(const double* __restrict__ gx, const double* __restrict__
   }
 }
 
-// PRO(g,p) of WAVES_EXPANDPRO for every projector of the present positions
-// into prox(LDG, NPRO), zero for NGL <= g < LDG (FP64 handles: the tile
-// loaders of the contractions then read whole columns), straight from the
-// positions: one thread per (g, atom) forms exp(-iG.R_a) as k_eigr does and
-// writes the atom's projectors, so no EIGR array is formed.
-__global__ void k_pro_f64_direct(int ngl, int ldg, const double* __restrict__ gx, const double* __restrict__ gy,
-                                 const double* __restrict__ gz, const double* __restrict__ r,
-                                 const int* __restrict__ ipro0, const int* __restrict__ nlmn,
-                                 const ProDesc* __restrict__ pdesc, const double* __restrict__ ylm,
-                                 const double* __restrict__ pro, double2* __restrict__ prox) {
-  const int a = blockIdx.y;
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= ldg) return;
-  const int p0 = ipro0[a], np = nlmn[a];
-  if (g >= ngl) {
-    for (int k = 0; k < np; ++k) prox[(size_t)g + (size_t)ldg * (p0 + k)] = make_double2(0.0, 0.0);
-    return;
-  }
-  double sn, cs;
-  sincos(gx[g] * r[3 * a] + gy[g] * r[3 * a + 1] + gz[g] * r[3 * a + 2], &sn, &cs);
-  const double2 ei = make_double2(cs, -sn);
-  for (int k = 0; k < np; ++k) {
-    const ProDesc d = pdesc[p0 + k];
-    const double sv = ylm[(size_t)g + (size_t)ngl * d.lm] * pro[(size_t)g + (size_t)ngl * d.ibare];
-    const double2 e = cmul(mipow(d.l), ei);
-    prox[(size_t)g + (size_t)ldg * (p0 + k)] = make_double2(sv * e.x, sv * e.y);
-  }
-}
-
 __device__ __forceinline__ double2 zero2() { return make_double2(0.0, 0.0); }
 
 // ---------------------------------------------------------------------------
@@ -410,15 +377,12 @@ __device__ __forceinline__ double2 zero2() { return make_double2(0.0, 0.0); }
 // for one or two operands X (psiA -> part, psiB -> part + dual_stride).
 // M = bands (blockIdx.y), N = projectors (blockIdx.x), K = g (blockIdx.z).
 // ---------------------------------------------------------------------------
-// TAB: the projector functions come from the expanded table prox(LDG, NPRO)
-// of the present positions (FP64 handles) instead of being formed in the loader.
-template <bool DUAL, bool TAB>
+template <bool DUAL>
 __global__ void __launch_bounds__(NT, 1) k_proj(const double2* __restrict__ psiA, const double2* __restrict__ psiB,
                                                 int ldg, int ngl, int nbh, int npro, int kchunk,
                                                 const ProDesc* __restrict__ pdesc, const double* __restrict__ ylm,
                                                 const double* __restrict__ pro, const double2* __restrict__ eigr,
-                                                double2* __restrict__ part, size_t dual_stride,
-                                                const double2* __restrict__ prox = nullptr) {
+                                                double2* __restrict__ part, size_t dual_stride) {
   extern __shared__ double sm[];
   __shared__ ProDesc sd[BN];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wm = warp >> 2, wn = warp & 3;
@@ -441,32 +405,10 @@ __global__ void __launch_bounds__(NT, 1) k_proj(const double2* __restrict__ psiA
     return (DUAL && g < kend && b < nbh) ? psiB[(size_t)g + (size_t)ldg * b] : zero2();
   };
   auto fb0 = [&](int row, int g) {
-    double2 v = zero2();
-    if (g < kend && n0 + row < npro) {
-      if constexpr (TAB) v = cconj(prox[(size_t)g + (size_t)ldg * (n0 + row)]);
-      else v = cconj(gen_pro(g, ngl, sd[row], ylm, pro, eigr));
-    }
-    return v;
+    return (g < kend && n0 + row < npro) ? cconj(gen_pro(g, ngl, sd[row], ylm, pro, eigr)) : zero2();
   };
-  if constexpr (TAB) {
-    auto pa0 = [&](int row, int g) -> const double2* {
-      const int b = m0 + row;
-      return (g < kend && b < nbh) ? psiA + (size_t)g + (size_t)ldg * b : nullptr;
-    };
-    auto pa1 = [&](int row, int g) -> const double2* {
-      const int b = m0 + row;
-      return (DUAL && g < kend && b < nbh) ? psiB + (size_t)g + (size_t)ldg * b : nullptr;
-    };
-    auto pb0 = [&](int row, int g) -> const double2* {
-      return (g < kend && n0 + row < npro) ? prox + (size_t)g + (size_t)ldg * (n0 + row) : nullptr;
-    };
-    double2* sm2 = reinterpret_cast<double2*>(sm);
-    if (DUAL) mainloop2<MP21, true, true, true, true>(sm2, kbeg, kend, pa0, pa1, pb0, pb0, NoConj(), NoConj(), acc, acc2);
-    else mainloop2<MP11, true, true, true, true>(sm2, kbeg, kend, pa0, pa0, pb0, pb0, NoConj(), NoConj(), acc, acc2);
-  } else {
-    if (DUAL) mainloop<MP21, true, true>(sm, kbeg, kend, fa0, fa1, fb0, fb0, acc, acc2);
-    else mainloop<MP11, true, true>(sm, kbeg, kend, fa0, fa0, fb0, fb0, acc, acc2);
-  }
+  if (DUAL) mainloop<MP21, true, true>(sm, kbeg, kend, fa0, fa1, fb0, fb0, acc, acc2);
+  else mainloop<MP11, true, true>(sm, kbeg, kend, fa0, fa0, fb0, fb0, acc, acc2);
   double2* out = part + (size_t)blockIdx.z * nbh * npro;
 #pragma unroll
   for (int mi = 0; mi < 4; ++mi)
@@ -516,15 +458,14 @@ __global__ void k_reduce_parts(const double2* __restrict__ part, int nz, size_t 
 // mode ADDPRO_OPSI : opsi  = (psi0 + PRO*C2) * dt^2/((1+annee) m_G)
 // mode ADDPRO_FUSED: both, then psim = a1 psi0 + a2 psim + a3/m_G hpsi
 // ---------------------------------------------------------------------------
-template <int MODE, bool TAB>
+template <int MODE>
 __global__ void __launch_bounds__(NT, 1) k_addpro(double2* __restrict__ hpsi, double2* __restrict__ opsi,
                                                   const double2* __restrict__ psi0, double2* __restrict__ psim,
                                                   const double* __restrict__ mpsi, int ldg, int ngl, int nbh,
                                                   int npro, const double2* __restrict__ c1,
                                                   const double2* __restrict__ c2, const ProDesc* __restrict__ pdesc,
                                                   const double* __restrict__ ylm, const double* __restrict__ pro,
-                                                  const double2* __restrict__ eigr, StepCoef sc,
-                                                  const double2* __restrict__ prox) {
+                                                  const double2* __restrict__ eigr, StepCoef sc) {
   constexpr bool USE_H = (MODE != ADDPRO_OPSI);
   constexpr bool USE_O = (MODE != ADDPRO_HPSI);
   extern __shared__ double sm[];
@@ -535,9 +476,7 @@ __global__ void __launch_bounds__(NT, 1) k_addpro(double2* __restrict__ hpsi, do
   acc2.zero();
   auto fa = [&](int row, int p) {
     int g = m0 + row;
-    if (!(g < ngl && p < npro)) return zero2();
-    if constexpr (TAB) return prox[(size_t)g + (size_t)ldg * p];
-    else return gen_pro(g, ngl, pdesc[p], ylm, pro, eigr);
+    return (g < ngl && p < npro) ? gen_pro(g, ngl, pdesc[p], ylm, pro, eigr) : zero2();
   };
   auto fb1 = [&](int row, int p) {
     int b = n0 + row;
@@ -547,31 +486,9 @@ __global__ void __launch_bounds__(NT, 1) k_addpro(double2* __restrict__ hpsi, do
     int b = n0 + row;
     return (b < nbh && p < npro) ? c2[(size_t)b + (size_t)nbh * p] : zero2();
   };
-  if constexpr (TAB) {
-    auto pa = [&](int row, int p) -> const double2* {
-      const int g = m0 + row;
-      return (g < ngl && p < npro) ? prox + (size_t)g + (size_t)ldg * p : nullptr;
-    };
-    auto pb1 = [&](int row, int p) -> const double2* {
-      const int b = n0 + row;
-      return (b < nbh && p < npro) ? c1 + (size_t)b + (size_t)nbh * p : nullptr;
-    };
-    auto pb2 = [&](int row, int p) -> const double2* {
-      const int b = n0 + row;
-      return (b < nbh && p < npro) ? c2 + (size_t)b + (size_t)nbh * p : nullptr;
-    };
-    double2* sm2 = reinterpret_cast<double2*>(sm);
-    if (MODE == ADDPRO_FUSED)
-      mainloop2<MP12, false, false, false, false>(sm2, 0, npro, pa, pa, pb1, pb2, NoConj(), NoConj(), acc, acc2);
-    else if (MODE == ADDPRO_HPSI)
-      mainloop2<MP11, false, false, false, false>(sm2, 0, npro, pa, pa, pb1, pb1, NoConj(), NoConj(), acc, acc2);
-    else
-      mainloop2<MP11, false, false, false, false>(sm2, 0, npro, pa, pa, pb2, pb2, NoConj(), NoConj(), acc2, acc);
-  } else {
-    if (MODE == ADDPRO_FUSED) mainloop<MP12, false, false>(sm, 0, npro, fa, fa, fb1, fb2, acc, acc2);
-    else if (MODE == ADDPRO_HPSI) mainloop<MP11, false, false>(sm, 0, npro, fa, fa, fb1, fb1, acc, acc2);
-    else mainloop<MP11, false, false>(sm, 0, npro, fa, fa, fb2, fb2, acc2, acc);
-  }
+  if (MODE == ADDPRO_FUSED) mainloop<MP12, false, false>(sm, 0, npro, fa, fa, fb1, fb2, acc, acc2);
+  else if (MODE == ADDPRO_HPSI) mainloop<MP11, false, false>(sm, 0, npro, fa, fa, fb1, fb1, acc, acc2);
+  else mainloop<MP11, false, false>(sm, 0, npro, fa, fa, fb2, fb2, acc2, acc);
 #pragma unroll
   for (int mi = 0; mi < 4; ++mi)
 #pragma unroll
@@ -599,192 +516,13 @@ __global__ void __launch_bounds__(NT, 1) k_addpro(double2* __restrict__ hpsi, do
           double2 p0 = psi0[k], pm = psim[k];
           double a1 = sc.a1, a2 = sc.a2, a3 = sc.a3 / mpsi[g];
           if (sc.fr) {  // cell friction ANNEEVEC(G) (src/paw_waves1.f90:6536-6540)
-            const double an = 1.0 + sc.fr[g];
-            a1 = 2.0 / an;
+            a1 = 2.0 * sc.fr[g];
             a2 = 1.0 - a1;
-            a3 = -sc.dt2 / an / mpsi[g];
+            a3 = -sc.dt2 * sc.fr[g] / mpsi[g];
           }
           psim[k] = make_double2(a1 * p0.x + a2 * pm.x + a3 * hv.x, a1 * p0.y + a2 * pm.y + a3 * hv.y);
         }
       }
-}
-
-// ---------------------------------------------------------------------------
-// Gram products for one or more (X, Y) pairs (blockIdx.z = split*npair + pair):
-//   T1(m,n) = sum_k conj(X(k,m)) Y(k,n)
-//   T2(m,n) = sum_k X(k,m) Y(-k,n)    (MINUS: k -> minusg[k])
-//           = sum_k X(k,m) Y(k,n)     (otherwise)
-// Layout: element (k, m) of an operand at ptr[k*sk + m*sm].
-// part[((split*npair + pair)*2 + t)*nm*nn + m + nm*n]
-// ---------------------------------------------------------------------------
-struct GramArgs {
-  GramPair pair[3];
-  int npair;
-  int nk, nm, nn;   // K, M, N extents
-  size_t sk, sm;    // strides of k and of m/n
-  int kchunk;
-};
-
-template <bool MINUS, bool KFAST>
-__global__ void __launch_bounds__(NT, 1) k_gram(GramArgs a, const int* __restrict__ minusg,
-                                                double2* __restrict__ part) {
-  extern __shared__ double sm[];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wm = warp >> 2, wn = warp & 3;
-  const int pair = blockIdx.z % a.npair, split = blockIdx.z / a.npair;
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  const double2* X = a.pair[pair].x;
-  const double2* Y = a.pair[pair].y;
-  const int kbeg = split * a.kchunk, kend = min(a.nk, kbeg + a.kchunk);
-  Acc t1, t2;
-  t1.zero();
-  t2.zero();
-  auto pa = [&](int row, int k) -> const double2* {
-    int m = m0 + row;
-    return (k < kend && m < a.nm) ? X + (size_t)k * a.sk + (size_t)m * a.sm : nullptr;
-  };
-  auto pb = [&](int row, int k) -> const double2* {
-    int n = n0 + row;
-    return (k < kend && n < a.nn) ? Y + (size_t)k * a.sk + (size_t)n * a.sm : nullptr;
-  };
-  auto pb2 = [&](int row, int k) -> const double2* {
-    int n = n0 + row;
-    if (!(k < kend && n < a.nn)) return nullptr;
-    int kk = MINUS ? minusg[k] : k;
-    return Y + (size_t)kk * a.sk + (size_t)n * a.sm;
-  };
-  mainloop2<MPGRAM, KFAST, KFAST, false, false>(reinterpret_cast<double2*>(sm), kbeg, kend, pa, pa, pb, pb2,
-                                                AllConj(), NoConj(), t1, t2);
-  const size_t mn = (size_t)a.nm * a.nn;
-  double2* o1 = part + ((size_t)blockIdx.z * 2 + 0) * mn;
-  double2* o2 = part + ((size_t)blockIdx.z * 2 + 1) * mn;
-#pragma unroll
-  for (int mi = 0; mi < 4; ++mi)
-#pragma unroll
-    for (int ni = 0; ni < 2; ++ni)
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        int m, n;
-        acc_mn(wm, wn, lane, mi, ni, e, m, n);
-        m += m0;
-        n += n0;
-        if (m < a.nm && n < a.nn) {
-          o1[(size_t)m + (size_t)a.nm * n] = make_double2(t1.r[mi][ni][e], t1.i[mi][ni][e]);
-          o2[(size_t)m + (size_t)a.nm * n] = make_double2(t2.r[mi][ni][e], t2.i[mi][ni][e]);
-        }
-      }
-}
-
-// ---------------------------------------------------------------------------
-//   ADDOPSI form (XMINUS): out(g,n) += sum_k X(g,k) L1(k,n) + conj(X(-g,k)) L2(k,n)
-//   ADDOPROJ form       : out(p,n) += sum_k X(p,k) L1(k,n) + conj(X(p,k)) L2(k,n)
-// X element (m, k) at X[m*sxm + k*sxk]; out element (m, n) at out[m*som + n*son];
-// L1/L2 (nk, nn) column-major complex.  M = blockIdx.x, N = blockIdx.y.
-// ---------------------------------------------------------------------------
-struct AddXArgs {
-  double2* out;
-  const double2* x;
-  const double2* l1;
-  const double2* l2;
-  int nm, nn, nk;
-  size_t sxm, sxk, som, son;
-};
-
-template <bool XMINUS, bool MFAST>
-__global__ void __launch_bounds__(NT, 1) k_addx(AddXArgs a, const int* __restrict__ minusg) {
-  extern __shared__ double sm[];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wm = warp >> 2, wn = warp & 3;
-  const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
-  Acc acc, dummy;
-  acc.zero();
-  const int ktot = 2 * a.nk;
-  // the second half of K takes conj(X(-g)): conjugated at the fragment read
-  auto pa = [&](int row, int kg) -> const double2* {
-    int m = m0 + row;
-    if (!(m < a.nm && kg < ktot)) return nullptr;
-    if (kg < a.nk) return a.x + (size_t)m * a.sxm + (size_t)kg * a.sxk;
-    int mm2 = XMINUS ? minusg[m] : m;
-    return a.x + (size_t)mm2 * a.sxm + (size_t)(kg - a.nk) * a.sxk;
-  };
-  auto pb = [&](int row, int kg) -> const double2* {
-    int n = n0 + row;
-    if (!(n < a.nn && kg < ktot)) return nullptr;
-    return kg < a.nk ? a.l1 + (size_t)kg + (size_t)a.nk * n : a.l2 + (size_t)(kg - a.nk) + (size_t)a.nk * n;
-  };
-  const int nk = a.nk;
-  auto second = [nk](int kg) { return kg >= nk; };
-  // the outputs' old values (out is not an operand), loaded before the
-  // products so that their latency overlaps the MMAs
-  double2 old[4][2][2];
-#pragma unroll
-  for (int mi = 0; mi < 4; ++mi)
-#pragma unroll
-    for (int ni = 0; ni < 2; ++ni)
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        int m, n;
-        acc_mn(wm, wn, lane, mi, ni, e, m, n);
-        m += m0;
-        n += n0;
-        old[mi][ni][e] = (m < a.nm && n < a.nn) ? a.out[(size_t)m * a.som + (size_t)n * a.son] : make_double2(0.0, 0.0);
-      }
-  mainloop2<MP11, !MFAST, true, false, false>(reinterpret_cast<double2*>(sm), 0, ktot, pa, pa, pb, pb, second,
-                                              second, acc, dummy);
-#pragma unroll
-  for (int mi = 0; mi < 4; ++mi)
-#pragma unroll
-    for (int ni = 0; ni < 2; ++ni)
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        int m, n;
-        acc_mn(wm, wn, lane, mi, ni, e, m, n);
-        m += m0;
-        n += n0;
-        if (m < a.nm && n < a.nn) {
-          size_t k = (size_t)m * a.som + (size_t)n * a.son;
-          const double2 o = old[mi][ni][e];
-          a.out[k] = make_double2(o.x + acc.r[mi][ni][e], o.y + acc.i[mi][ni][e]);
-        }
-      }
-}
-
-// out(b,p) += sum_k x(k,p) l1(k,b) + conj(x(k,p)) l2(k,b) for (NBH, NPRO)
-// arrays with the band index fastest.  A block of 256 threads forms 64 bands
-// x 4 projectors, one output per thread with K in order; L1, L2 and x pass
-// through shared memory kAopK values of k at a time, copied along k (the
-// contiguous index), so that no warp reads L1 or L2 at a stride of NBH.
-constexpr int kAopK = 16;
-__global__ void k_addoproj(double2* __restrict__ out, const double2* __restrict__ x, const double2* __restrict__ l1,
-                           const double2* __restrict__ l2, int npro, int nbh) {
-  __shared__ double2 s1[64][kAopK + 1], s2[64][kAopK + 1], sx[4][kAopK];
-  const int tb = threadIdx.x & 63, tp = threadIdx.x >> 6;
-  const int b0 = blockIdx.y * 64, p0 = blockIdx.x * 4;
-  const int b = b0 + tb, p = p0 + tp;
-  double sr = 0.0, si = 0.0;
-  for (int k0 = 0; k0 < nbh; k0 += kAopK) {
-    __syncthreads();  // the previous chunk is consumed
-    for (int i = threadIdx.x; i < 64 * kAopK; i += blockDim.x) {
-      const int kk = i % kAopK, bb = i / kAopK, k = k0 + kk, bg = b0 + bb;
-      const bool ok = k < nbh && bg < nbh;
-      s1[bb][kk] = ok ? l1[(size_t)k + (size_t)nbh * bg] : make_double2(0.0, 0.0);
-      s2[bb][kk] = ok ? l2[(size_t)k + (size_t)nbh * bg] : make_double2(0.0, 0.0);
-    }
-    if (threadIdx.x < 4 * kAopK) {
-      const int pp = threadIdx.x / kAopK, kk = threadIdx.x % kAopK, k = k0 + kk, pg = p0 + pp;
-      sx[pp][kk] = (k < nbh && pg < npro) ? x[(size_t)pg * nbh + k] : make_double2(0.0, 0.0);
-    }
-    __syncthreads();
-    const int kn = min(kAopK, nbh - k0);
-    for (int kk = 0; kk < kn; ++kk) {
-      const double2 xv = sx[tp][kk], av = s1[tb][kk], cv = s2[tb][kk];
-      sr += xv.x * av.x - xv.y * av.y + xv.x * cv.x + xv.y * cv.y;
-      si += xv.x * av.y + xv.y * av.x + xv.x * cv.y - xv.y * cv.x;
-    }
-  }
-  if (b < nbh && p < npro) {
-    const size_t t = (size_t)b + (size_t)nbh * p;
-    const double2 o = out[t];
-    out[t] = make_double2(o.x + sr, o.y + si);
-  }
 }
 
 // ---------------------------------------------------------------------------
@@ -795,14 +533,12 @@ __global__ void k_addoproj(double2* __restrict__ out, const double2* __restrict_
 // cancels in this sum (c(-G) = -conj(c(G)) for c = i Y P (-i)^l EIGR over the
 // full sphere), so it is not applied.
 // ---------------------------------------------------------------------------
-template <bool TAB>
 __global__ void __launch_bounds__(NT, 1) k_force(const double2* __restrict__ psi0, int ldg, int ngl, int nbh,
                                                  int npro, const double2* __restrict__ ded,
                                                  const ProDesc* __restrict__ pdesc, const double* __restrict__ ylm,
                                                  const double* __restrict__ pro, const double2* __restrict__ eigr,
                                                  const double* __restrict__ gx, const double* __restrict__ gy,
-                                                 const double* __restrict__ gz, double* __restrict__ fpart,
-                                                 const double2* __restrict__ prox) {
+                                                 const double* __restrict__ gz, double* __restrict__ fpart) {
   extern __shared__ double sm[];
   __shared__ double fred[BN][3][2];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wm = warp >> 2, wn = warp & 3;
@@ -817,22 +553,6 @@ __global__ void __launch_bounds__(NT, 1) k_force(const double2* __restrict__ psi
     int p = n0 + row;
     return (b < nbh && p < npro) ? ded + (size_t)b + (size_t)nbh * p : nullptr;
   };
-  // with the projector table, its values for this tile's outputs are loaded
-  // before the products so that their latency overlaps the MMAs
-  double2 pvt[4][2][2];
-  if constexpr (TAB) {
-#pragma unroll
-    for (int mi = 0; mi < 4; ++mi)
-#pragma unroll
-      for (int ni = 0; ni < 2; ++ni)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          int m, n;
-          acc_mn(wm, wn, lane, mi, ni, e, m, n);
-          const int g = m0 + m, p = n0 + n;
-          pvt[mi][ni][e] = (g < ngl && p < npro) ? prox[(size_t)g + (size_t)ldg * p] : make_double2(0.0, 0.0);
-        }
-  }
   mainloop2<MP11, false, true, true, true>(reinterpret_cast<double2*>(sm), 0, nbh, pa, pa, pb, pb, NoConj(),
                                            NoConj(), acc, dummy);
   // epilogue: per (g, p) contribution, reduced over g
@@ -852,19 +572,12 @@ __global__ void __launch_bounds__(NT, 1) k_force(const double2* __restrict__ psi
         int g = m0 + m, p = n0 + n;
         if (g < ngl && p < npro) {
           double2 dd = make_double2(acc.r[mi][ni][e], acc.i[mi][ni][e]);
-          double sv;
-          if constexpr (TAB) {
-            // Re(i PRO(g,p) conj(dd))
-            const double2 pv = pvt[mi][ni][e];
-            sv = -pv.y * dd.x + pv.x * dd.y;
-          } else {
-            ProDesc d = pdesc[p];
-            double pr = pro[(size_t)g + (size_t)ngl * d.ibare];
-            double y = ylm[(size_t)g + (size_t)ngl * d.lm];
-            // cw = i * P * (-i)^l * EIGR
-            double2 cw = cmul(make_double2(0.0, pr), cmul(mipow(d.l), eigr[(size_t)g + (size_t)ngl * d.iat]));
-            sv = (cw.x * dd.x + cw.y * dd.y) * y;  // Re(cw * conj(dd)) * Y
-          }
+          const ProDesc d = pdesc[p];
+          const double pr = pro[(size_t)g + (size_t)ngl * d.ibare];
+          const double y = ylm[(size_t)g + (size_t)ngl * d.lm];
+          // cw = i * P * (-i)^l * EIGR
+          const double2 cw = cmul(make_double2(0.0, pr), cmul(mipow(d.l), eigr[(size_t)g + (size_t)ngl * d.iat]));
+          const double sv = (cw.x * dd.x + cw.y * dd.y) * y;  // Re(cw * conj(dd)) * Y
           f[ni][e][0] += sv * gx[g];
           f[ni][e][1] += sv * gy[g];
           f[ni][e][2] += sv * gz[g];
@@ -898,137 +611,6 @@ __global__ void __launch_bounds__(NT, 1) k_force(const double2* __restrict__ psi
     int n = i / 3, c = i % 3;
     int p = n0 + n;
     if (p < npro) fpart[((size_t)blockIdx.x * npro + p) * 3 + c] = fred[n][c][0] + fred[n][c][1];
-  }
-}
-
-// Persistent form of k_force for the projector table and NBH <= 64: the
-// force contraction has a short K (the bands), so a CTA per output tile spends
-// most of its time filling its pipeline.  Here CTA (gi, pj) keeps the DEDPRO
-// tile of projector tile pj (all K) resident in shared memory and walks the G
-// tiles gi, gi + gstride, ...: the psi rows of the next G tile are copied
-// (16-byte cp.async) while the current one is multiplied and its epilogue
-// runs, and the G-weighted sums of every projector accumulate in registers
-// over all the CTA's tiles.  fpart(gi, p, c) then holds the CTA's partial sum.
-constexpr int kFpSlices = 4;                 // K slices of BK (NBH <= 64)
-constexpr int kFpASlice = BK * LDR;          // double2 of one [k][row] psi slice
-constexpr size_t kFpSmem = sizeof(double2) * ((size_t)kFpSlices * TILE2 + 2 * (size_t)kFpSlices * kFpASlice);
-__global__ void __launch_bounds__(NT, 1) k_force_p(const double2* __restrict__ psi0, int ldg, int ngl, int nbh,
-                                                   int npro, const double2* __restrict__ ded,
-                                                   const double* __restrict__ gx, const double* __restrict__ gy,
-                                                   const double* __restrict__ gz, double* __restrict__ fpart,
-                                                   const double2* __restrict__ prox, int gstride) {
-  extern __shared__ double sm[];
-  __shared__ double fred[BN][3][2];
-  double2* bsm = reinterpret_cast<double2*>(sm);  // [slice][TILE2], DEDPRO (row = projector, k = band)
-  double2* asm_ = bsm + kFpSlices * TILE2;        // [buffer][slice][kFpASlice], psi (k = band, row = G)
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wm = warp >> 2, wn = warp & 3;
-  const int gi = blockIdx.x, n0 = blockIdx.y * BN;
-  const int tm = (ngl + BM - 1) / BM;
-  const int nsl = (nbh + BK - 1) / BK;
-  // resident DEDPRO tile
-  for (int sl = 0; sl < nsl; ++sl)
-#pragma unroll
-    for (int q = 0; q < EPT; ++q) {
-      int row, kk;
-      tile_rc<true>(tid + q * NT, row, kk);
-      const int b = sl * BK + kk, pr = n0 + row;
-      cpa16(bsm + sl * TILE2 + toff<true>(row, kk), (b < nbh && pr < npro) ? ded + b + (size_t)nbh * pr : nullptr);
-    }
-  auto issue_a = [&](int t, int buf) {
-    const int m0 = t * BM;
-    for (int sl = 0; sl < nsl; ++sl)
-#pragma unroll
-      for (int q = 0; q < EPT; ++q) {
-        int row, kk;
-        tile_rc<false>(tid + q * NT, row, kk);
-        const int g = m0 + row, b = sl * BK + kk;
-        cpa16(asm_ + ((size_t)buf * kFpSlices + sl) * kFpASlice + toff<false>(row, kk),
-              (g < ngl && b < nbh) ? psi0 + (size_t)g + (size_t)ldg * b : nullptr);
-      }
-  };
-  if (gi < tm) issue_a(gi, 0);
-  cpa_commit();
-  double f[2][2][3];
-#pragma unroll
-  for (int ni = 0; ni < 2; ++ni)
-#pragma unroll
-    for (int e = 0; e < 2; ++e) f[ni][e][0] = f[ni][e][1] = f[ni][e][2] = 0.0;
-  int buf = 0;
-  for (int t = gi; t < tm; t += gstride, buf ^= 1) {
-    if (t + gstride < tm) issue_a(t + gstride, buf ^ 1);
-    cpa_commit();
-    cpa_wait<1>();  // this tile's psi rows (and the DEDPRO tile) have landed
-    __syncthreads();
-    const int m0 = t * BM;
-    // the projector-table values of this tile's outputs, loaded before the
-    // products so that their latency overlaps the MMAs
-    double2 pvt[4][2][2];
-#pragma unroll
-    for (int mi = 0; mi < 4; ++mi)
-#pragma unroll
-      for (int ni = 0; ni < 2; ++ni)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          int m, n;
-          acc_mn(wm, wn, lane, mi, ni, e, m, n);
-          const int g = m0 + m, p = n0 + n;
-          pvt[mi][ni][e] = (g < ngl && p < npro) ? prox[(size_t)g + (size_t)ldg * p] : make_double2(0.0, 0.0);
-        }
-    Acc acc;
-    acc.zero();
-    for (int sl = 0; sl < nsl; ++sl)
-      mma_slice2<false, true, true>(acc, asm_ + ((size_t)buf * kFpSlices + sl) * kFpASlice, bsm + sl * TILE2, wm,
-                                    wn, lane, sl * BK, NoConj());
-    acc.finish();
-#pragma unroll
-    for (int mi = 0; mi < 4; ++mi)
-#pragma unroll
-      for (int ni = 0; ni < 2; ++ni)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          int m, n;
-          acc_mn(wm, wn, lane, mi, ni, e, m, n);
-          const int g = m0 + m, p = n0 + n;
-          if (g < ngl && p < npro) {
-            // Re(i PRO(g,p) conj(dd))
-            const double2 pv = pvt[mi][ni][e];
-            const double sv = -pv.y * acc.r[mi][ni][e] + pv.x * acc.i[mi][ni][e];
-            f[ni][e][0] += sv * gx[g];
-            f[ni][e][1] += sv * gy[g];
-            f[ni][e][2] += sv * gz[g];
-          }
-        }
-    __syncthreads();  // the buffer is free for the copies of the tile after next
-  }
-  cpa_wait<0>();
-  // reduce across the 8 lanes that share (lane & 3) (different g rows)
-#pragma unroll
-  for (int ni = 0; ni < 2; ++ni)
-#pragma unroll
-    for (int e = 0; e < 2; ++e)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        double v = f[ni][e][c];
-        v += __shfl_xor_sync(0xffffffffu, v, 4);
-        v += __shfl_xor_sync(0xffffffffu, v, 8);
-        v += __shfl_xor_sync(0xffffffffu, v, 16);
-        f[ni][e][c] = v;
-      }
-  if (lane < 4) {
-#pragma unroll
-    for (int ni = 0; ni < 2; ++ni)
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        int n = wn * 16 + ni * 8 + 2 * lane + e;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) fred[n][c][wm] = f[ni][e][c];
-      }
-  }
-  __syncthreads();
-  for (int i = tid; i < BN * 3; i += NT) {
-    int n = i / 3, c = i % 3;
-    int p = n0 + n;
-    if (p < npro) fpart[((size_t)gi * npro + p) * 3 + c] = fred[n][c][0] + fred[n][c][1];
   }
 }
 
@@ -1155,40 +737,57 @@ static int choose_split(Handle* h, int tiles, int nk, int minchunk, double mul) 
   return std::min(want, maxs);
 }
 
+int eigr_room(Handle* h) {
+  if (h->g.eigr) return CUW_OK;
+  if (h->capturing) return h->fail(CUW_ERR_STATE, "structure factors allocated during graph capture");
+  h->touch();
+  if (cudaMalloc(&h->g.eigr, sizeof(double2) * (size_t)h->d.ngl * std::max(1, h->d.nat)) != cudaSuccess) {
+    cudaGetLastError();
+    h->g.eigr = nullptr;
+    return h->fail(CUW_ERR_NOMEM, "cudaMalloc of the structure factors failed");
+  }
+  return CUW_OK;
+}
+
+// Tables of the projectors at r_dev that the present path reads: the folded
+// FP64 table (FP64 products, symmetric G set), EIGR (FP64 products otherwise)
+// or EIGR and the fp32 table (tensor-core products of the mixed path).  Those
+// of a position buffer stay current until that buffer is written: R(+) of one
+// step is R(0) of the next.
 int eigr_compute(Handle* h, const double* r_dev) {
-  // EIGR (and the fp32 projector table) of the positions in a position buffer
-  // stay current until that buffer is written: R(+) of one step is R(0) of the
-  // next
   const bool pos = r_dev == h->g.r0 || r_dev == h->g.rp || r_dev == h->g.rm;
-  if (pos && r_dev == h->eigr_src) return CUW_OK;
+  const int need = h->tc_on() ? TAB_EIGR | TAB_F32 : (h->sym ? TAB_F64 : TAB_EIGR);
+  const bool same = pos && r_dev == h->eigr_src;
+  if (same && (h->tabs & need) == need) return CUW_OK;
+  if (!same) h->tabs = 0;
   h->eigr_src = nullptr;
-  if (!h->mixed() && h->npro > 0) {
-    // FP64 handles: the expanded projector table straight from the positions
-    // (the contractions read only the table, so EIGR is not formed)
-    if (!h->g.prox) {
-      if (h->capturing) return h->fail(CUW_ERR_STATE, "projector table allocated during graph capture");
-      h->touch();
-      CUW_TRY(cudaMalloc(&h->g.prox, sizeof(double2) * (size_t)h->ldg * h->npro));
-    }
-    const Device& g = h->g;
-    k_pro_f64_direct<<<dim3(ceil_div(h->ldg, 256), h->d.nat), 256, 0, h->stream>>>(
-        h->d.ngl, h->ldg, g.gx, g.gy, g.gz, r_dev, g.t_ipro0, g.t_nlmn, g.pdesc, g.ylm, g.pro, g.prox);
-    CUW_LAUNCH_CHECK("k_pro_f64_direct");
-  } else {
+  const int todo = need & ~h->tabs;
+  if (todo & TAB_F64) CUW_RET(fold_table(h, r_dev));
+  if (todo & TAB_EIGR) {
+    CUW_RET(eigr_room(h));
     dim3 grid(std::min(ceil_div(h->d.ngl, 256), 64), h->d.nat);
     k_eigr<<<grid, 256, 0, h->stream>>>(h->g.gx, h->g.gy, h->g.gz, r_dev, h->d.ngl, h->d.nat, h->g.eigr);
     CUW_LAUNCH_CHECK("k_eigr");
-    if (h->mixed()) CUW_RET(tc_pro_table(h));
   }
+  if (todo & TAB_F32) CUW_RET(tc_pro_table(h));
+  h->tabs = pos ? (h->tabs | todo) : 0;
   if (pos) h->eigr_src = r_dev;
   return CUW_OK;
 }
 
-// projA = Omega <p|psiA>, projB likewise when psiB != null; uses h->g.eigr
-int proj_compute(Handle* h, const double2* psiA, double2* projA, const double2* psiB, double2* projB) {
+// projA = Omega <p|psiA>, projB likewise when psiB != null, from the tables of
+// eigr_compute; `folded`: slots 0 and 1 of the folded arrays hold psiA and psiB
+int proj_compute(Handle* h, const double2* psiA, double2* projA, const double2* psiB, double2* projB, bool folded) {
   if (h->tc_on()) {
     CUW_RET(tc_proj(h, psiA, projA));
     return psiB ? tc_proj(h, psiB, projB) : CUW_OK;
+  }
+  if (h->sym) {
+    if (!folded) {
+      CUW_RET(fold_psi(h, psiA, 0));
+      if (psiB) CUW_RET(fold_psi(h, psiB, 1));
+    }
+    return fold_proj(h, projA, psiB ? projB : nullptr);
   }
   const int nbh = h->d.nbh, npro = h->npro, ngl = h->d.ngl;
   const int tn = ceil_div(npro, BN), tm = ceil_div(nbh, BM);
@@ -1199,24 +798,13 @@ int proj_compute(Handle* h, const double2* psiA, double2* projA, const double2* 
   const bool dual = (psiB != nullptr);
   CUW_RET(ensure_part(h, sizeof(double2) * one * (dual ? 2 : 1)));
   dim3 grid(tn, tm, ks);
-  // FP64 handles read the expanded projector table; the FP64 products of a
-  // mixed handle (start-up orthonormalisation, orthonormality test) form it
-  const bool tab = !h->mixed() && h->g.prox;
   const Device& g = h->g;
-  if (dual && tab)
-    k_proj<true, true><<<grid, NT, smem2_bytes<MP21>(), h->stream>>>(psiA, psiB, h->ldg, ngl, nbh, npro, kchunk,
-                                                                   g.pdesc, g.ylm, g.pro, g.eigr, g.part, one,
-                                                                   g.prox);
-  else if (dual)
-    k_proj<true, false><<<grid, NT, smem_bytes<MP21>(), h->stream>>>(psiA, psiB, h->ldg, ngl, nbh, npro, kchunk,
-                                                                    g.pdesc, g.ylm, g.pro, g.eigr, g.part, one);
-  else if (tab)
-    k_proj<false, true><<<grid, NT, smem2_bytes<MP11>(), h->stream>>>(psiA, nullptr, h->ldg, ngl, nbh, npro, kchunk,
-                                                                    g.pdesc, g.ylm, g.pro, g.eigr, g.part, 0,
-                                                                    g.prox);
+  if (dual)
+    k_proj<true><<<grid, NT, smem_bytes<MP21>(), h->stream>>>(psiA, psiB, h->ldg, ngl, nbh, npro, kchunk, g.pdesc,
+                                                              g.ylm, g.pro, g.eigr, g.part, one);
   else
-    k_proj<false, false><<<grid, NT, smem_bytes<MP11>(), h->stream>>>(psiA, nullptr, h->ldg, ngl, nbh, npro, kchunk,
-                                                                     g.pdesc, g.ylm, g.pro, g.eigr, g.part, 0);
+    k_proj<false><<<grid, NT, smem_bytes<MP11>(), h->stream>>>(psiA, nullptr, h->ldg, ngl, nbh, npro, kchunk, g.pdesc,
+                                                               g.ylm, g.pro, g.eigr, g.part, 0);
   CUW_LAUNCH_CHECK("k_proj");
   const size_t n = (size_t)nbh * npro;
   const int rb = std::min(ceil_div((int)std::min<size_t>(n, 1 << 30), 256), 4 * h->nsm);
@@ -1237,18 +825,14 @@ int addpro_run(Handle* h, int mode, const double2* hpc, const double2* opc) {
   sc.a2 = 1.0 - sc.a1;
   sc.a3 = -h->delt * h->delt / (1.0 + h->annee);
   sc.oscale = h->delt * h->delt / (1.0 + h->annee);  // src/paw_waves2.f90:148-156
-  sc.fr = h->fric_on ? h->g.anv : nullptr;
+  sc.fr = h->fric_on ? h->g.aninv : nullptr;
   sc.dt2 = h->delt * h->delt;
   if (h->tc_on()) return tc_addpro(h, mode, hpc, opc, sc);
+  if (h->sym) return fold_addpro(h, mode, hpc, opc, sc);
   Device& g = h->g;
-  const bool tab = !h->mixed() && g.prox;
-#define CUW_ADDPRO(MODE_, MP_)                                                                                  \
-  (tab ? k_addpro<MODE_, true><<<grid, NT, smem2_bytes<MP_>(), h->stream>>>(                                      \
-             g.hpsi, g.opsi, g.psi0, g.psim, g.mpsi, h->ldg, ngl, nbh, npro, hpc, opc, g.pdesc, g.ylm, g.pro,    \
-             g.eigr, sc, g.prox)                                                                                 \
-       : k_addpro<MODE_, false><<<grid, NT, smem_bytes<MP_>(), h->stream>>>(                                     \
-             g.hpsi, g.opsi, g.psi0, g.psim, g.mpsi, h->ldg, ngl, nbh, npro, hpc, opc, g.pdesc, g.ylm, g.pro,    \
-             g.eigr, sc, nullptr))
+#define CUW_ADDPRO(MODE_, MP_)                                                                                    \
+  k_addpro<MODE_><<<grid, NT, smem_bytes<MP_>(), h->stream>>>(g.hpsi, g.opsi, g.psi0, g.psim, g.mpsi, h->ldg, ngl, \
+                                                              nbh, npro, hpc, opc, g.pdesc, g.ylm, g.pro, g.eigr, sc)
   switch (mode) {
     case ADDPRO_HPSI: CUW_ADDPRO(ADDPRO_HPSI, MP11); break;
     case ADDPRO_OPSI: CUW_ADDPRO(ADDPRO_OPSI, MP11); break;
@@ -1374,103 +958,21 @@ int oproj_compute(Handle* h, const double2* proj, double2* out) {
   return CUW_OK;
 }
 
-// T(pair) products into h->g.part region [pair][t][nbh*nbh] after reduction at
-// offset `dst` (complex), scaled by `scale`.
-static int gram_run(Handle* h, const GramPair* pairs, int npair, bool minus, int nk, int nm, size_t sk, size_t sm,
-                    double scale, double2* dst) {
-  if (h->tc_on()) return tc_gram(h, pairs, npair, minus, nk, nm, sk, sm, scale, dst);
-  GramArgs a;
-  for (int i = 0; i < npair; ++i) a.pair[i] = pairs[i];
-  a.npair = npair;
-  a.nk = nk;
-  a.nm = nm;
-  a.nn = nm;
-  a.sk = sk;
-  a.sm = sm;
-  const int tiles = ceil_div(nm, BM) * ceil_div(nm, BN) * npair;
-  int ks = choose_split(h, tiles, nk, 128, h->split_gram);
-  a.kchunk = ceil_div(ceil_div(nk, ks), BK) * BK;
-  ks = ceil_div(nk, a.kchunk);
-  const size_t mn = (size_t)nm * nm;
-  CUW_RET(ensure_part(h, sizeof(double2) * mn * 2 * npair * ks));
-  dim3 grid(ceil_div(nm, BN), ceil_div(nm, BM), ks * npair);
-  if (minus) k_gram<true, true><<<grid, NT, smem2_bytes<MPGRAM>(), h->stream>>>(a, h->g.minusg, h->g.part);
-  else k_gram<false, false><<<grid, NT, smem2_bytes<MPGRAM>(), h->stream>>>(a, h->g.minusg, h->g.part);
-  CUW_LAUNCH_CHECK("k_gram");
-  // reduce over splits: layout part[(split*npair+pair)*2+t] -> dst[(pair*2+t)]
-  const size_t n = mn * 2 * npair;
-  const int rb = std::min(ceil_div((int)n, 256), 4 * h->nsm);
-  k_reduce_parts<<<rb, 256, 0, h->stream>>>(h->g.part, ks, n, n, scale, dst);
-  CUW_LAUNCH_CHECK("k_reduce_parts");
-  return CUW_OK;
-}
-
-int gram_planewave(Handle* h, const GramPair* pairs, int npair, double2* dst) {
-  return gram_run(h, pairs, npair, true, h->d.ngl, h->d.nbh, 1, (size_t)h->ldg, h->gweight, dst);
-}
-
-int gram_projections(Handle* h, const GramPair* pairs, int npair, double2* dst) {
-  return gram_run(h, pairs, npair, false, h->npro, h->d.nbh, (size_t)h->d.nbh, 1, 1.0, dst);
-}
-
-int addopsi_run(Handle* h, double2* psibar, const double2* opsi, const double2* l1, const double2* l2) {
-  AddXArgs a;
-  a.out = psibar;
-  a.x = opsi;
-  a.l1 = l1;
-  a.l2 = l2;
-  a.nm = h->d.ngl;
-  a.nn = h->d.nbh;
-  a.nk = h->d.nbh;
-  a.sxm = 1;
-  a.sxk = (size_t)h->ldg;
-  a.som = 1;
-  a.son = (size_t)h->ldg;
-  if (h->tc_on()) return tc_addx(h, true, a.out, a.x, a.l1, a.l2, a.nm, a.nn, a.nk, a.sxm, a.sxk, a.som, a.son);
-  dim3 grid(ceil_div(a.nm, BM), ceil_div(a.nn, BN));
-  k_addx<true, true><<<grid, NT, smem2_bytes<MP11>(), h->stream>>>(a, h->g.minusg);
-  CUW_LAUNCH_CHECK("k_addx");
-  return CUW_OK;
-}
-
-// ADDOPROJ for the (NBH, NPRO) projection arrays (src/paw_waves2.f90:687-758):
-// PROJ(b,p) += sum_k OPROJ(k,p) L1(k,b) + conj(OPROJ(k,p)) L2(k,b), in FP64 on
-// both paths.  The product is small (NPRO x NBH outputs, K = NBH), so one
-// thread per output with K in order beats a tiled GEMM, whose few CTAs
-// mostly fill and drain their pipeline.
-int addoproj_run(Handle* h, double2* proj, const double2* oproj, const double2* l1, const double2* l2) {
-  const int n = h->npro * h->d.nbh;
-  if (n == 0) return CUW_OK;
-  k_addoproj<<<dim3(ceil_div(h->npro, 4), ceil_div(h->d.nbh, 64)), 256, 0, h->stream>>>(proj, oproj, l1, l2, h->npro,
-                                                                                        h->d.nbh);
-  CUW_LAUNCH_CHECK("k_addoproj");
-  return CUW_OK;
-}
-
 int force_gemm(Handle* h, const double2* ded, double* force_dev) {
   const int ngl = h->d.ngl, nbh = h->d.nbh, npro = h->npro;
   int tm = ceil_div(ngl, BM);
-  const int tn = ceil_div(npro, BN);
-  CUW_RET(ensure_part(h, sizeof(double) * 3 * (size_t)std::max(tm, ceil_div(ngl, 128)) * npro));
+  // row groups of the partial sums: tiles of 64 or 128 G, or CTAs of the folded form
+  CUW_RET(ensure_part(h, sizeof(double) * 3 * (size_t)std::max(tm, 2 * h->nsm) * npro));
   double* fpart = reinterpret_cast<double*>(h->g.part);
   if (h->tc_on()) {
     CUW_RET(tc_force(h, ded, fpart, &tm));
-  } else if (!h->mixed() && h->g.prox && nbh <= kFpSlices * BK) {
-    // persistent: about one CTA per SM, each walking every gstride-th G tile
-    const int gstride = std::max(1, std::min(tm, h->nsm / tn));
-    k_force_p<<<dim3(gstride, tn), NT, kFpSmem, h->stream>>>(h->g.psi0, h->ldg, ngl, nbh, npro, ded, h->g.gx,
-                                                               h->g.gy, h->g.gz, fpart, h->g.prox, gstride);
-    CUW_LAUNCH_CHECK("k_force_p");
-    tm = gstride;
+  } else if (h->sym) {
+    CUW_RET(fold_psi(h, h->g.psi0, 0));
+    CUW_RET(fold_force(h, ded, fpart, &tm));
   } else {
-    if (!h->mixed() && h->g.prox)
-      k_force<true><<<dim3(tm, tn), NT, smem2_bytes<MP11>(), h->stream>>>(
-          h->g.psi0, h->ldg, ngl, nbh, npro, ded, h->g.pdesc, h->g.ylm, h->g.pro, h->g.eigr, h->g.gx, h->g.gy,
-          h->g.gz, fpart, h->g.prox);
-    else
-      k_force<false><<<dim3(tm, tn), NT, smem2_bytes<MP11>(), h->stream>>>(
-          h->g.psi0, h->ldg, ngl, nbh, npro, ded, h->g.pdesc, h->g.ylm, h->g.pro, h->g.eigr, h->g.gx, h->g.gy,
-          h->g.gz, fpart, nullptr);
+    k_force<<<dim3(tm, ceil_div(npro, BN)), NT, smem2_bytes<MP11>(), h->stream>>>(
+        h->g.psi0, h->ldg, ngl, nbh, npro, ded, h->g.pdesc, h->g.ylm, h->g.pro, h->g.eigr, h->g.gx, h->g.gy, h->g.gz,
+        fpart);
     CUW_LAUNCH_CHECK("k_force");
   }
   TabView t = tables(h);
@@ -1482,22 +984,13 @@ int force_gemm(Handle* h, const double2* ded, double* force_dev) {
 
 // dynamic shared memory above 48 KB for the pipelined contraction kernels
 int gemm_setup(Handle* h) {
-  CUW_TRY(smem_allow((const void*)k_proj<true, false>, (int)smem_bytes<MP21>()));
-  CUW_TRY(smem_allow((const void*)k_proj<false, false>, (int)smem_bytes<MP11>()));
-  CUW_TRY(smem_allow((const void*)k_proj<true, true>, (int)smem2_bytes<MP21>()));
-  CUW_TRY(smem_allow((const void*)k_proj<false, true>, (int)smem2_bytes<MP11>()));
-  CUW_TRY(smem_allow((const void*)k_addpro<ADDPRO_HPSI, false>, (int)smem_bytes<MP11>()));
-  CUW_TRY(smem_allow((const void*)k_addpro<ADDPRO_OPSI, false>, (int)smem_bytes<MP11>()));
-  CUW_TRY(smem_allow((const void*)k_addpro<ADDPRO_FUSED, false>, (int)smem_bytes<MP12>()));
-  CUW_TRY(smem_allow((const void*)k_addpro<ADDPRO_HPSI, true>, (int)smem2_bytes<MP11>()));
-  CUW_TRY(smem_allow((const void*)k_addpro<ADDPRO_OPSI, true>, (int)smem2_bytes<MP11>()));
-  CUW_TRY(smem_allow((const void*)k_addpro<ADDPRO_FUSED, true>, (int)smem2_bytes<MP12>()));
-  CUW_TRY(smem_allow((const void*)k_gram<true, true>, (int)smem2_bytes<MPGRAM>()));
-  CUW_TRY(smem_allow((const void*)k_gram<false, false>, (int)smem2_bytes<MPGRAM>()));
-  CUW_TRY(smem_allow((const void*)k_addx<true, true>, (int)smem2_bytes<MP11>()));
-  CUW_TRY(smem_allow((const void*)k_force<false>, (int)smem2_bytes<MP11>()));
-  CUW_TRY(smem_allow((const void*)k_force<true>, (int)smem2_bytes<MP11>()));
-  CUW_TRY(smem_allow((const void*)k_force_p, (int)kFpSmem));
+  CUW_TRY(smem_allow((const void*)k_proj<true>, (int)smem_bytes<MP21>()));
+  CUW_TRY(smem_allow((const void*)k_proj<false>, (int)smem_bytes<MP11>()));
+  CUW_TRY(smem_allow((const void*)k_addpro<ADDPRO_HPSI>, (int)smem_bytes<MP11>()));
+  CUW_TRY(smem_allow((const void*)k_addpro<ADDPRO_OPSI>, (int)smem_bytes<MP11>()));
+  CUW_TRY(smem_allow((const void*)k_addpro<ADDPRO_FUSED>, (int)smem_bytes<MP12>()));
+  CUW_TRY(smem_allow((const void*)k_force, (int)smem2_bytes<MP11>()));
+  CUW_RET(fold_kernels_setup(h));
   return CUW_OK;
 }
 
@@ -1574,7 +1067,7 @@ static int noalloc_scratch(double2** out) {
   if (!g_noalloc_ptr[dev]) {
     void* p = nullptr;
     if (cudaGetSymbolAddress(&p, g_noalloc_scratch) != cudaSuccess) return CUW_ERR_CUDA;
-    if (cuw::smem_allow((const void*)cuw::k_proj<false, false>, (int)cuw::smem_bytes<cuw::MP11>()) != cudaSuccess)
+    if (cuw::smem_allow((const void*)cuw::k_proj<false>, (int)cuw::smem_bytes<cuw::MP11>()) != cudaSuccess)
       return CUW_ERR_CUDA;
     g_noalloc_ptr[dev] = static_cast<double2*>(p);
   }
@@ -1610,7 +1103,7 @@ extern "C" int cuwaves_projections_noalloc(int ngl, int ldg, int nbh, int nat, i
   // every partial sum that the reduction reads is written by k_proj in this
   // call, so nothing in the array has to start at zero; with no error pending
   // before the launches, cudaGetLastError reports only their own failures
-  k_proj<false, false><<<dim3(tn, tm, ks), NT, smem_bytes<MP11>(), st>>>(
+  k_proj<false><<<dim3(tn, tm, ks), NT, smem_bytes<MP11>(), st>>>(
       reinterpret_cast<const double2*>(psi), nullptr, ldg, ngl, nbh, npro, kchunk,
       reinterpret_cast<const ProDesc*>(pdesc), ylm, pro, reinterpret_cast<const double2*>(eigr), scratch, 0);
   if (cudaGetLastError() != cudaSuccess) return CUW_ERR_CUDA;

@@ -1328,20 +1328,6 @@ __global__ void k_lambda12(const double* __restrict__ lam, int nb, int nbh, doub
   l2[idx] = make_double2(0.5 * (s1.x + s2.x), 0.5 * (s1.y + s2.y));
 }
 
-// X (real NB x NB) -> X1, X2 of WAVES_GRAMSCHMIDT (src/paw_waves2.f90:2109-2128)
-__global__ void k_fold_x(const double* __restrict__ x, int nb, int nbh, double2* __restrict__ x1,
-                         double2* __restrict__ x2) {
-  int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= nbh * nbh) return;
-  int ibh1 = idx % nbh, ibh2 = idx / nbh;
-  int a = 2 * ibh1, b = 2 * ibh1 + 1, c = 2 * ibh2, d = 2 * ibh2 + 1;
-  // CSVAR1 = X11 + i X12 ; CSVAR2 = -i X21 + X22
-  double2 s1 = make_double2(x[a + (size_t)nb * c], x[a + (size_t)nb * d]);
-  double2 s2 = make_double2(x[b + (size_t)nb * d], -x[b + (size_t)nb * c]);
-  x1[idx] = make_double2(0.5 * (s1.x + s2.x), 0.5 * (s1.y + s2.y));
-  x2[idx] = make_double2(0.5 * (s1.x - s2.x), 0.5 * (s1.y - s2.y));
-}
-
 // real LAMBDA -> RLAM0 (complex), and the extrapolation of WAVES$SWITCH
 __global__ void k_store_lambda(const double* __restrict__ lam, int n, double2* __restrict__ rlam0) {
   int idx = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1905,13 +1891,6 @@ int smap_run(Handle* h) {
   CUW_TRY(cudaMemsetAsync(g.ostatus, 0, sizeof(int) * 2, h->stream));
   k_smap<<<1, 32, (sizeof(double) + sizeof(int)) * (size_t)n, h->stream>>>(g.rlam0, n, g.smap, g.ostatus);
   CUW_LAUNCH_CHECK("k_smap");
-  return CUW_OK;
-}
-
-int fold_x_run(Handle* h, const double* x, double2* x1, double2* x2) {
-  const int nbh = h->d.nbh;
-  k_fold_x<<<ceil_div(nbh * nbh, 256), 256, 0, h->stream>>>(x, h->d.nb, nbh, x1, x2);
-  CUW_LAUNCH_CHECK("k_fold_x");
   return CUW_OK;
 }
 

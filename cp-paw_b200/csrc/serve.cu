@@ -111,12 +111,11 @@ size_t estimate_bytes(const cuw_dims& d, const int* isp) {
   b += 4 * nbh * npro * 16;                            // proj, oproj, hproj, pbuf
   b += 2 * nb * nb * 16 + 24 * nb * nb * 8;            // Lagrange and solve matrices
   b += ngl * (3 * 4 + 7 * 8) + ngl * (nbare + d.lmx) * 8;  // G set and tables
-  b += ngl * (size_t)d.nat * 16;                       // EIGR
   b += nr * 8;                                         // V(r)
   b += std::min(nbh * nr * 16, ((size_t)48 << 20) + nr * 16);  // FFT work grid
   b += (size_t)20 << 20;                               // split-K partials and small tables
-  if (d.precision == CUW_PREC_MIXED) b += ldg * npro * 8;  // fp32 projector table
-  else b += ldg * npro * 16;                               // fp64 projector table
+  if (d.precision == CUW_PREC_MIXED) b += ldg * npro * 8 + ngl * (size_t)d.nat * 16;  // fp32 projector table, EIGR
+  else b += ldg * npro * 8 + 2 * ldg * nbh * 16;  // folded fp64 projector table and wave functions
   return b;
 }
 

@@ -301,10 +301,9 @@ __global__ void __launch_bounds__(kThreads, 1)
           if (MODE == ADDPRO_FUSED) {
             double a1 = sc.a1, a2 = sc.a2, a3 = sc.a3 * rm;
             if (sc.fr) {  // cell friction ANNEEVEC(G) (src/paw_waves1.f90:6536-6540)
-              const double an = 1.0 + sc.fr[g];
-              a1 = 2.0 / an;
+              a1 = 2.0 * sc.fr[g];
               a2 = 1.0 - a1;
-              a3 = -sc.dt2 / an * rm;
+              a3 = -sc.dt2 * sc.fr[g] * rm;
             }
             psim[k[q]] = make_double2(a1 * p0v[q].x + a2 * pm[q].x + a3 * h2.x, a1 * p0v[q].y + a2 * pm[q].y + a3 * h2.y);
           }

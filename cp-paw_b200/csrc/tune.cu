@@ -84,6 +84,19 @@ int grid_room(Handle* h, int bands) {
   return CUW_OK;
 }
 
+// the step's three plane-wave overlaps, on PSI0 and PSIM (results into the
+// solve's scratch matrices)
+int overlaps(Handle* h) {
+  Device& g = h->g;
+  if (h->tc_on()) {
+    const GramPair p[3] = {{g.psi0, g.psi0}, {g.psim, g.psi0}, {g.psim, g.psim}};
+    return tc_gram(h, p, 3, true, h->d.ngl, h->d.nbh, 1, (size_t)h->ldg, h->gweight, g.tmat);
+  }
+  CUW_RET(fold_room(h));
+  const FoldPair p[3] = {{0, 0, g.pbuf, g.pbuf}, {1, 0, g.pbuf, g.pbuf}, {1, 1, g.pbuf, g.pbuf}};
+  return fold_gram(h, p, 3, g.mat, g.omat, g.oomat);
+}
+
 }  // namespace
 
 int autotune(Handle* h, double* out, int n) {
@@ -106,6 +119,7 @@ int autotune(Handle* h, double* out, int n) {
     CUW_RET(grid_room(h, c.batch));
     CUW_RET(fft_set_variant(h, c.fft_variant));
     h->dmma_tiles = c.dmma_tiles != 0;
+    CUW_RET(fold_rooms(h));
   } else {
     CUW_RET(eigr_compute(h, g.r0));
     // FFT band batch: the L2 rule's batch and even splits of the bands
@@ -145,14 +159,14 @@ int autotune(Handle* h, double* out, int n) {
     c.dmma_tiles = h->dmma_tiles ? 1 : 0;
     c.ms[3] = c.ms[4] = 0.0;
     if (h->mixed()) {
-      const GramPair pq[3] = {{g.psi0, g.psi0}, {g.psim, g.psi0}, {g.psim, g.psim}};
       h->split_proj = h->split_gram = 1.0;
       for (int fam = 0; fam < 2; ++fam) {
         h->dmma_tiles = fam == 1;
         double ms = 0.0;
+        CUW_RET(eigr_compute(h, g.r0));  // the tables of this family
         CUW_RET(time_best(h, [&] {
           int rc = proj_compute(h, g.psi0, g.pbuf, nullptr, nullptr);
-          if (rc == CUW_OK) rc = gram_planewave(h, pq, 3, g.tmat);
+          if (rc == CUW_OK) rc = overlaps(h);
           if (rc == CUW_OK) rc = addpro_run(h, ADDPRO_HPSI, g.hproj, g.oproj);
           return rc;
         }, 3, &ms));
@@ -160,6 +174,7 @@ int autotune(Handle* h, double* out, int n) {
       }
       c.dmma_tiles = c.ms[4] < c.ms[3] ? 1 : 0;
       h->dmma_tiles = c.dmma_tiles != 0;
+      CUW_RET(eigr_compute(h, g.r0));
       h->have_hpsi = false;
     }
     // split-K factors
@@ -175,11 +190,10 @@ int autotune(Handle* h, double* out, int n) {
         c.split_proj = m;
       }
     }
-    const GramPair pp[3] = {{g.psi0, g.psi0}, {g.psim, g.psi0}, {g.psim, g.psim}};
     for (double m : muls) {
       h->split_gram = m;
       double ms = 0.0;
-      CUW_RET(time_best(h, [&] { return gram_planewave(h, pp, 3, g.tmat); }, 3, &ms));
+      CUW_RET(time_best(h, [&] { return overlaps(h); }, 3, &ms));
       if (ms < c.ms[2]) {
         c.ms[2] = ms;
         c.split_gram = m;
