@@ -18,7 +18,6 @@
 
 namespace cuw {
 
-int unravel_run(Handle* h, const double2* pw, const double2* oc, int npair, double* o0, double* o1, double* o2);
 int jacobi_run(Handle* h, const double* s_dev, double* u, double* e, const int* gate);
 int lambda_init_run(Handle* h);
 int store_lambda_run(Handle* h);
@@ -382,46 +381,25 @@ static int force_dev_run(Handle* h, double* force_dev) {
 static int mark(Handle* h, int phase);
 // (enqueues only: the solve's status is read with the step's results).
 // fused: the step's ADDPRO has formed PSIM and OPSI (and left them folded in
-// slots 0 and 1 where it is the folded form)
+// slots 0 and 1, where it is a folded form)
 static int ortho_core(Handle* h, int max_iter, double eps, bool fused) {
   Device& g = h->g;
   // projections of PSIBAR and OPSI at R(+)
   CUW_RET(mark(h, 1));
   CUW_RET(eigr_compute(h, g.rp));
   CUW_RET(mark(h, 5));
-  // PSIBAR and OPSI stay fixed through the Gram products: their split forms
-  // are reused (the guard closes the scope on every way out)
-  struct ScopeGuard {
-    Handle* h;
-    ~ScopeGuard() {
-      if (h) tc_scope(h, false);
-    }
-  } guard{h->mixed() ? h : nullptr};
-  if (h->mixed()) tc_scope(h, true);
-  if (!h->tc_on() && !(fused && h->sym)) {
-    CUW_RET(fold_psi(h, g.psim, 0));
-    CUW_RET(fold_psi(h, g.opsi, 1));
+  const bool tc = h->tc_on();
+  if (!(fused && h->sym)) {
+    CUW_RET(tc ? tc_fold(h, g.psim, 0) : fold_psi(h, g.psim, 0));
+    CUW_RET(tc ? tc_fold(h, g.opsi, 1) : fold_psi(h, g.opsi, 1));
   }
   CUW_RET(proj_compute(h, g.psim, g.proj, g.opsi, g.oproj, true));
   CUW_RET(mark(h, 6));
   // DO*PROJ and DO*OPROJ
   CUW_RET(oproj_compute(h, g.proj, g.hproj));
   CUW_RET(oproj_compute(h, g.oproj, g.pbuf));
-  if (h->tc_on()) {
-    const size_t mn = (size_t)h->d.nbh * h->d.nbh;
-    double2* pw = g.tmat;
-    double2* oc = g.tmat + 6 * mn;
-    GramPair pc[3] = {{g.proj, g.hproj}, {g.oproj, g.hproj}, {g.oproj, g.pbuf}};
-    CUW_RET(tc_gram(h, pc, 3, false, h->npro, h->d.nbh, (size_t)h->d.nbh, 1, 1.0, oc));
-    GramPair pp[3] = {{g.psim, g.psim}, {g.opsi, g.psim}, {g.opsi, g.opsi}};
-    CUW_RET(tc_gram(h, pp, 3, true, h->d.ngl, h->d.nbh, 1, (size_t)h->ldg, h->gweight, pw));
-    CUW_RET(unravel_run(h, pw, oc, 3, g.mat, g.omat, g.oomat));
-  } else {
-    const FoldPair pp[3] = {{0, 0, g.proj, g.hproj}, {1, 0, g.oproj, g.hproj}, {1, 1, g.oproj, g.pbuf}};
-    CUW_RET(fold_gram(h, pp, 3, g.mat, g.omat, g.oomat));
-  }
-  if (h->mixed()) tc_scope(h, false);
-  guard.h = nullptr;
+  const FoldPair pp[3] = {{0, 0, g.proj, g.hproj}, {1, 0, g.oproj, g.hproj}, {1, 1, g.oproj, g.pbuf}};
+  CUW_RET(tc ? tc_gram(h, pp, 3, g.mat, g.omat, g.oomat) : fold_gram(h, pp, 3, g.mat, g.omat, g.oomat));
   CUW_RET(mark(h, 7));
   if (h->safeortho) {
     CUW_RET(lambda_init_run(h));
@@ -435,13 +413,7 @@ static int ortho_core(Handle* h, int max_iter, double eps, bool fused) {
     CUW_RET(ortho_y_general(h, g.mat, g.omat, g.oomat, h->swapstates ? g.smap : nullptr, g.lam, !h->swapstates));
   }
   CUW_RET(mark(h, 8));
-  if (h->tc_on()) {
-    CUW_RET(lambda12_run(h, g.lam, g.lam1c, g.lam2c));
-    CUW_RET(tc_addx(h, true, g.psim, g.opsi, g.lam1c, g.lam2c, h->d.ngl, h->d.nbh, h->d.nbh, 1, (size_t)h->ldg, 1,
-                    (size_t)h->ldg));
-  } else {
-    CUW_RET(fold_addx(h, 1, g.lam, g.psim));
-  }
+  CUW_RET(tc ? tc_addx(h, 1, g.lam, g.psim) : fold_addx(h, 1, g.lam, g.psim));
   CUW_RET(addoproj_run(h, g.proj, g.oproj, g.lam));
   CUW_RET(store_lambda_run(h));
   h->have_opsi = false;
@@ -508,9 +480,9 @@ static void free_all(Handle* h) {
                   g.minusg, g.gx, g.gy, g.gz, g.g2, g.pro, g.ylm, g.mpsi, g.bucket, g.pdesc, g.plane_iz, g.plane_rows, g.plane_off,
                   g.plane_g, g.plane_pos, g.zslot, g.v, g.grid, g.tw1, g.tw2, g.tw3, g.r0, g.rp, g.rm, g.force, g.mass,
                   g.eigr, g.dh, g.dover, g.occ, g.mat, g.omat, g.oomat, g.lam, g.lam2, g.lam0, g.u, g.u2, g.eig, g.haux, g.gamn,
-                  g.work, g.wk2, g.smat, g.emat, g.gt, g.xb, g.tb, g.maxpart, g.ostatus, g.smap, g.lam1c, g.lam2c, g.part, g.red, g.scal, g.tmat, g.t_ipro0,
-                  g.t_nlmn, g.t_isp, g.t_lnofp, g.t_mofp, g.t_lmn0ln, g.t_lox, g.pf, g.xminus[0], g.xminus[1], g.bpre[0],
-                  g.bpre[1], g.bsmall, g.jac_a, g.r_plus, g.r_minus, g.r_gx, g.r_gy, g.r_gz, g.r_g2, g.r_ylm,
+                  g.work, g.wk2, g.smat, g.emat, g.gt, g.xb, g.tb, g.maxpart, g.ostatus, g.smap, g.part, g.red, g.scal, g.t_ipro0,
+                  g.t_nlmn, g.t_isp, g.t_lnofp, g.t_mofp, g.t_lmn0ln, g.t_lox, g.pf, g.u32, g.bpre,
+                  g.bsmall, g.jac_a, g.r_plus, g.r_minus, g.r_gx, g.r_gy, g.r_gz, g.r_g2, g.r_ylm,
                   g.r_g0, g.r_v0, g.r_pscore, g.r_vbar, g.r_lmrx, g.qlm, g.r_rhog, g.r_vg, g.r_pot, g.r_vtot,
                   g.r_grid, g.r_part, g.fpot, g.vqlm, g.r_out, g.half, g.prox, g.uf, g.anv, g.aninv, g.dbucket, g.rmpsi};
   for (void* p : ptrs)
@@ -596,7 +568,6 @@ extern "C" int cuwaves_create(const cuw_dims* dims, cuw_handle** out) {
     const size_t nps = (size_t)h->ldg * d.nbh * sizeof(double2);
     const size_t npj = (size_t)d.nbh * std::max(1, h->npro) * sizeof(double2);
     const size_t nn = (size_t)d.nb * d.nb;
-    const size_t mn = (size_t)d.nbh * d.nbh;
 #define TRYA(p, b) \
   if ((rc = dev_alloc(h, reinterpret_cast<void**>(&(p)), (b))) != CUW_OK) break
     TRYA(g.psi0, nps); TRYA(g.psim, nps); TRYA(g.hpsi, nps); TRYA(g.opsi, nps);
@@ -622,8 +593,6 @@ extern "C" int cuwaves_create(const cuw_dims* dims, cuw_handle** out) {
     TRYA(g.smat, sizeof(double) * nn); TRYA(g.emat, sizeof(double) * nn); TRYA(g.gt, sizeof(double) * nn);
     TRYA(g.xb, sizeof(double) * nn); TRYA(g.tb, sizeof(double) * nn);
     TRYA(g.maxpart, sizeof(double) * 64); TRYA(g.ostatus, sizeof(int) * 16); TRYA(g.smap, sizeof(int) * d.nb);
-    TRYA(g.lam1c, sizeof(double2) * mn); TRYA(g.lam2c, sizeof(double2) * mn);
-    TRYA(g.tmat, sizeof(double2) * 12 * mn);
     TRYA(g.red, sizeof(double) * (4 * (size_t)d.nbh * (ceil_div(d.ngl, RG) + 1) + 8));
     TRYA(g.scal, sizeof(double) * (size_t)(2 * d.nb + 16));
 #undef TRYA
@@ -1733,7 +1702,7 @@ extern "C" int cuwaves_set_option(cuw_handle* hp, int option, double value) {
       if (value != 0.0 && value != 1.0) return h->fail(CUW_ERR_ARG, "CONTRACTION_TILES must be 0 or 1");
       if (!h->mixed() && value == 0.0) return h->fail(CUW_ERR_ARG, "FP64 handles have DMMA tiles only");
       h->dmma_tiles = value != 0.0;
-      return h->have_gset ? fold_rooms(h) : CUW_OK;
+      return CUW_OK;
     case CUW_OPT_SAFEORTHO:
       if (value != 0.0 && value != 1.0) return h->fail(CUW_ERR_ARG, "SAFEORTHO must be 0 or 1");
       h->safeortho = value != 0.0;

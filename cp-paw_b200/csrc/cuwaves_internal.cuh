@@ -93,19 +93,19 @@ struct Device {
   double *r0 = nullptr, *rp = nullptr, *rm = nullptr;  // (3, NAT)
   double *force = nullptr;       // (3, NAT)
   double *mass = nullptr;        // (NAT)
-  double2 *eigr = nullptr;       // (NGL, NAT) structure factors of the last position set
-  float2 *pf = nullptr;          // (LDG, NPRO) mixed path: PRO(g,p) of the last position set in fp32, 0 for g >= NGL
+  double2 *eigr = nullptr;       // (NGL, NAT) structure factors of the last position set (G sets without parity)
   // folded arrays of the FP64 products (fold.cu): the +-G pairs of the sphere,
   // P(r,p) of the last position set (LDU, NPRO) and two slots of U(r,n) (LDU, NB)
   int2 *half = nullptr;
   double *prox = nullptr;
   double *uf = nullptr;
-  double2 *xminus[2] = {nullptr, nullptr};  // (LDG, NBH) mixed path: X(-G) copies of wave-function arrays
-  float *bpre[2] = {nullptr, nullptr};       // mixed path: wave-function arrays split into tf32 B tiles
-  const double2 *bpre_src[2] = {nullptr, nullptr};  // arrays they hold (valid inside a solve scope)
-  float *bsmall = nullptr;                   // mixed path: small matrices split into tf32 B tiles (3 slots)
+  // the same in fp32 (mixed path), and the operands split into tf32 B tiles: the
+  // two slots of U, and the small matrix of the product under way
+  float *pf = nullptr;
+  float *u32 = nullptr;
+  float *bpre = nullptr;
+  float *bsmall = nullptr;
   double *jac_a = nullptr;                   // packed matrix of the eigensolver when NB is too large for shared memory
-  size_t bsmall_slot = 0;                    // floats per slot
   double2 *dh = nullptr;         // (LMNXX, LMNXX, NAT)
   double *dover = nullptr;       // (LNXX, LNXX, NSP)
   double *occ = nullptr;         // (NB)
@@ -120,8 +120,6 @@ struct Device {
   int *smap = nullptr;           // (NB) state order of WAVES_ORTHO_Y_C (SAFEORTHO = F, SWAPSTATES = T)
   // (NGL) ANNEEVEC, 1 / (1 + ANNEEVEC) and GSET%DBUCKET of the cell friction
   double *anv = nullptr, *aninv = nullptr, *dbucket = nullptr;
-  double2 *lam1c = nullptr, *lam2c = nullptr;  // (NBH, NBH) folded multipliers
-  double2 *tmat = nullptr;       // 12 (NBH, NBH) reduced Gram products
   // scratch for split-K partial sums and band reductions
   double2 *part = nullptr;
   size_t part_bytes = 0;
@@ -230,7 +228,7 @@ struct Handle {
   // of the split-tf32 tcgen05 tiles (128 x 128 x 8); set by the autotuner or
   // CUW_OPT_CONTRACTION_TILES
   bool dmma_tiles = false;
-  bool tc_on() const { return mixed() && !fp64_only && !dmma_tiles; }
+  bool tc_on() const { return mixed() && !fp64_only && !dmma_tiles && sym; }
   // relative accuracy to which each ORTHO_X iteration solves its Lyapunov
   // equation (0: to rounding).  Measured on Si64 over 40 CP steps against the
   // solve to rounding: 1e-6 moves the FP64 total energy by 3e-12 Ha and the
@@ -248,7 +246,6 @@ struct Handle {
   double emass = 0.0, emasscg2 = 0.0;
   int lyap_max_sweeps = 64;  // sweeps per Lyapunov solve before the fixed point counts as failed
   bool ortho_panel = true;   // ORTHO_X by the panel-staged cluster kernel where it applies (64 < NB <= 128)
-  bool tc_scope_open = false;
   // position buffer (r0, rp or rm) that the projector tables were built from,
   // and which of them (TAB_*) are current for it
   const double* eigr_src = nullptr;
@@ -376,16 +373,11 @@ int hoproj_compute(Handle* h, const double2* proj, double2* hout, double2* oout)
 int ortho_solve(Handle* h, int max_iter, double eps);
 int ortho_result(Handle* h, const int* st, int* iters);
 int addoproj_run(Handle* h, double2* proj, const double2* oproj, const double* lam);
-int lambda12_run(Handle* h, const double* lam_real, double2* l1, double2* l2);
 int band_reduce(Handle* h, int what, double* out_host, double* eig_host);
 int force_run(Handle* h, double* force_host);
 int force_gemm(Handle* h, const double2* ded, double* force_dev);
 int small_tables_setup(Handle* h);
 int gemm_setup(Handle* h);
-struct GramPair {
-  const double2* x;
-  const double2* y;
-};
 // folded FP64 products (fold.cu); slots 0 and 1 hold folded wave-function arrays
 struct FoldPair {
   int x, y;                // slots
@@ -394,9 +386,6 @@ struct FoldPair {
 int fold_setup(Handle* h, const std::vector<int>& minusg);
 int fold_kernels_setup(Handle* h);
 int fold_rooms(Handle* h);
-int fold_room(Handle* h);
-int eigr_room(Handle* h);
-int fold_table_room(Handle* h);
 int fold_table(Handle* h, const double* r_dev);
 int fold_psi(Handle* h, const double2* psi, int slot);
 int fold_proj(Handle* h, double2* proj0, double2* proj1);
@@ -405,6 +394,9 @@ int fold_gram(Handle* h, const FoldPair* pairs, int npair, double* o0, double* o
 // ADDPRO_FUSED leaves folded PSIM in slot 0 and OPSI in slot 1
 int fold_addpro(Handle* h, int mode, const double2* hpc, const double2* opc, const StepCoef& sc);
 int fold_addx(Handle* h, int slot, const double* lam, double2* out);
+// the one-centre part of fold_gram alone: kc FP64 partial matrices per pair
+int fold_oc_splits(const Handle* h, int npair);
+int fold_oc(Handle* h, const FoldPair* pairs, int npair, int kc, double* oc);
 int fold_force(Handle* h, const double2* ded, double* fpart, int* nt);
 int ensure_part(Handle* h, size_t bytes);  // split-K scratch h->g.part of at least `bytes`
 // Raises (never lowers) the dynamic shared-memory limit of kernel fn on the
@@ -412,19 +404,18 @@ int ensure_part(Handle* h, size_t bytes);  // split-K scratch h->g.part of at le
 // handles of the process: a handle of a smaller system must not lower the
 // limit that a larger one launches with.
 cudaError_t smem_allow(const void* fn, int bytes);
-// split-precision (tf32 x3) tensor-core versions, used when precision is
-// CUW_PREC_MIXED; same arguments and results as the FP64 functions above
+// split-precision (tf32 x3) tensor-core versions, used when tc_on(); tc_fold
+// puts a wave-function array into a slot of U in fp32, tc_split forms the split
+// B operands of slots 0 .. nset-1
 int tc_setup(Handle* h);
-int tc_pro_table(Handle* h);  // h->g.pf from h->g.eigr (mixed path)
-// Split wave-function operands computed inside a scope are reused by later
-// contractions of the same scope (the arrays do not change inside it).
-void tc_scope(Handle* h, bool open);
-int tc_proj(Handle* h, const double2* psi, double2* proj);
+int tc_rooms(Handle* h);
+int tc_pro_table(Handle* h, const double* r_dev);
+int tc_fold(Handle* h, const double2* psi, int slot);
+int tc_split(Handle* h, int nset);
+int tc_proj(Handle* h, double2* proj0, double2* proj1);
 int tc_addpro(Handle* h, int mode, const double2* hpc, const double2* opc, const StepCoef& sc);
-int tc_gram(Handle* h, const GramPair* pairs, int npair, bool minus, int nk, int nm, size_t sk, size_t sm,
-            double scale, double2* dst);
-int tc_addx(Handle* h, bool xminus, double2* out, const double2* x, const double2* l1, const double2* l2, int nm,
-            int nn, int nk, size_t sxm, size_t sxk, size_t som, size_t son);
+int tc_gram(Handle* h, const FoldPair* pairs, int npair, double* o0, double* o1, double* o2);
+int tc_addx(Handle* h, int slot, const double* lam, double2* out);
 int tc_force(Handle* h, const double2* ded, double* fpart, int* ntile);
 int propagate_run(Handle* h);
 int opsi_scale(Handle* h, double oscale);

@@ -35,6 +35,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <string>
 #include <vector>
 
 #include "cuwaves_internal.cuh"
@@ -315,8 +316,8 @@ __global__ void k_rproj_sum(const double2* __restrict__ part, int nz, int nbh, i
 
 // ---------------------------------------------------------------------------
 // Overlaps of up to three pairs: part[z][pair][i][j], z < ks: the plane-wave
-// sum over split z of U(r,i) V(r,j); z = ks: the one-centre sum over the
-// projectors of P_x(i,p) (DO P_y)(j,p)  (WAVES_OVERLAP + WAVES_1COVERLAP,
+// sum over split z of U(r,i) V(r,j); z >= ks: the one-centre sum over split z - ks
+// of the projectors of P_x(i,p) (DO P_y)(j,p)  (WAVES_OVERLAP + WAVES_1COVERLAP,
 // src/paw_waves2.f90:761-1022)
 // ---------------------------------------------------------------------------
 struct RGramArgs {
@@ -324,7 +325,7 @@ struct RGramArgs {
   const double* y[3];
   const double* px[3];  // projections, real view (n + NB p)
   const double* py[3];
-  int npair, nb, npro, nr, ldu, kchunk, ks;
+  int npair, nb, npro, nr, ldu, kchunk, ks, pchunk;
 };
 template <int MI, int NI>
 __global__ void __launch_bounds__(RT, 2) k_rgram(RGramArgs a, double* __restrict__ part) {
@@ -339,7 +340,8 @@ __global__ void __launch_bounds__(RT, 2) k_rgram(RGramArgs a, double* __restrict
     rmain<MI, NI, true, true>(rsm, x, m0, y, n0, z * a.kchunk, min(a.nr, (z + 1) * a.kchunk), acc);
   } else {
     const Op x{of(a.px), a.nb, a.nb}, y{of(a.py), a.nb, a.nb};
-    rmain<MI, NI, false, false>(rsm, x, m0, y, n0, 0, a.npro, acc);
+    const int k0 = (z - a.ks) * a.pchunk;
+    rmain<MI, NI, false, false>(rsm, x, m0, y, n0, k0, min(a.npro, k0 + a.pchunk), acc);
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
@@ -356,13 +358,13 @@ __global__ void __launch_bounds__(RT, 2) k_rgram(RGramArgs a, double* __restrict
   }
 }
 
-// out_pair(i + NB j) = scale * sum_z part[z][pair][i][j] + part[ks][pair][i][j]
-__global__ void k_rgram_sum(const double2* __restrict__ part, int ks, int nb, int npair, double scale,
+// out_pair(i + NB j) = scale * the ks plane-wave parts + the kc one-centre parts
+__global__ void k_rgram_sum(const double2* __restrict__ part, int ks, int kc, int nb, int npair, double scale,
                             double* __restrict__ o0, double* __restrict__ o1, double* __restrict__ o2) {
   const size_t per = (size_t)nb * nb / 2, n = per * npair;
   const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (t >= n) return;
-  const double2 s = sum_parts(part + t, ks, n), c = part[(size_t)ks * n + t];
+  const double2 s = sum_parts(part + t, ks, n), c = sum_parts(part + (size_t)ks * n + t, kc, n);
   const int pair = (int)(t / per);
   const size_t e = 2 * (t % per);
   const int i = (int)(e / nb), j = (int)(e % nb);
@@ -739,10 +741,17 @@ int fold_setup(Handle* h, const std::vector<int>& mg) {
     if (i <= mg[i]) half.push_back(make_int2(i, mg[i]));
   const int nh = (int)half.size(), ldu = ceil_div(2 * nh, 32) * 32;
   if (nh != h->nh) {
-    for (void** p : {(void**)&g.half, (void**)&g.uf, (void**)&g.prox}) {
-      if (*p) cudaFree(*p);
-      *p = nullptr;
-    }
+    auto drop = [](auto*& p) {
+      if (p) cudaFree(p);
+      p = nullptr;
+    };
+    drop(g.half);
+    drop(g.uf);
+    drop(g.prox);
+    drop(g.pf);
+    drop(g.u32);
+    drop(g.bpre);
+    drop(g.bsmall);
     h->nh = nh;
     h->ldu = ldu;
     CUW_TRY(cudaMalloc(&g.half, sizeof(int2) * nh));
@@ -760,51 +769,31 @@ int fold_setup(Handle* h, const std::vector<int>& mg) {
   return fold_rooms(h);
 }
 
-// Buffers of the tables and folded arrays that the handle's steps use, so that
-// no step allocates (steps are captured into graphs).
+// Buffers whose sizes follow from the folded sphere: two folded wave-function
+// arrays (rows of slot 1 follow slot 0's), the projector table or, for tables
+// without parity, EIGR, and the fp32 forms of the mixed path (whose start-up
+// orthonormalisation is FP64).  No later call allocates them, so that no step
+// captured into a graph does.
 int fold_rooms(Handle* h) {
-  if (!h->mixed() || h->dmma_tiles) {
-    CUW_RET(fold_room(h));
-    CUW_RET(h->sym ? fold_table_room(h) : eigr_room(h));
-  }
-  return h->mixed() ? eigr_room(h) : CUW_OK;
-}
-
-// the two folded FP64 wave-function arrays (rows of slot 1 follow slot 0's).
-// A mixed-precision handle allocates them, and the FP64 table below, at its
-// first FP64 product (start-up orthonormalisation, orthonormality test, DMMA
-// tiles).
-int fold_room(Handle* h) {
-  if (h->g.uf) return CUW_OK;
-  if (h->capturing) return h->fail(CUW_ERR_STATE, "folded wave functions allocated during graph capture");
-  h->touch();
-  const size_t n = sizeof(double) * (size_t)h->ldu * h->d.nb * 2;
-  if (cudaMalloc(&h->g.uf, n) != cudaSuccess) {
-    cudaGetLastError();
-    h->g.uf = nullptr;
-    return h->fail(CUW_ERR_NOMEM, "cudaMalloc of the folded wave functions failed");
-  }
-  CUW_TRY(cudaMemsetAsync(h->g.uf, 0, n, h->stream));
-  return CUW_OK;
-}
-int fold_table_room(Handle* h) {
-  if (h->g.prox || h->npro == 0) return CUW_OK;
-  if (h->capturing) return h->fail(CUW_ERR_STATE, "projector table allocated during graph capture");
-  h->touch();
-  const size_t n = sizeof(double) * (size_t)h->ldu * h->npro;
-  if (cudaMalloc(&h->g.prox, n) != cudaSuccess) {
-    cudaGetLastError();
-    h->g.prox = nullptr;
-    return h->fail(CUW_ERR_NOMEM, "cudaMalloc of the projector table failed");
-  }
-  CUW_TRY(cudaMemsetAsync(h->g.prox, 0, n, h->stream));
-  return CUW_OK;
+  auto room = [&](auto*& p, size_t n, const char* what) -> int {
+    if (p || n == 0) return CUW_OK;
+    if (cudaMalloc(&p, n * sizeof(*p)) != cudaSuccess) {
+      cudaGetLastError();
+      p = nullptr;
+      return h->fail(CUW_ERR_NOMEM, std::string("cudaMalloc of the ") + what + " failed");
+    }
+    return CUW_OK;
+  };
+  Device& g = h->g;
+  CUW_RET(room(g.uf, (size_t)h->ldu * h->d.nb * 2, "folded wave functions"));
+  if (h->sym) CUW_RET(room(g.prox, (size_t)h->ldu * h->npro, "projector table"));
+  else CUW_RET(room(g.eigr, (size_t)h->d.ngl * std::max(1, h->d.nat), "structure factors"));
+  return h->mixed() && h->sym ? tc_rooms(h) : CUW_OK;
 }
 
 static double* slot_ptr(const Handle* h, int slot) { return h->g.uf + (size_t)slot * h->d.nb * h->ldu; }
 
 int fold_psi(Handle* h, const double2* psi, int slot) {
-  CUW_RET(fold_room(h));
   k_fold<<<dim3(ceil_div(h->nh, 256), h->d.nbh), 256, 0, h->stream>>>(psi, h->g.half, h->nh, h->ldg, h->ldu,
                                                                       slot_ptr(h, slot));
   CUW_LAUNCH_CHECK("k_fold");
@@ -812,7 +801,6 @@ int fold_psi(Handle* h, const double2* psi, int slot) {
 }
 
 int fold_table(Handle* h, const double* r_dev) {
-  CUW_RET(fold_table_room(h));
   const Device& g = h->g;
   k_pro_fold<<<dim3(ceil_div(h->nh, 256), h->d.nat), 256, 0, h->stream>>>(h->nh, h->d.ngl, h->ldu, g.half, g.gx, g.gy,
                                                                           g.gz, r_dev, g.t_ipro0, g.t_nlmn, g.pdesc,
@@ -846,40 +834,69 @@ int fold_proj(Handle* h, double2* proj0, double2* proj1) {
   return CUW_OK;
 }
 
-int fold_gram(Handle* h, const FoldPair* pairs, int npair, double* o0, double* o1, double* o2) {
+static int gram_args(Handle* h, const FoldPair* pairs, int npair, RGramArgs* a) {
   if (npair < 1 || npair > 3) return h->fail(CUW_ERR_ARG, "overlaps: one to three pairs");
-  RGramArgs a{};
+  *a = RGramArgs{};
   for (int i = 0; i < npair; ++i) {
-    a.x[i] = slot_ptr(h, pairs[i].x);
-    a.y[i] = slot_ptr(h, pairs[i].y);
-    a.px[i] = reinterpret_cast<const double*>(pairs[i].px);
-    a.py[i] = reinterpret_cast<const double*>(pairs[i].py);
+    a->x[i] = slot_ptr(h, pairs[i].x);
+    a->y[i] = slot_ptr(h, pairs[i].y);
+    a->px[i] = reinterpret_cast<const double*>(pairs[i].px);
+    a->py[i] = reinterpret_cast<const double*>(pairs[i].py);
   }
-  const int nb = h->d.nb, nr = 2 * h->nh;
-  a.npair = npair;
-  a.nb = nb;
-  a.npro = h->npro;
-  a.nr = nr;
-  a.ldu = h->ldu;
-  RTile t = pick_tile(h, nb, nb);
+  a->npair = npair;
+  a->nb = h->d.nb;
+  a->npro = h->npro;
+  a->nr = 2 * h->nh;
+  a->ldu = h->ldu;
+  return CUW_OK;
+}
+static RTile gram_tile(const Handle* h) {
+  RTile t = pick_tile(h, h->d.nb, h->d.nb);
   t.mi = t.ni == 8 ? 4 : 2;
-  const int tiles = ceil_div(nb, 16 * t.ni) * ceil_div(nb, 16 * t.mi) * npair;
-  // one split's worth of CTAs forms the one-centre sums
-  int ks = std::max(1, rsplit(h, tiles, nr, h->split_gram) - 1);
-  a.kchunk = ceil_div(ceil_div(nr, ks), RK) * RK;
-  a.ks = ks = ceil_div(nr, a.kchunk);
-  CUW_RET(ensure_part(h, sizeof(double) * (size_t)(ks + 1) * npair * nb * nb));
-  double* part = reinterpret_cast<double*>(h->g.part);
-  const dim3 grid(ceil_div(nb, 16 * t.ni), ceil_div(nb, 16 * t.mi), (ks + 1) * npair);
+  return t;
+}
+static int gram_launch(Handle* h, const RGramArgs& a, RTile t, int nz, double* part) {
+  const dim3 grid(ceil_div(a.nb, 16 * t.ni), ceil_div(a.nb, 16 * t.mi), nz * a.npair);
 #define L(MI, NI) k_rgram<MI, NI><<<grid, RT, rsmem<MI, NI>(), h->stream>>>(a, part)
   RTILE_SWITCH_K(t, L);
 #undef L
   CUW_LAUNCH_CHECK("k_rgram");
+  return CUW_OK;
+}
+
+int fold_gram(Handle* h, const FoldPair* pairs, int npair, double* o0, double* o1, double* o2) {
+  RGramArgs a;
+  CUW_RET(gram_args(h, pairs, npair, &a));
+  const RTile t = gram_tile(h);
+  const int tiles = ceil_div(a.nb, 16 * t.ni) * ceil_div(a.nb, 16 * t.mi) * npair;
+  // the one-centre sums take splits of about the same length
+  const int ks0 = rsplit(h, tiles, a.nr, h->split_gram);
+  a.pchunk = std::max(RK, ceil_div(std::min(a.npro, ceil_div(a.nr, ks0)), RK) * RK);
+  const int kc = ceil_div(a.npro, a.pchunk), ks1 = std::max(1, ks0 - kc);
+  a.kchunk = ceil_div(ceil_div(a.nr, ks1), RK) * RK;
+  const int ks = a.ks = ceil_div(a.nr, a.kchunk), nb = a.nb;
+  CUW_RET(ensure_part(h, sizeof(double) * (size_t)(ks + kc) * npair * nb * nb));
+  CUW_RET(gram_launch(h, a, t, ks + kc, reinterpret_cast<double*>(h->g.part)));
   const size_t n = (size_t)nb * nb / 2 * npair;
-  k_rgram_sum<<<(unsigned)((n + 127) / 128), 128, 0, h->stream>>>(h->g.part, ks, nb, npair, 0.5 * h->gweight, o0, o1,
-                                                                  o2);
+  k_rgram_sum<<<(unsigned)((n + 127) / 128), 128, 0, h->stream>>>(h->g.part, ks, kc, nb, npair, 0.5 * h->gweight, o0,
+                                                                  o1, o2);
   CUW_LAUNCH_CHECK("k_rgram_sum");
   return CUW_OK;
+}
+
+// one wave of CTAs, at least 32 projectors each
+int fold_oc_splits(const Handle* h, int npair) {
+  const RTile t = gram_tile(h);
+  const int nb = h->d.nb, tiles = ceil_div(nb, 16 * t.ni) * ceil_div(nb, 16 * t.mi) * npair;
+  const int want = std::max(1, std::min(2 * h->nsm / std::max(1, tiles), ceil_div(h->npro, 32)));
+  return ceil_div(h->npro, std::max(RK, ceil_div(ceil_div(h->npro, want), RK) * RK));
+}
+int fold_oc(Handle* h, const FoldPair* pairs, int npair, int kc, double* oc) {
+  if (kc == 0) return CUW_OK;
+  RGramArgs a;
+  CUW_RET(gram_args(h, pairs, npair, &a));
+  a.pchunk = ceil_div(ceil_div(a.npro, kc), RK) * RK;
+  return gram_launch(h, a, gram_tile(h), kc, oc);
 }
 
 // opsi *= oscale / m_G (src/paw_waves2.f90:140-162)
@@ -895,8 +912,7 @@ int fold_addpro(Handle* h, int mode, const double2* hpc, const double2* opc, con
   const int nb = h->d.nb, npro = h->npro;
   const Op p{g.prox, h->ldu, 2 * h->nh};
   if (mode == ADDPRO_FUSED) {
-    CUW_RET(fold_room(h));
-    const RStepArgs a{g.hpsi, g.opsi, g.psim, g.psi0, g.rmpsi, g.half, slot_ptr(h, 0), slot_ptr(h, 1),
+      const RStepArgs a{g.hpsi, g.opsi, g.psim, g.psi0, g.rmpsi, g.half, slot_ptr(h, 0), slot_ptr(h, 1),
                       h->ldg, h->ldu, h->nh, h->d.nbh, sc};
     const Op c1{reinterpret_cast<const double*>(hpc), nb, nb}, c2{reinterpret_cast<const double*>(opc), nb, nb};
     const RTile t = pick_tile(h, 2 * h->nh, 2 * nb);

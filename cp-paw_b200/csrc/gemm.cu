@@ -737,26 +737,14 @@ static int choose_split(Handle* h, int tiles, int nk, int minchunk, double mul) 
   return std::min(want, maxs);
 }
 
-int eigr_room(Handle* h) {
-  if (h->g.eigr) return CUW_OK;
-  if (h->capturing) return h->fail(CUW_ERR_STATE, "structure factors allocated during graph capture");
-  h->touch();
-  if (cudaMalloc(&h->g.eigr, sizeof(double2) * (size_t)h->d.ngl * std::max(1, h->d.nat)) != cudaSuccess) {
-    cudaGetLastError();
-    h->g.eigr = nullptr;
-    return h->fail(CUW_ERR_NOMEM, "cudaMalloc of the structure factors failed");
-  }
-  return CUW_OK;
-}
-
 // Tables of the projectors at r_dev that the present path reads: the folded
-// FP64 table (FP64 products, symmetric G set), EIGR (FP64 products otherwise)
-// or EIGR and the fp32 table (tensor-core products of the mixed path).  Those
+// table in FP64 or, for the tensor-core products of the mixed path, in fp32, or
+// EIGR for a G set without parity.  Those
 // of a position buffer stay current until that buffer is written: R(+) of one
 // step is R(0) of the next.
 int eigr_compute(Handle* h, const double* r_dev) {
   const bool pos = r_dev == h->g.r0 || r_dev == h->g.rp || r_dev == h->g.rm;
-  const int need = h->tc_on() ? TAB_EIGR | TAB_F32 : (h->sym ? TAB_F64 : TAB_EIGR);
+  const int need = h->tc_on() ? TAB_F32 : (h->sym ? TAB_F64 : TAB_EIGR);
   const bool same = pos && r_dev == h->eigr_src;
   if (same && (h->tabs & need) == need) return CUW_OK;
   if (!same) h->tabs = 0;
@@ -764,12 +752,11 @@ int eigr_compute(Handle* h, const double* r_dev) {
   const int todo = need & ~h->tabs;
   if (todo & TAB_F64) CUW_RET(fold_table(h, r_dev));
   if (todo & TAB_EIGR) {
-    CUW_RET(eigr_room(h));
     dim3 grid(std::min(ceil_div(h->d.ngl, 256), 64), h->d.nat);
     k_eigr<<<grid, 256, 0, h->stream>>>(h->g.gx, h->g.gy, h->g.gz, r_dev, h->d.ngl, h->d.nat, h->g.eigr);
     CUW_LAUNCH_CHECK("k_eigr");
   }
-  if (todo & TAB_F32) CUW_RET(tc_pro_table(h));
+  if (todo & TAB_F32) CUW_RET(tc_pro_table(h, r_dev));
   h->tabs = pos ? (h->tabs | todo) : 0;
   if (pos) h->eigr_src = r_dev;
   return CUW_OK;
@@ -779,8 +766,12 @@ int eigr_compute(Handle* h, const double* r_dev) {
 // eigr_compute; `folded`: slots 0 and 1 of the folded arrays hold psiA and psiB
 int proj_compute(Handle* h, const double2* psiA, double2* projA, const double2* psiB, double2* projB, bool folded) {
   if (h->tc_on()) {
-    CUW_RET(tc_proj(h, psiA, projA));
-    return psiB ? tc_proj(h, psiB, projB) : CUW_OK;
+    if (!folded) {
+      CUW_RET(tc_fold(h, psiA, 0));
+      if (psiB) CUW_RET(tc_fold(h, psiB, 1));
+    }
+    CUW_RET(tc_split(h, psiB ? 2 : 1));
+    return tc_proj(h, projA, psiB ? projB : nullptr);
   }
   if (h->sym) {
     if (!folded) {
@@ -965,6 +956,7 @@ int force_gemm(Handle* h, const double2* ded, double* force_dev) {
   CUW_RET(ensure_part(h, sizeof(double) * 3 * (size_t)std::max(tm, 2 * h->nsm) * npro));
   double* fpart = reinterpret_cast<double*>(h->g.part);
   if (h->tc_on()) {
+    CUW_RET(tc_fold(h, h->g.psi0, 0));
     CUW_RET(tc_force(h, ded, fpart, &tm));
   } else if (h->sym) {
     CUW_RET(fold_psi(h, h->g.psi0, 0));

@@ -1,15 +1,11 @@
 // Orthonormality constraint of the CP step on the device (FP64 throughout).
 //
-//   k_unravel       WAVES_OVERLAP + WAVES_1COVERLAP unravelling of super wave
-//                   functions into real NB x NB matrices (src/paw_waves2.f90:797-848,
-//                   999-1020) and their sum (:262-289)
 //   k_lambda_init   symmetrisation and occupation scaling of RLAM0 (:295-303, 352-359)
 //   k_jacobi        eigenpairs of 0.5*(CHIPSI+CHIPSI^T) (LIB$DIAGR8 -> DSYEV,
 //                   src/paw_library.f90:572-631, 1555-1620) by parallel cyclic Jacobi
 //   k_ortho_x       the iteration of WAVES_ORTHO_X (src/paw_waves2.f90:1844-2022)
 //                   as one thread-block cluster; every wait is a hardware cluster
 //                   barrier and the loop is bounded by max_iter
-//   k_lambda12      LAMBDA1/LAMBDA2 of WAVES_ADDOPSI (:583-595)
 //   k_switch_lambda Lagrange extrapolation of WAVES$SWITCH (:2249-2296)
 //   k_ortho_y       WAVES_ORTHO_Y_C (:1025-1338) for WAVES_GRAMSCHMIDT (:2025-2177);
 //                   its matrices are real at the Gamma point, so it runs in real
@@ -42,33 +38,6 @@ constexpr int kStFallbacks = 9, kStRediag = 10;
 // replayed as a CUDA graph): a gated kernel does nothing unless the ORTHO_X
 // status it is given says that the fixed point failed.
 __device__ __forceinline__ bool gate_closed(const int* gate) { return gate && *gate != kFixedPointFailed; }
-
-// ---------------------------------------------------------------------------
-// T[pair][t] (NBH x NBH complex) -> real (NB x NB) matrices
-//   pw : plane-wave part, t=0 <X|Y>, t=1 sum X(G) Y(-G)     (both times Omega)
-//   oc : one-centre part, t=0 CMAT1, t=1 CMAT2
-// ---------------------------------------------------------------------------
-__global__ void k_unravel(const double2* __restrict__ pw, const double2* __restrict__ oc, int npair, int nbh,
-                          double* __restrict__ out0, double* __restrict__ out1, double* __restrict__ out2) {
-  const int nb = 2 * nbh;
-  const size_t mn = (size_t)nbh * nbh;
-  int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  int pair = blockIdx.y;
-  if (idx >= (int)mn || pair >= npair) return;
-  int i = idx % nbh, j = idx / nbh;
-  double* out = pair == 0 ? out0 : (pair == 1 ? out1 : out2);
-  double2 t1 = pw[(pair * 2 + 0) * mn + idx], t2 = pw[(pair * 2 + 1) * mn + idx];
-  double2 c1 = oc[(pair * 2 + 0) * mn + idx], c2 = oc[(pair * 2 + 1) * mn + idx];
-  // one-centre: cs1 = 0.5(C1+C2), cs2 = 0.5(C1-C2)
-  double cs1r = 0.5 * (c1.x + c2.x), cs1i = 0.5 * (c1.y + c2.y);
-  double cs2r = 0.5 * (c1.x - c2.x), cs2i = 0.5 * (c1.y - c2.y);
-  double re = 0.5 * t1.x, im = 0.5 * t1.y, re2 = 0.5 * t2.x, im2 = 0.5 * t2.y;
-  const int a = 2 * i, b = 2 * j;
-  out[a + (size_t)nb * b] = cs1r + (re + re2);
-  out[a + (size_t)nb * (b + 1)] = cs1i + (im + im2);
-  out[(a + 1) + (size_t)nb * b] = -cs2i + (-im + im2);
-  out[(a + 1) + (size_t)nb * (b + 1)] = cs2r + (re - re2);
-}
 
 // Lambda = sym(RLAM0) scaled by 0.5*f_i/(f_i+f_j); real part
 __global__ void k_lambda_init(const double2* __restrict__ rlam0, const double* __restrict__ occ, int nb,
@@ -1314,20 +1283,6 @@ __global__ void __launch_bounds__(256) k_small_gemm(const double* A, int tA, con
   gemm_tile<2, 2, 32>(A, tA != 0, B, tB != 0, n, i0, min(n, i0 + 32), j0, min(n, j0 + 32), C, smA, smB);
 }
 
-// LAMBDA1/LAMBDA2 (NBH x NBH complex) from real LAMBDA (NB x NB)
-__global__ void k_lambda12(const double* __restrict__ lam, int nb, int nbh, double2* __restrict__ l1,
-                           double2* __restrict__ l2) {
-  int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= nbh * nbh) return;
-  int ibh1 = idx % nbh, ibh2 = idx / nbh;
-  int a = 2 * ibh1, b = 2 * ibh1 + 1, c = 2 * ibh2, d = 2 * ibh2 + 1;
-  // CSVAR1 = L(a,c) + i L(a,d); CSVAR2 = i L(b,c) - L(b,d)
-  double2 s1 = make_double2(lam[a + (size_t)nb * c], lam[a + (size_t)nb * d]);
-  double2 s2 = make_double2(-lam[b + (size_t)nb * d], lam[b + (size_t)nb * c]);
-  l1[idx] = make_double2(0.5 * (s1.x - s2.x), 0.5 * (s1.y - s2.y));
-  l2[idx] = make_double2(0.5 * (s1.x + s2.x), 0.5 * (s1.y + s2.y));
-}
-
 // real LAMBDA -> RLAM0 (complex), and the extrapolation of WAVES$SWITCH
 __global__ void k_store_lambda(const double* __restrict__ lam, int n, double2* __restrict__ rlam0) {
   int idx = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1481,21 +1436,6 @@ __global__ void __launch_bounds__(1024) k_ortho_y(const double* __restrict__ s1,
 // ---------------------------------------------------------------------------
 // host orchestration
 // ---------------------------------------------------------------------------
-
-int unravel_run(Handle* h, const double2* pw, const double2* oc, int npair, double* o0, double* o1, double* o2) {
-  const int nbh = h->d.nbh;
-  dim3 grid(ceil_div(nbh * nbh, 256), npair);
-  k_unravel<<<grid, 256, 0, h->stream>>>(pw, oc, npair, nbh, o0, o1, o2);
-  CUW_LAUNCH_CHECK("k_unravel");
-  return CUW_OK;
-}
-
-int lambda12_run(Handle* h, const double* lam_real, double2* l1, double2* l2) {
-  const int nbh = h->d.nbh;
-  k_lambda12<<<ceil_div(nbh * nbh, 256), 256, 0, h->stream>>>(lam_real, h->d.nb, nbh, l1, l2);
-  CUW_LAUNCH_CHECK("k_lambda12");
-  return CUW_OK;
-}
 
 int jacobi_run(Handle* h, const double* s_dev, double* u, double* e, const int* gate) {
   const int n = h->d.nb;

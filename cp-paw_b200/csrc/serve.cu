@@ -114,7 +114,7 @@ size_t estimate_bytes(const cuw_dims& d, const int* isp) {
   b += nr * 8;                                         // V(r)
   b += std::min(nbh * nr * 16, ((size_t)48 << 20) + nr * 16);  // FFT work grid
   b += (size_t)20 << 20;                               // split-K partials and small tables
-  if (d.precision == CUW_PREC_MIXED) b += ldg * npro * 8 + ngl * (size_t)d.nat * 16;  // fp32 projector table, EIGR
+  if (d.precision == CUW_PREC_MIXED) b += ldg * npro * 8 + ngl * (size_t)d.nat * 16;  // projector tables (fp32, start-up fp64)
   else b += ldg * npro * 8 + 2 * ldg * nbh * 16;  // folded fp64 projector table and wave functions
   return b;
 }

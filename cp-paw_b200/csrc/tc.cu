@@ -23,51 +23,46 @@
 namespace cuw {
 namespace {
 
-// Real K values per chunk: 16 (two MMA steps of K = 8), i.e. eight complex K.
+// Real K values per chunk: 16 (two MMA steps of K = 8).
 // The accumulation run stays one MMA step: the tensor core's truncating fp32
 // accumulation was measured on B200 at a signed mean error of -3.7e-8 /
 // -8.7e-8 / -1.8e-7 of |C| for runs of 8 / 16 / 32 real K, and one step keeps
 // the energy bias below 1e-6 Ha/atom.
-constexpr int kCK = 8, kNSplit = 8;
+constexpr int kCK = 16, kNSplit = 8;
 
-// Raw slot layouts (bytes) of the A operands.  TMA boxes land row-major; boxes
-// whose rows are read down a column by the converters use the 64- or 128-byte
-// swizzle, so that eight consecutive rows hit distinct banks.  The B operands
-// arrive already split (k_bsplit) as one bulk copy per chunk.
-constexpr int kRawProj = 8192;    // Pf 128 p x 8 g (64-byte rows, 64B swizzle)
-constexpr int kRawAddpro = 8192;  // Pf 8 p x 128 g (1 KB rows)
-constexpr int kRawGram = 16384;   // X, X(-k): 64 rows of 8 k (128B swizzle), or X: 8 rows of 64 (1 KB)
-constexpr int kRawAddx = 32768;   // X, second-half X: 8 k x 128 m (2 KB rows) or 128 m x 8 k (128B swizzle)
-constexpr int kRawForce = 16384;  // psi0 8 b x 128 g (2 KB rows)
+// Every contraction is a real product over the folded half sphere (fold.cu):
+// A rows are projectors, bands or sphere rows r, and a raw A slot is one TMA box
+// of 16 K values of 128 rows in fp32: either K contiguous (64-byte rows, 64-byte
+// swizzle, so that eight consecutive rows read down a column hit distinct banks)
+// or row contiguous (16 rows of 512 bytes).  The B operands arrive already split
+// (k_bsplit) as one bulk copy per chunk.
+constexpr int kRawFold = 8192;
 constexpr int kRawGemm = 36864;   // A, B 128 rows x 16 doubles (144-byte rows, element copies)
 // Chunks travel in pairs through the copy and conversion hand-overs (the last
 // template argument): each hand-over costs several hundred cycles whatever it
 // carries, and pairs took 10-20 % off these kernels on B200 (Si64 and Si128
 // projections, back-projection, Gram; more raw slots than listed here gained
 // nothing).  Stage and slot counts below count pairs.
-using ProjPipe = tc::Pipe<4, 4, kRawProj, true, 2, 2, 2>;
-using AddproPipe = tc::Pipe<4, 4, kRawAddpro, true, 2, 2, 2>;
-using GramPipe = tc::Pipe<4, 2, kRawGram, true, 2, 2, 2>;
-using AddxPipe = tc::Pipe<3, 2, kRawAddx, true, 2, 2, 2>;
-using ForcePipe = tc::Pipe<4, 2, kRawForce, true, 2, 2, 2>;
+using ProjPipe = tc::Pipe<4, 4, kRawFold, true, 2, 2, 2>;
+using AddproPipe = tc::Pipe<4, 4, kRawFold, true, 2, 2, 2>;
+using GramPipe = tc::Pipe<4, 4, kRawFold, true, 2, 2, 2>;
+using AddxPipe = tc::Pipe<4, 4, kRawFold, true, 2, 2, 2>;
+using ForcePipe = tc::Pipe<4, 4, kRawFold, true, 2, 2, 2>;
 using GemmPipe = tc::Pipe<kNSplit, 2, kRawGemm, false>;
 constexpr int kThreads = ProjPipe::kThreads;
-constexpr int kNC = ProjPipe::kCols / 2;  // complex output columns per drain thread
 constexpr int kBTile = 4096;              // floats of one split B chunk (hi and lo tiles)
 static_assert(ProjPipe::kSmem <= 232448 && GramPipe::kSmem <= 232448 && AddxPipe::kSmem <= 232448 &&
                   GemmPipe::kSmem <= 232448 && ForcePipe::kSmem <= 232448 && AddproPipe::kSmem <= 232448,
               "shared memory");
-// k_tc_force reuses the stage and raw buffers for a 128 x 64 FP64 tile, rows
-// padded to an odd number of doubles so that the column stores of a warp (one
-// row per lane) spread over the banks
-constexpr int kSvLd = 65;
-static_assert(ForcePipe::kSplitBytes + ForcePipe::kNRaw * ForcePipe::kG * kRawForce >= sizeof(double) * (128 * kSvLd + 4 * 128 + 4 * 192),
+// rows of the force kernels' FP64 tiles are padded to an odd number of doubles
+// so that the column stores of a warp (one row per lane) spread over the banks
+constexpr int kSvLd = 65, kSvLd1 = 129;
+static_assert(ForcePipe::kSplitBytes + ForcePipe::kNRaw * ForcePipe::kG * kRawFold >=
+                  sizeof(double) * (128 * kSvLd1 + 4 * 128 + 4 * 384),
               "stage area too small");
 
-// offset of 16-byte chunk e of row r in a box with 128-byte (64-byte) rows
-// under the TMA 128-byte (64-byte) swizzle: chunk bits 4-6 (4-5) of the
-// address are XORed with bits 7-9 (7-8)
-__device__ __forceinline__ int sw128(int r, int e) { return r * 128 + ((e ^ (r & 7)) << 4); }
+// offset of 16-byte piece e of row r in a box with 64-byte rows under the TMA
+// 64-byte swizzle: address bits 4-5 are XORed with bits 7-8
 __device__ __forceinline__ int sw64(int r, int e) { return r * 64 + ((e ^ ((r >> 1) & 3)) << 4); }
 
 template <class T>
@@ -75,7 +70,6 @@ __device__ __forceinline__ T at(const unsigned char* raw, int byte) {
   return *reinterpret_cast<const T*>(raw + byte);
 }
 __device__ __forceinline__ double2 dz() { return make_double2(0.0, 0.0); }
-__device__ __forceinline__ double2 cj(double2 a) { return make_double2(a.x, -a.y); }
 
 // B functors of the pipelines that do not use them
 struct NoLoadB {
@@ -89,11 +83,17 @@ __device__ __forceinline__ void load_bsplit(tc::Copier& cp, int lane, const floa
   if (lane == 0) cp.bulk(0, bs + ((size_t)tile * nchk + chunk) * kBTile, 4 * kBTile);
 }
 
-// complex value i of an A row as real K values 2i, 2i+1 (conj: -Im)
-template <bool CONJ, class C2>
-__device__ __forceinline__ void a_put(float (&v)[8], int i, C2 a) {
-  v[2 * i] = (float)a.x;
-  v[2 * i + 1] = CONJ ? -(float)a.y : (float)a.y;
+// the eight K values 8 kh.. of A row r in a K-contiguous / row-contiguous box
+__device__ __forceinline__ void a_kfast(const unsigned char* raw, int r, int kh, float (&v)[8]) {
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const float4 x = at<float4>(raw, sw64(r, 2 * kh + i));
+    v[4 * i] = x.x, v[4 * i + 1] = x.y, v[4 * i + 2] = x.z, v[4 * i + 3] = x.w;
+  }
+}
+__device__ __forceinline__ void a_mfast(const unsigned char* raw, int r, int kh, float (&v)[8]) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = at<float>(raw, (8 * kh + i) * 512 + 4 * r);
 }
 
 // ---------------------------------------------------------------------------
@@ -146,415 +146,382 @@ __global__ void __launch_bounds__(kThreads, 1)
   tc::pipe_run<GemmPipe>((K + 15) / 16, load, no_b, a_row, convert_b, finish, err);
 }
 
-// out[i] = scale * sum_z part[z*n + i], summed in FP64 in a fixed order
-__global__ void k_tc_reduce(const float2* __restrict__ part, int nz, size_t n, double scale,
-                            double2* __restrict__ out) {
+// fp32 partial sums `stride` apart, summed in FP64 in split order, eight loads
+// in flight
+__device__ __forceinline__ double2 sum_parts(const float2* __restrict__ part, int nz, size_t stride) {
+  double2 s = dz();
+  int z = 0;
+  for (; z + 8 <= nz; z += 8) {
+    float2 v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = part[(size_t)(z + j) * stride];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      s.x += (double)v[j].x;
+      s.y += (double)v[j].y;
+    }
+  }
+  for (; z < nz; ++z) {
+    const float2 v = part[(size_t)z * stride];
+    s.x += (double)v.x;
+    s.y += (double)v.y;
+  }
+  return s;
+}
+
+// PROJ(b, p) of one or two arrays from part[z][p][set][b]
+__global__ void k_tc_proj_sum(const float2* __restrict__ part, int nz, int nbh, int nset, int npro, double scale,
+                              double2* __restrict__ out0, double2* __restrict__ out1) {
+  const int nw = nset * nbh;
+  const size_t n = (size_t)nw * npro;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    double sx = 0.0, sy = 0.0;
-    int z = 0;
-    for (; z + 8 <= nz; z += 8) {  // eight loads in flight, added in split order
-      float2 v[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) v[j] = part[(size_t)(z + j) * n + i];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        sx += (double)v[j].x;
-        sy += (double)v[j].y;
-      }
-    }
-    for (; z < nz; ++z) {
-      const float2 v = part[(size_t)z * n + i];
-      sx += (double)v.x;
-      sy += (double)v.y;
-    }
-    out[i] = make_double2(sx * scale, sy * scale);
+    const double2 s = sum_parts(part + i, nz, n);
+    const int b = (int)(i % nw);
+    const size_t p = i / nw;
+    (b < nbh ? out0 : out1)[(b < nbh ? b : b - nbh) + (size_t)nbh * p] = cscale(s, scale);
   }
 }
 
-// Projector table of the mixed path: pf[p*ldg + g] = fp32(PRO(g,p)) with
-// PRO(g,p) = Y_lm(g) P_ln(|g|) (-i)^l EIGR(g,a) (WAVES_EXPANDPRO,
-// src/paw_waves1.f90:6070-6109) evaluated in FP64, zero for g >= NGL.  The
-// single rounding to fp32 is the one the split into tf32 pairs starts from.
-__global__ void k_pro_f32(int ngl, int ldg, const int* __restrict__ ipro0, const int* __restrict__ nlmn,
+// out_pair(i + NB j) = scale * sum_z part[z][pair][i][j] + one-centre sum
+// oc[z][pair][i][j] (FP64, kc splits)
+__global__ void k_tc_gram_sum(const float2* __restrict__ part, int nz, const double2* __restrict__ oc, int kc, int nb,
+                              int npair, double scale, double* __restrict__ o0, double* __restrict__ o1,
+                              double* __restrict__ o2) {
+  const size_t per = (size_t)nb * nb / 2, n = per * npair;
+  const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  if (t >= n) return;
+  const double2 s = sum_parts(part + t, nz, n);
+  double2 c = dz();
+  for (int z = 0; z < kc; ++z) c = cadd(c, oc[(size_t)z * n + t]);
+  const int pair = (int)(t / per);
+  const size_t e = 2 * (t % per);
+  const int i = (int)(e / nb), j = (int)(e % nb);
+  double* o = pair == 0 ? o0 : (pair == 1 ? o1 : o2);
+  o[i + (size_t)nb * j] = s.x * scale + c.x;
+  o[i + (size_t)nb * (j + 1)] = s.y * scale + c.y;
+}
+
+// Folded projector table of the mixed path: P(r, p) in fp32 (k_pro_fold of
+// fold.cu evaluates the same in FP64).  The single rounding to fp32 is the one
+// the split into tf32 pairs starts from.
+__global__ void k_pro_f32(int nh, int ngl, int ldu, const int2* __restrict__ half, const double* __restrict__ gx,
+                          const double* __restrict__ gy, const double* __restrict__ gz, const double* __restrict__ r,
+                          const int* __restrict__ ipro0, const int* __restrict__ nlmn,
                           const ProDesc* __restrict__ pdesc, const double* __restrict__ ylm,
-                          const double* __restrict__ pro, const double2* __restrict__ eigr, float2* __restrict__ pf) {
-  // one thread per (g, atom): EIGR(g, a) read once for all projectors of the atom
-  const int a = blockIdx.y, p0 = ipro0[a], np = nlmn[a];
-  for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < ldg; g += gridDim.x * blockDim.x) {
-    if (g >= ngl) {
-      for (int k = 0; k < np; ++k) pf[(size_t)(p0 + k) * ldg + g] = make_float2(0.f, 0.f);
-      continue;
-    }
-    const double2 e = eigr[(size_t)g + (size_t)ngl * a];
-    for (int k = 0; k < np; ++k) {
-      const ProDesc d = pdesc[p0 + k];
-      const double s = ylm[(size_t)g + (size_t)ngl * d.lm] * pro[(size_t)g + (size_t)ngl * d.ibare];
-      const double2 em = cmul(mipow(d.l), e);
-      pf[(size_t)(p0 + k) * ldg + g] = make_float2((float)(s * em.x), (float)(s * em.y));
-    }
+                          const double* __restrict__ pro, float* __restrict__ pf) {
+  const int a = blockIdx.y, h = blockIdx.x * blockDim.x + threadIdx.x;
+  if (h >= nh) return;
+  const int g = half[h].x, p0 = ipro0[a], np = nlmn[a];
+  double sn, cs;
+  sincos(gx[g] * r[3 * a] + gy[g] * r[3 * a + 1] + gz[g] * r[3 * a + 2], &sn, &cs);
+  const double2 ei = make_double2(cs, -sn);
+  for (int k = 0; k < np; ++k) {
+    const ProDesc d = pdesc[p0 + k];
+    const double sv = ylm[(size_t)g + (size_t)ngl * d.lm] * pro[(size_t)g + (size_t)ngl * d.ibare];
+    const double2 e = cmul(mipow(d.l), ei);
+    *reinterpret_cast<float2*>(pf + (size_t)ldu * (p0 + k) + 2 * h) = make_float2((float)(sv * e.x), (float)(sv * e.y));
   }
 }
 
+// U(r, n) of a wave-function array in fp32 (k_fold of fold.cu; the sums and
+// differences are formed in FP64)
+__global__ void k_fold_f32(const double2* __restrict__ psi, const int2* __restrict__ half, int nh, int ldg, int ldu,
+                           float* __restrict__ u) {
+  const int h = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y;
+  if (h >= nh) return;
+  const int2 g = half[h];
+  const double2* p = psi + (size_t)ldg * b;
+  const double2 x = p[g.x], y = p[g.y];
+  const bool self = g.x == g.y;
+  float* o = u + (size_t)ldu * (2 * b) + 2 * h;
+  *reinterpret_cast<float2*>(o) = make_float2((float)(self ? x.x : x.x + y.x), (float)(self ? x.x : x.y - y.y));
+  *reinterpret_cast<float2*>(o + ldu) = make_float2((float)(self ? x.y : x.y + y.y), (float)(self ? x.y : y.x - x.x));
+}
+
 // ---------------------------------------------------------------------------
-// <p|psi> partial sums (WAVES_PROJECTIONS, src/paw_waves1.f90:5746-5905):
-// part[z][p][b] = sum_{g in split z} conj(PRO(g,p)) psi(g,b)   (float2)
-// M = 128 projectors (blockIdx.x), N = 64 bands (blockIdx.y), K = g (blockIdx.z)
+// Products with K along the half sphere: part[z][i][n] = sum_{r in split z}
+// A(r,i) B(r,n), fp32.
+//   projections (WAVES_PROJECTIONS, src/paw_waves1.f90:5746-5905): A = P, B = U
+//     of one or two arrays (column tiles of the second follow the first's)
+//   overlaps (PLANEWAVE$SCALARPRODUCT, src/paw_fft.f90:2344-2422): A = U of x,
+//     B = U of y for up to three pairs (blockIdx.z = split*npair + pair)
+// Rows tile blockIdx.x, column tile blockIdx.y.
 // ---------------------------------------------------------------------------
+struct TcTnArgs {
+  int npair, nk, kchunk, nchk;
+  int nrow, ncol;       // rows of A, columns of one array
+  int tps, ldp;         // column tiles of one array, row length of part
+  const float* bs[3];   // split B of each pair
+};
+struct TcTnMaps {
+  CUtensorMap a[3];
+};
+template <class P>
 __global__ void __launch_bounds__(kThreads, 1)
-    k_tc_proj(const __grid_constant__ CUtensorMap tm_pf, const float* __restrict__ bpsi, int nchk, int ngl, int nbh,
-              int npro, int kchunk, float2* __restrict__ part, int* __restrict__ err) {
-  const int m0 = blockIdx.x * 128, b0 = blockIdx.y * 64;
-  const int gbeg = blockIdx.z * kchunk, gend = min(ngl, gbeg + kchunk);
-  // raw slot: Pf box 128 p x 8 g (64-byte rows, 64B swizzle); zeros past NGL
-  // and NPRO.  Chunks never straddle a split boundary (kchunk is a multiple of 8).
+    k_tc_tn(TcTnArgs a, const __grid_constant__ TcTnMaps tm, float* __restrict__ part, int* __restrict__ err) {
+  const int pair = blockIdx.z % a.npair, split = blockIdx.z / a.npair;
+  const int m0 = blockIdx.x * 128;
+  const int kbeg = split * a.kchunk, kend = min(a.nk, kbeg + a.kchunk);
+  const float* bs = a.bs[pair];
+  // zeros past NK and the rows; chunks never straddle a split boundary (kchunk
+  // is a multiple of 16)
   auto load = [&](int c, int lane, tc::Copier& cp) {
-    if (lane == 0) cp.tensor(0, &tm_pf, 2 * (gbeg + c * kCK), m0, 8192);
+    if (lane == 0) cp.tensor(0, &tm.a[pair], kbeg + c * kCK, m0, kRawFold);
   };
-  auto load_b = [&](int c, int lane, tc::Copier& cp) { load_bsplit(cp, lane, bpsi, nchk, blockIdx.y, gbeg / kCK + c); };
-  auto a_row = [&](int c, const unsigned char* raw, int r, int kh, float (&v)[8]) {  // conj(Pf) row p
+  auto load_b = [&](int c, int lane, tc::Copier& cp) { load_bsplit(cp, lane, bs, a.nchk, blockIdx.y, kbeg / kCK + c); };
+  auto a_row = [&](int c, const unsigned char* raw, int r, int kh, float (&v)[8]) { a_kfast(raw, r, kh, v); };
+  auto finish = [&](const float (&acc)[P::kCols], int row, int col0) {
+    const int i = m0 + row;
+    if (i >= a.nrow) return;
+    const int set = blockIdx.y / a.tps, n0 = 128 * (blockIdx.y - set * a.tps) + col0;
+    float* out = part + ((size_t)blockIdx.z * a.nrow + i) * a.ldp + (size_t)set * a.ncol + n0;
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const float4 x = at<float4>(raw, sw64(r, 2 * kh + i));
-      v[4 * i] = x.x, v[4 * i + 1] = -x.y, v[4 * i + 2] = x.z, v[4 * i + 3] = -x.w;
-    }
-  };
-  auto finish = [&](const float (&acc)[ProjPipe::kCols], int row, int col0) {
-    const int p = m0 + row;
-    if (p >= npro) return;
-    float2* out = part + ((size_t)blockIdx.z * npro + p) * nbh;
-    const int bb = b0 + col0 / 2;
-#pragma unroll
-    for (int j = 0; j < kNC; ++j)
-      if (bb + j < nbh) out[bb + j] = make_float2(acc[2 * j], acc[2 * j + 1]);
+    for (int j = 0; j < P::kCols; j += 2)
+      if (n0 + j < a.ncol) *reinterpret_cast<float2*>(out + j) = make_float2(acc[j], acc[j + 1]);
   };
   NoConvertB no_cb;
-  const int nchunk = gend > gbeg ? (gend - gbeg + kCK - 1) / kCK : 0;
-  tc::pipe_run<ProjPipe>(nchunk, load, load_b, a_row, no_cb, finish, err);
+  const int nchunk = kend > kbeg ? (kend - kbeg + kCK - 1) / kCK : 0;
+  tc::pipe_run<P>(nchunk, load, load_b, a_row, no_cb, finish, err);
+}
+
+// the value at this lane's G from the row values of a pair (adjacent lanes):
+// even rows hold s and take G (s + i t), odd rows hold t and take -G (s - i t)
+__device__ __forceinline__ double2 unfold(double2 v, bool odd) {
+  double2 o;
+  o.x = __shfl_xor_sync(0xffffffffu, v.x, 1);
+  o.y = __shfl_xor_sync(0xffffffffu, v.y, 1);
+  return odd ? make_double2(o.x + v.y, o.y - v.x) : make_double2(v.x - o.y, v.y + o.x);
+}
+// the row value of U (u of even rows, w of odd rows) from this lane's psi
+__device__ __forceinline__ double2 refold(double2 v, bool odd, bool self) {
+  double2 o;
+  o.x = __shfl_xor_sync(0xffffffffu, v.x, 1);
+  o.y = __shfl_xor_sync(0xffffffffu, v.y, 1);
+  if (self) return odd ? o : v;
+  return odd ? make_double2(o.y - v.y, v.x - o.x) : make_double2(v.x + o.x, v.y + o.y);
 }
 
 // ---------------------------------------------------------------------------
 // ADDPRO with the step epilogues (WAVES_ADDPRO, src/paw_waves1.f90:5908-6067,
-// and the epilogues of the FP64 k_addpro): 128 g x 32 bands per CTA (band
-// tile blockIdx.x, G tile blockIdx.y), the tile columns hold C1 (hproj)
-// products for the bands, then C2 (oproj) products.
+// and the epilogues of the FP64 form): 128 sphere rows (64 pairs) x 32 super
+// wave functions per CTA (column tile blockIdx.x, row tile blockIdx.y), the tile
+// columns hold C1 (hproj) products, then C2 (oproj) products.  FUSED leaves the
+// folded psim and opsi in um and uo.
 // ---------------------------------------------------------------------------
+struct TcAddproArgs {
+  double2 *hpsi, *opsi, *psim;
+  const double2* psi0;
+  const double* rmpsi;
+  const int2* half;
+  float *um, *uo;
+  int ldg, ldu, nh, nbh, npro, nchk;
+  const float* bc;
+  StepCoef sc;
+};
 template <int MODE>
 __global__ void __launch_bounds__(kThreads, 1)
-    k_tc_addpro(double2* __restrict__ hpsi, double2* __restrict__ opsi, const double2* __restrict__ psi0,
-                double2* __restrict__ psim, const double* __restrict__ mpsi, int ldg, int ngl, int nbh, int npro,
-                const __grid_constant__ CUtensorMap tm_pf, const float* __restrict__ bc, int nchk, StepCoef sc,
-                int* __restrict__ err) {
+    k_tc_addpro(TcAddproArgs a, const __grid_constant__ CUtensorMap tm_pf, int* __restrict__ err) {
   constexpr bool USE_H = (MODE != ADDPRO_OPSI);
   constexpr bool USE_O = (MODE != ADDPRO_HPSI);
-  // the band tiles of one G tile are consecutive blocks (blockIdx.x), so the
-  // second read of the G tile's projector rows comes from L2
-  const int g0 = blockIdx.y * 128, b0 = blockIdx.x * 32;
-  // raw slot: Pf box 8 p x 128 g (1 KB rows); zeros past NGL and NPRO.  B:
-  // [C1 | C2] of bands b0..b0+31, split (k_bsplit, zero where unused)
+  // the column tiles of one row tile are consecutive blocks (blockIdx.x), so the
+  // second read of the row tile's projectors comes from L2
+  const int m0 = blockIdx.y * 128, b0 = blockIdx.x * 32;
   auto load = [&](int c, int lane, tc::Copier& cp) {
-    if (lane == 0) cp.tensor(0, &tm_pf, 2 * g0, c * kCK, 8192);
+    if (lane == 0) cp.tensor(0, &tm_pf, m0, c * kCK, kRawFold);
   };
-  auto load_b = [&](int c, int lane, tc::Copier& cp) { load_bsplit(cp, lane, bc, nchk, blockIdx.x, c); };
-  auto a_row = [&](int c, const unsigned char* raw, int r, int kh, float (&v)[8]) {  // Pf(g, p), K = p
-#pragma unroll
-    for (int i = 0; i < 4; ++i) a_put<false>(v, i, at<float2>(raw, (4 * kh + i) * 1024 + r * 8));
-  };
+  auto load_b = [&](int c, int lane, tc::Copier& cp) { load_bsplit(cp, lane, a.bc, a.nchk, blockIdx.x, c); };
+  auto a_row = [&](int c, const unsigned char* raw, int r, int kh, float (&v)[8]) { a_mfast(raw, r, kh, v); };
   auto finish = [&](const float (&acc)[AddproPipe::kCols], int row, int col0) {
-    const int g = g0 + row;
-    if (g >= ngl) return;
-    const double rm = 1.0 / mpsi[g];
-    const bool hcol = col0 < 64;  // columns 0..63: C1 (H) products, 64..127: C2 (O)
-    const int bl0 = (col0 & 63) / 2;
+    const int r = m0 + row;
+    const bool rok = r < 2 * a.nh, odd = row & 1;
+    const int2 gp = rok ? a.half[r >> 1] : make_int2(0, 0);
+    const bool self = gp.x == gp.y, mine = rok && !(odd && self);
+    const int g = odd ? gp.y : gp.x;
+    const double rm = a.rmpsi[g];
+    const bool hcol = col0 < 64;  // columns 0..63: C1 (H) products, 64..127: C2 (O); uniform in a warp
+    const int bl0 = b0 + (col0 & 63) / 2;
+    if (hcol ? !USE_H : !USE_O) return;
+    double a1 = a.sc.a1, a2 = a.sc.a2, a3 = a.sc.a3 * rm;
+    if (MODE == ADDPRO_FUSED && a.sc.fr) {  // cell friction ANNEEVEC(G) (src/paw_waves1.f90:6536-6540)
+      const double ai = a.sc.fr[g];
+      a1 = 2.0 * ai;
+      a2 = 1.0 - a1;
+      a3 = -a.sc.dt2 * ai * rm;
+    }
     // columns in groups of kB whose loads are all issued before any store of
     // the group (the arrays may alias as far as the compiler knows, so a load
     // after a store would wait for it: one memory round trip per group, not
     // two per column)
     constexpr int kB = 2;
 #pragma unroll
-    for (int j0 = 0; j0 < kNC; j0 += kB) {
+    for (int j0 = 0; j0 < AddproPipe::kCols / 2; j0 += kB) {
       double2 hv[kB], p0v[kB], pm[kB];
-      size_t k[kB];
-      bool ok[kB];
 #pragma unroll
       for (int q = 0; q < kB; ++q) {
-        const int b = b0 + bl0 + j0 + q;
-        ok[q] = b < nbh;
-        k[q] = (size_t)g + (size_t)ldg * (ok[q] ? b : 0);
-        if (hcol && USE_H) {
-          hv[q] = ok[q] ? hpsi[k[q]] : dz();
+        const int b = bl0 + j0 + q;
+        const size_t k = mine && b < a.nbh ? (size_t)g + (size_t)a.ldg * b : 0;
+        if (hcol) {
+          hv[q] = a.hpsi[k];
           if (MODE == ADDPRO_FUSED) {
-            p0v[q] = ok[q] ? psi0[k[q]] : dz();
-            pm[q] = ok[q] ? psim[k[q]] : dz();
+            p0v[q] = a.psi0[k];
+            pm[q] = a.psim[k];
           }
-        } else if (!hcol && USE_O) {
-          p0v[q] = ok[q] ? psi0[k[q]] : dz();
+        } else {
+          p0v[q] = a.psi0[k];
         }
       }
 #pragma unroll
       for (int q = 0; q < kB; ++q) {
-        if (!ok[q]) continue;
-        const int j = j0 + q;
-        const double2 v = make_double2((double)acc[2 * j], (double)acc[2 * j + 1]);
-        if (hcol && USE_H) {
+        const int b = bl0 + j0 + q, j = j0 + q;
+        const bool bok = b < a.nbh, ok = mine && bok;
+        const size_t k = (size_t)g + (size_t)a.ldg * b;
+        const double2 v = unfold(make_double2((double)acc[2 * j], (double)acc[2 * j + 1]), odd);
+        double2 res = dz();  // psi(+) or O psi at this lane's G
+        if (hcol) {
           const double2 h2 = cadd(hv[q], v);
-          hpsi[k[q]] = h2;
+          if (ok) a.hpsi[k] = h2;
           if (MODE == ADDPRO_FUSED) {
-            double a1 = sc.a1, a2 = sc.a2, a3 = sc.a3 * rm;
-            if (sc.fr) {  // cell friction ANNEEVEC(G) (src/paw_waves1.f90:6536-6540)
-              a1 = 2.0 * sc.fr[g];
-              a2 = 1.0 - a1;
-              a3 = -sc.dt2 * sc.fr[g] * rm;
-            }
-            psim[k[q]] = make_double2(a1 * p0v[q].x + a2 * pm[q].x + a3 * h2.x, a1 * p0v[q].y + a2 * pm[q].y + a3 * h2.y);
+            res = make_double2(a1 * p0v[q].x + a2 * pm[q].x + a3 * h2.x, a1 * p0v[q].y + a2 * pm[q].y + a3 * h2.y);
+            if (ok) a.psim[k] = res;
           }
-        } else if (!hcol && USE_O) {
-          const double s = sc.oscale * rm;
-          opsi[k[q]] = make_double2((p0v[q].x + v.x) * s, (p0v[q].y + v.y) * s);
+        } else {
+          const double s = a.sc.oscale * rm;
+          res = make_double2((p0v[q].x + v.x) * s, (p0v[q].y + v.y) * s);
+          if (ok) a.opsi[k] = res;
+        }
+        if (MODE == ADDPRO_FUSED) {
+          const double2 f = refold(res, odd, self);
+          if (rok && bok) {
+            float* u = (hcol ? a.um : a.uo) + (size_t)a.ldu * (2 * b) + r;
+            u[0] = (float)f.x;
+            u[a.ldu] = (float)f.y;
+          }
         }
       }
     }
   };
   NoConvertB no_cb;
-  tc::pipe_run<AddproPipe>((npro + kCK - 1) / kCK, load, load_b, a_row, no_cb, finish, err);
+  tc::pipe_run<AddproPipe>(a.nchk, load, load_b, a_row, no_cb, finish, err);
 }
 
 // ---------------------------------------------------------------------------
-// Gram products (PLANEWAVE$SCALARPRODUCT, src/paw_fft.f90:2344-2422, for
-// WAVES_OVERLAP and WAVES_1COVERLAP): for pair (X, Y)
-//   T1(m,n) = sum_k conj(X(k,m)) Y(k,n)
-//   T2(m,n) = sum_k X(k,m) Y(-k,n) = sum_k X(-k,m) Y(k,n)   (MINUS; the sphere
-//             is closed under k -> -k), else sum_k X(k,m) Y(k,n)
-// Tile rows 0..63: conj(X) for T1, rows 64..127: X(-k) for T2, sharing the
-// Y columns.  Partials part[z][t][m + nm n] (float2), z = split*npair + pair.
+// psi(+) += O|psi0> Lambda (WAVES_ADDOPSI, src/paw_waves2.f90:547-615): U of the
+// operand times the real Lambda, unfolded into out
 // ---------------------------------------------------------------------------
-struct TcGramArgs {
-  int npair, nk, nm, kchunk, nchk;
-  bool kfast;            // X(k, m) contiguous in k (plane waves); else in m (projections)
-  const float* ybs[3];   // Y of each pair, split (k_bsplit)
-};
-// TMA maps of the pairs: X and X(-k) (plane waves with MINUS)
-struct TcGramMaps {
-  CUtensorMap x[3], xm[3];
-};
-
-template <bool MINUS>
 __global__ void __launch_bounds__(kThreads, 1)
-    k_tc_gram(TcGramArgs a, const __grid_constant__ TcGramMaps tm, float2* __restrict__ part, int* __restrict__ err) {
-  const int pair = blockIdx.z % a.npair, split = blockIdx.z / a.npair;
-  const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
-  const int kbeg = split * a.kchunk, kend = min(a.nk, kbeg + a.kchunk);
-  const bool kfast = a.kfast;
-  // raw slot: X at 0, X(-k) at 8K (MINUS).  kfast: boxes of 64 rows (m) of
-  // eight k (128-byte rows, 128B swizzle); otherwise 8 rows (k) of 64 m (1 KB
-  // rows).  Zeros past NK and NM.
-  constexpr int XM = 8192;
-  const float* ybs = a.ybs[pair];
+    k_tc_addx(double2* __restrict__ out, const int2* __restrict__ half, int nh, int ldg, int nbh, int nchk,
+              const float* __restrict__ ls, const __grid_constant__ CUtensorMap tm_u, int* __restrict__ err) {
+  const int m0 = blockIdx.x * 128;
   auto load = [&](int c, int lane, tc::Copier& cp) {
-    if (lane == 0) {
-      const int k0 = kbeg + c * kCK;
-      if (kfast) {
-        cp.tensor(0, &tm.x[pair], 2 * k0, m0, 8192);
-        if (MINUS) cp.tensor(XM, &tm.xm[pair], 2 * k0, m0, 8192);
-      } else {
-        cp.tensor(0, &tm.x[pair], 2 * m0, k0, 8192);
-      }
-    }
+    if (lane == 0) cp.tensor(0, &tm_u, m0, c * kCK, kRawFold);
   };
-  auto load_b = [&](int c, int lane, tc::Copier& cp) { load_bsplit(cp, lane, ybs, a.nchk, blockIdx.x, kbeg / kCK + c); };
-  auto xoff = [&](int r, int e) { return kfast ? sw128(r, e) : e * 1024 + r * 16; };
-  auto a_row = [&](int c, const unsigned char* raw, int r, int kh, float (&v)[8]) {
-    // rows 0..63 conj X(k), rows 64..127 X(-k) (MINUS) or X(k)
-    const int ml = r & 63;
-    const int base = (MINUS && r >= 64) ? XM : 0;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const double2 x = at<double2>(raw, base + xoff(ml, 4 * kh + i));
-      if (r < 64) a_put<true>(v, i, x);
-      else a_put<false>(v, i, x);
-    }
-  };
-  auto finish = [&](const float (&acc)[GramPipe::kCols], int row, int col0) {
-    const int t = row >> 6, m = m0 + (row & 63);
-    if (m >= a.nm) return;
-    const size_t mn = (size_t)a.nm * a.nm;
-    float2* out = part + ((size_t)blockIdx.z * 2 + t) * mn;
-    const int nb = n0 + col0 / 2;
-#pragma unroll
-    for (int j = 0; j < kNC; ++j)
-      if (nb + j < a.nm) out[(size_t)m + (size_t)a.nm * (nb + j)] = make_float2(acc[2 * j], acc[2 * j + 1]);
-  };
-  NoConvertB no_cb;
-  const int nchunk = kend > kbeg ? (kend - kbeg + kCK - 1) / kCK : 0;
-  tc::pipe_run<GramPipe>(nchunk, load, load_b, a_row, no_cb, finish, err);
-}
-
-// ---------------------------------------------------------------------------
-// ADDOPSI / ADDOPROJ (src/paw_waves2.f90:547-615, 687-758):
-//   out(m,n) += sum_k X(m,k) L1(k,n) + conj(X(m',k)) L2(k,n),
-//   m' = minusg[m] (XMINUS) or m.  K runs over both halves (2 nk).
-// ---------------------------------------------------------------------------
-struct TcAddXArgs {
-  double2* out;
-  int nm, nn, nk, nchk;
-  size_t som, son;
-  bool mfast;       // X(m, k) contiguous in m (plane waves); else in k (projections)
-  const float* lbs; // [L1; L2], split (k_bsplit)
-};
-// TMA maps: X for K < NK, the second-half X (conj X(m') for K >= NK)
-struct TcAddXMaps {
-  CUtensorMap x, x2;
-};
-
-__global__ void __launch_bounds__(kThreads, 1)
-    k_tc_addx(TcAddXArgs a, const __grid_constant__ TcAddXMaps tm, int* __restrict__ err) {
-  const int m0 = blockIdx.x * 128, n0 = blockIdx.y * 64;
-  const int ktot = 2 * a.nk;
-  const bool mfast = a.mfast;
-  (void)n0;
-  // raw slot: X at 0 and the second-half X at 16K: mfast boxes of 8 rows (k)
-  // of 128 m (2 KB rows), else 128 rows (m) of eight k (128B swizzle).
-  // Second-half boxes start at k = kg0 - NK, negative for a chunk that
-  // straddles NK: rows or columns outside the arrays read as zero.
-  constexpr int X2 = 16384;
-  auto load = [&](int c, int lane, tc::Copier& cp) {
-    if (lane == 0) {
-      const int kg0 = c * kCK, k2 = kg0 - a.nk;
-      if (kg0 < a.nk) {
-        if (mfast) cp.tensor(0, &tm.x, 2 * m0, kg0, 16384);
-        else cp.tensor(0, &tm.x, 2 * kg0, m0, 16384);
-      }
-      if (kg0 + kCK > a.nk) {
-        if (mfast) cp.tensor(X2, &tm.x2, 2 * m0, k2, 16384);
-        else cp.tensor(X2, &tm.x2, 2 * k2, m0, 16384);
-      }
-    }
-  };
-  auto load_b = [&](int c, int lane, tc::Copier& cp) { load_bsplit(cp, lane, a.lbs, a.nchk, blockIdx.y, c); };
-  auto a_row = [&](int c, const unsigned char* raw, int r, int kh, float (&v)[8]) {  // X(m,k) | conj X(m',k)
-    const int kg0 = c * kCK + 4 * kh;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int e = 4 * kh + i;
-      const bool first = kg0 + i < a.nk;
-      const double2 x = (kg0 + i < ktot) ? at<double2>(raw, (first ? 0 : X2) + (mfast ? e * 2048 + r * 16 : sw128(r, e))) : dz();
-      if (first) a_put<false>(v, i, x);
-      else a_put<true>(v, i, x);
-    }
-  };
+  auto load_b = [&](int c, int lane, tc::Copier& cp) { load_bsplit(cp, lane, ls, nchk, blockIdx.y, c); };
+  auto a_row = [&](int c, const unsigned char* raw, int r, int kh, float (&v)[8]) { a_mfast(raw, r, kh, v); };
   auto finish = [&](const float (&acc)[AddxPipe::kCols], int row, int col0) {
-    const int m = m0 + row;
-    if (m >= a.nm) return;
-    const int nb = blockIdx.y * 64 + col0 / 2;
+    const int r = m0 + row;
+    const bool rok = r < 2 * nh, odd = row & 1;
+    const int2 gp = rok ? half[r >> 1] : make_int2(0, 0);
+    const bool self = gp.x == gp.y, mine = rok && !(odd && self);
+    const int g = odd ? gp.y : gp.x, b0 = (blockIdx.y * 128 + col0) / 2;
     // four columns' loads before their stores (one memory round trip per group)
 #pragma unroll
-    for (int j0 = 0; j0 < kNC; j0 += 4) {
+    for (int j0 = 0; j0 < AddxPipe::kCols / 2; j0 += 4) {
       double2 o[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        const int j = j0 + q;
-        o[q] = nb + j < a.nn ? a.out[(size_t)m * a.som + (size_t)(nb + j) * a.son] : dz();
+        const int b = b0 + j0 + q;
+        o[q] = out[mine && b < nbh ? (size_t)g + (size_t)ldg * b : 0];
       }
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        const int j = j0 + q;
-        if (nb + j < a.nn)
-          a.out[(size_t)m * a.som + (size_t)(nb + j) * a.son] =
-              make_double2(o[q].x + (double)acc[2 * j], o[q].y + (double)acc[2 * j + 1]);
+        const int b = b0 + j0 + q, j = j0 + q;
+        const double2 w = make_double2((double)acc[2 * j], (double)acc[2 * j + 1]), v = unfold(w, odd);
+        if (mine && b < nbh)
+          out[(size_t)g + (size_t)ldg * b] =
+              self ? cadd(o[q], w) : make_double2(o[q].x + 0.5 * v.x, o[q].y + 0.5 * v.y);
       }
     }
   };
   NoConvertB no_cb;
-  tc::pipe_run<AddxPipe>((ktot + kCK - 1) / kCK, load, load_b, a_row, no_cb, finish, err);
+  tc::pipe_run<AddxPipe>(nchk, load, load_b, a_row, no_cb, finish, err);
 }
 
 // ---------------------------------------------------------------------------
 // Forces (WAVES_DEDPRO + WAVES_PROFORCE, src/paw_waves1.f90:5694-5743,
-// 6112-6234): D(g,p) = sum_b psi0(g,b) conj(E(b,p)) on the tensor cores for
-// 128 g x 64 projectors, then sv(g,p) = Re[i P (-i)^l EIGR conj(D)] Y_lm in the
-// drain warps (into the freed stage buffers) and fpart[tile][p][c] =
-// sum_g sv(g,p) G_c(g) by the whole CTA.
+// 6112-6234): D(r,p) = sum_n U(r,n) E(n,p) on the tensor cores for 128 sphere
+// rows x 128 projectors, then sv(r,p) = +-P(r^1,p) D(r,p) in the drain warps
+// (into the freed stage buffers) and fpart[tile][p][c] = sum_r sv(r,p) G_c by
+// the whole CTA.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(kThreads, 1)
-    k_tc_force(const __grid_constant__ CUtensorMap tm_psi, const float* __restrict__ be, int nchk, int ngl, int nbh,
-               int npro, const ProDesc* __restrict__ pdesc, const double* __restrict__ ylm,
-               const double* __restrict__ pro, const double2* __restrict__ eigr, const double* __restrict__ gx,
+    k_tc_force(const __grid_constant__ CUtensorMap tm_u, const float* __restrict__ be, int nchk, int nh, int npro,
+               int ldu, const float* __restrict__ pf, const int2* __restrict__ half, const double* __restrict__ gx,
                const double* __restrict__ gy, const double* __restrict__ gz, double* __restrict__ fpart,
                int* __restrict__ err) {
-  const int g0 = blockIdx.x * 128, p0 = blockIdx.y * 64;
-  // raw slot: psi0 box 8 b x 128 g (2 KB rows); zeros past NGL and NBH.  B:
-  // conj(E) of projectors p0..p0+63, split (k_bsplit)
+  const int m0 = blockIdx.x * 128, p0 = blockIdx.y * 128;
   auto load = [&](int c, int lane, tc::Copier& cp) {
-    if (lane == 0) cp.tensor(0, &tm_psi, 2 * g0, c * kCK, 16384);
+    if (lane == 0) cp.tensor(0, &tm_u, m0, c * kCK, kRawFold);
   };
   auto load_b = [&](int c, int lane, tc::Copier& cp) { load_bsplit(cp, lane, be, nchk, blockIdx.y, c); };
-  auto a_row = [&](int c, const unsigned char* raw, int r, int kh, float (&v)[8]) {  // psi0(g, b), K = b
-#pragma unroll
-    for (int i = 0; i < 4; ++i) a_put<false>(v, i, at<double2>(raw, (4 * kh + i) * 2048 + r * 16));
-  };
-  // [128][kSvLd], over the stage and raw buffers: when a drain thread finishes,
+  auto a_row = [&](int c, const unsigned char* raw, int r, int kh, float (&v)[8]) { a_mfast(raw, r, kh, v); };
+  // [128][kSvLd1], over the stage and raw buffers: when a drain thread finishes,
   // every chunk has been converted and multiplied and no copy is in flight
   double* sv = reinterpret_cast<double*>(tc::pipe_stage_base());
   auto finish = [&](const float (&acc)[ForcePipe::kCols], int row, int col0) {
-    const int g = g0 + row, pb = col0 / 2;
+    const int r = m0 + row;
+    const double sg = (row & 1) ? 1.0 : -1.0;
 #pragma unroll
-    for (int j = 0; j < kNC; ++j) {
-      const int p = p0 + pb + j;
-      double v = 0.0;
-      if (g < ngl && p < npro) {
-        const ProDesc d = pdesc[p];
-        const double pr = pro[(size_t)g + (size_t)ngl * d.ibare];
-        const double y = ylm[(size_t)g + (size_t)ngl * d.lm];
-        const double2 cw = cmul(make_double2(0.0, pr), cmul(mipow(d.l), eigr[(size_t)g + (size_t)ngl * d.iat]));
-        v = (cw.x * (double)acc[2 * j] + cw.y * (double)acc[2 * j + 1]) * y;
-      }
-      sv[row * kSvLd + pb + j] = v;
+    for (int j = 0; j < ForcePipe::kCols; ++j) {
+      const int p = p0 + col0 + j;
+      sv[row * kSvLd1 + col0 + j] =
+          (r < 2 * nh && p < npro) ? sg * (double)__ldg(&pf[(size_t)ldu * p + (r ^ 1)]) * (double)acc[j] : 0.0;
     }
   };
   NoConvertB no_cb;
-  tc::pipe_run<ForcePipe>((nbh + kCK - 1) / kCK, load, load_b, a_row, no_cb, finish, err);
+  tc::pipe_run<ForcePipe>(nchk, load, load_b, a_row, no_cb, finish, err);
   // pipe_run ended with a CTA barrier: sv is complete (if a wait ran out the
   // error flag is set and the caller discards the result).  G components of the
-  // tile, then fpart = sum_g sv(g,p) G_c(g) in four row quarters combined in a
+  // rows, then fpart = sum_r sv(r,p) G_c in four row quarters combined in a
   // fixed order
-  double* gsh = sv + 128 * kSvLd;  // [128][4]
-  double* qsum = gsh + 4 * 128;    // [4][192]
+  double* gsh = sv + 128 * kSvLd1;  // [128][4]
+  double* qsum = gsh + 4 * 128;     // [4][384]
   for (int i = threadIdx.x; i < 3 * 128; i += blockDim.x) {
-    const int c = i / 128, r = i % 128, g = g0 + r;
-    gsh[4 * r + c] = g < ngl ? (c == 0 ? gx : (c == 1 ? gy : gz))[g] : 0.0;
+    const int c = i / 128, row = i % 128, r = m0 + row;
+    gsh[4 * row + c] = r < 2 * nh ? (c == 0 ? gx : (c == 1 ? gy : gz))[half[r >> 1].x] : 0.0;
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < 4 * 192; i += blockDim.x) {
-    const int qr = i / 192, k = i % 192, pl = k / 3, c = k % 3;
+  for (int i = threadIdx.x; i < 4 * 384; i += blockDim.x) {
+    const int qr = i / 384, k = i % 384, pl = k / 3, c = k % 3;
     double s = 0.0;
 #pragma unroll 8
-    for (int r = 32 * qr; r < 32 * qr + 32; ++r) s += sv[r * kSvLd + pl] * gsh[4 * r + c];
+    for (int r = 32 * qr; r < 32 * qr + 32; ++r) s += sv[r * kSvLd1 + pl] * gsh[4 * r + c];
     qsum[i] = s;
   }
   __syncthreads();
-  for (int k = threadIdx.x; k < 192; k += blockDim.x) {
+  for (int k = threadIdx.x; k < 384; k += blockDim.x) {
     const int pl = k / 3, c = k % 3, p = p0 + pl;
-    if (p < npro) fpart[((size_t)blockIdx.x * npro + p) * 3 + c] = ((qsum[k] + qsum[192 + k]) + qsum[384 + k]) + qsum[576 + k];
+    if (p < npro) fpart[((size_t)blockIdx.x * npro + p) * 3 + c] = ((qsum[k] + qsum[384 + k]) + qsum[768 + k]) + qsum[1152 + k];
   }
 }
 
 // ---------------------------------------------------------------------------
 // Forces, persistent form for NBH <= 64 (an even number of K chunks, at most
-// eight): the same D(g,p) = sum_b psi0(g,b) conj(E(b,p)) and force sums as
-// k_tc_force, but one CTA per SM walks a contiguous run of (g tile, projector
-// tile) items.  The split psi0 rows of a g tile (all of K: 8 chunks x 32 TMEM
-// columns) stay in tensor memory for every projector tile of that g tile, so
-// only the pre-split conj(E) chunks stream.  Each item accumulates in one of
-// two TMEM regions (two chunks at a time: cross terms, then hi*hi); the drain
-// warps copy the region to registers and release it at once, so the MMAs of
-// the next items run while the drains form sv(g,p) = Re[i pf(g,p) conj(D)]
-// from the FP32 projector table and the G-weighted column sums of this item.
+// eight): the same D(r,p) = sum_n U(r,n) E(n,p) and force sums as k_tc_force,
+// but one CTA per SM walks a contiguous run of (row tile, projector tile) items.
+// The split U rows of a row tile (all of K: 8 chunks x 32 TMEM columns) stay in
+// tensor memory for every projector tile of that row tile, so only the pre-split
+// E chunks stream.  Each item accumulates in one of two TMEM regions (two chunks
+// at a time: cross terms, then hi*hi); the drain warps copy the region to
+// registers and release it at once, so the MMAs of the next items run while the
+// drains form sv(r,p) = +-P(r^1,p) D(r,p) from the fp32 projector table and the
+// G-weighted column sums of this item, 64 projectors at a time.
 //   warp 0   TMEM allocation, MMA issue (one thread)
-//   warp 1   TMA copies of raw psi0 chunks (two raw slots, one per converter group)
-//   warp 2   bulk copies of the split conj(E) chunks into kFNS stages
-//   3..10    converters (two groups of four warps, alternate chunks of a g tile)
+//   warp 1   TMA copies of raw U chunks (two raw slots, one per converter group)
+//   warp 2   bulk copies of the split E chunks into kFNS stages
+//   3..10    converters (two groups of four warps, alternate chunks of a row tile)
 //   11..26   drains and the per-item force epilogue
-// Barriers: rawfull/rawempty (raw psi0 slots), afull[c] (A chunk c of the
-// current g tile in TMEM), afree (MMAs of the last item of a g tile done),
+// Barriers: rawfull/rawempty (raw U slots), afull[c] (A chunk c of the
+// current row tile in TMEM), afree (MMAs of the last item of a row tile done),
 // sfull/sfree (B stages), bfull/bempty (accumulation regions, one item each).
 // Every wait is bounded; the drain group decides to leave by one vote per item
 // (a reduction barrier all 16 drain warps reach), so none of them is left at a
@@ -563,19 +530,19 @@ __global__ void __launch_bounds__(kThreads, 1)
 // ---------------------------------------------------------------------------
 constexpr int kFNS = 6;        // B stages (16 KB each)
 constexpr int kFMaxChunks = 8; // K chunks of a resident A tile (TMEM columns 256..511)
-constexpr size_t kForcePSmem = (size_t)kFNS * 16384 + 2 * 16384 +
+constexpr size_t kForcePSmem = (size_t)kFNS * 16384 + 2 * kRawFold +
                                sizeof(double) * (128 * kSvLd + 4 * 128 + 4 * 192) + 1024 + 512;
 static_assert(kForcePSmem <= 232448, "shared memory");
 
 __global__ void __launch_bounds__(kThreads, 1)
-    k_tc_force_p(const __grid_constant__ CUtensorMap tm_psi, const float* __restrict__ be, int nchk, int ngl, int npro,
-                 int ldg, int tn, int nitems, const float2* __restrict__ pf, const double* __restrict__ gx,
-                 const double* __restrict__ gy, const double* __restrict__ gz, double* __restrict__ fpart,
-                 int* __restrict__ err) {
+    k_tc_force_p(const __grid_constant__ CUtensorMap tm_u, const float* __restrict__ be, int nchk, int nh, int npro,
+                 int ldu, int tn, int nitems, const float* __restrict__ pf, const int2* __restrict__ half,
+                 const double* __restrict__ gx, const double* __restrict__ gy, const double* __restrict__ gz,
+                 double* __restrict__ fpart, int* __restrict__ err) {
   using namespace tc;
   float* st = pipe_stage_base();
   unsigned char* raw0 = reinterpret_cast<unsigned char*>(st) + (size_t)kFNS * 16384;
-  double* sv = reinterpret_cast<double*>(raw0 + 2 * 16384);  // [128][kSvLd]
+  double* sv = reinterpret_cast<double*>(raw0 + 2 * kRawFold);  // [128][kSvLd]
   double* gsh = sv + 128 * kSvLd;                            // [128][4]
   double* qsum = gsh + 4 * 128;                              // [4][192]
   uint64_t* rawfull = reinterpret_cast<uint64_t*>(qsum + 4 * 192);
@@ -592,7 +559,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   const long long G = gridDim.x;
   const int w0 = (int)((long long)blockIdx.x * nitems / G), w1 = (int)((long long)(blockIdx.x + 1) * nitems / G);
   const int m_first = w0 / tn;
-  const int nm = w1 > w0 ? (w1 - 1) / tn - m_first + 1 : 0;  // g tiles of this CTA
+  const int nm = w1 > w0 ? (w1 - 1) / tn - m_first + 1 : 0;  // row tiles of this CTA
   if (tid == 0) {
     for (int i = 0; i < 2; ++i) {
       mbar_init(&rawfull[i], 1);
@@ -681,7 +648,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
     }
   } else if (warp == 1) {
-    // raw psi0 chunks: chunk c of the im-th g tile goes to slot c % 2 (the slot
+    // raw U chunks: chunk c of the im-th row tile goes to slot c % 2 (the slot
     // of converter group c % 2)
     int issued = 0;
     const int total = nm * nchk;
@@ -698,8 +665,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         break;
       }
       if (lane == 0) {
-        tma_load_2d(raw0 + slot * 16384, &tm_psi, 2 * 128 * m, c * kCK, &rawfull[slot]);
-        mbar_arrive_expect_tx(&rawfull[slot], 16384);
+        tma_load_2d(raw0 + slot * kRawFold, &tm_u, 128 * m, c * kCK, &rawfull[slot]);
+        mbar_arrive_expect_tx(&rawfull[slot], kRawFold);
       }
       issued = q + 1;
     }
@@ -733,7 +700,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (*abort_flag && lane == 0)
       for (int q = max(0, issued - kFNS); q < issued; ++q) mbar_wait(&sfull[q % kFNS], (q / kFNS) & 1, kWaitCycles);
   } else if (warp < 11) {
-    // converters: group grp owns chunks grp, grp + 2, ... of every g tile
+    // converters: group grp owns chunks grp, grp + 2, ... of every row tile
     const int grp = (warp - 3) >> 2;
     const int arow = 32 * (warp & 3) + lane;
     const uint32_t tlane = (uint32_t)(32 * (warp & 3)) << 16;
@@ -748,18 +715,17 @@ __global__ void __launch_bounds__(kThreads, 1)
           if (lane == 0) raise();
           break;
         }
-        const unsigned char* raw = raw0 + slot * 16384;
+        const unsigned char* raw = raw0 + slot * kRawFold;
 #pragma unroll
         for (int kh = 0; kh < 2; ++kh) {
+          float v[8];
+          a_mfast(raw, arow, kh, v);
           uint32_t hi[8], lo[8];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const double2 x = at<double2>(raw, (4 * kh + i) * 2048 + arow * 16);
-            float h0, l0, h1, l1;
-            split_tf32f((float)x.x, h0, l0);
-            split_tf32f((float)x.y, h1, l1);
-            hi[2 * i] = __float_as_uint(h0), lo[2 * i] = __float_as_uint(l0);
-            hi[2 * i + 1] = __float_as_uint(h1), lo[2 * i + 1] = __float_as_uint(l1);
+          for (int i = 0; i < 8; ++i) {
+            float h0, l0;
+            split_tf32f(v[i], h0, l0);
+            hi[i] = __float_as_uint(h0), lo[i] = __float_as_uint(l0);
           }
           const uint32_t ta = tmem + tlane + (uint32_t)(256 + 32 * c + 8 * kh);
           tmem_st8(ta, hi);
@@ -774,12 +740,13 @@ __global__ void __launch_bounds__(kThreads, 1)
   } else {
     const int q = warp & 3, dw = warp - 11, col0 = 32 * (dw / 4), dt = tid - 11 * 32;
     const uint32_t lane_base = ((uint32_t)(32 * q) << 16) + (uint32_t)col0;
-    const int row = 32 * q + lane, pb = col0 / 2;
+    const int row = 32 * q + lane;
+    const double sg = (row & 1) ? 1.0 : -1.0;
     // expected truncation loss: a quarter unit in the last place per K=8 step
     const float half_ulps = kLossPerStep * (float)(2 * nchk);
     int it = 0;
     for (int w = w0; w < w1; ++w, ++it) {
-      const int m = w / tn, n = w % tn, g = m * 128 + row, r = it & 1;
+      const int m = w / tn, n = w % tn, rr = m * 128 + row, r = it & 1;
       bool got = mbar_wait(&bfull[r], (it >> 1) & 1, kWaitCycles);
       got = __all_sync(0xffffffffu, got && !*abort_flag);
       float acc[32];
@@ -799,39 +766,47 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (dt == 0) raise();
         break;
       }
-      // G components of the item's g tile ([row][4]: the three components of
-      // a row in different banks); sv(g,p) = Re[i pf(g,p) conj(D)], with the
-      // sixteen table loads of a thread in flight together
+      // G components of the item's row tile ([row][4]: the three components of
+      // a row in different banks)
       if (dt < 128) {
-        const int gg = m * 128 + dt;
-        const bool in = gg < ngl;
-        gsh[4 * dt] = in ? gx[gg] : 0.0;
-        gsh[4 * dt + 1] = in ? gy[gg] : 0.0;
-        gsh[4 * dt + 2] = in ? gz[gg] : 0.0;
+        const int r1 = m * 128 + dt;
+        const int g = r1 < 2 * nh ? half[r1 >> 1].x : -1;
+        gsh[4 * dt] = g >= 0 ? gx[g] : 0.0;
+        gsh[4 * dt + 1] = g >= 0 ? gy[g] : 0.0;
+        gsh[4 * dt + 2] = g >= 0 ? gz[g] : 0.0;
       }
-      float2 pfv[16];
+#pragma unroll 1
+      for (int hb = 0; hb < 2; ++hb) {  // projectors 64 hb .. 64 hb + 63 of the item
+        if ((col0 >> 6) == hb) {
+          // thirty-two table loads of a thread, sixteen in flight together
 #pragma unroll
-      for (int jx = 0; jx < 16; ++jx) {
-        const int p = n * 64 + pb + jx;
-        pfv[jx] = (g < ngl && p < npro) ? __ldg(&pf[(size_t)p * ldg + g]) : make_float2(0.f, 0.f);
-      }
+          for (int jb = 0; jb < 32; jb += 16) {
+            float pfv[16];
 #pragma unroll
-      for (int jx = 0; jx < 16; ++jx)
-        sv[row * kSvLd + pb + jx] = -(double)pfv[jx].y * (double)acc[2 * jx] + (double)pfv[jx].x * (double)acc[2 * jx + 1];
-      bar_sync(1, 512);
-      // fpart[m][p][c] = sum_g sv(g,p) G_c(g): four row quarters, fixed order
-      for (int t = dt; t < 4 * 192; t += 512) {
-        const int qr = t / 192, k = t % 192, pl = k / 3, c = k % 3;
-        double sum = 0.0;
+            for (int jx = 0; jx < 16; ++jx) {
+              const int p = n * 128 + col0 + jb + jx;
+              pfv[jx] = (rr < 2 * nh && p < npro) ? __ldg(&pf[(size_t)p * ldu + (rr ^ 1)]) : 0.f;
+            }
+#pragma unroll
+            for (int jx = 0; jx < 16; ++jx)
+              sv[row * kSvLd + (col0 & 63) + jb + jx] = sg * (double)pfv[jx] * (double)acc[jb + jx];
+          }
+        }
+        bar_sync(1, 512);
+        // fpart[m][p][c] = sum_r sv(r,p) G_c: four row quarters, fixed order
+        for (int t = dt; t < 4 * 192; t += 512) {
+          const int qr = t / 192, k = t % 192, pl = k / 3, c = k % 3;
+          double sum = 0.0;
 #pragma unroll 8
-        for (int rw = 32 * qr; rw < 32 * qr + 32; ++rw) sum += sv[rw * kSvLd + pl] * gsh[4 * rw + c];
-        qsum[t] = sum;
-      }
-      bar_sync(1, 512);
-      if (dt < 192) {
-        const int pl = dt / 3, c = dt % 3, p = n * 64 + pl;
-        if (p < npro)
-          fpart[((size_t)m * npro + p) * 3 + c] = ((qsum[dt] + qsum[192 + dt]) + qsum[384 + dt]) + qsum[576 + dt];
+          for (int rw = 32 * qr; rw < 32 * qr + 32; ++rw) sum += sv[rw * kSvLd + pl] * gsh[4 * rw + c];
+          qsum[t] = sum;
+        }
+        bar_sync(1, 512);
+        if (dt < 192) {
+          const int pl = dt / 3, c = dt % 3, p = n * 128 + 64 * hb + pl;
+          if (p < npro)
+            fpart[((size_t)m * npro + p) * 3 + c] = ((qsum[dt] + qsum[192 + dt]) + qsum[384 + dt]) + qsum[576 + dt];
+        }
       }
       bar_sync(1, 512);
     }
@@ -845,62 +820,53 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
 }
 
-// Source of a split B operand: value(row, h) of complex output column `row`
-// at complex K index h
-//   kind 0: x[h + ld*row]            kind 1: x[row + ld*h]
-//   kind 2: conj x[h + ld*row]       kind 3: h < nk1 ? x[h + ld*row] : x2[h - nk1 + ld*row]
-//   kind 4: tile of 32 rows of x then 32 rows of x2, each as kind 1 (null: zero)
+// Source of a split B operand: value(row, k)
+//   kind 0: xf[k + ld*row]  (fp32)   kind 1: x[k + ld*row]
+//   kind 2: tile of 64 rows of x then 64 rows of x2, each x[row + ld*k] (null: zero)
 struct BSplitSrc {
   int kind;
-  const double2* x;
-  const double2* x2;
+  const double* x;
+  const double* x2;
+  const float* xf;
   long long ld;
-  int nrow, nk, nk1;
+  int nrow, nk;
+  int tps;              // tiles of one array (kind 0); the next array's tiles
+  long long set_stride; // follow, its values set_stride further
 };
 
-// B operand in real form, split into tf32 hi/lo tiles in the shared-memory
-// layout of the pipeline (tc_pipe.cuh): block (tile, chunk) of 4096 floats =
-// hi then lo, element (R, k) of 128 real rows x 16 real K at
-// (k/4)*512 + R*4 + k%4; real rows 2j / 2j+1 of complex column j are
-// (Re c, -Im c) / (Im c, Re c).  Zero outside the source.
+// B operand split into tf32 hi/lo tiles in the shared-memory layout of the
+// pipeline (tc_pipe.cuh): block (tile, chunk) of 4096 floats = hi then lo,
+// element (row, k) of 128 rows x 16 K at (k/4)*512 + row*4 + k%4.  Zero outside
+// the source.
 __global__ void k_bsplit(BSplitSrc b, int nchk, float* __restrict__ out) {
   const int tile = blockIdx.y, c = blockIdx.x;
   float* o = out + ((size_t)tile * nchk + c) * kBTile;
   for (int it = threadIdx.x; it < 512; it += blockDim.x) {
-    const int R = it & 127, kg = it >> 7, j = R >> 1;
-    double2 v[2];
+    const int R = it & 127, kg = it >> 7, k0 = c * kCK + 4 * kg;
+    float w[4] = {0.f, 0.f, 0.f, 0.f};
+    if (b.kind == 0) {
+      const int set = tile / b.tps, row = 128 * (tile - set * b.tps) + R;
+      // (rows are padded to 32 values, zero past NK)
+      if (row < b.nrow && k0 < b.nk) {
+        const float4 x = *reinterpret_cast<const float4*>(b.xf + set * b.set_stride + k0 + b.ld * row);
+        w[0] = x.x, w[1] = x.y, w[2] = x.z, w[3] = x.w;
+      }
+    } else {
+      const int row = b.kind == 1 ? 128 * tile + R : 64 * tile + (R & 63);
+      const double* src = b.kind == 1 || R < 64 ? b.x : b.x2;
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const int h = c * kCK + 2 * kg + e;
-      v[e] = dz();
-      if (h >= b.nk) continue;
-      if (b.kind == 4) {
-        const double2* src = j < 32 ? b.x : b.x2;
-        const int row = 32 * tile + (j & 31);
-        if (src && row < b.nrow) v[e] = src[(size_t)row + (size_t)b.ld * h];
-      } else {
-        const int row = 64 * tile + j;
-        if (row >= b.nrow) continue;
-        if (b.kind == 0) v[e] = b.x[(size_t)h + (size_t)b.ld * row];
-        else if (b.kind == 1) v[e] = b.x[(size_t)row + (size_t)b.ld * h];
-        else if (b.kind == 2) v[e] = cj(b.x[(size_t)h + (size_t)b.ld * row]);
-        else v[e] = h < b.nk1 ? b.x[(size_t)h + (size_t)b.ld * row] : b.x2[(size_t)(h - b.nk1) + (size_t)b.ld * row];
+      for (int e = 0; e < 4; ++e) {
+        const int k = k0 + e;
+        if (src && row < b.nrow && k < b.nk) w[e] = (float)(b.kind == 1 ? src[k + b.ld * row] : src[row + b.ld * k]);
       }
     }
-    double w[4];
-    if ((R & 1) == 0) w[0] = v[0].x, w[1] = -v[0].y, w[2] = v[1].x, w[3] = -v[1].y;
-    else w[0] = v[0].y, w[1] = v[0].x, w[2] = v[1].y, w[3] = v[1].x;
-    tc::store_split4(o, o + 2048, kg * 128 + R, w[0], w[1], w[2], w[3]);
-  }
-}
-
-// dst(g, b) = src(-g, b) for g < NGL, 0 in the padding (ld = ldg)
-__global__ void k_minus_copy(const double2* __restrict__ src, double2* __restrict__ dst,
-                             const int* __restrict__ minusg, int ngl, int ldg, int nbh) {
-  const size_t n = (size_t)ldg * nbh;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const int g = (int)(i % ldg);
-    dst[i] = g < ngl ? src[(size_t)minusg[g] + (i - g)] : dz();
+    float4 h, l;
+    tc::split_tf32f(w[0], h.x, l.x);
+    tc::split_tf32f(w[1], h.y, l.y);
+    tc::split_tf32f(w[2], h.z, l.z);
+    tc::split_tf32f(w[3], h.w, l.w);
+    reinterpret_cast<float4*>(o)[kg * 128 + R] = h;
+    reinterpret_cast<float4*>(o + 2048)[kg * 128 + R] = l;
   }
 }
 
@@ -938,40 +904,49 @@ static EncodeTiled encode_tiled() {
   return fn;
 }
 
-// 2-D map of `rows` rows of `inner` real elements (FP64 or fp32), rows `ld`
-// elements apart, box bx x by; elements outside read as zero
-static int make_map(Handle* h, CUtensorMap* m, const void* base, bool f64, long long inner, long long rows,
-                    long long ld, int bx, int by, CUtensorMapSwizzle sw) {
+// 2-D map of `rows` rows of `inner` fp32 values, rows `ld` values apart, box bx
+// x by; elements outside read as zero
+static int make_map(Handle* h, CUtensorMap* m, const float* base, long long inner, long long rows, long long ld, int bx,
+                    int by, CUtensorMapSwizzle sw) {
   const EncodeTiled fn = encode_tiled();
   if (!fn) return h->fail(CUW_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
-  const long long es = f64 ? 8 : 4;
   const cuuint64_t dims[2] = {(cuuint64_t)std::max(1ll, inner), (cuuint64_t)std::max(1ll, rows)};
-  const cuuint64_t strides[1] = {(cuuint64_t)(ld * es)};
+  const cuuint64_t strides[1] = {(cuuint64_t)(ld * 4)};
   const cuuint32_t box[2] = {(cuuint32_t)bx, (cuuint32_t)by};
   const cuuint32_t estr[2] = {1, 1};
-  const CUresult r = fn(m, f64 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2,
-                        const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
-                        CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  const CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(base), dims, strides, box, estr,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return h->fail(CUW_ERR_CUDA, "cuTensorMapEncodeTiled failed: " + std::to_string((int)r));
   return CUW_OK;
 }
-// complex (ld, cols) array of FP64 pairs: rows = columns of the array
-static int map_c(Handle* h, CUtensorMap* m, const double2* base, long long n, long long cols, long long ld, int bx,
-                 int by, CUtensorMapSwizzle sw) {
-  return make_map(h, m, base, true, 2 * n, cols, 2 * ld, bx, by, sw);
+// a folded array (rows of 2 nh sphere values) as K-contiguous or row-contiguous
+// A operand
+static int map_kfast(Handle* h, CUtensorMap* m, const float* base, int rows) {
+  return make_map(h, m, base, 2 * h->nh, rows, h->ldu, 16, 128, CU_TENSOR_MAP_SWIZZLE_64B);
 }
+static int map_mfast(Handle* h, CUtensorMap* m, const float* base, int rows) {
+  return make_map(h, m, base, 2 * h->nh, rows, h->ldu, 128, 16, CU_TENSOR_MAP_SWIZZLE_NONE);
+}
+static float* u32_slot(const Handle* h, int slot) { return h->g.u32 + (size_t)slot * h->d.nb * h->ldu; }
+static int tiles_per_array(const Handle* h) { return ceil_div(h->d.nb, 128); }
 
 int tc_setup(Handle* h) {
-  CUW_TRY(smem_allow((const void*)k_tc_proj, (int)ProjPipe::kSmem));
+  CUW_TRY(smem_allow((const void*)k_tc_tn<ProjPipe>, (int)ProjPipe::kSmem));
+  CUW_TRY(smem_allow((const void*)k_tc_tn<GramPipe>, (int)GramPipe::kSmem));
   CUW_TRY(smem_allow((const void*)k_tc_addpro<ADDPRO_HPSI>, (int)AddproPipe::kSmem));
   CUW_TRY(smem_allow((const void*)k_tc_addpro<ADDPRO_OPSI>, (int)AddproPipe::kSmem));
   CUW_TRY(smem_allow((const void*)k_tc_addpro<ADDPRO_FUSED>, (int)AddproPipe::kSmem));
-  CUW_TRY(smem_allow((const void*)k_tc_gram<true>, (int)GramPipe::kSmem));
-  CUW_TRY(smem_allow((const void*)k_tc_gram<false>, (int)GramPipe::kSmem));
   CUW_TRY(smem_allow((const void*)k_tc_addx, (int)AddxPipe::kSmem));
   CUW_TRY(smem_allow((const void*)k_tc_force, (int)ForcePipe::kSmem));
   CUW_TRY(smem_allow((const void*)k_tc_force_p, (int)kForcePSmem));
   if (!encode_tiled()) return h->fail(CUW_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
+  return CUW_OK;
+}
+
+// buffers whose sizes follow from the folded sphere (called with a new G set)
+int tc_rooms(Handle* h) {
+  Device& g = h->g;
   auto alloc = [&](void** p, size_t bytes) -> int {
     if (*p) return CUW_OK;
     if (cudaMalloc(p, bytes) != cudaSuccess) {
@@ -979,37 +954,42 @@ int tc_setup(Handle* h) {
       *p = nullptr;
       return h->fail(CUW_ERR_NOMEM, "cudaMalloc of mixed-path scratch failed");
     }
-    CUW_TRY(cudaMemsetAsync(*p, 0, bytes, h->stream));
     return CUW_OK;
   };
-  CUW_RET(alloc(reinterpret_cast<void**>(&h->g.pf), sizeof(float2) * (size_t)h->ldg * std::max(1, h->npro)));
-  for (int i = 0; i < 2; ++i)
-    CUW_RET(alloc(reinterpret_cast<void**>(&h->g.xminus[i]), sizeof(double2) * (size_t)h->ldg * h->d.nbh));
-  const size_t psi_split = (size_t)kBTile * ceil_div(h->d.nbh, 64) * ceil_div(h->d.ngl, kCK);
-  for (int i = 0; i < 2; ++i) CUW_RET(alloc(reinterpret_cast<void**>(&h->g.bpre[i]), sizeof(float) * psi_split));
-  // largest small-matrix operand: [C1 | C2] of ADDPRO, tiles of 32 bands
-  const int np = std::max(1, h->npro), nb = h->d.nbh;
-  size_t slot = (size_t)ceil_div(nb, 32) * ceil_div(np, kCK);
-  slot = std::max(slot, (size_t)ceil_div(np, 64) * ceil_div(nb, kCK));
-  slot = std::max(slot, (size_t)ceil_div(nb, 64) * ceil_div(np, kCK));
-  slot = std::max(slot, (size_t)ceil_div(nb, 64) * ceil_div(2 * nb, kCK));
-  h->g.bsmall_slot = slot * kBTile;
-  CUW_RET(alloc(reinterpret_cast<void**>(&h->g.bsmall), sizeof(float) * 3 * h->g.bsmall_slot));
+  const int np = std::max(1, h->npro), nb = h->d.nb;
+  CUW_RET(alloc(reinterpret_cast<void**>(&g.pf), sizeof(float) * (size_t)h->ldu * np));
+  if (!g.u32) {
+    CUW_RET(alloc(reinterpret_cast<void**>(&g.u32), sizeof(float) * (size_t)h->ldu * nb * 2));
+    // the padding of the rows is read as K values past the sphere (k_bsplit)
+    if (h->ldu > 2 * h->nh)
+      CUW_TRY(cudaMemset2DAsync(g.u32 + 2 * h->nh, sizeof(float) * h->ldu, 0, sizeof(float) * (h->ldu - 2 * h->nh),
+                                (size_t)2 * nb, h->stream));
+  }
+  CUW_RET(alloc(reinterpret_cast<void**>(&g.bpre),
+                sizeof(float) * kBTile * 2 * (size_t)tiles_per_array(h) * ceil_div(2 * h->nh, kCK)));
+  // largest small-matrix operand: [C1 | C2] of ADDPRO, DEDPRO or Lambda
+  size_t slot = (size_t)ceil_div(nb, 64) * ceil_div(np, kCK);
+  slot = std::max(slot, (size_t)ceil_div(np, 128) * ceil_div(nb, kCK));
+  slot = std::max(slot, (size_t)ceil_div(nb, 128) * ceil_div(nb, kCK));
+  CUW_RET(alloc(reinterpret_cast<void**>(&g.bsmall), sizeof(float) * slot * kBTile));
   return CUW_OK;
 }
 
-int tc_pro_table(Handle* h) {
+int tc_pro_table(Handle* h, const double* r_dev) {
   if (h->npro == 0) return CUW_OK;
-  const dim3 grid(std::min(ceil_div(h->ldg, 256), 64), h->d.nat);
-  k_pro_f32<<<grid, 256, 0, h->stream>>>(h->d.ngl, h->ldg, h->g.t_ipro0, h->g.t_nlmn, h->g.pdesc, h->g.ylm, h->g.pro,
-                                         h->g.eigr, h->g.pf);
+  const Device& g = h->g;
+  k_pro_f32<<<dim3(ceil_div(h->nh, 256), h->d.nat), 256, 0, h->stream>>>(h->nh, h->d.ngl, h->ldu, g.half, g.gx, g.gy,
+                                                                         g.gz, r_dev, g.t_ipro0, g.t_nlmn, g.pdesc,
+                                                                         g.ylm, g.pro, g.pf);
   CUW_LAUNCH_CHECK("k_pro_f32");
   return CUW_OK;
 }
 
-void tc_scope(Handle* h, bool open) {
-  h->tc_scope_open = open;
-  h->g.bpre_src[0] = h->g.bpre_src[1] = nullptr;
+int tc_fold(Handle* h, const double2* psi, int slot) {
+  k_fold_f32<<<dim3(ceil_div(h->nh, 256), h->d.nbh), 256, 0, h->stream>>>(psi, h->g.half, h->nh, h->ldg, h->ldu,
+                                                                          u32_slot(h, slot));
+  CUW_LAUNCH_CHECK("k_fold_f32");
+  return CUW_OK;
 }
 
 static int tc_bsplit(Handle* h, const BSplitSrc& b, int ntile, int nchk, float* out) {
@@ -1017,213 +997,153 @@ static int tc_bsplit(Handle* h, const BSplitSrc& b, int ntile, int nchk, float* 
   CUW_LAUNCH_CHECK("k_bsplit");
   return CUW_OK;
 }
-// split form of wave-function array psi (B operand, rows = bands, K = g)
-static int tc_bsplit_psi(Handle* h, const double2* psi, const float** out) {
-  Device& g = h->g;
-  for (int i = 0; i < 2; ++i)
-    if (h->tc_scope_open && g.bpre_src[i] == psi) {
-      *out = g.bpre[i];
-      return CUW_OK;
-    }
-  const int i = g.bpre_src[0] ? 1 : 0;
-  BSplitSrc b{0, psi, nullptr, (long long)h->ldg, h->d.nbh, h->d.ngl, 0};
-  CUW_RET(tc_bsplit(h, b, ceil_div(h->d.nbh, 64), ceil_div(h->d.ngl, kCK), g.bpre[i]));
-  if (h->tc_scope_open) g.bpre_src[i] = psi;
-  *out = g.bpre[i];
-  return CUW_OK;
-}
-// split form of a small matrix into slot `slot` of h->g.bsmall
-static int tc_bsplit_small(Handle* h, const BSplitSrc& b, int ntile, int nchk, int slot, const float** out) {
-  if ((size_t)ntile * nchk * kBTile > h->g.bsmall_slot) return h->fail(CUW_ERR_STATE, "split operand scratch too small");
-  float* dst = h->g.bsmall + (size_t)slot * h->g.bsmall_slot;
-  CUW_RET(tc_bsplit(h, b, ntile, nchk, dst));
-  *out = dst;
-  return CUW_OK;
+
+// split forms of folded slots 0 .. nset-1 (B operands of tc_proj and tc_gram)
+int tc_split(Handle* h, int nset) {
+  BSplitSrc b{};
+  b.xf = h->g.u32;
+  b.ld = h->ldu;
+  b.nrow = h->d.nb;
+  b.nk = 2 * h->nh;
+  b.tps = tiles_per_array(h);
+  b.set_stride = (long long)h->d.nb * h->ldu;
+  return tc_bsplit(h, b, nset * b.tps, ceil_div(2 * h->nh, kCK), h->g.bpre);
 }
 
-// X(-G) copy of a wave-function array into scratch slot i
-static int tc_minus(Handle* h, const double2* x, int i, const double2** out) {
-  const size_t n = (size_t)h->ldg * h->d.nbh;
-  const int blocks = (int)std::min<size_t>((n + 255) / 256, (size_t)8 * h->nsm);
-  k_minus_copy<<<blocks, 256, 0, h->stream>>>(x, h->g.xminus[i], h->g.minusg, h->d.ngl, h->ldg, h->d.nbh);
-  CUW_LAUNCH_CHECK("k_minus_copy");
-  *out = h->g.xminus[i];
-  return CUW_OK;
-}
-
-static int tc_reduce(Handle* h, const float2* part, int nz, size_t n, double scale, double2* out) {
-  const int rb = (int)std::min<size_t>((n + 255) / 256, (size_t)4 * h->nsm);
-  k_tc_reduce<<<rb, 256, 0, h->stream>>>(part, nz, n, scale, out);
-  CUW_LAUNCH_CHECK("k_tc_reduce");
-  return CUW_OK;
-}
-
-int tc_proj(Handle* h, const double2* psi, double2* proj) {
-  const int nbh = h->d.nbh, npro = h->npro, ngl = h->d.ngl;
-  const int tn = ceil_div(npro, 128), tb = ceil_div(nbh, 64);
-  int ks = tc_splits(h, tn * tb, ngl, h->split_proj);
-  const int kchunk = ceil_div(ceil_div(ngl, ks), kCK) * kCK;
-  ks = ceil_div(ngl, kchunk);
-  const size_t n = (size_t)nbh * npro;
+// PROJ of slot 0 (and slot 1 when proj1 is given), from the split forms
+int tc_proj(Handle* h, double2* proj0, double2* proj1) {
+  const int nb = h->d.nb, npro = h->npro, nset = proj1 ? 2 : 1;
+  TcTnArgs a{};
+  a.npair = 1;
+  a.nk = 2 * h->nh;
+  a.nrow = npro;
+  a.ncol = nb;
+  a.tps = tiles_per_array(h);
+  a.ldp = nset * nb;
+  a.nchk = ceil_div(a.nk, kCK);
+  a.bs[0] = h->g.bpre;
+  TcTnMaps tm;
+  CUW_RET(map_kfast(h, &tm.a[0], h->g.pf, npro));
+  tm.a[1] = tm.a[2] = tm.a[0];
+  const int tn = ceil_div(npro, 128), tb = nset * a.tps;
+  int ks = tc_splits(h, tn * tb, a.nk, h->split_proj);
+  a.kchunk = ceil_div(ceil_div(a.nk, ks), kCK) * kCK;
+  ks = ceil_div(a.nk, a.kchunk);
+  const size_t n = (size_t)nset * h->d.nbh * npro;
   CUW_RET(ensure_part(h, sizeof(float2) * n * ks));
-  float2* part = reinterpret_cast<float2*>(h->g.part);
-  CUtensorMap tpf;
-  CUW_RET(make_map(h, &tpf, h->g.pf, false, 2ll * ngl, npro, 2ll * h->ldg, 16, 128, CU_TENSOR_MAP_SWIZZLE_64B));
-  const float* bpsi = nullptr;
-  CUW_RET(tc_bsplit_psi(h, psi, &bpsi));
-  k_tc_proj<<<dim3(tn, tb, ks), kThreads, ProjPipe::kSmem, h->stream>>>(tpf, bpsi, ceil_div(ngl, kCK), ngl, nbh, npro,
-                                                                         kchunk, part, tc_err(h));
-  CUW_LAUNCH_CHECK("k_tc_proj");
-  return tc_reduce(h, part, ks, n, h->gweight, proj);
+  k_tc_tn<ProjPipe><<<dim3(tn, tb, ks), kThreads, ProjPipe::kSmem, h->stream>>>(a, tm, reinterpret_cast<float*>(h->g.part),
+                                                                      tc_err(h));
+  CUW_LAUNCH_CHECK("k_tc_tn");
+  k_tc_proj_sum<<<(unsigned)std::min<size_t>((n + 127) / 128, (size_t)16 * h->nsm), 128, 0, h->stream>>>(
+      reinterpret_cast<const float2*>(h->g.part), ks, h->d.nbh, nset, npro, h->gweight, proj0, proj1);
+  CUW_LAUNCH_CHECK("k_tc_proj_sum");
+  return CUW_OK;
 }
 
 int tc_addpro(Handle* h, int mode, const double2* hpc, const double2* opc, const StepCoef& sc) {
-  const int ngl = h->d.ngl, nbh = h->d.nbh, npro = h->npro;
-  const dim3 grid(ceil_div(nbh, 32), ceil_div(ngl, 128));
   Device& g = h->g;
+  const int nb = h->d.nb, npro = h->npro;
   CUtensorMap tpf;
-  CUW_RET(make_map(h, &tpf, g.pf, false, 2ll * ngl, npro, 2ll * h->ldg, 256, 8, CU_TENSOR_MAP_SWIZZLE_NONE));
+  CUW_RET(map_mfast(h, &tpf, g.pf, npro));
   const int nchk = ceil_div(npro, kCK);
-  const float* bc = nullptr;
-  BSplitSrc b{4, mode == ADDPRO_OPSI ? nullptr : hpc, mode == ADDPRO_HPSI ? nullptr : opc, (long long)nbh, nbh, npro, 0};
-  CUW_RET(tc_bsplit_small(h, b, ceil_div(nbh, 32), nchk, 0, &bc));
-#define TC_ADDPRO(M)                                                                                            \
-  k_tc_addpro<M><<<grid, kThreads, AddproPipe::kSmem, h->stream>>>(g.hpsi, g.opsi, g.psi0, g.psim, g.mpsi, h->ldg, \
-                                                                   ngl, nbh, npro, tpf, bc, nchk, sc, tc_err(h))
-  if (mode == ADDPRO_HPSI) TC_ADDPRO(ADDPRO_HPSI);
-  else if (mode == ADDPRO_OPSI) TC_ADDPRO(ADDPRO_OPSI);
-  else TC_ADDPRO(ADDPRO_FUSED);
-#undef TC_ADDPRO
+  BSplitSrc b{};
+  b.kind = 2;
+  b.x = mode == ADDPRO_OPSI ? nullptr : reinterpret_cast<const double*>(hpc);
+  b.x2 = mode == ADDPRO_HPSI ? nullptr : reinterpret_cast<const double*>(opc);
+  b.ld = nb;
+  b.nrow = nb;
+  b.nk = npro;
+  CUW_RET(tc_bsplit(h, b, ceil_div(nb, 64), nchk, g.bsmall));
+  const TcAddproArgs a{g.hpsi, g.opsi, g.psim, g.psi0, g.rmpsi, g.half, u32_slot(h, 0), u32_slot(h, 1),
+                       h->ldg, h->ldu, h->nh, h->d.nbh, npro, nchk, g.bsmall, sc};
+  const dim3 grid(ceil_div(nb, 64), ceil_div(2 * h->nh, 128));
+  if (mode == ADDPRO_HPSI) k_tc_addpro<ADDPRO_HPSI><<<grid, kThreads, AddproPipe::kSmem, h->stream>>>(a, tpf, tc_err(h));
+  else if (mode == ADDPRO_OPSI) k_tc_addpro<ADDPRO_OPSI><<<grid, kThreads, AddproPipe::kSmem, h->stream>>>(a, tpf, tc_err(h));
+  else k_tc_addpro<ADDPRO_FUSED><<<grid, kThreads, AddproPipe::kSmem, h->stream>>>(a, tpf, tc_err(h));
   CUW_LAUNCH_CHECK("k_tc_addpro");
   return CUW_OK;
 }
 
-int tc_gram(Handle* h, const GramPair* pairs, int npair, bool minus, int nk, int nm, size_t sk, size_t sm,
-            double scale, double2* dst) {
-  if (npair < 1 || npair > 3) return h->fail(CUW_ERR_ARG, "Gram product: one to three pairs");
-  TcGramArgs a{};
+int tc_gram(Handle* h, const FoldPair* pairs, int npair, double* o0, double* o1, double* o2) {
+  if (npair < 1 || npair > 3) return h->fail(CUW_ERR_ARG, "overlaps: one to three pairs");
+  const int nb = h->d.nb, tps = tiles_per_array(h);
+  TcTnArgs a{};
   a.npair = npair;
-  a.nk = nk;
-  a.nm = nm;
-  a.kfast = sk == 1;
-  a.nchk = ceil_div(nk, kCK);
-  if (!a.kfast && sm != 1) return h->fail(CUW_ERR_UNSUPPORTED, "Gram product with neither index contiguous");
-  if (minus && !a.kfast) return h->fail(CUW_ERR_UNSUPPORTED, "X(-k) Gram product of projections");
-  TcGramMaps tm{};
-  // X(-k) copies of the distinct X arrays (at most two: PSIBAR and OPSI)
-  const double2* src[2] = {nullptr, nullptr};
-  const double2* mcopy[2] = {nullptr, nullptr};
-  const double2* ydone[3] = {nullptr, nullptr, nullptr};
-  int nsmall = 0;
-  for (int i = 0; i < npair; ++i) {
-    const double2 *x = pairs[i].x, *y = pairs[i].y;
-    if (a.kfast) {
-      CUW_RET(map_c(h, &tm.x[i], x, nk, nm, (long long)sm, 16, 64, CU_TENSOR_MAP_SWIZZLE_128B));
-      CUW_RET(tc_bsplit_psi(h, y, &a.ybs[i]));
-    } else {
-      CUW_RET(map_c(h, &tm.x[i], x, nm, nk, (long long)sk, 128, 8, CU_TENSOR_MAP_SWIZZLE_NONE));
-      int same = -1;
-      for (int j = 0; j < i; ++j)
-        if (ydone[j] == y) same = j;
-      if (same >= 0) {
-        a.ybs[i] = a.ybs[same];
-      } else {
-        BSplitSrc b{1, y, nullptr, (long long)sk, nm, nk, 0};
-        CUW_RET(tc_bsplit_small(h, b, ceil_div(nm, 64), a.nchk, nsmall++, &a.ybs[i]));
-      }
-      ydone[i] = y;
-    }
-    tm.xm[i] = tm.x[i];
-    if (minus) {
-      if (sm != (size_t)h->ldg || nk != h->d.ngl || nm != h->d.nbh)
-        return h->fail(CUW_ERR_UNSUPPORTED, "X(-k) Gram product of a non wave-function array");
-      int slot = -1;
-      for (int j = 0; j < 2; ++j)
-        if (src[j] == x) slot = j;
-      if (slot < 0) {
-        slot = src[0] ? 1 : 0;
-        if (src[slot]) return h->fail(CUW_ERR_UNSUPPORTED, "more than two X arrays in one Gram call");
-        src[slot] = x;
-        CUW_RET(tc_minus(h, x, slot, &mcopy[slot]));
-      }
-      CUW_RET(map_c(h, &tm.xm[i], mcopy[slot], nk, nm, (long long)sm, 16, 64, CU_TENSOR_MAP_SWIZZLE_128B));
-    }
+  a.nk = 2 * h->nh;
+  a.nrow = a.ncol = a.ldp = nb;
+  a.tps = tps;
+  a.nchk = ceil_div(a.nk, kCK);
+  TcTnMaps tm;
+  for (int i = 0; i < 3; ++i) {
+    const FoldPair& q = pairs[std::min(i, npair - 1)];
+    CUW_RET(map_kfast(h, &tm.a[i], u32_slot(h, q.x), nb));
+    a.bs[i] = h->g.bpre + (size_t)q.y * tps * a.nchk * kBTile;
   }
-  for (int i = npair; i < 3; ++i) {
-    tm.x[i] = tm.xm[i] = tm.x[0];
-    a.ybs[i] = a.ybs[0];
-  }
-  const int tiles = ceil_div(nm, 64) * ceil_div(nm, 64) * npair;
-  int ks = tc_splits(h, tiles, nk, h->split_gram);
-  a.kchunk = ceil_div(ceil_div(nk, ks), kCK) * kCK;
-  ks = ceil_div(nk, a.kchunk);
-  const size_t mn = (size_t)nm * nm;
-  CUW_RET(ensure_part(h, sizeof(float2) * mn * 2 * npair * ks));
-  float2* part = reinterpret_cast<float2*>(h->g.part);
-  const dim3 grid(ceil_div(nm, 64), ceil_div(nm, 64), ks * npair);
-  if (minus) k_tc_gram<true><<<grid, kThreads, GramPipe::kSmem, h->stream>>>(a, tm, part, tc_err(h));
-  else k_tc_gram<false><<<grid, kThreads, GramPipe::kSmem, h->stream>>>(a, tm, part, tc_err(h));
-  CUW_LAUNCH_CHECK("k_tc_gram");
-  return tc_reduce(h, part, ks, mn * 2 * npair, scale, dst);
+  int ks = tc_splits(h, tps * tps * npair, a.nk, h->split_gram);
+  a.kchunk = ceil_div(ceil_div(a.nk, ks), kCK) * kCK;
+  ks = ceil_div(a.nk, a.kchunk);
+  // the one-centre sums stay in FP64, behind the fp32 partials
+  const size_t n = (size_t)nb * nb * npair;
+  const int kc = fold_oc_splits(h, npair);
+  const size_t off = (sizeof(float) * n * ks + 255) / 256 * 256;
+  CUW_RET(ensure_part(h, off + sizeof(double) * n * kc));
+  double* oc = reinterpret_cast<double*>(reinterpret_cast<char*>(h->g.part) + off);
+  CUW_RET(fold_oc(h, pairs, npair, kc, oc));
+  k_tc_tn<GramPipe><<<dim3(tps, tps, ks * npair), kThreads, GramPipe::kSmem, h->stream>>>(
+      a, tm, reinterpret_cast<float*>(h->g.part), tc_err(h));
+  CUW_LAUNCH_CHECK("k_tc_tn");
+  k_tc_gram_sum<<<(unsigned)((n / 2 + 127) / 128), 128, 0, h->stream>>>(reinterpret_cast<const float2*>(h->g.part), ks,
+                                                                        reinterpret_cast<const double2*>(oc), kc, nb,
+                                                                        npair, 0.5 * h->gweight, o0, o1, o2);
+  CUW_LAUNCH_CHECK("k_tc_gram_sum");
+  return CUW_OK;
 }
 
-int tc_addx(Handle* h, bool xminus, double2* out, const double2* x, const double2* l1, const double2* l2, int nm,
-            int nn, int nk, size_t sxm, size_t sxk, size_t som, size_t son) {
-  TcAddXArgs a;
-  a.out = out;
-  a.nm = nm;
-  a.nn = nn;
-  a.nk = nk;
-  a.som = som;
-  a.son = son;
-  a.mfast = sxm == 1;
-  a.nchk = ceil_div(2 * nk, kCK);
-  TcAddXMaps tm;
-  if (a.mfast) {
-    const double2* x2 = x;
-    if (xminus) {
-      if (sxk != (size_t)h->ldg || nm != h->d.ngl || nk != h->d.nbh)
-        return h->fail(CUW_ERR_UNSUPPORTED, "X(-G) update of a non wave-function array");
-      CUW_RET(tc_minus(h, x, 0, &x2));
-    }
-    CUW_RET(map_c(h, &tm.x, x, nm, nk, (long long)sxk, 256, 8, CU_TENSOR_MAP_SWIZZLE_NONE));
-    CUW_RET(map_c(h, &tm.x2, x2, nm, nk, (long long)sxk, 256, 8, CU_TENSOR_MAP_SWIZZLE_NONE));
-  } else {
-    if (sxk != 1 || xminus) return h->fail(CUW_ERR_UNSUPPORTED, "projection update with gathered rows");
-    CUW_RET(map_c(h, &tm.x, x, nk, nm, (long long)sxm, 16, 128, CU_TENSOR_MAP_SWIZZLE_128B));
-    tm.x2 = tm.x;
-  }
-  BSplitSrc b{3, l1, l2, (long long)nk, nn, 2 * nk, nk};
-  CUW_RET(tc_bsplit_small(h, b, ceil_div(nn, 64), a.nchk, 0, &a.lbs));
-  const dim3 grid(ceil_div(nm, 128), ceil_div(nn, 64));
-  k_tc_addx<<<grid, kThreads, AddxPipe::kSmem, h->stream>>>(a, tm, tc_err(h));
+int tc_addx(Handle* h, int slot, const double* lam, double2* out) {
+  const int nb = h->d.nb, nchk = ceil_div(nb, kCK);
+  CUtensorMap tu;
+  CUW_RET(map_mfast(h, &tu, u32_slot(h, slot), nb));
+  BSplitSrc b{};
+  b.kind = 1;
+  b.x = lam;
+  b.ld = nb;
+  b.nrow = nb;
+  b.nk = nb;
+  CUW_RET(tc_bsplit(h, b, ceil_div(nb, 128), nchk, h->g.bsmall));
+  const dim3 grid(ceil_div(2 * h->nh, 128), ceil_div(nb, 128));
+  k_tc_addx<<<grid, kThreads, AddxPipe::kSmem, h->stream>>>(out, h->g.half, h->nh, h->ldg, h->d.nbh, nchk, h->g.bsmall,
+                                                            tu, tc_err(h));
   CUW_LAUNCH_CHECK("k_tc_addx");
   return CUW_OK;
 }
 
+// force partial sums of slot 0 with E = ded; *ntile row tiles
 int tc_force(Handle* h, const double2* ded, double* fpart, int* ntile) {
-  const int ngl = h->d.ngl, nbh = h->d.nbh, npro = h->npro;
-  const int tm = ceil_div(ngl, 128), tn = ceil_div(npro, 64);
-  CUtensorMap tps;
-  CUW_RET(map_c(h, &tps, h->g.psi0, ngl, nbh, h->ldg, 256, 8, CU_TENSOR_MAP_SWIZZLE_NONE));
-  const int nchk = ceil_div(nbh, kCK);
-  const float* be = nullptr;
-  BSplitSrc b{2, ded, nullptr, (long long)nbh, npro, nbh, 0};
-  CUW_RET(tc_bsplit_small(h, b, tn, nchk, 0, &be));
+  const Device& g = h->g;
+  const int nb = h->d.nb, npro = h->npro;
+  const int tm = ceil_div(2 * h->nh, 128), tn = ceil_div(npro, 128);
+  CUtensorMap tu;
+  CUW_RET(map_mfast(h, &tu, u32_slot(h, 0), nb));
+  const int nchk = ceil_div(nb, kCK);
+  BSplitSrc b{};
+  b.kind = 1;
+  b.x = reinterpret_cast<const double*>(ded);
+  b.ld = nb;
+  b.nrow = npro;
+  b.nk = nb;
+  CUW_RET(tc_bsplit(h, b, tn, nchk, g.bsmall));
+  *ntile = tm;
   if (nchk % 2 == 0 && nchk <= kFMaxChunks) {
-    // persistent form: the psi0 tile stays in tensor memory across projector tiles
+    // persistent form: the U tile stays in tensor memory across projector tiles
     const int nitems = tm * tn;
     k_tc_force_p<<<std::min(nitems, h->nsm), kThreads, kForcePSmem, h->stream>>>(
-        tps, be, nchk, ngl, npro, h->ldg, tn, nitems, h->g.pf, h->g.gx, h->g.gy, h->g.gz, fpart, tc_err(h));
+        tu, g.bsmall, nchk, h->nh, npro, h->ldu, tn, nitems, g.pf, g.half, g.gx, g.gy, g.gz, fpart, tc_err(h));
     CUW_LAUNCH_CHECK("k_tc_force_p");
-    *ntile = tm;
     return CUW_OK;
   }
-  k_tc_force<<<dim3(tm, tn), kThreads, ForcePipe::kSmem, h->stream>>>(tps, be, nchk, ngl, nbh, npro, h->g.pdesc,
-                                                                      h->g.ylm, h->g.pro, h->g.eigr, h->g.gx,
-                                                                      h->g.gy, h->g.gz, fpart, tc_err(h));
+  k_tc_force<<<dim3(tm, tn), kThreads, ForcePipe::kSmem, h->stream>>>(tu, g.bsmall, nchk, h->nh, npro, h->ldu, g.pf,
+                                                                     g.half, g.gx, g.gy, g.gz, fpart, tc_err(h));
   CUW_LAUNCH_CHECK("k_tc_force");
-  *ntile = tm;
   return CUW_OK;
 }
 

@@ -88,12 +88,8 @@ int grid_room(Handle* h, int bands) {
 // solve's scratch matrices)
 int overlaps(Handle* h) {
   Device& g = h->g;
-  if (h->tc_on()) {
-    const GramPair p[3] = {{g.psi0, g.psi0}, {g.psim, g.psi0}, {g.psim, g.psim}};
-    return tc_gram(h, p, 3, true, h->d.ngl, h->d.nbh, 1, (size_t)h->ldg, h->gweight, g.tmat);
-  }
-  CUW_RET(fold_room(h));
   const FoldPair p[3] = {{0, 0, g.pbuf, g.pbuf}, {1, 0, g.pbuf, g.pbuf}, {1, 1, g.pbuf, g.pbuf}};
+  if (h->tc_on()) return tc_gram(h, p, 3, g.mat, g.omat, g.oomat);
   return fold_gram(h, p, 3, g.mat, g.omat, g.oomat);
 }
 
@@ -119,7 +115,6 @@ int autotune(Handle* h, double* out, int n) {
     CUW_RET(grid_room(h, c.batch));
     CUW_RET(fft_set_variant(h, c.fft_variant));
     h->dmma_tiles = c.dmma_tiles != 0;
-    CUW_RET(fold_rooms(h));
   } else {
     CUW_RET(eigr_compute(h, g.r0));
     // FFT band batch: the L2 rule's batch and even splits of the bands
