@@ -10,8 +10,8 @@
 // B200 layout: three kernels per band batch.
 //   gtor_plane : sphere -> xy-plane in shared memory, x then y transforms,
 //                plane written to the work grid (only occupied planes).
-//   zcol_v     : z columns of 16 x-points: inverse z transform, V(r) and the
-//                1/N scale, forward z transform, in shared memory.
+//   zcol       : z columns: inverse z transform, V(r) and the 1/N scale, forward
+//                z transform, between registers and one shared-memory tile.
 //   rtog_plane : forward y then x transforms of a plane, gathered back onto
 //                the sphere with 1/2|G|^2 (+bucket) psi added.
 // Each 1-D transform is a mixed-radix Stockham autosort (radix 2,3,4,5,7,8,11)
@@ -148,28 +148,157 @@ struct Bfly<8> {
   }
 };
 
-// generic prime radix through the twiddle table of the axis (tw[k] = W_N^k)
+// cos and sin of 2 pi k / R, k = 0 .. R/2, of the butterflies whose twiddles
+// are not handled above
 template <int R>
-struct BflyGeneric {
+__host__ __device__ constexpr double root_c(int k) {
+  constexpr double c7[4] = {1.0, 0.623489801858733530525, -0.222520933956314404288, -0.900968867902419126236};
+  constexpr double c9[5] = {1.0, 0.766044443118978035202, 0.173648177666930348851, -0.5, -0.939692620785908384054};
+  constexpr double c11[6] = {1.0, 0.841253532831181168861, 0.415415013001886425529, -0.142314838273285140443,
+                             -0.654860733945285064056, -0.959492973614497389890};
+  constexpr double c16[9] = {1.0, 0.923879532511286756128, 0.707106781186547524400, 0.382683432365089771728, 0.0,
+                             -0.382683432365089771728, -0.707106781186547524400, -0.923879532511286756128, -1.0};
+  return R == 7 ? c7[k] : (R == 9 ? c9[k] : (R == 11 ? c11[k] : c16[k]));
+}
+template <int R>
+__host__ __device__ constexpr double root_s(int k) {
+  constexpr double s7[4] = {0.0, 0.781831482468029808708, 0.974927912181823607018, 0.433883739117558120476};
+  constexpr double s9[5] = {0.0, 0.642787609686539326323, 0.984807753012208059367, 0.866025403784438646764,
+                            0.342020143325668733044};
+  constexpr double s11[6] = {0.0, 0.540640817455597582108, 0.909631995354518371412, 0.989821441880932732377,
+                             0.755749574354258283774, 0.281732556841429697711};
+  constexpr double s16[9] = {0.0, 0.382683432365089771728, 0.707106781186547524400, 0.923879532511286756128, 1.0,
+                             0.923879532511286756128, 0.707106781186547524400, 0.382683432365089771728, 0.0};
+  return R == 7 ? s7[k] : (R == 9 ? s9[k] : (R == 11 ? s11[k] : s16[k]));
+}
+
+// odd prime radix: the symmetric and antisymmetric sums of v[q], v[R-q] with
+// real constants
+template <int R>
+struct BflyPrime {
   template <class C>
-  __device__ __forceinline__ static void run(C (&v)[R], typename CT<C>::R, const C* tw, int n) {
-    C out[R];
-    const int step = n / R;
+  __device__ __forceinline__ static void run(C (&v)[R], typename CT<C>::R sgn, const C*, int) {
+    using T = typename CT<C>::R;
+    constexpr int H = R / 2;
+    C p[H], m[H];
+    const C a = v[0];
+    C t = a;
 #pragma unroll
-    for (int s = 0; s < R; ++s) {
-      C acc = v[0];
-#pragma unroll
-      for (int q = 1; q < R; ++q) acc = cadd(acc, cmul(v[q], tw[((q * s) % R) * step]));
-      out[s] = acc;
+    for (int q = 0; q < H; ++q) {
+      p[q] = cadd(v[q + 1], v[R - 1 - q]);
+      m[q] = csub(v[q + 1], v[R - 1 - q]);
+      t = cadd(t, p[q]);
     }
+    v[0] = t;
 #pragma unroll
-    for (int s = 0; s < R; ++s) v[s] = out[s];
+    for (int k = 1; k <= H; ++k) {
+      C r = a, i = CT<C>::mk(0, 0);
+#pragma unroll
+      for (int q = 1; q <= H; ++q) {
+        const int e = (q * k) % R, f = e <= H ? e : R - e;
+        const T c = (T)root_c<R>(f), d = (T)(e <= H ? root_s<R>(f) : -root_s<R>(f));
+        r.x += c * p[q - 1].x;
+        r.y += c * p[q - 1].y;
+        i.x += d * m[q - 1].x;
+        i.y += d * m[q - 1].y;
+      }
+      i = mul_i(i, sgn);
+      v[k] = cadd(r, i);
+      v[R - k] = csub(r, i);
+    }
   }
 };
 template <>
-struct Bfly<7> : BflyGeneric<7> {};
+struct Bfly<7> : BflyPrime<7> {};
 template <>
-struct Bfly<11> : BflyGeneric<11> {};
+struct Bfly<11> : BflyPrime<11> {};
+
+// radix A*B with coprime A and B, without twiddles: element (B a + A b) mod R
+// of the input and element k = (ka mod A, kb mod B) of the output
+template <int A, int B>
+__host__ __device__ constexpr int crt(int ka, int kb) {
+  for (int k = 0; k < A * B; ++k)
+    if (k % A == ka && k % B == kb) return k;
+  return 0;
+}
+template <int A, int B>
+struct BflyCoprime {
+  template <class C>
+  __device__ __forceinline__ static void run(C (&v)[A * B], typename CT<C>::R sgn, const C*, int) {
+    constexpr int R = A * B;
+    C y[B][A];
+#pragma unroll
+    for (int b = 0; b < B; ++b) {
+#pragma unroll
+      for (int a = 0; a < A; ++a) y[b][a] = v[(B * a + A * b) % R];
+      Bfly<A>::run(y[b], sgn, (const C*)nullptr, 0);
+    }
+#pragma unroll
+    for (int a = 0; a < A; ++a) {
+      C z[B];
+#pragma unroll
+      for (int b = 0; b < B; ++b) z[b] = y[b][a];
+      Bfly<B>::run(z, sgn, (const C*)nullptr, 0);
+#pragma unroll
+      for (int b = 0; b < B; ++b) v[crt<A, B>(a, b)] = z[b];
+    }
+  }
+};
+template <>
+struct Bfly<6> : BflyCoprime<2, 3> {};
+template <>
+struct Bfly<10> : BflyCoprime<2, 5> {};
+template <>
+struct Bfly<12> : BflyCoprime<4, 3> {};
+
+// radix Q*Q with constant twiddles
+template <int Q>
+struct BflySquare {
+  template <class C>
+  __device__ __forceinline__ static void run(C (&v)[Q * Q], typename CT<C>::R sgn, const C*, int) {
+    using T = typename CT<C>::R;
+    constexpr int R = Q * Q;
+    C y[Q][Q];
+#pragma unroll
+    for (int b = 0; b < Q; ++b) {
+#pragma unroll
+      for (int a = 0; a < Q; ++a) y[b][a] = v[b + Q * a];
+      Bfly<Q>::run(y[b], sgn, (const C*)nullptr, 0);
+#pragma unroll
+      for (int a = 1; a < Q; ++a) {
+        if (b == 0) continue;
+        const int e = a * b, f = e <= R / 2 ? e : R - e;
+        const T c = (T)root_c<R>(f), d = (T)(e <= R / 2 ? root_s<R>(f) : -root_s<R>(f));
+        y[b][a] = cmul(y[b][a], CT<C>::mk(c, sgn * d));
+      }
+    }
+#pragma unroll
+    for (int a = 0; a < Q; ++a) {
+      C z[Q];
+#pragma unroll
+      for (int b = 0; b < Q; ++b) z[b] = y[b][a];
+      Bfly<Q>::run(z, sgn, (const C*)nullptr, 0);
+#pragma unroll
+      for (int b = 0; b < Q; ++b) v[a + Q * b] = z[b];
+    }
+  }
+};
+template <>
+struct Bfly<9> : BflySquare<3> {};
+template <>
+struct Bfly<16> : BflySquare<4> {};
+
+// N = r1 * r2 (r1 <= r2) with the two factors as even as the butterflies allow
+// (both at most 12, or 8 x 16); {0, 0} when N has no such split
+struct Split2 {
+  int r1, r2;
+};
+__host__ __device__ constexpr bool has_bfly(int r) { return (r >= 2 && r <= 12) || r == 16; }
+__host__ __device__ constexpr Split2 split2(int N) {
+  for (int a = 12; a >= 2; --a)
+    if (N % a == 0 && a <= N / a && has_bfly(N / a)) return Split2{a, N / a};
+  return Split2{0, 0};
+}
 
 // One Stockham stage on lines [line0, line0+nl) of length n held in shared
 // memory: element e of line L lives at buf[L*ls + e*es].  tw[k] = exp(sgn*2 pi i k/n).
@@ -239,9 +368,7 @@ struct AxisArg {
 //   bit 0: 16 instead of 8 complex values per thread and stage (more lines
 //          per pass, fewer barrier-separated passes, more registers);
 //   bit 1: the radix stages in ascending instead of descending order;
-//   bit 2: on 64^3 grids, the z transforms exchange values between the lanes
-//          of a column by warp shuffles instead of shared memory (k_zcol_v64).
-// Variants 0, 1 and 2 are V = 0, 1, 2; variant 3 is V = 4 (64^3 grids only).
+// Variants 0, 1 and 2 are V = 0, 1, 2; 64^3 grids have variant 3, both bits.
 // ---------------------------------------------------------------------------
 struct RadixList {
   int n;
@@ -486,20 +613,14 @@ __global__ void __launch_bounds__(kPlaneThreads, 2)
   for (int i = threadIdx.x; i < npl; i += blockDim.x) dst[i] = plane[i + row_of<N1>(i, nr1)];
 }
 
-constexpr int kTX = 16;  // x columns per z-column block, generic kernels
-// x columns per z-column block of a grid with compile-time lengths: a whole x
-// row up to 64 (fewer when the z lines are long, so that two blocks of the FP64
-// tile [N3][TX] still fit an SM), which amortises the block's fixed work
-// (twiddles, plane map, barriers) over more columns
-__host__ __device__ constexpr int tx_of(int n1, int n3) {
-  return n1 == 0 ? kTX : (n1 < 64 ? (n3 * n1 * 16 <= 100000 ? n1 : 32) : (n3 * 64 * 16 <= 100000 ? 64 : 56));
-}
-
-template <class C, int N, int TX>
+// z columns of any length: Stockham stages on a tile of kTX columns of a y row
+constexpr int kTX = 16;
+template <class C>
 __global__ void __launch_bounds__(kPlaneThreads, 2)
     k_zcol_v(C* __restrict__ grid, const double* __restrict__ v, const int* __restrict__ zslot, int nzp, int nr1,
              int nr2, AxisArg a3, const double2* __restrict__ tw3g, double scale) {
   using T = typename CT<C>::R;
+  constexpr int TX = kTX;
   extern __shared__ __align__(16) unsigned char smraw[];
   C* sm = reinterpret_cast<C*>(smraw);
   const int nr3 = a3.n;
@@ -519,7 +640,7 @@ __global__ void __launch_bounds__(kPlaneThreads, 2)
     tile[i] = val;
   }
   __syncthreads();
-  xform<N>(tile, a3, TX, 1, TX, false, tw, (T)1);
+  xform<0>(tile, a3, TX, 1, TX, false, tw, (T)1);
   for (int i = threadIdx.x; i < nr3 * TX; i += blockDim.x) {
     int iz = i / TX, x = i % TX;
     double vv = 0.0;
@@ -530,7 +651,7 @@ __global__ void __launch_bounds__(kPlaneThreads, 2)
   // forward transform: conjugated twiddles
   for (int k = threadIdx.x; k < nr3; k += blockDim.x) tw[k].y = -tw[k].y;
   __syncthreads();
-  xform<N>(tile, a3, TX, 1, TX, false, tw, (T)-1);
+  xform<0>(tile, a3, TX, 1, TX, false, tw, (T)-1);
   for (int i = threadIdx.x; i < nr3 * TX; i += blockDim.x) {
     int iz = i / TX, x = i % TX;
     int s = zslot[iz];
@@ -538,138 +659,180 @@ __global__ void __launch_bounds__(kPlaneThreads, 2)
   }
 }
 
-// z transforms of one y row for a 64^3 grid without block-wide barriers.
-// Each x column is transformed by the 8 lanes t = 0..7 of a warp quarter-group
-// as 64 = 8 x 8 (Cooley-Tukey): a radix-8 DFT over the lane's strided elements
-// x[t + 8r], the twiddles exp(sgn 2 pi i t k1/64), a transpose through the
-// column's own 64 shared-memory slots, and a radix-8 DFT across the lanes, which
-// leaves X[t + 8 k2] in lane t, the same distribution as the input.  V(r) is
-// applied in registers between the G->R and the R->G transforms, so the only
-// block barriers are around the coalesced load and store of the tile.
+// z transforms of lengths N = R1 R2 with both factors in one butterfly: kZX
+// consecutive columns of the xy plane per block (whatever rows they lie in),
+// one column per lane, and R2 warps.  Warp t takes x[t + R2 r] from the work
+// grid into registers, a radix-R1 butterfly and the twiddles, and leaves
+// element (k1, t) in shared memory; warp k1 reads its row (k1, .), and after a
+// radix-R2 butterfly holds X[k1 + R1 k2] = psi(z).  V(r) is applied there in
+// registers, and the R->G transform runs the same two steps backwards: radix R2
+// over k2, twiddles, the same row of slots, and warp m1's radix-R1 butterfly
+// gives x[m1 + R2 m2], which goes straight to the work grid.  Shared memory is
+// crossed twice and there are two barriers a band; every slot is written by the
+// thread that read it last, so the next band needs no barrier of its own.
+// V of the block's columns stays in registers over the `nbb` bands of a block.
 //
-// Shared-memory banks: the tile's row stride kZ64Ld = 68 and the rotated slot
-// order of the transpose ((t + k1) mod 8) put the lanes of one wavefront
-// (8 lanes of 16 bytes, or 16 lanes of 8 bytes) on different bank groups in
-// every access.
-constexpr int kZ64Ld = 68;
-constexpr int kZ64Smem = 64 * kZ64Ld + 2 * 64;  // elements: tile and two twiddle tables
-// bytes of shared memory of k_zcol_v64<C>: the elements above and the y row of
-// V(r) * scale as [64 z][kZ64Ld] real numbers of the work-grid precision
+// What bounds it: the work grid's bytes from L2 (the batch is sized for it)
+// and the barriers' latency, hidden by 2 to 4 blocks an SM.  The Stockham
+// stages that it replaces crossed shared memory once more for every radix and
+// for the copies in and out, with two block barriers each: 32 bands of 72^3 in
+// FP32 took 384 us and take 42, of 64^3 69 (by a kernel of its own) and 62; a
+// whole CP step of Si128 (56 x 56 x 110, FP64) 12.6 ms and 11.0 ms.
+constexpr int kZX = 32;
+template <int N>
+constexpr int kZThreads = kZX * split2(N).r2;
+// blocks an SM that the register limit leaves room for: about 64 registers a
+// thread in FP32 and 128 in FP64
+template <class C, int N>
+constexpr int kZBlocks = ((sizeof(C) == 8 ? 1024 : 512) + kZThreads<N> / 4) / kZThreads<N>;
+
+// shared memory of a z kernel with TX columns: tile, twiddles, plane offsets
 template <class C>
-constexpr int z64_smem_bytes() { return kZ64Smem * (int)sizeof(C) + 64 * kZ64Ld * (int)sizeof(typename CT<C>::R); }
+constexpr int z_smem(int n, int tx) { return (int)((n * tx + n) * sizeof(C) + n * sizeof(int)); }
 
-// b[j] = a[(j + sh) & 7] (sh = +-t) for a run-time shift, by three stages of
-// selects: the register indices stay compile-time constants
-template <class C>
-__device__ __forceinline__ void rot8(C (&a)[8], int sh) {
-#pragma unroll
-  for (int bit = 1; bit < 8; bit <<= 1) {
-    const bool on = (sh & bit) != 0;
-    C b[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) b[j] = on ? a[(j + bit) & 7] : a[j];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) a[j] = b[j];
-  }
-}
-__device__ __forceinline__ float2 shfl_c(float2 v, int src) {
-  return make_float2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
-}
-__device__ __forceinline__ double2 shfl_c(double2 v, int src) {
-  return make_double2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
-}
-
-// on entry a[r] = x[t + 8r]; on exit a[k] = X[t + 8k], X[k] = sum_n x[n] tw[nk mod 64]
-// with tw[k] = exp(sgn 2 pi i k/64).  Between the two radix-8 DFTs the 8 x 8
-// transpose among the column's lanes (lane t then holds element t of every
-// lane): through the column's shared-memory slots col[q * kZ64Ld], or (SHFL)
-// by warp shuffles among the 8 lanes, which are `lane0 + 4 t` of the warp:
-// round r sends element (t - r) mod 8 to lane (t - r) mod 8 and receives
-// element t of lane (t + r) mod 8; the array is rotated by t before and after
-// so that every round uses a fixed register.
-template <class C, bool SHFL>
-__device__ __forceinline__ void z64(C (&a)[8], C* col, int t, const C* tw, typename CT<C>::R sgn) {
-  Bfly<8>::run(a, sgn, tw, 64);
-#pragma unroll
-  for (int k1 = 1; k1 < 8; ++k1) a[k1] = cmul(a[k1], tw[t * k1]);
-  if constexpr (SHFL) {
-    const int lane = threadIdx.x & 31, l0 = lane & 3;
-    rot8(a, t);  // a[j] = old a[(j + t) mod 8]
-    C b[8];
-#pragma unroll
-    for (int r = 0; r < 8; ++r) {
-      // send old a[(t - r) mod 8] = rotated a[(-r) mod 8]
-      const C v = a[(8 - r) & 7];
-      b[r] = shfl_c(v, l0 + 4 * ((t + r) & 7));  // element t of lane (t + r) mod 8
-    }
-    // b[r] holds element t of lane (t + r) mod 8: a[n1] = b[(n1 - t) mod 8]
-#pragma unroll
-    for (int j = 0; j < 8; ++j) a[j] = b[j];
-    rot8(a, 8 - t);
-  } else {
-    __syncwarp();  // the lanes' earlier reads of the slots are done
-#pragma unroll
-    for (int k1 = 0; k1 < 8; ++k1) col[(k1 * 8 + ((t + k1) & 7)) * kZ64Ld] = a[k1];
-    __syncwarp();
-#pragma unroll
-    for (int n1 = 0; n1 < 8; ++n1) a[n1] = col[(t * 8 + ((n1 + t) & 7)) * kZ64Ld];
-  }
-  Bfly<8>::run(a, sgn, tw, 64);
-}
-
-template <class C, bool SHFL>
-__global__ void __launch_bounds__(kPlaneThreads, 2)
-    k_zcol_v64(C* __restrict__ grid, const double* __restrict__ v, const int* __restrict__ zslot, int nzp, int nr2,
-               const double2* __restrict__ tw3g, double scale) {
+template <class C, int N>
+__global__ void __launch_bounds__(kZThreads<N>, kZBlocks<C, N>)
+    k_zcol(C* __restrict__ grid, const double* __restrict__ v, const int* __restrict__ zslot, int nzp, int npl,
+           const double2* __restrict__ tw3g, double scale, int nb, int nbb) {
   using T = typename CT<C>::R;
+  constexpr int R1 = split2(N).r1, R2 = split2(N).r2;
   extern __shared__ __align__(16) unsigned char smraw[];
-  C* sm = reinterpret_cast<C*>(smraw);
-  C* tile = sm;               // [64 z][kZ64Ld], x columns 0..63
-  C* twp = sm + 64 * kZ64Ld;  // exp(+2 pi i k/64)
-  C* twm = twp + 64;          // exp(-2 pi i k/64)
-  T* vrow = reinterpret_cast<T*>(twm + 64);  // [64 z][kZ64Ld]: V(x, iy, z) * scale
-  const int iy = blockIdx.x, bl = blockIdx.y;
-  const size_t npl = (size_t)64 * nr2;
-  C* gb = grid + (size_t)bl * nzp * npl;
-  load_tw(twp, tw3g, 64, +1.0);
-  load_tw(twm, tw3g, 64, -1.0);
-  for (int i = threadIdx.x; i < 64 * 64; i += blockDim.x) {
-    const int iz = i >> 6, x = i & 63, s = zslot[iz];
-    tile[iz * kZ64Ld + x] = s >= 0 ? gb[(size_t)s * npl + (size_t)iy * 64 + x] : CT<C>::mk(0, 0);
-    vrow[iz * kZ64Ld + x] = (T)(v[(size_t)x + 64 * ((size_t)iy + (size_t)nr2 * iz)] * scale);
+  C* buf = reinterpret_cast<C*>(smraw);  // [R1][R2][kZX]
+  C* tw = buf + N * kZX;
+  int* zs = reinterpret_cast<int*>(tw + N);
+  const int x = threadIdx.x % kZX, j = threadIdx.x / kZX;
+  const int c = blockIdx.x * kZX + x;
+  const bool in = c < npl;
+  load_tw(tw, tw3g, N, +1.0);
+  for (int i = threadIdx.x; i < N; i += blockDim.x) zs[i] = zslot[i];
+  T vr[R2];
+  if (j < R1) {
+#pragma unroll
+    for (int k = 0; k < R2; ++k) vr[k] = in ? (T)(v[(size_t)(j + R1 * k) * npl + c] * scale) : (T)0;
   }
   __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int t = lane >> 2, l = lane & 3;
-  for (int round = 0; round < 2; ++round) {  // 8 warps x 2 rounds x 4 columns
-    const int x = warp * 8 + round * 4 + l;
-    C* col = tile + x;
-    C a[8];
+  const int b1 = min(nb, ((int)blockIdx.y + 1) * nbb);
+  for (int bl = blockIdx.y * nbb; bl < b1; ++bl) {
+    C* gb = grid + (size_t)bl * nzp * npl + c;
+    C a[R1];
 #pragma unroll
-    for (int r = 0; r < 8; ++r) a[r] = col[(t + 8 * r) * kZ64Ld];
-    z64<C, SHFL>(a, col, t, twp, (T)1);
+    for (int r = 0; r < R1; ++r) {
+      const int s = zs[j + R2 * r];
+      a[r] = in && s >= 0 ? gb[(size_t)s * npl] : CT<C>::mk(0, 0);
+    }
+    Bfly<R1>::run(a, (T)1, (const C*)nullptr, 0);
+    C* slot = buf + j * kZX + x;
+    slot[0] = a[0];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) a[k] = cscale(a[k], vrow[(t + 8 * k) * kZ64Ld + x]);
-    z64<C, SHFL>(a, col, t, twm, (T)-1);
-    __syncwarp();  // the transpose reads are done before the slots take the result
+    for (int k = 1; k < R1; ++k) slot[k * R2 * kZX] = cmul(a[k], tw[k * j]);
+    __syncthreads();
+    if (j < R1) {
+      C b[R2];
+      C* row = buf + j * R2 * kZX + x;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) col[(t + 8 * k) * kZ64Ld] = a[k];
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < 64 * 64; i += blockDim.x) {
-    const int iz = i >> 6, x = i & 63, s = zslot[iz];
-    if (s >= 0) gb[(size_t)s * npl + (size_t)iy * 64 + x] = tile[iz * kZ64Ld + x];
+      for (int t = 0; t < R2; ++t) b[t] = row[t * kZX];
+      Bfly<R2>::run(b, (T)1, (const C*)nullptr, 0);
+#pragma unroll
+      for (int k = 0; k < R2; ++k) b[k] = cscale(b[k], vr[k]);
+      Bfly<R2>::run(b, (T)-1, (const C*)nullptr, 0);
+      row[0] = b[0];
+#pragma unroll
+      for (int m = 1; m < R2; ++m) row[m * kZX] = cmulc(b[m], tw[m * j]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < R1; ++k) a[k] = slot[k * R2 * kZX];
+    Bfly<R1>::run(a, (T)-1, (const C*)nullptr, 0);
+#pragma unroll
+    for (int m = 0; m < R1; ++m) {
+      const int s = zs[j + R2 * m];
+      if (in && s >= 0) gb[(size_t)s * npl] = a[m];
+    }
   }
 }
 
 // Pseudo density of WAVES_DENSITY (src/paw_waves1.f90:5377-5500) for super
 // wave functions at the Gamma point: after the x/y passes of k_gtor_plane, the
-// G->R z transform of kRhoTX x columns of every band of the batch in turn, and
-// rho(r) += f1 Re(psi)^2 + f2 Im(psi)^2 (= Re[psi (s1 conj psi + s2 psi)] with
-// s1,2 = (f1 +- f2)/2, :5474-5496) in FP64, bands in order, so that the sum is
-// deterministic; `first` starts rho from zero, else the batch adds to it.
-constexpr int kRhoTX = 16;
+// G->R z transform of the block's x columns of every band of the batch in turn,
+// and rho(r) += f1 Re(psi)^2 + f2 Im(psi)^2 (= Re[psi (s1 conj psi + s2 psi)]
+// with s1,2 = (f1 +- f2)/2, :5474-5496) in FP64, bands in order, so that the
+// sum is deterministic; `first` starts rho from zero, else the batch adds to it.
+// Lengths N = R1 R2 take the first two steps of k_zcol, with rho(r) of the
+// thread's points in registers and the next band's elements loaded before the
+// current band's second step; kRhoX columns a block, because the bands are a
+// serial chain and more blocks in flight hide its barriers.
+constexpr int kRhoX = 16;
+template <int N>
+constexpr int kRhoThreads = (kRhoX * split2(N).r2 + 31) / 32 * 32;
+
 template <class C, int N>
+__global__ void __launch_bounds__(kRhoThreads<N>, 2)
+    k_zrho(const C* __restrict__ grid, const int* __restrict__ zslot, int nzp, int npl,
+           const double2* __restrict__ tw3g, const double* __restrict__ occ, int nb, int b0, int nbatch,
+           double* __restrict__ rho, int first) {
+  using T = typename CT<C>::R;
+  constexpr int R1 = split2(N).r1, R2 = split2(N).r2;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  C* buf = reinterpret_cast<C*>(smraw);  // [R1][R2][kRhoX]
+  C* tw = buf + N * kRhoX;
+  int* zs = reinterpret_cast<int*>(tw + N);
+  const int x = threadIdx.x % kRhoX, j = threadIdx.x / kRhoX;
+  const int c = blockIdx.x * kRhoX + x;
+  const bool in = c < npl, one = j < R2, two = j < R1;  // the block is padded to whole warps
+  load_tw(tw, tw3g, N, +1.0);
+  for (int i = threadIdx.x; i < N; i += blockDim.x) zs[i] = zslot[i];
+  double acc[R2];
+#pragma unroll
+  for (int k = 0; k < R2; ++k) acc[k] = !first && in && two ? rho[(size_t)(j + R1 * k) * npl + c] : 0.0;
+  __syncthreads();
+  C a[R1];
+  auto load = [&](int bl) {
+    const C* gb = grid + (size_t)bl * nzp * npl + c;
+#pragma unroll
+    for (int r = 0; r < R1; ++r) {
+      const int s = one ? zs[j + R2 * r] : -1;
+      a[r] = in && s >= 0 ? gb[(size_t)s * npl] : CT<C>::mk(0, 0);
+    }
+  };
+  load(0);
+  for (int bl = 0; bl < nbatch; ++bl) {
+    const int b = b0 + bl;
+    const double f1 = occ[2 * b], f2 = 2 * b + 1 < nb ? occ[2 * b + 1] : 0.0;
+    const bool live = f1 != 0.0 || f2 != 0.0;  // the same for the whole block
+    if (live) {
+      Bfly<R1>::run(a, (T)1, (const C*)nullptr, 0);
+      if (one) {
+        C* slot = buf + j * kRhoX + x;
+        slot[0] = a[0];
+#pragma unroll
+        for (int k = 1; k < R1; ++k) slot[k * R2 * kRhoX] = cmul(a[k], tw[k * j]);
+      }
+    }
+    if (bl + 1 < nbatch) load(bl + 1);
+    if (!live) continue;
+    __syncthreads();
+    if (two) {
+      C d[R2];
+      const C* row = buf + j * R2 * kRhoX + x;
+#pragma unroll
+      for (int t = 0; t < R2; ++t) d[t] = row[t * kRhoX];
+      Bfly<R2>::run(d, (T)1, (const C*)nullptr, 0);
+#pragma unroll
+      for (int k = 0; k < R2; ++k) {
+        const double re = (double)d[k].x, im = (double)d[k].y;
+        acc[k] += f1 * re * re + f2 * im * im;
+      }
+    }
+    __syncthreads();  // the rows are read before the next band writes them
+  }
+#pragma unroll
+  for (int k = 0; k < R2; ++k)
+    if (in && two) rho[(size_t)(j + R1 * k) * npl + c] = acc[k];
+}
+
+// the same for any other length: Stockham stages on a tile of kRhoTX columns
+constexpr int kRhoTX = 16;
+template <class C>
 __global__ void __launch_bounds__(kPlaneThreads, 2)
     k_zcol_rho(const C* __restrict__ grid, const int* __restrict__ zslot, int nzp, int nr1, int nr2, AxisArg a3,
                const double2* __restrict__ tw3g, const double* __restrict__ occ, int nb, int b0, int nbatch,
@@ -706,7 +869,7 @@ __global__ void __launch_bounds__(kPlaneThreads, 2)
       tile[i] = val;
     }
     __syncthreads();
-    xform<N>(tile, a3, TX, 1, TX, false, tw, (T)1);
+    xform<0>(tile, a3, TX, 1, TX, false, tw, (T)1);
 #pragma unroll
     for (int e = 0; e < EPT; ++e) {
       const int i = threadIdx.x + e * blockDim.x;
@@ -834,17 +997,88 @@ bool plan_axis(int n, AxisPlan& p) {
 
 }  // namespace
 
-// out = FFT_RTOG[ V * FFT_GTOR[psi] ] (+ 1/2 G^2 psi + bucket psi when add_kinetic)
-template <class C, int N1, int N2, int N3, int V>
-static int fft_vpsi_t(Handle* h, const double2* psi, double2* out, bool add_kinetic) {
-  constexpr int TX = tx_of(N1, N3);
-  const int nr1 = h->d.nr1, nr2 = h->d.nr2, nr3 = h->d.nr3;
-  const int smem_plane = (int)(((size_t)nr2 * plane_stride(nr1) + nr1 + nr2) * sizeof(C));
-  const int smem_z = (int)(((size_t)nr3 * TX + nr3) * sizeof(C));
-  const int tp = kPlaneThreads;
-  const int tz = kPlaneThreads;
-  AxisArg a1 = make_axis(h->ax[0]), a2 = make_axis(h->ax[1]), a3 = make_axis(h->ax[2]);
+// z lengths with two-step kernels: those of the grids above and the other
+// lengths up to 128 that the grids of larger or finer cells take
+#define CUW_Z_LENGTHS(F)                                                                                     \
+  F(18) F(20) F(24) F(28) F(30) F(32) F(36) F(40) F(42) F(44) F(48) F(50) F(54) F(56) F(60) F(64) F(66) F(70) F(72) \
+  F(80) F(84) F(88) F(90) F(96) F(100) F(108) F(110) F(120) F(128)
+
+// shared-memory limits of the z kernels of this grid (outside any capture)
+template <class C>
+static int z_setup(Handle* h) {
+  const int n = h->d.nr3;
+  switch (n) {
+#define CUW_Z(N)                                                                  \
+  case N:                                                                         \
+    CUW_TRY(smem_allow((const void*)k_zcol<C, N>, z_smem<C>(N, kZX)));              \
+    return smem_allow((const void*)k_zrho<C, N>, z_smem<C>(N, kRhoX)) == cudaSuccess ? CUW_OK : CUW_ERR_CUDA;
+    CUW_Z_LENGTHS(CUW_Z)
+#undef CUW_Z
+    default: break;
+  }
+  CUW_TRY(smem_allow((const void*)k_zcol_v<C>, (int)(((size_t)n * kTX + n) * sizeof(C))));
+  CUW_TRY(smem_allow((const void*)k_zcol_rho<C>, (int)(((size_t)n * kRhoTX + n) * sizeof(C))));
+  return CUW_OK;
+}
+
+// z transforms and V(r) of nb bands of the work grid
+template <class C>
+static int z_vpsi(Handle* h, int nb) {
+  const int nr1 = h->d.nr1, nr2 = h->d.nr2, nr3 = h->d.nr3, npl = nr1 * nr2;
   const double scale = 1.0 / ((double)nr1 * nr2 * nr3);
+  Device& g = h->g;
+  C* grid = reinterpret_cast<C*>(g.grid);
+  // bands per block: V is read once for all of them; up to 4 while the launch
+  // still has eight blocks for every SM
+  const int nx = ceil_div(npl, kZX);
+  const int nbb = std::max(1, std::min(4, nx * nb / (8 * h->nsm)));
+  const dim3 gr(nx, ceil_div(nb, nbb));
+  switch (nr3) {
+#define CUW_Z(N)                                                                                                 \
+  case N:                                                                                                        \
+    k_zcol<C, N><<<gr, kZThreads<N>, z_smem<C>(N, kZX), h->stream>>>(grid, g.v, g.zslot, h->nzp, npl, g.tw3, scale, \
+                                                                     nb, nbb);                                   \
+    break;
+    CUW_Z_LENGTHS(CUW_Z)
+#undef CUW_Z
+    default:
+      k_zcol_v<C><<<dim3(nr2 * ceil_div(nr1, kTX), nb), kPlaneThreads, ((size_t)nr3 * kTX + nr3) * sizeof(C),
+                    h->stream>>>(grid, g.v, g.zslot, h->nzp, nr1, nr2, make_axis(h->ax[2]), g.tw3, scale);
+  }
+  CUW_LAUNCH_CHECK("k_zcol");
+  return CUW_OK;
+}
+
+// z transforms and density of nb bands from band b0
+template <class C>
+static int z_rho(Handle* h, double* rho, int b0, int nb) {
+  const int nr1 = h->d.nr1, nr2 = h->d.nr2, nr3 = h->d.nr3, npl = nr1 * nr2;
+  Device& g = h->g;
+  const C* grid = reinterpret_cast<const C*>(g.grid);
+  switch (nr3) {
+#define CUW_Z(N)                                                                                                     \
+  case N:                                                                                                            \
+    k_zrho<C, N><<<ceil_div(npl, kRhoX), kRhoThreads<N>, z_smem<C>(N, kRhoX), h->stream>>>(                            \
+        grid, g.zslot, h->nzp, npl, g.tw3, g.occ, h->d.nb, b0, nb, rho, b0 == 0);                                      \
+    break;
+    CUW_Z_LENGTHS(CUW_Z)
+#undef CUW_Z
+    default:
+      if (nr3 * kRhoTX > 8 * kPlaneThreads) return h->fail(CUW_ERR_UNSUPPORTED, "density: NR3 above 128");
+      k_zcol_rho<C><<<nr2 * ceil_div(nr1, kRhoTX), kPlaneThreads, ((size_t)nr3 * kRhoTX + nr3) * sizeof(C), h->stream>>>(
+          grid, g.zslot, h->nzp, nr1, nr2, make_axis(h->ax[2]), g.tw3, g.occ, h->d.nb, b0, nb, rho, b0 == 0);
+  }
+  CUW_LAUNCH_CHECK("k_zrho");
+  return CUW_OK;
+}
+
+// out = FFT_RTOG[ V * FFT_GTOR[psi] ] (+ 1/2 G^2 psi + bucket psi when add_kinetic)
+template <class C, int N1, int N2, int V>
+static int fft_vpsi_t(Handle* h, const double2* psi, double2* out, bool add_kinetic) {
+  const int nr1 = h->d.nr1, nr2 = h->d.nr2;
+  const int smem_plane = (int)(((size_t)nr2 * plane_stride(nr1) + nr1 + nr2) * sizeof(C));
+  const int tp = kPlaneThreads;
+  AxisArg a1 = make_axis(h->ax[0]), a2 = make_axis(h->ax[1]);
   Device& g = h->g;
   C* grid = reinterpret_cast<C*>(g.grid);
   for (int b0 = 0; b0 < h->d.nbh; b0 += h->batch) {
@@ -853,16 +1087,7 @@ static int fft_vpsi_t(Handle* h, const double2* psi, double2* out, bool add_kine
                                                                            g.plane_pos, g.plane_rows, grid, h->nzp,
                                                                            a1, a2, g.tw1, g.tw2);
     CUW_LAUNCH_CHECK("k_gtor_plane");
-    if constexpr (N1 == 64 && N3 == 64) {
-      k_zcol_v64<C, (V & 4) != 0><<<dim3(nr2, nb), tz, z64_smem_bytes<C>(), h->stream>>>(grid, g.v, g.zslot, h->nzp, nr2,
-                                                                                 g.tw3, scale);
-      CUW_LAUNCH_CHECK("k_zcol_v64");
-    } else {
-      const int nxb = (nr1 + TX - 1) / TX;
-      k_zcol_v<C, N3, TX><<<dim3(nr2 * nxb, nb), tz, smem_z, h->stream>>>(grid, g.v, g.zslot, h->nzp, nr1, nr2, a3,
-                                                                       g.tw3, scale);
-      CUW_LAUNCH_CHECK("k_zcol_v");
-    }
+    CUW_RET(z_vpsi<C>(h, nb));
     k_rtog_plane<C, N1, N2, V><<<dim3(h->nzp, nb), tp, smem_plane, h->stream>>>(grid, h->nzp, g.plane_off, g.plane_g,
                                                                       g.plane_pos, g.plane_rows, out, psi, h->ldg, b0, g.g2,
                                                                       g.bucket, add_kinetic ? 1 : 0, a1, a2,
@@ -875,59 +1100,49 @@ static int fft_vpsi_t(Handle* h, const double2* psi, double2* out, bool add_kine
 
 // rho = sum over the bands of this set of f |psi(r)|^2 terms (WAVES_DENSITY
 // for TINV at Gamma), batch by batch through the work grid
-template <class C, int N1, int N2, int N3, int V>
+template <class C, int N1, int N2, int V>
 static int fft_density_t(Handle* h, const double2* psi, double* rho) {
-  const int nr1 = h->d.nr1, nr2 = h->d.nr2, nr3 = h->d.nr3;
-  if (nr3 * kRhoTX > 8 * kPlaneThreads) return h->fail(CUW_ERR_UNSUPPORTED, "density: NR3 above 128");
+  const int nr1 = h->d.nr1, nr2 = h->d.nr2;
   const int smem_plane = (int)(((size_t)nr2 * plane_stride(nr1) + nr1 + nr2) * sizeof(C));
-  const int smem_rho = (int)(((size_t)nr3 * kRhoTX + nr3) * sizeof(C));
-  AxisArg a1 = make_axis(h->ax[0]), a2 = make_axis(h->ax[1]), a3 = make_axis(h->ax[2]);
+  AxisArg a1 = make_axis(h->ax[0]), a2 = make_axis(h->ax[1]);
   Device& g = h->g;
   C* grid = reinterpret_cast<C*>(g.grid);
-  const int nxb = (nr1 + kRhoTX - 1) / kRhoTX;
   for (int b0 = 0; b0 < h->d.nbh; b0 += h->batch) {
     const int nb = std::min(h->batch, h->d.nbh - b0);
     k_gtor_plane<C, N1, N2, V><<<dim3(h->nzp, nb), kPlaneThreads, smem_plane, h->stream>>>(
         psi, h->ldg, b0, g.plane_off, g.plane_g, g.plane_pos, g.plane_rows, grid, h->nzp, a1, a2, g.tw1, g.tw2);
     CUW_LAUNCH_CHECK("k_gtor_plane");
-    k_zcol_rho<C, N3><<<nr2 * nxb, kPlaneThreads, smem_rho, h->stream>>>(grid, g.zslot, h->nzp, nr1, nr2, a3, g.tw3,
-                                                                       g.occ, h->d.nb, b0, nb, rho, b0 == 0);
-    CUW_LAUNCH_CHECK("k_zcol_rho");
+    CUW_RET(z_rho<C>(h, rho, b0, nb));
   }
   return CUW_OK;
 }
 
 // kernels of work-grid type C and length N (0: any length): shared-memory
 // limits and the launcher
-template <class C, int N1, int N2, int N3, int V>
+template <class C, int N1, int N2, int V>
 static int fft_select_v(Handle* h, int smem_plane) {
-  constexpr int TX = tx_of(N1, N3);
-  const int smem_z = (int)(((size_t)h->d.nr3 * TX + h->d.nr3) * sizeof(C));
   CUW_TRY(smem_allow((const void*)k_gtor_plane<C, N1, N2, V>, smem_plane));
   CUW_TRY(smem_allow((const void*)k_rtog_plane<C, N1, N2, V>, smem_plane));
-  if constexpr (N1 == 64 && N3 == 64)
-    CUW_TRY(smem_allow((const void*)k_zcol_v64<C, (V & 4) != 0>, z64_smem_bytes<C>()));
-  else CUW_TRY(smem_allow((const void*)k_zcol_v<C, N3, TX>, smem_z));
-  CUW_TRY(smem_allow((const void*)k_zcol_rho<C, N3>, (int)(((size_t)h->d.nr3 * kRhoTX + h->d.nr3) * sizeof(C))));
-  h->fft_run = &fft_vpsi_t<C, N1, N2, N3, V>;
-  h->fft_rho = &fft_density_t<C, N1, N2, N3, V>;
+  CUW_RET(z_setup<C>(h));
+  h->fft_run = &fft_vpsi_t<C, N1, N2, V>;
+  h->fft_rho = &fft_density_t<C, N1, N2, V>;
   return CUW_OK;
 }
 // the plan variant h->fft_variant of a grid with compiled lengths (variant 0
 // for the kernels with run-time lengths)
-template <class C, int N1, int N2, int N3>
+template <class C, int N1, int N2>
 static int fft_select(Handle* h, int smem_plane) {
   if constexpr (N1 > 0) {
     switch (h->fft_variant) {
-      case 1: return fft_select_v<C, N1, N2, N3, 1>(h, smem_plane);
-      case 2: return fft_select_v<C, N1, N2, N3, 2>(h, smem_plane);
+      case 1: return fft_select_v<C, N1, N2, 1>(h, smem_plane);
+      case 2: return fft_select_v<C, N1, N2, 2>(h, smem_plane);
       case 3:
-        if constexpr (N1 == 64 && N3 == 64) return fft_select_v<C, N1, N2, N3, 4>(h, smem_plane);
+        if constexpr (N1 == 64 && N2 == 64) return fft_select_v<C, N1, N2, 3>(h, smem_plane);
         break;
       default: break;
     }
   }
-  return fft_select_v<C, N1, N2, N3, 0>(h, smem_plane);
+  return fft_select_v<C, N1, N2, 0>(h, smem_plane);
 }
 
 // Kernels of the handle's grid and plan variant: grids of the table get
@@ -942,14 +1157,14 @@ static int fft_choose(Handle* h) {
 #define CUW_FFT_GRID(A, B, Z)                                                                        \
   if (!found && nr1 == A && nr2 == B && nr3 == Z) {                                                  \
     found = true;                                                                                    \
-    rc = h->mixed() ? fft_select<float2, A, B, Z>(h, smem_plane) : fft_select<double2, A, B, Z>(h, smem_plane); \
+    rc = h->mixed() ? fft_select<float2, A, B>(h, smem_plane) : fft_select<double2, A, B>(h, smem_plane); \
   }
   CUW_FFT_GRIDS
 #undef CUW_FFT_GRID
   h->fft_compiled = found;
   if (!found) {
     h->fft_variant = 0;
-    rc = h->mixed() ? fft_select<float2, 0, 0, 0>(h, smem_plane) : fft_select<double2, 0, 0, 0>(h, smem_plane);
+    rc = h->mixed() ? fft_select<float2, 0, 0>(h, smem_plane) : fft_select<double2, 0, 0>(h, smem_plane);
   }
   return rc;
 }
@@ -1081,7 +1296,7 @@ int fft_density(Handle* h, const double2* psi, double* rho) {
 
 // plan variant v (0 .. fft_variants()-1) of the compiled kernels; grids with
 // run-time lengths have variant 0 only
-// the shuffle variant (3) changes only the 64-point z kernel
+// variant 3 exists for 64^3 grids only
 static bool z64_grid(const Handle* h) { return h->d.nr1 == 64 && h->d.nr2 == 64 && h->d.nr3 == 64; }
 int fft_variants(const Handle* h) { return !h->fft_compiled ? 1 : (z64_grid(h) ? kFftVariants : kFftVariants - 1); }
 int fft_set_variant(Handle* h, int v) {
