@@ -14,9 +14,11 @@
 //                z transform, between registers and one shared-memory tile.
 //   rtog_plane : forward y then x transforms of a plane, gathered back onto
 //                the sphere with 1/2|G|^2 (+bucket) psi added.
-// Each 1-D transform is a mixed-radix Stockham autosort (radix 2,3,4,5,7,8,11)
-// whose butterflies run in registers; every stage reads all of its inputs into
-// registers before a barrier and writes after it, so it works in place.
+// A 1-D transform of a common length is two butterflies in registers with one
+// exchange through shared memory (N = R1 R2, factors up to 12 or 16); any other
+// length with prime factors up to 11 takes the Stockham stages (radix
+// 2,3,4,5,7,8,11), which read all of their inputs into registers before a
+// barrier and write after it, and so work in place.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -358,23 +360,15 @@ struct AxisArg {
 };
 
 // ---------------------------------------------------------------------------
-// Compile-time specialisation for the common grid lengths: every divisor of
+// Compile-time specialisation of the Stockham stages: every divisor of
 // the index arithmetic is a constant, the stages are inlined and the block
 // size is fixed (kPlaneThreads), so the lines per chunk are constant too.
-// ---------------------------------------------------------------------------
-//
-// Plan variants V (chosen per handle by the autotuner, src/paw_library.f90
-// LIB_FFTW3 leaves the same choice to FFTW's measured planning):
-//   bit 0: 16 instead of 8 complex values per thread and stage (more lines
-//          per pass, fewer barrier-separated passes, more registers);
-//   bit 1: the radix stages in ascending instead of descending order;
-// Variants 0, 1 and 2 are V = 0, 1, 2; 64^3 grids have variant 3, both bits.
 // ---------------------------------------------------------------------------
 struct RadixList {
   int n;
   int r[8];
 };
-__host__ __device__ constexpr RadixList radices_of(int N, int V = 0) {
+__host__ __device__ constexpr RadixList radices_of(int N) {
   RadixList L{0, {0, 0, 0, 0, 0, 0, 0, 0}};
   int m = N;
   const int order[7] = {8, 4, 2, 3, 5, 7, 11};
@@ -383,39 +377,23 @@ __host__ __device__ constexpr RadixList radices_of(int N, int V = 0) {
       L.r[L.n++] = order[i];
       m /= order[i];
     }
-  if (V & 2)
-    for (int a = 0, b = L.n - 1; a < b; ++a, --b) {
-      const int t = L.r[a];
-      L.r[a] = L.r[b];
-      L.r[b] = t;
-    }
   return L;
 }
-__host__ __device__ constexpr int values_of(int V) { return (V & 1) ? 16 : kMaxV; }
-__host__ __device__ constexpr int bpt_v(int r, int mv) { return (mv / r) > 0 ? (mv / r) : 1; }
-__host__ __device__ constexpr int chunk_lines(int N, int V = 0) {
-  RadixList L = radices_of(N, V);
+__host__ __device__ constexpr int chunk_lines(int N) {
+  RadixList L = radices_of(N);
   int lc = 1 << 30;
   for (int s = 0; s < L.n; ++s) {
-    int cap = (kPlaneThreads * bpt_v(L.r[s], values_of(V)) * L.r[s]) / N;
+    int cap = (kPlaneThreads * bpt_of(L.r[s]) * L.r[s]) / N;
     if (cap < 1) cap = 1;
     lc = lc < cap ? lc : cap;
   }
   return lc;
 }
-constexpr int kFftVariants = 4;
 
-// Line l of a transform lives at row (row0 + l) mod nrows of the buffer
-// (row0 = 0 and nrows above every line index: the identity).
-__device__ __forceinline__ int line_row(int l, int row0, int nrows) {
-  const int r = row0 + l;
-  return r >= nrows ? r - nrows : r;
-}
-
-template <int N, int R, int NS, int LC, int MV, class C>
+template <int N, int R, int NS, int LC, class C>
 __device__ __forceinline__ void stage_fixed(C* buf, int line0, int nl, int ls, int es, bool jfast, const C* tw,
-                                            typename CT<C>::R sgn, int row0, int nrows) {
-  constexpr int BPT = bpt_v(R, MV);
+                                            typename CT<C>::R sgn) {
+  constexpr int BPT = bpt_of(R);
   constexpr int NQ = N / R;
   constexpr int TSTEP = N / (NS * R);
   // jfast: index space nl*NQ (line = bf / NQ); otherwise the full chunk LC*NQ
@@ -434,7 +412,7 @@ __device__ __forceinline__ void stage_fixed(C* buf, int line0, int nl, int ls, i
     const int k = j % NS;
     off_[t] = line * N + ((j / NS) * NS * R + k);  // (line, destination index) packed
     if (act[t]) {
-      C* base = buf + (size_t)line_row(line0 + line, row0, nrows) * ls;
+      C* base = buf + (size_t)(line0 + line) * ls;
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         C x = base[(size_t)(j + r * NQ) * es];
@@ -449,7 +427,7 @@ __device__ __forceinline__ void stage_fixed(C* buf, int line0, int nl, int ls, i
   for (int t = 0; t < BPT; ++t) {
     if (act[t]) {
       const int line = off_[t] / N, idxd = off_[t] % N;
-      C* base = buf + (size_t)line_row(line0 + line, row0, nrows) * ls;
+      C* base = buf + (size_t)(line0 + line) * ls;
 #pragma unroll
       for (int r = 0; r < R; ++r) base[(size_t)(idxd + r * NS) * es] = v[t][r];
     }
@@ -457,24 +435,23 @@ __device__ __forceinline__ void stage_fixed(C* buf, int line0, int nl, int ls, i
   __syncthreads();
 }
 
-template <int N, int S, int NS, int LC, int V, class C>
+template <int N, int S, int NS, int LC, class C>
 __device__ __forceinline__ void stages_fixed(C* buf, int line0, int nl, int ls, int es, bool jfast, const C* tw,
-                                             typename CT<C>::R sgn, int row0, int nrows) {
-  constexpr RadixList L = radices_of(N, V);
+                                             typename CT<C>::R sgn) {
+  constexpr RadixList L = radices_of(N);
   if constexpr (S < L.n) {
     constexpr int R = L.r[S];
-    stage_fixed<N, R, NS, LC, values_of(V)>(buf, line0, nl, ls, es, jfast, tw, sgn, row0, nrows);
-    stages_fixed<N, S + 1, NS * R, LC, V>(buf, line0, nl, ls, es, jfast, tw, sgn, row0, nrows);
+    stage_fixed<N, R, NS, LC>(buf, line0, nl, ls, es, jfast, tw, sgn);
+    stages_fixed<N, S + 1, NS * R, LC>(buf, line0, nl, ls, es, jfast, tw, sgn);
   }
 }
 
-template <int N, int V = 0, class C>
-__device__ void transform_fixed(C* buf, int nlines, int ls, int es, bool jfast, const C* tw, typename CT<C>::R sgn,
-                                int row0 = 0, int nrows = 1 << 30) {
-  constexpr int LC = chunk_lines(N, V);
+template <int N, class C>
+__device__ void transform_fixed(C* buf, int nlines, int ls, int es, bool jfast, const C* tw, typename CT<C>::R sgn) {
+  constexpr int LC = chunk_lines(N);
   for (int l0 = 0; l0 < nlines; l0 += LC) {
     const int nl = min(LC, nlines - l0);
-    stages_fixed<N, 0, 1, LC, V>(buf, l0, nl, ls, es, jfast, tw, sgn, row0, nrows);
+    stages_fixed<N, 0, 1, LC>(buf, l0, nl, ls, es, jfast, tw, sgn);
   }
 }
 
@@ -528,26 +505,6 @@ __device__ void transform(C* buf, const AxisArg& ax, int nlines, int ls, int es,
   }
 }
 
-// N > 0: the transform of compile-time length N, inlined alone into the
-// kernel (its registers then fit without spills); N == 0: run-time dispatch.
-template <int N, int V = 0, class C>
-__device__ __forceinline__ void xform(C* buf, const AxisArg& ax, int nlines, int ls, int es, bool jfast,
-                                      const C* tw, typename CT<C>::R sgn) {
-  if constexpr (N > 0) transform_fixed<N, V>(buf, nlines, ls, es, jfast, tw, sgn);
-  else transform(buf, ax, nlines, ls, es, jfast, tw, sgn);
-}
-
-// The x lines of an xy plane restricted to the rows that hold G vectors:
-// rows (y0 + l) mod nr2 for l < ny (the plane's rows form one range of signed
-// y).  The other rows are zero before the G->R transform and are not read
-// after the R->G transform.  Kernels with run-time lengths transform every row.
-template <int N, int V = 0, class C>
-__device__ __forceinline__ void xform_rows(C* buf, const AxisArg& ax, int y0, int ny, int nr2, int ls,
-                                           const C* tw, typename CT<C>::R sgn) {
-  if constexpr (N > 0) transform_fixed<N, V>(buf, ny, ls, 1, false, tw, sgn, y0, nr2);
-  else transform(buf, ax, nr2, ls, 1, false, tw, sgn);
-}
-
 // load twiddles exp(sgn*2 pi i k/n) from the FP64 table exp(+2 pi i k/n)
 template <class C>
 __device__ void load_tw(C* dst, const double2* src, int n, double sgn) {
@@ -574,21 +531,13 @@ __device__ __forceinline__ double2 to_d2(float2 a) { return make_double2((double
 // scattered writes of the first radix-8 stage of the x lines (stride 8
 // elements) hit one bank group eight times.
 __host__ __device__ constexpr int plane_stride(int nr1) { return nr1 + 1; }
-// row index of the dense plane offset i (i / NR1, with a constant divisor when
-// the kernel is specialised for one length)
-template <int N>
-__device__ __forceinline__ int row_of(int i, int nr1) {
-  if constexpr (N > 0) return i / N;
-  else return i / nr1;
-}
-
 // ---------------------------------------------------------------------------
 // The kernels take the work-grid type C (double2 or float2); the sphere
 // coefficients psi/out stay FP64 and are converted at the gather/scatter.
-template <class C, int N1, int N2, int V>
+template <class C>
 __global__ void __launch_bounds__(kPlaneThreads, 2)
-    k_gtor_plane(const double2* __restrict__ psi, int ldg, int b0, const int* __restrict__ plane_off,
-                 const int* __restrict__ plane_g, const int* __restrict__ plane_pos, const int2* __restrict__ plane_rows,
+    k_gtor_any(const double2* __restrict__ psi, int ldg, int b0, const int* __restrict__ plane_off,
+                 const int* __restrict__ plane_g, const int* __restrict__ plane_pos,
                  C* __restrict__ grid, int nzp, AxisArg a1, AxisArg a2, const double2* __restrict__ tw1g,
                  const double2* __restrict__ tw2g) {
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -606,11 +555,10 @@ __global__ void __launch_bounds__(kPlaneThreads, 2)
   for (int k = plane_off[p] + threadIdx.x; k < plane_off[p + 1]; k += blockDim.x)
     plane[plane_pos[k]] = from_d2<C>(src[plane_g[k]]);
   __syncthreads();
-  const int2 rows = plane_rows[p];
-  xform_rows<N1, V>(plane, a1, rows.x, rows.y, nr2, ps, tw1, (typename CT<C>::R)1);  // x lines
-  xform<N2, V>(plane, a2, nr1, 1, ps, false, tw2, (typename CT<C>::R)1);               // y lines
+  transform(plane, a1, nr2, ps, 1, false, tw1, (typename CT<C>::R)1);   // x lines
+  transform(plane, a2, nr1, 1, ps, false, tw2, (typename CT<C>::R)1);   // y lines
   C* dst = grid + ((size_t)bl * nzp + p) * npl;
-  for (int i = threadIdx.x; i < npl; i += blockDim.x) dst[i] = plane[i + row_of<N1>(i, nr1)];
+  for (int i = threadIdx.x; i < npl; i += blockDim.x) dst[i] = plane[i + i / nr1];
 }
 
 // z columns of any length: Stockham stages on a tile of kTX columns of a y row
@@ -640,7 +588,7 @@ __global__ void __launch_bounds__(kPlaneThreads, 2)
     tile[i] = val;
   }
   __syncthreads();
-  xform<0>(tile, a3, TX, 1, TX, false, tw, (T)1);
+  transform(tile, a3, TX, 1, TX, false, tw, (T)1);
   for (int i = threadIdx.x; i < nr3 * TX; i += blockDim.x) {
     int iz = i / TX, x = i % TX;
     double vv = 0.0;
@@ -651,7 +599,7 @@ __global__ void __launch_bounds__(kPlaneThreads, 2)
   // forward transform: conjugated twiddles
   for (int k = threadIdx.x; k < nr3; k += blockDim.x) tw[k].y = -tw[k].y;
   __syncthreads();
-  xform<0>(tile, a3, TX, 1, TX, false, tw, (T)-1);
+  transform(tile, a3, TX, 1, TX, false, tw, (T)-1);
   for (int i = threadIdx.x; i < nr3 * TX; i += blockDim.x) {
     int iz = i / TX, x = i % TX;
     int s = zslot[iz];
@@ -869,7 +817,7 @@ __global__ void __launch_bounds__(kPlaneThreads, 2)
       tile[i] = val;
     }
     __syncthreads();
-    xform<0>(tile, a3, TX, 1, TX, false, tw, (T)1);
+    transform(tile, a3, TX, 1, TX, false, tw, (T)1);
 #pragma unroll
     for (int e = 0; e < EPT; ++e) {
       const int i = threadIdx.x + e * blockDim.x;
@@ -886,11 +834,211 @@ __global__ void __launch_bounds__(kPlaneThreads, 2)
   }
 }
 
+// xy planes of compiled lengths, each axis N = R1 R2 in two register steps that
+// work in place: a thread reads the R1 (then R2) elements of its butterfly from
+// shared memory and writes its results to the same slots, so that a step needs
+// one barrier and no staging.  The digit reversal this leaves is taken out
+// where the values are permuted anyway: x line slot r + R1 t holds x = t + R2 r
+// when the sphere is scattered (k_gtor_plane), and slot R2 k1 + k2 holds
+// x = k1 + R1 k2 when it is gathered (k_rtog_plane).  The last y step of G->R
+// writes the work grid itself, and the first one of R->G reads it, so the plane
+// crosses shared memory three and a half times.  Only the rows that hold G
+// vectors (y0 + l mod N2, l < ny; one range of signed y) are cleared, get x
+// transforms, and are read by the first y step or written by the last.
+//
+// What bounds them: shared-memory passes and the barriers between them (a plane
+// is 33 to 150 KB, so few blocks share an SM).  Before, every radix of a
+// Stockham stage crossed shared memory with two barriers and the plane was
+// copied in and out: 32 bands of 72^3 in FP32, G->R 63.3 -> 28.6 us and R->G
+// 97.0 -> 33.8 us; 16 bands of 72^3 in FP64, G->R 44.7 -> 26.1 us.
+//
+// Plan variants V (chosen per handle by the autotuner; src/paw_library.f90
+// LIB_FFTW3 leaves the same choice to FFTW's measured planning):
+//   bit 0: 512 instead of 256 threads a plane;
+//   bit 1: R1 and R2 exchanged.
+// V = 0 is the default: H|psi> of 32 H2O on 72^3 takes 497, 552 and 498 us with
+// V = 0, 1, 2 in FP64 and 307, 324 and 306 us in mixed precision; the tuner
+// finds the handles where another order of the factors is ahead.
+// Variants 0, 1 and 2 are V = 0, 1, 2; 64^3 grids also have variant 3, both.
+constexpr int kFftVariants = 4;
+__host__ __device__ constexpr int plane_threads(int V) { return (V & 1) ? 2 * kPlaneThreads : kPlaneThreads; }
+template <int N, int V>
+struct Axis2 {
+  static constexpr int R1 = (V & 2) ? split2(N).r2 : split2(N).r1;
+  static constexpr int R2 = (V & 2) ? split2(N).r1 : split2(N).r2;
+};
+// blocks an SM that registers are budgeted for: 64 registers a thread in FP32, 128 in FP64
+template <class C, int V>
+constexpr int kPlaneBlocks = (sizeof(C) == 8 ? 1024 : 512) / plane_threads(V);
+
+// R elements at p, p + st, ..., through a butterfly; element k times exp(sgn 2 pi i k e / N)
+template <int R, class C>
+__device__ __forceinline__ void take(C (&a)[R], const C* p, int st) {
+#pragma unroll
+  for (int r = 0; r < R; ++r) a[r] = p[r * st];
+}
+template <int R, bool TW, class C>
+__device__ __forceinline__ void put(const C (&a)[R], C* p, int st, const C* tw, int e) {
+  p[0] = a[0];
+#pragma unroll
+  for (int k = 1; k < R; ++k) p[k * st] = TW ? cmul(a[k], tw[k * e]) : a[k];
+}
+
 template <class C, int N1, int N2, int V>
-__global__ void __launch_bounds__(kPlaneThreads, 2)
+__global__ void __launch_bounds__(plane_threads(V), kPlaneBlocks<C, V>)
+    k_gtor_plane(const double2* __restrict__ psi, int ldg, int b0, const int* __restrict__ plane_off,
+                 const int* __restrict__ plane_g, const int* __restrict__ plane_pos, const int2* __restrict__ plane_rows,
+                 C* __restrict__ grid, int nzp, const double2* __restrict__ tw1g, const double2* __restrict__ tw2g) {
+  using T = typename CT<C>::R;
+  constexpr int NT = plane_threads(V), PS = plane_stride(N1);
+  constexpr int A1 = Axis2<N1, V>::R1, A2 = Axis2<N1, V>::R2, B1 = Axis2<N2, V>::R1, B2 = Axis2<N2, V>::R2;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  C* plane = reinterpret_cast<C*>(smraw);  // [N2][PS]
+  C* tw1 = plane + N2 * PS;
+  C* tw2 = tw1 + N1;
+  const int p = blockIdx.x, bl = blockIdx.y, b = b0 + bl;
+  const int2 rows = plane_rows[p];
+  const int y0 = rows.x, ny = rows.y;
+  for (int i = threadIdx.x; i < ny * N1; i += NT) {
+    int y = y0 + i / N1;
+    if (y >= N2) y -= N2;
+    plane[y * PS + i % N1] = CT<C>::mk(0, 0);
+  }
+  load_tw(tw1, tw1g, N1, +1.0);
+  load_tw(tw2, tw2g, N2, +1.0);
+  __syncthreads();
+  const double2* src = psi + (size_t)ldg * b;
+  for (int k = plane_off[p] + threadIdx.x; k < plane_off[p + 1]; k += NT) {
+    const int pos = plane_pos[k], x = pos % PS;
+    plane[pos - x + x / A2 + A1 * (x % A2)] = from_d2<C>(src[plane_g[k]]);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < ny * A2; i += NT) {  // x, radix A1
+    const int t = i / ny;
+    int y = y0 + i - t * ny;
+    if (y >= N2) y -= N2;
+    C a[A1], *q = plane + y * PS + A1 * t;
+    take(a, q, 1);
+    Bfly<A1>::run(a, (T)1, (const C*)nullptr, 0);
+    put<A1, true>(a, q, 1, tw1, t);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < ny * A1; i += NT) {  // x, radix A2
+    const int k1 = i / ny;
+    int y = y0 + i - k1 * ny;
+    if (y >= N2) y -= N2;
+    C a[A2], *q = plane + y * PS + k1;
+    take(a, q, A1);
+    Bfly<A2>::run(a, (T)1, (const C*)nullptr, 0);
+    put<A2, false>(a, q, A1, tw1, 0);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < N1 * B2; i += NT) {  // y, radix B1
+    const int t = i / N1, x = i % N1;
+    C a[B1], *q = plane + t * PS + x;
+#pragma unroll
+    for (int r = 0; r < B1; ++r) {
+      int l = t + B2 * r - y0;  // rows outside the range hold nothing
+      if (l < 0) l += N2;
+      a[r] = l < ny ? q[r * B2 * PS] : CT<C>::mk(0, 0);
+    }
+    Bfly<B1>::run(a, (T)1, (const C*)nullptr, 0);
+    put<B1, true>(a, q, B2 * PS, tw2, t);
+  }
+  __syncthreads();
+  C* dst = grid + ((size_t)bl * nzp + p) * (N1 * N2);
+  for (int i = threadIdx.x; i < N1 * B1; i += NT) {  // y, radix B2
+    const int k1 = i / N1, x = i % N1;
+    C a[B2];
+    take(a, plane + k1 * B2 * PS + x, PS);
+    Bfly<B2>::run(a, (T)1, (const C*)nullptr, 0);
+    put<B2, false>(a, dst + k1 * N1 + x, B1 * N1, tw2, 0);
+  }
+}
+
+template <class C, int N1, int N2, int V>
+__global__ void __launch_bounds__(plane_threads(V), kPlaneBlocks<C, V>)
     k_rtog_plane(const C* __restrict__ grid, int nzp, const int* __restrict__ plane_off,
+                 const int* __restrict__ plane_g, const int* __restrict__ plane_pos, const int2* __restrict__ plane_rows,
+                 double2* __restrict__ out, const double2* __restrict__ psi, int ldg, int b0,
+                 const double* __restrict__ g2, const double* __restrict__ bucket, int add_kin,
+                 const double2* __restrict__ tw1g, const double2* __restrict__ tw2g) {
+  using T = typename CT<C>::R;
+  constexpr int NT = plane_threads(V), PS = plane_stride(N1);
+  constexpr int A1 = Axis2<N1, V>::R1, A2 = Axis2<N1, V>::R2, B1 = Axis2<N2, V>::R1, B2 = Axis2<N2, V>::R2;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  C* plane = reinterpret_cast<C*>(smraw);  // [N2][PS]
+  C* tw1 = plane + N2 * PS;
+  C* tw2 = tw1 + N1;
+  const int p = blockIdx.x, bl = blockIdx.y, b = b0 + bl;
+  const int2 rows = plane_rows[p];
+  const int y0 = rows.x, ny = rows.y;
+  load_tw(tw1, tw1g, N1, -1.0);
+  load_tw(tw2, tw2g, N2, -1.0);
+  __syncthreads();
+  const C* srcp = grid + ((size_t)bl * nzp + p) * (N1 * N2);
+  for (int i = threadIdx.x; i < N1 * B2; i += NT) {  // y, radix B1
+    const int t = i / N1, x = i % N1;
+    C a[B1];
+    take(a, srcp + t * N1 + x, B2 * N1);
+    Bfly<B1>::run(a, (T)-1, (const C*)nullptr, 0);
+    put<B1, true>(a, plane + B1 * t * PS + x, PS, tw2, t);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < N1 * B1; i += NT) {  // y, radix B2
+    const int k1 = i / N1, x = i % N1;
+    C a[B2], *q = plane + k1 * PS + x;
+    take(a, q, B1 * PS);
+    Bfly<B2>::run(a, (T)-1, (const C*)nullptr, 0);
+#pragma unroll
+    for (int k = 0; k < B2; ++k) {
+      int l = k1 + B1 * k - y0;  // rows outside the range are not read
+      if (l < 0) l += N2;
+      if (l < ny) q[k * B1 * PS] = a[k];
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < ny * A2; i += NT) {  // x, radix A1
+    const int t = i / ny;
+    int y = y0 + i - t * ny;
+    if (y >= N2) y -= N2;
+    C a[A1], *q = plane + y * PS + t;
+    take(a, q, A2);
+    Bfly<A1>::run(a, (T)-1, (const C*)nullptr, 0);
+    put<A1, true>(a, q, A2, tw1, t);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < ny * A1; i += NT) {  // x, radix A2
+    const int k1 = i / ny;
+    int y = y0 + i - k1 * ny;
+    if (y >= N2) y -= N2;
+    C a[A2], *q = plane + y * PS + A2 * k1;
+    take(a, q, 1);
+    Bfly<A2>::run(a, (T)-1, (const C*)nullptr, 0);
+    put<A2, false>(a, q, 1, tw1, 0);
+  }
+  __syncthreads();
+  double2* dst = out + (size_t)ldg * b;
+  const double2* ps = psi + (size_t)ldg * b;
+  for (int k = plane_off[p] + threadIdx.x; k < plane_off[p + 1]; k += NT) {
+    const int g = plane_g[k], pos = plane_pos[k], x = pos % PS;
+    double2 val = to_d2(plane[pos - x + x / A1 + A2 * (x % A1)]);
+    if (add_kin) {
+      const double kin = 0.5 * g2[g] + (bucket ? bucket[g] : 0.0);
+      const double2 c = ps[g];
+      val.x += kin * c.x;
+      val.y += kin * c.y;
+    }
+    dst[g] = val;
+  }
+}
+
+// planes of any other lengths: Stockham stages on every line
+template <class C>
+__global__ void __launch_bounds__(kPlaneThreads, 2)
+    k_rtog_any(const C* __restrict__ grid, int nzp, const int* __restrict__ plane_off,
                  const int* __restrict__ plane_g, const int* __restrict__ plane_pos,
-                 const int2* __restrict__ plane_rows, double2* __restrict__ out,
+                 double2* __restrict__ out,
                  const double2* __restrict__ psi, int ldg, int b0, const double* __restrict__ g2,
                  const double* __restrict__ bucket, int add_kin, AxisArg a1, AxisArg a2,
                  const double2* __restrict__ tw1g, const double2* __restrict__ tw2g) {
@@ -902,13 +1050,12 @@ __global__ void __launch_bounds__(kPlaneThreads, 2)
   C* tw2 = tw1 + nr1;
   const int p = blockIdx.x, bl = blockIdx.y, b = b0 + bl;
   const C* srcp = grid + ((size_t)bl * nzp + p) * npl;
-  for (int i = threadIdx.x; i < npl; i += blockDim.x) plane[i + row_of<N1>(i, nr1)] = srcp[i];
+  for (int i = threadIdx.x; i < npl; i += blockDim.x) plane[i + i / nr1] = srcp[i];
   load_tw(tw1, tw1g, nr1, -1.0);
   load_tw(tw2, tw2g, nr2, -1.0);
   __syncthreads();
-  xform<N2, V>(plane, a2, nr1, 1, pst, false, tw2, (typename CT<C>::R)-1);  // y lines
-  const int2 rows = plane_rows[p];
-  xform_rows<N1, V>(plane, a1, rows.x, rows.y, nr2, pst, tw1, (typename CT<C>::R)-1);  // x lines
+  transform(plane, a2, nr1, 1, pst, false, tw2, (typename CT<C>::R)-1);  // y lines
+  transform(plane, a1, nr2, pst, 1, false, tw1, (typename CT<C>::R)-1);  // x lines
   double2* dst = out + (size_t)ldg * b;
   const double2* ps = psi + (size_t)ldg * b;
   for (int k = plane_off[p] + threadIdx.x; k < plane_off[p + 1]; k += blockDim.x) {
@@ -947,7 +1094,7 @@ __global__ void __launch_bounds__(kPlaneThreads)
       tile[r * (n + 1) + x] = grid[(size_t)(row0 + r) * nr1 + x];
     }
     __syncthreads();
-    xform<0>(tile, ax, nl, n + 1, 1, false, tw, sgn);
+    transform(tile, ax, nl, n + 1, 1, false, tw, sgn);
     for (int i = threadIdx.x; i < nl * n; i += blockDim.x) {
       const int r = i / n, x = i % n;
       grid[(size_t)(row0 + r) * nr1 + x] = tile[r * (n + 1) + x];
@@ -965,7 +1112,7 @@ __global__ void __launch_bounds__(kPlaneThreads)
     tile[i] = x < nl ? grid[base + (size_t)e * es + x0 + x] : make_double2(0.0, 0.0);
   }
   __syncthreads();
-  xform<0>(tile, ax, TX, 1, TX, false, tw, sgn);
+  transform(tile, ax, TX, 1, TX, false, tw, sgn);
   for (int i = threadIdx.x; i < n * TX; i += blockDim.x) {
     const int e = i / TX, x = i % TX;
     if (x < nl) grid[base + (size_t)e * es + x0 + x] = tile[i];
@@ -1072,57 +1219,81 @@ static int z_rho(Handle* h, double* rho, int b0, int nb) {
   return CUW_OK;
 }
 
+// x and y transforms of the planes of nb bands from band b0, and back
+template <class C, int N1, int N2, int V>
+static int planes_gtor(Handle* h, const double2* psi, int b0, int nb, int smem) {
+  Device& g = h->g;
+  C* grid = reinterpret_cast<C*>(g.grid);
+  const dim3 gr(h->nzp, nb);
+  if constexpr (N1 > 0)
+    k_gtor_plane<C, N1, N2, V><<<gr, plane_threads(V), smem, h->stream>>>(
+        psi, h->ldg, b0, g.plane_off, g.plane_g, g.plane_pos, g.plane_rows, grid, h->nzp, g.tw1, g.tw2);
+  else
+    k_gtor_any<C><<<gr, kPlaneThreads, smem, h->stream>>>(psi, h->ldg, b0, g.plane_off, g.plane_g, g.plane_pos, grid,
+                                                          h->nzp, make_axis(h->ax[0]), make_axis(h->ax[1]), g.tw1,
+                                                          g.tw2);
+  CUW_LAUNCH_CHECK("k_gtor_plane");
+  return CUW_OK;
+}
+template <class C, int N1, int N2, int V>
+static int planes_rtog(Handle* h, const double2* psi, double2* out, int add_kinetic, int b0, int nb, int smem) {
+  Device& g = h->g;
+  const C* grid = reinterpret_cast<const C*>(g.grid);
+  const dim3 gr(h->nzp, nb);
+  if constexpr (N1 > 0)
+    k_rtog_plane<C, N1, N2, V><<<gr, plane_threads(V), smem, h->stream>>>(
+        grid, h->nzp, g.plane_off, g.plane_g, g.plane_pos, g.plane_rows, out, psi, h->ldg, b0, g.g2, g.bucket,
+        add_kinetic, g.tw1, g.tw2);
+  else
+    k_rtog_any<C><<<gr, kPlaneThreads, smem, h->stream>>>(grid, h->nzp, g.plane_off, g.plane_g, g.plane_pos, out, psi,
+                                                          h->ldg, b0, g.g2, g.bucket, add_kinetic,
+                                                          make_axis(h->ax[0]), make_axis(h->ax[1]), g.tw1, g.tw2);
+  CUW_LAUNCH_CHECK("k_rtog_plane");
+  return CUW_OK;
+}
+template <class C>
+static int plane_smem(const Handle* h) {
+  return (int)(((size_t)h->d.nr2 * plane_stride(h->d.nr1) + h->d.nr1 + h->d.nr2) * sizeof(C));
+}
+
 // out = FFT_RTOG[ V * FFT_GTOR[psi] ] (+ 1/2 G^2 psi + bucket psi when add_kinetic)
 template <class C, int N1, int N2, int V>
 static int fft_vpsi_t(Handle* h, const double2* psi, double2* out, bool add_kinetic) {
-  const int nr1 = h->d.nr1, nr2 = h->d.nr2;
-  const int smem_plane = (int)(((size_t)nr2 * plane_stride(nr1) + nr1 + nr2) * sizeof(C));
-  const int tp = kPlaneThreads;
-  AxisArg a1 = make_axis(h->ax[0]), a2 = make_axis(h->ax[1]);
-  Device& g = h->g;
-  C* grid = reinterpret_cast<C*>(g.grid);
+  const int smem = plane_smem<C>(h);
   for (int b0 = 0; b0 < h->d.nbh; b0 += h->batch) {
     const int nb = std::min(h->batch, h->d.nbh - b0);
-    k_gtor_plane<C, N1, N2, V><<<dim3(h->nzp, nb), tp, smem_plane, h->stream>>>(psi, h->ldg, b0, g.plane_off, g.plane_g,
-                                                                           g.plane_pos, g.plane_rows, grid, h->nzp,
-                                                                           a1, a2, g.tw1, g.tw2);
-    CUW_LAUNCH_CHECK("k_gtor_plane");
+    CUW_RET((planes_gtor<C, N1, N2, V>(h, psi, b0, nb, smem)));
     CUW_RET(z_vpsi<C>(h, nb));
-    k_rtog_plane<C, N1, N2, V><<<dim3(h->nzp, nb), tp, smem_plane, h->stream>>>(grid, h->nzp, g.plane_off, g.plane_g,
-                                                                      g.plane_pos, g.plane_rows, out, psi, h->ldg, b0, g.g2,
-                                                                      g.bucket, add_kinetic ? 1 : 0, a1, a2,
-                                                                      g.tw1, g.tw2);
-    CUW_LAUNCH_CHECK("k_rtog_plane");
+    CUW_RET((planes_rtog<C, N1, N2, V>(h, psi, out, add_kinetic ? 1 : 0, b0, nb, smem)));
   }
   return CUW_OK;
 }
-
 
 // rho = sum over the bands of this set of f |psi(r)|^2 terms (WAVES_DENSITY
 // for TINV at Gamma), batch by batch through the work grid
 template <class C, int N1, int N2, int V>
 static int fft_density_t(Handle* h, const double2* psi, double* rho) {
-  const int nr1 = h->d.nr1, nr2 = h->d.nr2;
-  const int smem_plane = (int)(((size_t)nr2 * plane_stride(nr1) + nr1 + nr2) * sizeof(C));
-  AxisArg a1 = make_axis(h->ax[0]), a2 = make_axis(h->ax[1]);
-  Device& g = h->g;
-  C* grid = reinterpret_cast<C*>(g.grid);
+  const int smem = plane_smem<C>(h);
   for (int b0 = 0; b0 < h->d.nbh; b0 += h->batch) {
     const int nb = std::min(h->batch, h->d.nbh - b0);
-    k_gtor_plane<C, N1, N2, V><<<dim3(h->nzp, nb), kPlaneThreads, smem_plane, h->stream>>>(
-        psi, h->ldg, b0, g.plane_off, g.plane_g, g.plane_pos, g.plane_rows, grid, h->nzp, a1, a2, g.tw1, g.tw2);
-    CUW_LAUNCH_CHECK("k_gtor_plane");
+    CUW_RET((planes_gtor<C, N1, N2, V>(h, psi, b0, nb, smem)));
     CUW_RET(z_rho<C>(h, rho, b0, nb));
   }
   return CUW_OK;
 }
 
-// kernels of work-grid type C and length N (0: any length): shared-memory
-// limits and the launcher
+// kernels of work-grid type C and xy lengths N1, N2 (0: any lengths):
+// shared-memory limits and the launchers
 template <class C, int N1, int N2, int V>
-static int fft_select_v(Handle* h, int smem_plane) {
-  CUW_TRY(smem_allow((const void*)k_gtor_plane<C, N1, N2, V>, smem_plane));
-  CUW_TRY(smem_allow((const void*)k_rtog_plane<C, N1, N2, V>, smem_plane));
+static int fft_select_v(Handle* h) {
+  const int smem = plane_smem<C>(h);
+  if constexpr (N1 > 0) {
+    CUW_TRY(smem_allow((const void*)k_gtor_plane<C, N1, N2, V>, smem));
+    CUW_TRY(smem_allow((const void*)k_rtog_plane<C, N1, N2, V>, smem));
+  } else {
+    CUW_TRY(smem_allow((const void*)k_gtor_any<C>, smem));
+    CUW_TRY(smem_allow((const void*)k_rtog_any<C>, smem));
+  }
   CUW_RET(z_setup<C>(h));
   h->fft_run = &fft_vpsi_t<C, N1, N2, V>;
   h->fft_rho = &fft_density_t<C, N1, N2, V>;
@@ -1131,18 +1302,18 @@ static int fft_select_v(Handle* h, int smem_plane) {
 // the plan variant h->fft_variant of a grid with compiled lengths (variant 0
 // for the kernels with run-time lengths)
 template <class C, int N1, int N2>
-static int fft_select(Handle* h, int smem_plane) {
+static int fft_select(Handle* h) {
   if constexpr (N1 > 0) {
     switch (h->fft_variant) {
-      case 1: return fft_select_v<C, N1, N2, 1>(h, smem_plane);
-      case 2: return fft_select_v<C, N1, N2, 2>(h, smem_plane);
+      case 1: return fft_select_v<C, N1, N2, 1>(h);
+      case 2: return fft_select_v<C, N1, N2, 2>(h);
       case 3:
-        if constexpr (N1 == 64 && N2 == 64) return fft_select_v<C, N1, N2, 3>(h, smem_plane);
+        if constexpr (N1 == 64 && N2 == 64) return fft_select_v<C, N1, N2, 3>(h);
         break;
       default: break;
     }
   }
-  return fft_select_v<C, N1, N2, 0>(h, smem_plane);
+  return fft_select_v<C, N1, N2, 0>(h);
 }
 
 // Kernels of the handle's grid and plan variant: grids of the table get
@@ -1150,21 +1321,19 @@ static int fft_select(Handle* h, int smem_plane) {
 // constant); any other grid takes the kernels with run-time lengths.
 static int fft_choose(Handle* h) {
   const int nr1 = h->d.nr1, nr2 = h->d.nr2, nr3 = h->d.nr3;
-  const size_t es = h->mixed() ? sizeof(float2) : sizeof(double2);
-  const int smem_plane = (int)(((size_t)nr2 * plane_stride(nr1) + nr1 + nr2) * es);
   int rc = CUW_OK;
   bool found = false;
 #define CUW_FFT_GRID(A, B, Z)                                                                        \
   if (!found && nr1 == A && nr2 == B && nr3 == Z) {                                                  \
     found = true;                                                                                    \
-    rc = h->mixed() ? fft_select<float2, A, B>(h, smem_plane) : fft_select<double2, A, B>(h, smem_plane); \
+    rc = h->mixed() ? fft_select<float2, A, B>(h) : fft_select<double2, A, B>(h); \
   }
   CUW_FFT_GRIDS
 #undef CUW_FFT_GRID
   h->fft_compiled = found;
   if (!found) {
     h->fft_variant = 0;
-    rc = h->mixed() ? fft_select<float2, 0, 0>(h, smem_plane) : fft_select<double2, 0, 0>(h, smem_plane);
+    rc = h->mixed() ? fft_select<float2, 0, 0>(h) : fft_select<double2, 0, 0>(h);
   }
   return rc;
 }
