@@ -6,6 +6,7 @@
 //   k_ortho_x       the iteration of WAVES_ORTHO_X (src/paw_waves2.f90:1844-2022)
 //                   as one thread-block cluster; every wait is a hardware cluster
 //                   barrier and the loop is bounded by max_iter
+//   k_ortho_x_small the same for at most 32 bands, as one CTA
 //   k_switch_lambda Lagrange extrapolation of WAVES$SWITCH (:2249-2296)
 //   k_ortho_y       WAVES_ORTHO_Y_C (:1025-1338) for WAVES_GRAMSCHMIDT (:2025-2177);
 //                   its matrices are real at the Gamma point, so it runs in real
@@ -924,6 +925,272 @@ __global__ void __launch_bounds__(512) k_ortho_x(OrthoArgs a) {
 }
 
 // ---------------------------------------------------------------------------
+// ORTHO_X for n <= 32 as one CTA of NB x NB warps (NB = n / 8 rounded up), with
+// every matrix in shared memory for the whole solve: warp (r, c) owns the 8 x 8
+// block (r, c) of each product (FP64 tensor cores, m8n8k4, two accumulation
+// chains).  One layout serves both orientations of both operands: columns at a
+// stride LD = 8 NB + 4, which is 4 or 12 mod 16 doubles, so a fragment's 16
+// lanes fall on 16 banks whether they run along rows or columns.  The
+// arithmetic, the phases and the stopping rules are those of k_ortho_x; the
+// products are latency, so what counts is that a phase is a few MMA steps and
+// one block barrier, without staging through global memory or padding to 128:
+// a solve of 8 bands took 327 us in k_ortho_x<1,1> and takes 18 us, and a CP
+// step of Si2 (8 bands) 422 and 145 us, of Si8 (16 bands) 436 and 206 us.
+//
+// The kernel also takes over the small launches around the iteration:
+//   mode 0: U, e diagonalise the current matrix exactly;
+//   mode 1: U is an earlier eigenbasis: S = sym(CHIPSI), B = U^T S U, e = diag B,
+//           E = B - diag B; S, Lambda and B go to global memory for the fallback;
+//   mode 2 (gated, after the Jacobi of B): U <- U V, Lambda from its saved copy.
+// ---------------------------------------------------------------------------
+struct SmallArgs {
+  int mode;
+  double* u;        // eigenbasis; written in mode 2
+  const double* v;  // eigenvectors of B (mode 2)
+  double* smat;     // written in mode 1
+  double* b;        // written in mode 1
+  double* e;        // written in mode 1
+  double* lam0;     // written in mode 1, read in mode 2
+};
+constexpr int kSmallN = 32;
+template <int NB>
+constexpr int small_smem() { return (int)sizeof(double) * (9 * 8 * NB * (8 * NB + 4) + 8 * NB + 4 * NB * NB); }
+
+// maximum over the warp of non-negative doubles, whose bit patterns order as integers
+__device__ __forceinline__ double warp_max_pos(double v) {
+  const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
+  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+  return __hiloint2double((int)mh, (int)ml);
+}
+
+template <int NB>
+__global__ void __launch_bounds__(32 * NB * NB) k_ortho_x_small(OrthoArgs a, SmallArgs s) {
+  if (gate_closed(a.gate)) return;
+  constexpr int NP = 8 * NB, LD = NP + 4, SZ = NP * LD, NW = NB * NB, NT = 32 * NW;
+  extern __shared__ double sm[];
+  double *CC = sm, *CP = CC + SZ, *U = CP + SZ, *E = U + SZ, *L = E + SZ, *H = L + SZ, *W = H + SZ, *X0 = W + SZ,
+         *X1 = X0 + SZ, *ee = X1 + SZ, *red = ee + NP;  // red: two sets of 2 NW maxima
+  const int n = a.n, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int fr = lane >> 2, fk = lane & 3, r0 = (warp % NB) * 8, c0 = (warp / NB) * 8;
+  const int i = r0 + fr, j = c0 + 2 * fk;  // this lane's elements (i, j) and (i, j + 1)
+  bool ok[2];
+#pragma unroll
+  for (int e = 0; e < 2; ++e) ok[e] = i < n && j + e < n;
+  auto load = [&](double* M, const double* src) {
+    for (int t = tid; t < NP * NP; t += NT) {
+      const int p = t % NP, q = t / NP;
+      M[p + LD * q] = p < n && q < n ? src[p + n * q] : 0.0;
+    }
+  };
+  // v += op(A) op(B) of this warp's block
+  auto product = [&](const double* A, bool tA, const double* B, bool tB, double (&v)[2]) {
+    double w[2] = {0.0, 0.0};
+#pragma unroll
+    for (int k = 0; k < NP; k += 8) {
+      const int k0 = k + fk, k1 = k + 4 + fk;
+      dmma(v, tA ? A[k0 + LD * (r0 + fr)] : A[r0 + fr + LD * k0], tB ? B[c0 + fr + LD * k0] : B[k0 + LD * (c0 + fr)]);
+      dmma(w, tA ? A[k1 + LD * (r0 + fr)] : A[r0 + fr + LD * k1], tB ? B[c0 + fr + LD * k1] : B[k1 + LD * (c0 + fr)]);
+    }
+    v[0] += w[0];
+    v[1] += w[1];
+  };
+  auto put = [&](double* M, const double (&v)[2]) {
+    M[i + LD * j] = v[0];
+    M[i + LD * (j + 1)] = v[1];
+  };
+  auto max2 = [&](double& x, double& y, int set) {
+    x = warp_max_pos(x);
+    y = warp_max_pos(y);
+    if (NW > 1) {
+      double* r = red + set * 2 * NW;
+      if (lane == 0) {
+        r[warp] = x;
+        r[NW + warp] = y;
+      }
+      __syncthreads();
+      x = warp_max_pos(lane < NW ? r[lane] : 0.0);
+      y = warp_max_pos(lane < NW ? r[NW + lane] : 0.0);
+    } else {
+      __syncwarp();
+    }
+  };
+  load(CC, a.chichi);
+  load(CP, a.chipsi);
+  load(U, s.u);
+  load(L, s.mode == 2 ? s.lam0 : a.lam);
+  if (s.mode == 2) load(X0, s.v);
+  if (s.mode != 1)
+    for (int t = tid; t < NP; t += NT) ee[t] = t < n ? a.e[t] : 0.5;
+  __syncthreads();
+  if (s.mode == 1) {
+    double v[2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      v[e] = 0.5 * (CP[i + LD * (j + e)] + CP[j + e + LD * i]);
+      if (ok[e]) {
+        s.smat[i + n * (j + e)] = v[e];
+        s.lam0[i + n * (j + e)] = L[i + LD * (j + e)];
+      }
+    }
+    put(W, v);
+    __syncthreads();
+    v[0] = v[1] = 0.0;
+    product(W, false, U, false, v);
+    put(H, v);
+    __syncthreads();
+    v[0] = v[1] = 0.0;
+    product(U, true, H, false, v);
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      if (ok[e]) s.b[i + n * (j + e)] = v[e];
+      if (i == j + e) {
+        ee[i] = i < n ? v[e] : 0.5;
+        if (i < n) s.e[i] = v[e];
+        v[e] = 0.0;
+      }
+    }
+    put(E, v);
+    __syncthreads();
+  } else if (s.mode == 2) {
+    double v[2] = {0.0, 0.0};
+    product(U, false, X0, false, v);
+    __syncthreads();
+    put(U, v);
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+      if (ok[e]) s.u[i + n * (j + e)] = v[e];
+    __syncthreads();
+  }
+  double cpv[2], ps[2], rden[2], lv[2];
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    const int jj = j + e;
+    cpv[e] = CP[i + LD * jj];
+    ps[e] = ok[e] ? a.psipsi[min(i, jj) + n * max(i, jj)] - (i == jj ? 1.0 : 0.0) : 0.0;
+    rden[e] = ok[e] ? 1.0 / (ee[i] + ee[jj]) : 0.0;
+    lv[e] = L[i + LD * jj];
+  }
+  int status = CUW_ERR_NOT_CONVERGED, iters = a.max_iter, sweeps = 0;
+  double rho_known = 0.0;
+  for (int iter = 1; iter <= a.max_iter; ++iter) {
+    // HAUX = CHICHI LAMBDA + CHIPSI
+    double v[2] = {cpv[0], cpv[1]};
+    product(CC, false, L, false, v);
+    put(H, v);
+    __syncthreads();
+    // W = LAMBDA^T HAUX + CHIPSI^T LAMBDA + PSIPSI - 1
+    v[0] = ps[0];
+    v[1] = ps[1];
+    product(L, true, H, false, v);
+    product(CP, true, L, false, v);
+    put(W, v);
+    double digam = 0.0, unused = 0.0;
+#pragma unroll
+    for (int e = 0; e < 2; ++e) digam = v[e] != v[e] ? INFINITY : fmax(digam, fabs(v[e]));
+    max2(digam, unused, 0);  // its barrier also ends the writes of W
+    if (digam < a.eps) {
+      status = CUW_OK;
+      iters = iter;
+      break;
+    }
+    if (!(digam <= 1e200)) {
+      status = CUW_ERR_DIVERGED;
+      iters = iter;
+      break;
+    }
+    // HAUX = U^T W, Gamma in the basis U = HAUX U, X = Gamma / (e_i + e_j)
+    v[0] = v[1] = 0.0;
+    product(U, true, W, false, v);
+    put(H, v);
+    __syncthreads();
+    double gt[2] = {0.0, 0.0}, xp[2], xq[2];
+    product(H, false, U, false, gt);
+#pragma unroll
+    for (int e = 0; e < 2; ++e) xq[e] = xp[e] = gt[e] * rden[e];
+    put(X0, xp);
+    __syncthreads();
+    double *xcur = X0, *xnext = X1;
+    bool failed = false;
+    if (s.mode == 1) {  // the fixed point of lyap_fast
+      double prev = INFINITY, rho = rho_known, omega = 1.0;
+      const int cheb0 = rho > 0.0 ? 0 : 2;
+      for (int it2 = 0; it2 < a.max_inner; ++it2) {
+        double ex[2] = {0.0, 0.0}, xe[2] = {0.0, 0.0}, dx = 0.0, xm = 0.0;
+        product(E, false, xcur, false, ex);
+        product(xcur, false, E, false, xe);
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const double xn = omega * ((gt[e] - ex[e] - xe[e]) * rden[e] - xq[e]) + xq[e];
+          dx = fmax(dx, fabs(xn - xp[e]));
+          xm = fmax(xm, fabs(xn));
+          xq[e] = xp[e];
+          xp[e] = xn;
+        }
+        put(xnext, xp);
+        max2(dx, xm, it2 & 1);  // its barrier also ends the writes of xnext
+        double* t = xcur;
+        xcur = xnext;
+        xnext = t;
+        ++sweeps;
+        const double ratio = dx / prev;
+        if (lyap_stop(dx, xm, prev, it2, a.max_inner, a.lyap_tol, failed)) break;
+        if (it2 == cheb0) {
+          if (cheb0 == 2) rho_known = rho = fmin(0.9, fmax(0.05, 1.1 * ratio));
+          omega = 1.0 / (1.0 - 0.5 * rho * rho);
+        } else if (it2 > cheb0) {
+          omega = 1.0 / (1.0 - 0.25 * rho * rho * omega);
+        }
+      }
+    }
+    if (failed) {
+      status = kFixedPointFailed;
+      iters = iter;
+      break;
+    }
+    // HAUX = U X, W = HAUX U^T
+    v[0] = v[1] = 0.0;
+    product(U, false, xcur, false, v);
+    put(H, v);
+    __syncthreads();
+    v[0] = v[1] = 0.0;
+    product(H, false, U, true, v);
+    if (a.occ_equal) {
+#pragma unroll
+      for (int e = 0; e < 2; ++e) lv[e] -= v[e];
+    } else {
+      // LAMBDA(I,J) -= 2 OCCI/(OCCI+OCCJ) W(I,J); then occupation symmetrisation
+      put(W, v);
+      __syncthreads();
+      const double dsmall = 1e-12;
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        if (!ok[e]) continue;
+        const int jj = j + e;
+        const double oi = a.occ[i], oj = a.occ[jj], occi = oi + dsmall, occj = oj + dsmall;
+        if (oi < oj) {
+          const double lji = L[jj + LD * i] - 2.0 * occj / (occj + occi) * W[jj + LD * i];
+          lv[e] = lji * occi / occj;
+        } else {
+          lv[e] = lv[e] - 2.0 * occi / (occi + occj) * v[e];
+        }
+      }
+      __syncthreads();
+    }
+    put(L, lv);
+    __syncthreads();
+  }
+#pragma unroll
+  for (int e = 0; e < 2; ++e)
+    if (ok[e]) a.lam[i + n * (j + e)] = lv[e];
+  if (tid == 0) {
+    a.status[0] = status;
+    a.status[1] = iters;
+    a.inner[0] += sweeps;
+  }
+}
+
+// ---------------------------------------------------------------------------
 // ORTHO_X for 64 < n <= 128 with equal occupations, as one cluster of 16 CTAs
 // in a 4 x 4 grid: CTA (ri, ci) owns the 32 x 32 tile (ri, ci) of every
 // product.  The matrices live in global memory (L2: 128 KB each); a product
@@ -1506,10 +1773,10 @@ __global__ void k_copy_gated(const double* __restrict__ src1, double* __restrict
 // g.u / g.eig; use_e: g.u diagonalises an earlier CHIPSI only and g.emat holds
 // the off-diagonal rest.  Status and iteration count go to g.ostatus[0..1];
 // gate: launch gated on the status of an earlier launch (gate_closed).
-static int ortho_x_launch(Handle* h, int use_e, int max_iter, double eps, const int* gate) {
+static OrthoArgs ortho_x_args(const Handle* h, int use_e, int max_iter, double eps, const int* gate) {
   const int n = h->d.nb;
-  Device& g = h->g;
-  OrthoArgs a;
+  const Device& g = h->g;
+  OrthoArgs a = {};
   a.n = n;
   a.chichi = g.oomat;
   a.psipsi = g.mat;
@@ -1538,6 +1805,31 @@ static int ortho_x_launch(Handle* h, int use_e, int max_iter, double eps, const 
   a.occ_equal = 1;
   for (int i = 1; i < n; ++i)
     if (h->occ_h[i] != h->occ_h[0]) a.occ_equal = 0;
+  return a;
+}
+
+// n <= kSmallN: the iteration and the launches around it in one CTA
+static int ortho_small_launch(Handle* h, int mode, int max_iter, double eps, const int* gate) {
+  const Device& g = h->g;
+  const OrthoArgs a = ortho_x_args(h, mode == 1, max_iter, eps, gate);
+  const SmallArgs s = {mode, g.u, g.wk2, g.smat, g.work, g.eig, g.lam0};
+#define CUW_SMALL(NB)                                                            \
+  {                                                                              \
+    CUW_TRY(smem_allow((const void*)k_ortho_x_small<NB>, small_smem<NB>()));       \
+    k_ortho_x_small<NB><<<1, 32 * NB * NB, small_smem<NB>(), h->stream>>>(a, s);   \
+  }
+  if (a.n <= 8) CUW_SMALL(1)
+  else if (a.n <= 16) CUW_SMALL(2)
+  else if (a.n <= 24) CUW_SMALL(3)
+  else CUW_SMALL(4)
+#undef CUW_SMALL
+  CUW_LAUNCH_CHECK("k_ortho_x_small");
+  return CUW_OK;
+}
+
+static int ortho_x_launch(Handle* h, int use_e, int max_iter, double eps, const int* gate) {
+  OrthoArgs a = ortho_x_args(h, use_e, max_iter, eps, gate);
+  const int n = a.n;
   // cluster of 16 CTAs (non-portable size), else 8, 4, ... ; tile rows/cols
   // per CTA are at most 16*MR x 16*MC with MR, MC in {1,2,4}
   cudaLaunchConfig_t cfg = {};
@@ -1574,10 +1866,7 @@ static int ortho_x_launch(Handle* h, int use_e, int max_iter, double eps, const 
       cudaGetLastError();
     }
   }
-  // NB <= 32: one CTA holds every tile (products of at most 32^3 take it well
-  // under a microsecond, less than one cluster barrier), which also leaves the
-  // other SMs to the other sets of a batch; larger NB start from 16 CTAs
-  int cs = n <= 32 ? 1 : 16;
+  int cs = 16;
   cudaError_t e = cudaSuccess;
   bool launched = false;
   for (; cs >= 1 && !launched; cs /= 2) {
@@ -1660,6 +1949,19 @@ int ortho_solve(Handle* h, int max_iter, double eps) {
   const int n = h->d.nb;
   Device& g = h->g;
   const int nn = n * n;
+  if (n <= kSmallN) {
+    if (h->have_u) {
+      const int* gate = g.ostatus;  // status of the first launch
+      CUW_RET(ortho_small_launch(h, 1, max_iter, eps, nullptr));
+      CUW_RET(jacobi_run(h, g.work, g.wk2, g.eig, gate));
+      return ortho_small_launch(h, 2, max_iter, eps, gate);
+    }
+    k_symmetrize<<<ceil_div(nn, 256), 256, 0, h->stream>>>(g.omat, n, g.smat, nullptr, g.lam0);
+    CUW_LAUNCH_CHECK("k_symmetrize");
+    CUW_RET(jacobi_run(h, g.smat, g.u, g.eig, nullptr));
+    h->have_u = true;
+    return ortho_small_launch(h, 0, max_iter, eps, nullptr);
+  }
   const dim3 tg(ceil_div(n, 32), ceil_div(n, 32));
   // with an eigenbasis, Lambda is saved to lam0 in the same launch
   k_symmetrize<<<ceil_div(n * n, 256), 256, 0, h->stream>>>(g.omat, n, g.smat, h->have_u ? g.lam : nullptr, g.lam0);

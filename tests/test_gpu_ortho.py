@@ -1,0 +1,57 @@
+"""ORTHO_X of up to 32 bands, which one CTA solves in shared memory: band counts
+on both sides of every multiple of 8, equal and unequal occupations, the first
+solve (exact eigenbasis), later ones (fixed point in the earlier eigenbasis) and
+a state far from the earlier one (rediagonalisation)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+import cuwaves  # noqa: E402
+from cuwaves import CUW_PSI0, CUW_PSIM, systems  # noqa: E402
+
+
+@pytest.mark.parametrize("equal", [True, False])
+@pytest.mark.parametrize("nb", [2, 6, 8, 10, 14, 16, 18, 22, 24, 26, 30, 32, 34])
+def test_small_ortho(nb, equal, oracle):
+    """Against the oracle.  Both stop when the residual is below 1e-8 of the
+    constraint, at the same iteration; what differs between them before that is
+    the Lyapunov solve's tolerance, below 1e-9 of the result."""
+    sy = systems.si_cell(1, epw_psi_ry=12.0)
+    sy.nb = nb
+    inp = systems.build_inputs(sy)
+    occ = np.array(inp["occ"], dtype=np.float64)
+    occ[:] = 2.0
+    if not equal:
+        occ[-1] = 0.5
+        occ[0] = 1.5
+    w = cuwaves.open_waves(inp).setup()
+    cpu = oracle.open_oracle(inp).setup()
+    for b in (w, cpu):
+        b.set_occ(occ)
+    w.initialize()
+
+    def same():
+        for which in (CUW_PSI0, CUW_PSIM):
+            cpu.upload_psi(which, w.download_psi(which))
+        cpu.set_proj(w.get_proj())
+        cpu.set_rlam0(w.get_rlam0())
+
+    for step in range(4):
+        if step == 3:  # another basis of the same space: the earlier eigenbasis is no help
+            nbh = inp["nbh"]
+            for which in (CUW_PSI0, CUW_PSIM):
+                w.upload_psi(which, w.download_psi(which)[np.arange(nbh)[::-1]])
+            w.projections()
+            w.set_rlam0(np.zeros((nb, nb), dtype=complex))
+        w.hpsi()
+        w.propagate()
+        same()
+        assert w.orthogonalize() == cpu.orthogonalize(), step
+        for which in (CUW_PSIM,):
+            a, b = w.download_psi(which), cpu.download_psi(which)
+            assert np.abs(a - b).max() < 1e-9 * np.abs(b).max(), step
+        assert np.abs(w.get_rlam0() - cpu.get_rlam0()).max() < 1e-8, step
+        w.switch()
+    w.close()
+    cpu.close()
