@@ -53,49 +53,94 @@ struct BandFinal {
   unsigned* count;
 };
 
-__global__ void k_band_sums(int mode, const double2* __restrict__ x, const double2* __restrict__ y, int ldg, int ngl,
-                            const double* __restrict__ w1, const double* __restrict__ w2,
-                            const int* __restrict__ minusg, double* __restrict__ part, int nblk, int rg,
-                            BandFinal fin) {
+// What bounds it: latency (two dependent loads, a reduction and the last
+// block's sums; the set's coefficients are 13 MB for 64 pairs of bands of
+// Si64).  A thread takes whole pairs +-G, so every coefficient is read once,
+// four pairs in flight; the block sums go through shuffles.  Against one load
+// pair at a time and a shared-memory tree: Si64 17.4 -> 14.9 us, Si2 11 -> 7 us.
+struct BandSum {
+  double q[4];
+};
+template <int MODE>
+__device__ __forceinline__ void band_add(BandSum& s, double2 a, double2 c, double2 ya, double2 yc, double w, double wb,
+                                         bool bucket) {
+  if (MODE == 2) {
+    s.q[0] += a.x * ya.x + a.y * ya.y;
+    s.q[1] += a.x * ya.y - a.y * ya.x;
+    s.q[2] += a.x * yc.x - a.y * yc.y;
+    s.q[3] += a.x * yc.y + a.y * yc.x;
+    return;
+  }
+  const double n2 = a.x * a.x + a.y * a.y;
+  const double cr = a.x * c.x - a.y * c.y;  // Re(conj(a) conj(c)) = Re(a c)
+  s.q[0] += w * n2;
+  s.q[1] += w * cr;
+  if (MODE == 0 && bucket) {
+    s.q[2] += wb * n2;
+    s.q[3] += wb * cr;
+  }
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(RB)
+    k_band_sums(const double2* __restrict__ x, const double2* __restrict__ y, int ldg, int nh,
+                const double* __restrict__ w1, const double* __restrict__ w2, const int2* __restrict__ half,
+                double* __restrict__ part, int nblk, int rg, BandFinal fin) {
+  constexpr int U = 4;
   const int b = blockIdx.y, blk = blockIdx.x;
   const double2* xb = x + (size_t)ldg * b;
-  const double2* yb = y ? y + (size_t)ldg * b : nullptr;
-  double q[4] = {0.0, 0.0, 0.0, 0.0};
-  const int g0 = blk * rg, g1 = min(ngl, g0 + rg);
-  for (int g = g0 + threadIdx.x; g < g1; g += RB) {
-    int mg = minusg[g];
-    if (mode == 0) {
-      double2 a = xb[g], c = xb[mg];
-      double n2 = a.x * a.x + a.y * a.y;
-      double cr = a.x * c.x - a.y * c.y;  // Re(conj(a) conj(c)) = Re(a c)
-      q[0] += w1[g] * n2;
-      q[1] += w1[g] * cr;
-      if (w2) {
-        q[2] += w2[g] * n2;
-        q[3] += w2[g] * cr;
+  const double2* yb = MODE ? y + (size_t)ldg * b : nullptr;
+  const double2 zero = make_double2(0.0, 0.0);
+  BandSum s = {{0.0, 0.0, 0.0, 0.0}};
+  const int g1 = min(nh, (blk + 1) * rg);
+  for (int g0 = blk * rg + threadIdx.x; g0 < g1; g0 += U * RB) {
+    int2 h[U];
+    double2 a[U], c[U], ya[U], yc[U];
+    double wa[U], wc[U], ba[U], bc[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) h[u] = g0 + u * RB < g1 ? half[g0 + u * RB] : make_int2(-1, -1);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const bool in = h[u].x >= 0;
+      a[u] = in ? xb[h[u].x] : zero;
+      c[u] = in ? xb[h[u].y] : zero;
+      if (MODE) {
+        ya[u] = in ? yb[h[u].x] : zero;
+        yc[u] = in ? yb[h[u].y] : zero;
       }
-    } else if (mode == 1) {
-      double2 d = csub(xb[g], yb[g]);
-      double2 dm = csub(xb[mg], yb[mg]);
-      q[0] += w1[g] * (d.x * d.x + d.y * d.y);
-      q[1] += w1[g] * (d.x * dm.x - d.y * dm.y);
-    } else {
-      double2 a = xb[g], hv = yb[g], hm = yb[mg];
-      q[0] += a.x * hv.x + a.y * hv.y;
-      q[1] += a.x * hv.y - a.y * hv.x;
-      q[2] += a.x * hm.x - a.y * hm.y;
-      q[3] += a.x * hm.y + a.y * hm.x;
+      if (MODE < 2) {
+        wa[u] = in ? w1[h[u].x] : 0.0;
+        wc[u] = in ? w1[h[u].y] : 0.0;
+      }
+      if (MODE == 0 && w2) {
+        ba[u] = in ? w2[h[u].x] : 0.0;
+        bc[u] = in ? w2[h[u].y] : 0.0;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (MODE == 1) {
+        a[u] = csub(a[u], ya[u]);
+        c[u] = csub(c[u], yc[u]);
+      }
+      band_add<MODE>(s, a[u], c[u], ya[u], yc[u], wa[u], ba[u], w2 != nullptr);
+      if (h[u].x != h[u].y) band_add<MODE>(s, c[u], a[u], yc[u], ya[u], wc[u], bc[u], w2 != nullptr);
     }
   }
-  __shared__ double red[4][RB];
-  for (int k = 0; k < 4; ++k) red[k][threadIdx.x] = q[k];
-  __syncthreads();
-  for (int s = RB / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s)
-      for (int k = 0; k < 4; ++k) red[k][threadIdx.x] += red[k][threadIdx.x + s];
-    __syncthreads();
+  __shared__ double red[4][RB / 32];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s.q[k] += __shfl_xor_sync(0xffffffffu, s.q[k], o);
+    if ((threadIdx.x & 31) == 0) red[k][threadIdx.x >> 5] = s.q[k];
   }
-  if (threadIdx.x < 4) part[((size_t)b * nblk + blk) * 4 + threadIdx.x] = red[threadIdx.x][0];
+  __syncthreads();
+  if (threadIdx.x < 4) {
+    double t = 0.0;
+#pragma unroll
+    for (int w = 0; w < RB / 32; ++w) t += red[threadIdx.x][w];
+    part[((size_t)b * nblk + blk) * 4 + threadIdx.x] = t;
+  }
   if (!fin.count) return;
   __shared__ bool last;
   __threadfence();  // this block's partials before its count
@@ -104,7 +149,7 @@ __global__ void k_band_sums(int mode, const double2* __restrict__ x, const doubl
   if (!last) return;
   __threadfence();
   extern __shared__ double fsh[];
-  energy_final_block(mode, part, nblk, fin.occ, gridDim.y, fin.gweight, fin.dt2, fin.tbucket, fin.out, fin.scalar,
+  energy_final_block(MODE, part, nblk, fin.occ, gridDim.y, fin.gweight, fin.dt2, fin.tbucket, fin.out, fin.scalar,
                      fsh);
   if (threadIdx.x == 0) *fin.count = 0u;
 }
@@ -112,7 +157,7 @@ __global__ void k_band_sums(int mode, const double2* __restrict__ x, const doubl
 // scalar results from band sums and occupations (the last block of
 // k_band_sums): the block sums the block
 // partials of every band (the order of the former two-kernel form), forms the
-// per-band terms in parallel, and thread 0 adds them in band order
+// per-band terms in parallel, and a warp adds them
 //   out[0] EKIN or WAVEKINETIC energy; out[1 + i] per-band values
 //   scalar (when not null) also receives out[0]
 // The partials are read through L2: other blocks of the same launch wrote them.
@@ -163,9 +208,12 @@ __device__ void energy_final_block(int mode, const double* __restrict__ part, in
     term[b] = e;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < 32) {
     double e = 0.0;
-    for (int b = 0; b < nbh; ++b) e += term[b];
+    for (int b = threadIdx.x; b < nbh; b += 32) e += term[b];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+    if (threadIdx.x) return;
     out[0] = (mode == 2) ? e : e * gweight;
     if (scalar) scalar[0] = out[0];
   }
@@ -279,26 +327,27 @@ __global__ void k_add_vec(double* __restrict__ a, const double* __restrict__ b, 
 // the band sums of mode over G, then (by the launch's last block) the scalar
 // results: out_dev[0] the energy, out_dev[1..] per band, scalar[0] (when not
 // null) the energy again
-static int band_sums_run(Handle* h, int mode, const double2* x, const double2* y, const double* w1, const double* w2,
+template <int MODE>
+static int band_sums_run(Handle* h, const double2* x, const double2* y, const double* w1, const double* w2,
                          double* out_dev, double* scalar) {
   const int nmax = ceil_div(h->d.ngl, RG);  // partial slots per band in g.red
   const size_t sm = sizeof(double) * 5 * (size_t)h->d.nbh;
-  if (sm > 48 * 1024) CUW_TRY(smem_allow((const void*)k_band_sums, (int)sm));
-  if (h->band_bps == 0) {
+  if (sm > 48 * 1024) CUW_TRY(smem_allow((const void*)k_band_sums<MODE>, (int)sm));
+  if (h->band_bps[MODE] == 0) {
     int bps = 0;
-    CUW_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_band_sums, RB, sm));
-    h->band_bps = std::max(1, bps);
+    CUW_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_band_sums<MODE>, RB, sm));
+    h->band_bps[MODE] = std::max(1, bps);
   }
   // one wave of blocks on the SMs the set may use (a second, nearly empty
-  // wave would double the time): G ranges of a multiple of RB per block
-  int nblk = std::min(nmax, std::max(1, h->nsm * h->band_bps / h->d.nbh));
-  const int rg = ceil_div(ceil_div(h->d.ngl, nblk), RB) * RB;
-  nblk = ceil_div(h->d.ngl, rg);
+  // wave would double the time): a multiple of RB pairs +-G per block
+  int nblk = std::min(nmax, std::max(1, h->nsm * h->band_bps[MODE] / h->d.nbh));
+  const int rg = ceil_div(ceil_div(h->nh, nblk), RB) * RB;
+  nblk = ceil_div(h->nh, rg);
   Device& g = h->g;
   BandFinal fin{g.occ, h->gweight, h->delt * h->delt, h->tbucket ? 1 : 0, out_dev, scalar,
                 reinterpret_cast<unsigned*>(g.red + 4 * (size_t)h->d.nbh * (nmax + 1))};
-  k_band_sums<<<dim3(nblk, h->d.nbh), RB, sm, h->stream>>>(mode, x, y, h->ldg, h->d.ngl, w1, w2, g.minusg, g.red,
-                                                           nblk, rg, fin);
+  k_band_sums<MODE><<<dim3(nblk, h->d.nbh), RB, sm, h->stream>>>(x, y, h->ldg, h->nh, w1, w2, g.half, g.red, nblk, rg,
+                                                                 fin);
   CUW_LAUNCH_CHECK("k_band_sums");
   return CUW_OK;
 }
@@ -308,9 +357,9 @@ static int band_sums_run(Handle* h, int mode, const double2* x, const double2* y
 static int energy_run(Handle* h, int mode, double* out_dev, double* scalar = nullptr) {
   Device& g = h->g;
   if (mode == RED_EKIN)
-    return band_sums_run(h, 0, g.psi0, nullptr, g.g2, h->tbucket ? g.bucket : nullptr, out_dev, scalar);
-  if (mode == RED_WAVEKIN) return band_sums_run(h, 1, g.psi0, g.psim, g.mpsi, nullptr, out_dev, scalar);
-  return band_sums_run(h, 2, g.psi0, g.hpsi, nullptr, nullptr, out_dev, scalar);
+    return band_sums_run<0>(h, g.psi0, nullptr, g.g2, h->tbucket ? g.bucket : nullptr, out_dev, scalar);
+  if (mode == RED_WAVEKIN) return band_sums_run<1>(h, g.psi0, g.psim, g.mpsi, nullptr, out_dev, scalar);
+  return band_sums_run<2>(h, g.psi0, g.hpsi, nullptr, nullptr, out_dev, scalar);
 }
 
 cudaError_t smem_allow(const void* fn, int bytes) {
@@ -396,8 +445,7 @@ static int ortho_core(Handle* h, int max_iter, double eps, bool fused) {
   CUW_RET(proj_compute(h, g.psim, g.proj, g.opsi, g.oproj, true));
   CUW_RET(mark(h, 6));
   // DO*PROJ and DO*OPROJ
-  CUW_RET(oproj_compute(h, g.proj, g.hproj));
-  CUW_RET(oproj_compute(h, g.oproj, g.pbuf));
+  CUW_RET(oproj_compute(h, g.proj, g.hproj, g.oproj, g.pbuf));
   const FoldPair pp[3] = {{0, 0, g.proj, g.hproj}, {1, 0, g.oproj, g.hproj}, {1, 1, g.oproj, g.pbuf}};
   CUW_RET(tc ? tc_gram(h, pp, 3, g.mat, g.omat, g.oomat) : fold_gram(h, pp, 3, g.mat, g.omat, g.oomat));
   CUW_RET(mark(h, 7));

@@ -165,7 +165,7 @@ struct Handle {
   // page-locked host block of cuwaves_cp_step's results (8 sums, the 16 status
   // words, the forces): one copy each and one wait per step
   double* res_h = nullptr;
-  int band_bps = 0;  // resident blocks per SM of the band-sum kernel (0: not yet queried)
+  int band_bps[3] = {0, 0, 0};  // resident blocks per SM of the band-sum kernels (0: not yet queried)
   int nzp = 0;                   // occupied z planes
   int batch = 0;                 // bands per FFT batch
   int grid_bands = 0;            // bands the FFT work grid has room for
@@ -319,6 +319,35 @@ __device__ __forceinline__ float2 cmulc(float2 a, float2 b) {
 }
 __device__ __forceinline__ float2 cscale(float2 a, float s) { return make_float2(a.x * s, a.y * s); }
 
+// Sum over split-K partials for output i: scale * part[z][i] (z < nz) + oc[z][i]
+// (z < kc), every array n wide.  A block of 32 x kSumZ threads has kSumZ threads
+// on each of 32 outputs, each with every kSumZ-th split (the outputs of small
+// sets are too few to hide the latency of 140 splits one after another: the
+// overlaps of 32 bands took 27 us and take 12); the result is valid in the threads with threadIdx.y == 0.
+constexpr int kSumZ = 8;
+__device__ __forceinline__ double2 split_get(const double2* p) { return *p; }
+__device__ __forceinline__ double2 split_get(const float2* p) { return make_double2((double)p->x, (double)p->y); }
+template <class P>
+__device__ __forceinline__ double2 split_sum(const P* __restrict__ part, int nz, size_t n, size_t i, double scale,
+                                             const double2* __restrict__ oc, int kc) {
+  __shared__ double2 sh[kSumZ][32];
+  double2 s = make_double2(0.0, 0.0);
+  if (i < n) {
+#pragma unroll 4
+    for (int z = threadIdx.y; z < nz; z += kSumZ) s = cadd(s, split_get(part + (size_t)z * n + i));
+    s = cscale(s, scale);
+#pragma unroll 4
+    for (int z = threadIdx.y; z < kc; z += kSumZ) s = cadd(s, oc[(size_t)z * n + i]);
+  }
+  sh[threadIdx.y][threadIdx.x] = s;
+  __syncthreads();
+  if (threadIdx.y == 0) {
+#pragma unroll
+    for (int y = 1; y < kSumZ; ++y) s = cadd(s, sh[y][threadIdx.x]);
+  }
+  return s;
+}
+
 // (-i)^l
 __device__ __forceinline__ double2 mipow(int l) {
   switch (l & 3) {
@@ -371,7 +400,8 @@ int proj_compute(Handle* h, const double2* psiA, double2* projA, const double2* 
                  bool folded = false);
 int addpro_run(Handle* h, int mode, const double2* hpc, const double2* opc);
 int hproj_compute(Handle* h, const double2* proj, double2* out);
-int oproj_compute(Handle* h, const double2* proj, double2* out);
+int oproj_compute(Handle* h, const double2* proj, double2* out, const double2* proj2 = nullptr,
+                  double2* out2 = nullptr);
 int hoproj_compute(Handle* h, const double2* proj, double2* hout, double2* oout);
 int ortho_solve(Handle* h, int max_iter, double eps);
 int ortho_result(Handle* h, const int* st, int* iters);

@@ -286,32 +286,18 @@ __global__ void __launch_bounds__(RT, 2) k_rproj(Op p, Op u, int kchunk, int nr,
   }
 }
 
-// sum of nz partial values `stride` apart, eight loads in flight, in split order
-__device__ __forceinline__ double2 sum_parts(const double2* __restrict__ part, int nz, size_t stride) {
-  double2 s = make_double2(0.0, 0.0);
-  int z = 0;
-  for (; z + 8 <= nz; z += 8) {
-    double2 v[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] = part[(size_t)(z + j) * stride];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) s = cadd(s, v[j]);
-  }
-  for (; z < nz; ++z) s = cadd(s, part[(size_t)z * stride]);
-  return s;
-}
-
-// PROJ(b, p) of one or two wave-function arrays (nbh super wave functions each)
-__global__ void k_rproj_sum(const double2* __restrict__ part, int nz, int nbh, int nset, int npro, double scale,
-                            double2* __restrict__ out0, double2* __restrict__ out1) {
+// PROJ(b, p) of one or two wave-function arrays (nbh super wave functions each);
+// the split sums are those of split_sum (cuwaves_internal.cuh)
+__global__ void __launch_bounds__(32 * kSumZ)
+    k_rproj_sum(const double2* __restrict__ part, int nz, int nbh, int nset, int npro, double scale,
+                double2* __restrict__ out0, double2* __restrict__ out1) {
   const int nw = nset * nbh;
-  const size_t n = (size_t)nw * npro;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const double2 s = sum_parts(part + i, nz, n);
-    const int b = (int)(i % nw);
-    const size_t p = i / nw;
-    (b < nbh ? out0 : out1)[(b < nbh ? b : b - nbh) + (size_t)nbh * p] = cscale(s, scale);
-  }
+  const size_t n = (size_t)nw * npro, i = blockIdx.x * (size_t)32 + threadIdx.x;
+  const double2 s = split_sum(part, nz, n, i, scale, (const double2*)nullptr, 0);
+  if (threadIdx.y || i >= n) return;
+  const int b = (int)(i % nw);
+  const size_t p = i / nw;
+  (b < nbh ? out0 : out1)[(b < nbh ? b : b - nbh) + (size_t)nbh * p] = s;
 }
 
 // ---------------------------------------------------------------------------
@@ -359,18 +345,18 @@ __global__ void __launch_bounds__(RT, 2) k_rgram(RGramArgs a, double* __restrict
 }
 
 // out_pair(i + NB j) = scale * the ks plane-wave parts + the kc one-centre parts
-__global__ void k_rgram_sum(const double2* __restrict__ part, int ks, int kc, int nb, int npair, double scale,
-                            double* __restrict__ o0, double* __restrict__ o1, double* __restrict__ o2) {
-  const size_t per = (size_t)nb * nb / 2, n = per * npair;
-  const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  const double2 s = sum_parts(part + t, ks, n), c = sum_parts(part + (size_t)ks * n + t, kc, n);
+__global__ void __launch_bounds__(32 * kSumZ)
+    k_rgram_sum(const double2* __restrict__ part, int ks, int kc, int nb, int npair, double scale,
+                double* __restrict__ o0, double* __restrict__ o1, double* __restrict__ o2) {
+  const size_t per = (size_t)nb * nb / 2, n = per * npair, t = blockIdx.x * (size_t)32 + threadIdx.x;
+  const double2 s = split_sum(part, ks, n, t, scale, part + (size_t)ks * n, kc);
+  if (threadIdx.y || t >= n) return;
   const int pair = (int)(t / per);
   const size_t e = 2 * (t % per);
   const int i = (int)(e / nb), j = (int)(e % nb);
   double* o = pair == 0 ? o0 : (pair == 1 ? o1 : o2);
-  o[i + (size_t)nb * j] = s.x * scale + c.x;
-  o[i + (size_t)nb * (j + 1)] = s.y * scale + c.y;
+  o[i + (size_t)nb * j] = s.x;
+  o[i + (size_t)nb * (j + 1)] = s.y;
 }
 
 // The complex value at this lane's G from the row values v = (Re, Im) of a
@@ -653,37 +639,51 @@ __global__ void __launch_bounds__(RT, 2) k_rforce(Op u, Op ded, const double* __
 }
 
 // PROJ(n, p) += sum_m O(m, p) Lambda(m, n) on the real views (n + NB p) of the
-// projection arrays (WAVES_ADDOPROJ, src/paw_waves2.f90:687-758).  A block
-// forms 64 n x 8 p, two p per thread with m in order; Lambda and O pass
-// through shared memory 32 values of m at a time.
-constexpr int kAopK = 32;
-__global__ void __launch_bounds__(256) k_raddoproj(double* __restrict__ out, const double* __restrict__ x,
+// projection arrays (WAVES_ADDOPROJ, src/paw_waves2.f90:687-758).  A warp forms
+// 8 n x 16 p on the FP64 tensor cores straight from global memory (L2): both
+// operands run along m, and lane k of a fragment takes m = 8 s + 2 k and the
+// next one with one 16-byte load (NB is even), so a load fills the fragments
+// of two MMAs.  The sum is short (NB terms), so what counts is that all of its
+// loads are in flight at once: 128 bands and 512 projectors take 9.1 us, and
+// took 19.5 us through shared memory, 32 values of m at a time.
+__global__ void __launch_bounds__(128) k_raddoproj(double* __restrict__ out, const double* __restrict__ x,
                                                    const double* __restrict__ lam, int npro, int nb) {
-  __shared__ double sl[64][kAopK + 1], sx[8][kAopK];
-  const int tn = threadIdx.x & 63, tp = threadIdx.x >> 6;
-  const int n = blockIdx.y * 64 + tn, p0 = blockIdx.x * 8;
-  double s0 = 0.0, s1 = 0.0;
-  for (int k0 = 0; k0 < nb; k0 += kAopK) {
-    __syncthreads();  // the previous chunk is consumed
-    for (int i = threadIdx.x; i < 64 * kAopK; i += blockDim.x) {
-      const int kk = i % kAopK, nn = i / kAopK, m = k0 + kk, ng = blockIdx.y * 64 + nn;
-      sl[nn][kk] = (m < nb && ng < nb) ? lam[m + (size_t)nb * ng] : 0.0;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, fr = lane >> 2, fk = lane & 3;
+  const int n0 = (blockIdx.y * 4 + warp) * 8, p0 = blockIdx.x * 16;
+  if (n0 >= nb) return;  // the whole warp
+  const double2 zero = make_double2(0.0, 0.0);
+  const bool an = n0 + fr < nb, b0 = p0 + fr < npro, b1 = p0 + 8 + fr < npro;
+  const double* la = lam + (size_t)nb * (an ? n0 + fr : 0);
+  const double* x0 = x + (size_t)nb * (b0 ? p0 + fr : 0);
+  const double* x1 = x + (size_t)nb * (b1 ? p0 + 8 + fr : 0);
+  double c0[2] = {0.0, 0.0}, c1[2] = {0.0, 0.0};
+  constexpr int U = 8;
+  for (int m0 = 0; m0 < nb; m0 += 8 * U) {
+    double2 a[U], v0[U], v1[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int m = m0 + 8 * u + 2 * fk;
+      const bool in = m < nb;
+      a[u] = in && an ? *reinterpret_cast<const double2*>(la + m) : zero;
+      v0[u] = in && b0 ? *reinterpret_cast<const double2*>(x0 + m) : zero;
+      v1[u] = in && b1 ? *reinterpret_cast<const double2*>(x1 + m) : zero;
     }
-    {
-      const int kk = threadIdx.x % kAopK, pp = threadIdx.x / kAopK, m = k0 + kk, pg = p0 + pp;
-      sx[pp][kk] = (m < nb && pg < npro) ? x[m + (size_t)nb * pg] : 0.0;
-    }
-    __syncthreads();
-#pragma unroll 8
-    for (int kk = 0; kk < kAopK; ++kk) {
-      const double l = sl[tn][kk];
-      s0 += sx[tp][kk] * l;
-      s1 += sx[tp + 4][kk] * l;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      dmma(c0, a[u].x, v0[u].x);
+      dmma(c1, a[u].x, v1[u].x);
+      dmma(c0, a[u].y, v0[u].y);
+      dmma(c1, a[u].y, v1[u].y);
     }
   }
+  const int n = n0 + fr;
   if (n >= nb) return;
-  if (p0 + tp < npro) out[n + (size_t)nb * (p0 + tp)] += s0;
-  if (p0 + tp + 4 < npro) out[n + (size_t)nb * (p0 + tp + 4)] += s1;
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    const int p = p0 + 2 * fk + e;
+    if (p < npro) out[n + (size_t)nb * p] += c0[e];
+    if (p + 8 < npro) out[n + (size_t)nb * (p + 8)] += c1[e];
+  }
 }
 
 }  // namespace
@@ -828,7 +828,7 @@ int fold_proj(Handle* h, double2* proj0, double2* proj1) {
 #undef L
   CUW_LAUNCH_CHECK("k_rproj");
   const size_t n = (size_t)nt / 2 * npro;
-  k_rproj_sum<<<(unsigned)std::min<size_t>((n + 127) / 128, (size_t)16 * h->nsm), 128, 0, h->stream>>>(
+  k_rproj_sum<<<(unsigned)((n + 31) / 32), dim3(32, kSumZ), 0, h->stream>>>(
       h->g.part, ks, h->d.nbh, nset, npro, h->gweight, proj0, proj1);
   CUW_LAUNCH_CHECK("k_rproj_sum");
   return CUW_OK;
@@ -878,8 +878,8 @@ int fold_gram(Handle* h, const FoldPair* pairs, int npair, double* o0, double* o
   CUW_RET(ensure_part(h, sizeof(double) * (size_t)(ks + kc) * npair * nb * nb));
   CUW_RET(gram_launch(h, a, t, ks + kc, reinterpret_cast<double*>(h->g.part)));
   const size_t n = (size_t)nb * nb / 2 * npair;
-  k_rgram_sum<<<(unsigned)((n + 127) / 128), 128, 0, h->stream>>>(h->g.part, ks, kc, nb, npair, 0.5 * h->gweight, o0,
-                                                                  o1, o2);
+  k_rgram_sum<<<(unsigned)((n + 31) / 32), dim3(32, kSumZ), 0, h->stream>>>(h->g.part, ks, kc, nb, npair,
+                                                                            0.5 * h->gweight, o0, o1, o2);
   CUW_LAUNCH_CHECK("k_rgram_sum");
   return CUW_OK;
 }
@@ -951,7 +951,7 @@ int fold_addx(Handle* h, int slot, const double* lam, double2* out) {
 
 int addoproj_run(Handle* h, double2* proj, const double2* oproj, const double* lam) {
   if (h->npro == 0) return CUW_OK;
-  k_raddoproj<<<dim3(ceil_div(h->npro, 8), ceil_div(h->d.nb, 64)), 256, 0, h->stream>>>(
+  k_raddoproj<<<dim3(ceil_div(h->npro, 16), ceil_div(h->d.nb, 32)), 128, 0, h->stream>>>(
       reinterpret_cast<double*>(proj), reinterpret_cast<const double*>(oproj), lam, h->npro, h->d.nb);
   CUW_LAUNCH_CHECK("k_raddoproj");
   return CUW_OK;

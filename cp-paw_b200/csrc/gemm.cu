@@ -622,18 +622,26 @@ __global__ void k_force_final(const double* __restrict__ fpart, int ntile, int n
   const int p0 = ipro0[a], np = nlmn[a];
   const int total = ntile * np;
   double s = 0.0;
-  for (int k = threadIdx.x; k < total; k += blockDim.x) {
-    int t = k / np, p = p0 + k % np;
-    s += fpart[((size_t)t * npro + p) * 3 + c];
+  // eight partial sums in flight: the sums are latency, not bytes
+  for (int k0 = threadIdx.x; k0 < total; k0 += 8 * blockDim.x) {
+    double v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int k = k0 + u * blockDim.x, t = k / np;
+      v[u] = k < total ? fpart[((size_t)t * npro + p0 + k - t * np) * 3 + c] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) s += v[u];
   }
-  __shared__ double red[128];
-  red[threadIdx.x] = s;
+  __shared__ double red[8];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
   __syncthreads();
-  for (int w = 64; w > 0; w >>= 1) {
-    if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-    __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < (int)blockDim.x / 32; ++w) s += red[w];
+    force[3 * a + c] = gweight * 2.0 * s;
   }
-  if (threadIdx.x == 0) force[3 * a + c] = gweight * 2.0 * red[0];
 }
 
 // ---------------------------------------------------------------------------
@@ -690,9 +698,14 @@ __device__ __forceinline__ void oproj_at(size_t i, const double2* __restrict__ p
 __global__ void k_oproj(const double2* __restrict__ proj, const double* __restrict__ dover, int lnxx,
                         const ProDesc* __restrict__ pdesc, const int* __restrict__ ipro0, const int* __restrict__ isp,
                         const int* __restrict__ lnofp, const int* __restrict__ mofp, const int* __restrict__ lmn0ln,
-                        const int* __restrict__ lox, int maxln, int nbh, int npro, double2* __restrict__ out) {
+                        const int* __restrict__ lox, int maxln, int nbh, int npro, double2* __restrict__ out,
+                        const double2* __restrict__ proj2, double2* __restrict__ out2) {
   size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (i >= (size_t)nbh * npro) return;
+  if (blockIdx.y) {
+    proj = proj2;
+    out = out2;
+  }
   oproj_at(i, proj, dover, lnxx, pdesc, ipro0, isp, lnofp, mofp, lmn0ln, lox, maxln, nbh, out);
 }
 
@@ -939,12 +952,13 @@ int hoproj_compute(Handle* h, const double2* proj, double2* hout, double2* oout)
   return CUW_OK;
 }
 
-int oproj_compute(Handle* h, const double2* proj, double2* out) {
+// DO * PROJ of one or two projection arrays
+int oproj_compute(Handle* h, const double2* proj, double2* out, const double2* proj2, double2* out2) {
   TabView t = tables(h);
   size_t n = (size_t)h->d.nbh * h->npro;
-  k_oproj<<<(unsigned)((n + 255) / 256), 256, 0, h->stream>>>(proj, h->g.dover, h->lnxx, h->g.pdesc, t.ipro0, t.isp,
-                                                              t.lnofp, t.mofp, t.lmn0ln, t.lox, CUW_MAXLN, h->d.nbh,
-                                                              h->npro, out);
+  k_oproj<<<dim3((unsigned)((n + 255) / 256), proj2 ? 2 : 1), 256, 0, h->stream>>>(
+      proj, h->g.dover, h->lnxx, h->g.pdesc, t.ipro0, t.isp, t.lnofp, t.mofp, t.lmn0ln, t.lox, CUW_MAXLN, h->d.nbh,
+      h->npro, out, proj2, out2);
   CUW_LAUNCH_CHECK("k_oproj");
   return CUW_OK;
 }
@@ -968,7 +982,7 @@ int force_gemm(Handle* h, const double2* ded, double* force_dev) {
     CUW_LAUNCH_CHECK("k_force");
   }
   TabView t = tables(h);
-  k_force_final<<<dim3(3, h->d.nat), 128, 0, h->stream>>>(fpart, tm, npro, t.ipro0, t.nlmn, h->d.nat, h->gweight,
+  k_force_final<<<dim3(3, h->d.nat), 256, 0, h->stream>>>(fpart, tm, npro, t.ipro0, t.nlmn, h->d.nat, h->gweight,
                                                           force_dev);
   CUW_LAUNCH_CHECK("k_force_final");
   return CUW_OK;

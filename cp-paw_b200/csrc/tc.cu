@@ -146,59 +146,33 @@ __global__ void __launch_bounds__(kThreads, 1)
   tc::pipe_run<GemmPipe>((K + 15) / 16, load, no_b, a_row, convert_b, finish, err);
 }
 
-// fp32 partial sums `stride` apart, summed in FP64 in split order, eight loads
-// in flight
-__device__ __forceinline__ double2 sum_parts(const float2* __restrict__ part, int nz, size_t stride) {
-  double2 s = dz();
-  int z = 0;
-  for (; z + 8 <= nz; z += 8) {
-    float2 v[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] = part[(size_t)(z + j) * stride];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      s.x += (double)v[j].x;
-      s.y += (double)v[j].y;
-    }
-  }
-  for (; z < nz; ++z) {
-    const float2 v = part[(size_t)z * stride];
-    s.x += (double)v.x;
-    s.y += (double)v.y;
-  }
-  return s;
-}
-
 // PROJ(b, p) of one or two arrays from part[z][p][set][b]
-__global__ void k_tc_proj_sum(const float2* __restrict__ part, int nz, int nbh, int nset, int npro, double scale,
-                              double2* __restrict__ out0, double2* __restrict__ out1) {
+__global__ void __launch_bounds__(32 * kSumZ)
+    k_tc_proj_sum(const float2* __restrict__ part, int nz, int nbh, int nset, int npro, double scale,
+                  double2* __restrict__ out0, double2* __restrict__ out1) {
   const int nw = nset * nbh;
-  const size_t n = (size_t)nw * npro;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const double2 s = sum_parts(part + i, nz, n);
-    const int b = (int)(i % nw);
-    const size_t p = i / nw;
-    (b < nbh ? out0 : out1)[(b < nbh ? b : b - nbh) + (size_t)nbh * p] = cscale(s, scale);
-  }
+  const size_t n = (size_t)nw * npro, i = blockIdx.x * (size_t)32 + threadIdx.x;
+  const double2 s = split_sum(part, nz, n, i, scale, (const double2*)nullptr, 0);
+  if (threadIdx.y || i >= n) return;
+  const int b = (int)(i % nw);
+  const size_t p = i / nw;
+  (b < nbh ? out0 : out1)[(b < nbh ? b : b - nbh) + (size_t)nbh * p] = s;
 }
 
 // out_pair(i + NB j) = scale * sum_z part[z][pair][i][j] + one-centre sum
 // oc[z][pair][i][j] (FP64, kc splits)
-__global__ void k_tc_gram_sum(const float2* __restrict__ part, int nz, const double2* __restrict__ oc, int kc, int nb,
-                              int npair, double scale, double* __restrict__ o0, double* __restrict__ o1,
-                              double* __restrict__ o2) {
-  const size_t per = (size_t)nb * nb / 2, n = per * npair;
-  const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  const double2 s = sum_parts(part + t, nz, n);
-  double2 c = dz();
-  for (int z = 0; z < kc; ++z) c = cadd(c, oc[(size_t)z * n + t]);
+__global__ void __launch_bounds__(32 * kSumZ)
+    k_tc_gram_sum(const float2* __restrict__ part, int nz, const double2* __restrict__ oc, int kc, int nb, int npair,
+                  double scale, double* __restrict__ o0, double* __restrict__ o1, double* __restrict__ o2) {
+  const size_t per = (size_t)nb * nb / 2, n = per * npair, t = blockIdx.x * (size_t)32 + threadIdx.x;
+  const double2 s = split_sum(part, nz, n, t, scale, oc, kc);
+  if (threadIdx.y || t >= n) return;
   const int pair = (int)(t / per);
   const size_t e = 2 * (t % per);
   const int i = (int)(e / nb), j = (int)(e % nb);
   double* o = pair == 0 ? o0 : (pair == 1 ? o1 : o2);
-  o[i + (size_t)nb * j] = s.x * scale + c.x;
-  o[i + (size_t)nb * (j + 1)] = s.y * scale + c.y;
+  o[i + (size_t)nb * j] = s.x;
+  o[i + (size_t)nb * (j + 1)] = s.y;
 }
 
 // Folded projector table of the mixed path: P(r, p) in fp32 (k_pro_fold of
@@ -1034,7 +1008,7 @@ int tc_proj(Handle* h, double2* proj0, double2* proj1) {
   k_tc_tn<ProjPipe><<<dim3(tn, tb, ks), kThreads, ProjPipe::kSmem, h->stream>>>(a, tm, reinterpret_cast<float*>(h->g.part),
                                                                       tc_err(h));
   CUW_LAUNCH_CHECK("k_tc_tn");
-  k_tc_proj_sum<<<(unsigned)std::min<size_t>((n + 127) / 128, (size_t)16 * h->nsm), 128, 0, h->stream>>>(
+  k_tc_proj_sum<<<(unsigned)((n + 31) / 32), dim3(32, kSumZ), 0, h->stream>>>(
       reinterpret_cast<const float2*>(h->g.part), ks, h->d.nbh, nset, npro, h->gweight, proj0, proj1);
   CUW_LAUNCH_CHECK("k_tc_proj_sum");
   return CUW_OK;
@@ -1092,9 +1066,9 @@ int tc_gram(Handle* h, const FoldPair* pairs, int npair, double* o0, double* o1,
   k_tc_tn<GramPipe><<<dim3(tps, tps, ks * npair), kThreads, GramPipe::kSmem, h->stream>>>(
       a, tm, reinterpret_cast<float*>(h->g.part), tc_err(h));
   CUW_LAUNCH_CHECK("k_tc_tn");
-  k_tc_gram_sum<<<(unsigned)((n / 2 + 127) / 128), 128, 0, h->stream>>>(reinterpret_cast<const float2*>(h->g.part), ks,
-                                                                        reinterpret_cast<const double2*>(oc), kc, nb,
-                                                                        npair, 0.5 * h->gweight, o0, o1, o2);
+  k_tc_gram_sum<<<(unsigned)((n / 2 + 31) / 32), dim3(32, kSumZ), 0, h->stream>>>(
+      reinterpret_cast<const float2*>(h->g.part), ks, reinterpret_cast<const double2*>(oc), kc, nb, npair,
+      0.5 * h->gweight, o0, o1, o2);
   CUW_LAUNCH_CHECK("k_tc_gram_sum");
   return CUW_OK;
 }
