@@ -708,13 +708,15 @@ __global__ void __launch_bounds__(kZThreads<N>, kZBlocks<C, N>)
 // Lengths N = R1 R2 take the first two steps of k_zcol, with rho(r) of the
 // thread's points in registers and the next band's elements loaded before the
 // current band's second step; kRhoX columns a block, because the bands are a
-// serial chain and more blocks in flight hide its barriers.
+// serial chain and more blocks in flight hide its barriers.  The register limit
+// leaves room for 480 threads an SM: at 72^3 in FP64 the 324 blocks then fit
+// one wave (three an SM), 16 bands in 31.9 us; with two an SM they took 49.0.
 constexpr int kRhoX = 16;
 template <int N>
 constexpr int kRhoThreads = (kRhoX * split2(N).r2 + 31) / 32 * 32;
 
 template <class C, int N>
-__global__ void __launch_bounds__(kRhoThreads<N>, 2)
+__global__ void __launch_bounds__(kRhoThreads<N>, 480 / kRhoThreads<N>)
     k_zrho(const C* __restrict__ grid, const int* __restrict__ zslot, int nzp, int npl,
            const double2* __restrict__ tw3g, const double* __restrict__ occ, int nb, int b0, int nbatch,
            double* __restrict__ rho, int first) {
