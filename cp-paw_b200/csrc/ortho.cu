@@ -1541,6 +1541,55 @@ __global__ void __launch_bounds__(512, 1) k_ortho_x_pnl(OrthoArgs a) {
   cl.sync();
 }
 
+// C = A^T B for n x n matrices (n even): a warp forms 8 x 16 on the FP64 tensor
+// cores straight from L2.  Both operands run along the summation index, and
+// lane k of a fragment takes two neighbouring terms with one 16-byte load, all
+// loads of 64 terms in flight (128 bands: 10.4 us in 32 x 32 shared-memory
+// tiles).  With e, the diagonal goes there and to b, the rest to b and em.
+__global__ void __launch_bounds__(128) k_gemm_tn(const double* __restrict__ A, const double* __restrict__ B, int n,
+                                                 double* __restrict__ b, double* __restrict__ e,
+                                                 double* __restrict__ em) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, fr = lane >> 2, fk = lane & 3;
+  const int i0 = (blockIdx.x * 4 + warp) * 8, j0 = blockIdx.y * 16;
+  if (i0 >= n) return;  // the whole warp
+  const double2 zero = make_double2(0.0, 0.0);
+  const bool ai = i0 + fr < n, b0 = j0 + fr < n, b1 = j0 + 8 + fr < n;
+  const double* pa = A + (size_t)n * (ai ? i0 + fr : 0);
+  const double* p0 = B + (size_t)n * (b0 ? j0 + fr : 0);
+  const double* p1 = B + (size_t)n * (b1 ? j0 + 8 + fr : 0);
+  double c0[2] = {0.0, 0.0}, c1[2] = {0.0, 0.0};
+  constexpr int U = 8;
+  for (int m0 = 0; m0 < n; m0 += 8 * U) {
+    double2 a[U], v0[U], v1[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int m = m0 + 8 * u + 2 * fk;
+      const bool in = m < n;
+      a[u] = in && ai ? *reinterpret_cast<const double2*>(pa + m) : zero;
+      v0[u] = in && b0 ? *reinterpret_cast<const double2*>(p0 + m) : zero;
+      v1[u] = in && b1 ? *reinterpret_cast<const double2*>(p1 + m) : zero;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      dmma(c0, a[u].x, v0[u].x);
+      dmma(c1, a[u].x, v1[u].x);
+      dmma(c0, a[u].y, v0[u].y);
+      dmma(c1, a[u].y, v1[u].y);
+    }
+  }
+  const int i = i0 + fr;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int j = j0 + (k >> 1) * 8 + 2 * fk + (k & 1);
+    if (i >= n || j >= n) continue;
+    const double v = k < 2 ? c0[k] : c1[k - 2];
+    b[i + (size_t)n * j] = v;
+    if (!e) continue;
+    em[i + (size_t)n * j] = i == j ? 0.0 : v;
+    if (i == j) e[i] = v;
+  }
+}
+
 // C = op(A) op(B) for n x n matrices, one 32x32 tile per CTA
 __global__ void __launch_bounds__(256) k_small_gemm(const double* A, int tA, const double* B, int tB, int n, double* C,
                                                     const int* gate) {
@@ -1761,18 +1810,6 @@ int jacobi_run(Handle* h, const double* s_dev, double* u, double* e, const int* 
   return CUW_OK;
 }
 
-// diag(B) -> e, B with its diagonal removed -> E
-__global__ void k_split_diag(const double* __restrict__ b, int n, double* __restrict__ e, double* __restrict__ emat,
-                             const int* gate) {
-  if (gate_closed(gate)) return;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n * n; k += gridDim.x * blockDim.x) {
-    const int i = k % n, j = k / n;
-    const double v = b[k];
-    if (i == j) e[i] = v;
-    emat[k] = (i == j) ? 0.0 : v;
-  }
-}
-
 // dst1 = src1 and dst2 = src2 (n elements each) unless the gate is closed
 __global__ void k_copy_gated(const double* __restrict__ src1, double* __restrict__ dst1,
                              const double* __restrict__ src2, double* __restrict__ dst2, int n, const int* gate) {
@@ -1936,17 +1973,16 @@ static int ortho_x_launch(Handle* h, int use_e, int max_iter, double eps, const 
   return CUW_OK;
 }
 
-// B = U^T S U -> g.work, its diagonal -> g.eig and off-diagonal rest -> g.emat
-static int rotate_to_basis(Handle* h, const int* gate) {
+// B = U^T S U -> g.u2, its diagonal -> g.eig and off-diagonal rest -> g.emat (S is
+// symmetric, so both products are of the A^T B form)
+static int rotate_to_basis(Handle* h) {
   const int n = h->d.nb;
   Device& g = h->g;
-  const dim3 tg(ceil_div(n, 32), ceil_div(n, 32));
-  k_small_gemm<<<tg, 256, 0, h->stream>>>(g.smat, 0, g.u, 0, n, g.haux, gate);
-  CUW_LAUNCH_CHECK("k_small_gemm");
-  k_small_gemm<<<tg, 256, 0, h->stream>>>(g.u, 1, g.haux, 0, n, g.work, gate);
-  CUW_LAUNCH_CHECK("k_small_gemm");
-  k_split_diag<<<ceil_div(n * n, 256), 256, 0, h->stream>>>(g.work, n, g.eig, g.emat, gate);
-  CUW_LAUNCH_CHECK("k_split_diag");
+  const dim3 tg(ceil_div(n, 32), ceil_div(n, 16));
+  k_gemm_tn<<<tg, 128, 0, h->stream>>>(g.smat, g.u, n, g.haux, nullptr, nullptr);
+  CUW_LAUNCH_CHECK("k_gemm_tn");
+  k_gemm_tn<<<tg, 128, 0, h->stream>>>(g.u, g.haux, n, g.u2, g.eig, g.emat);
+  CUW_LAUNCH_CHECK("k_gemm_tn");
   return CUW_OK;
 }
 
@@ -1983,13 +2019,12 @@ int ortho_solve(Handle* h, int max_iter, double eps) {
   if (h->have_u) {
     const int* gate = g.ostatus;  // status of the first launch
     const int cb = std::min(ceil_div(nn, 256), 2 * h->nsm);
-    CUW_RET(rotate_to_basis(h, nullptr));
+    CUW_RET(rotate_to_basis(h));
     CUW_RET(ortho_x_launch(h, 1, max_iter, eps, nullptr));
-    CUW_RET(rotate_to_basis(h, gate));  // g.work was overwritten by the iteration
-    CUW_RET(jacobi_run(h, g.work, g.wk2, g.eig, gate));
-    k_small_gemm<<<tg, 256, 0, h->stream>>>(g.u, 0, g.wk2, 0, n, g.u2, gate);
+    CUW_RET(jacobi_run(h, g.u2, g.wk2, g.eig, gate));
+    k_small_gemm<<<tg, 256, 0, h->stream>>>(g.u, 0, g.wk2, 0, n, g.haux, gate);
     CUW_LAUNCH_CHECK("k_small_gemm");
-    k_copy_gated<<<cb, 256, 0, h->stream>>>(g.u2, g.u, g.lam0, g.lam, nn, gate);
+    k_copy_gated<<<cb, 256, 0, h->stream>>>(g.haux, g.u, g.lam0, g.lam, nn, gate);
     CUW_LAUNCH_CHECK("k_copy_gated");
     CUW_RET(ortho_x_launch(h, 0, max_iter, eps, gate));
   } else {
