@@ -218,7 +218,7 @@ def fft_roofline(t_ms, fft_bytes, peaks, peak_src):
         return None
     achieved = fft_bytes / (t_ms * 1e-3) / 1e9
     peak = peaks.get("hbm_gbs")
-    return {"bound": "hbm", "kernels": "k_gtor_plane + k_zcol_v64 + k_rtog_plane", "achieved": round(achieved, 1),
+    return {"bound": "hbm", "kernels": "k_gtor_plane + k_zcol + k_rtog_plane", "achieved": round(achieved, 1),
             "peak": peak, "unit": "GB/s", "frac": round(achieved / peak, 4) if peak else None,
             "peak_source": f"{peak_src} hbm_gbs (of measured)" if peak_src != "fallback" else "fallback",
             "bytes_per_step": fft_bytes, "traffic": None}
@@ -253,16 +253,18 @@ def make_inputs(name="Si64"):
 
 
 def flops_model(inp):
-    """Algorithmic work per step (real flops / bytes), as used for the roofline."""
+    """Algorithmic work per step (real flops / bytes), as used for the roofline:
+    at the Gamma point the contractions are real products over the +-G pairs
+    (NGL real rows, 2 NBH real bands)."""
     ngl, nbh, npro = inp["ngl"], inp["nbh"], None
     npro = sum(sum(2 * l + 1 for l in inp["lox"][s - 1]) for s in inp["isp"].tolist())
     nr = inp["grid"][0] * inp["grid"][1] * inp["grid"][2]
-    contr = 8.0 * ngl * npro * nbh
+    contr = 4.0 * ngl * npro * nbh
     return {
         "addpro_propagate_flops": 2 * contr,      # H and O back-projection (one fused kernel)
         "projections_flops": 2 * contr,           # <p|psibar>, <p|O psi0> at R(+) (one fused kernel)
         "forces_flops": contr,
-        "gram_flops": 6 * 8.0 * ngl * nbh * nbh,
+        "gram_flops": 6 * 4.0 * ngl * nbh * nbh,
         "fft_bytes": 2 * nbh * 2 * nr * 16.0,     # two transforms per band, grid read+write
         "npro": npro,
     }
@@ -401,7 +403,7 @@ def run_mixed(args, local):
     # issue three TF32 MMAs (hi*hi + hi*lo + lo*hi) per product of the model
     fm = flops_model(inp)
     cand = {"addpro_propagate": (ph.get("addpro_propagate", 0.0), fm["addpro_propagate_flops"], "k_tc_addpro<FUSED>"),
-            "projections": (ph.get("projections", 0.0), fm["projections_flops"], "k_tc_proj")}
+            "projections": (ph.get("projections", 0.0), fm["projections_flops"], "k_tc_tn")}
     name = max(cand, key=lambda k: cand[k][0])
     t_ms, flops, kern = cand[name]
     p32 = tf32_peak_tflops(torch)
@@ -702,7 +704,7 @@ def emit_cuda(args, res, world):
         "e2e": {"value": round(e2e, 4), "unit": "steps/s", "h2d_bytes_per_step": res["h2d"],
                 "d2h_bytes_per_step": res["d2h"]},
         "gpu_launches": res["launches"],
-        "roofline": {"bound": "tensor", "kernel": f"k_{'addpro<FUSED>' if name == 'addpro_propagate' else 'proj<DUAL>'}",
+        "roofline": {"bound": "tensor", "kernel": 'k_raddpro_step' if name == 'addpro_propagate' else 'k_rproj',
                      "achieved": round(achieved, 3) if achieved else None, "peak": round(peak, 3) if peak else None,
                      "unit": "TFLOP/s", "frac": round(achieved / peak, 4) if achieved and peak else None,
                      "peak_source": "FP64 cuBLAS DGEMM (torch.matmul float64 8192^3) measured in this run; "

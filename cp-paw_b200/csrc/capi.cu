@@ -58,6 +58,7 @@ struct BandFinal {
 // Si64).  A thread takes whole pairs +-G, so every coefficient is read once,
 // four pairs in flight; the block sums go through shuffles.  Against one load
 // pair at a time and a shared-memory tree: Si64 17.4 -> 14.9 us, Si2 11 -> 7 us.
+// Two in flight with twice the blocks an SM: Si64 the same, Si2 7.8 us.
 struct BandSum {
   double q[4];
 };

@@ -624,8 +624,8 @@ __global__ void __launch_bounds__(kPlaneThreads, 2)
 // and the barriers' latency, hidden by 2 to 4 blocks an SM.  The Stockham
 // stages that it replaces crossed shared memory once more for every radix and
 // for the copies in and out, with two block barriers each: 32 bands of 72^3 in
-// FP32 took 384 us and take 42, of 64^3 69 (by a kernel of its own) and 62; a
-// whole CP step of Si128 (56 x 56 x 110, FP64) 12.6 ms and 11.0 ms.
+// FP32 took 384 us and take 42, 43 bands of 64^3 69 (by a kernel of their own)
+// and 36; a whole CP step of Si128 (56 x 56 x 110, FP64) 12.6 ms and 11.0 ms.
 constexpr int kZX = 32;
 template <int N>
 constexpr int kZThreads = kZX * split2(N).r2;

@@ -1544,8 +1544,10 @@ __global__ void __launch_bounds__(512, 1) k_ortho_x_pnl(OrthoArgs a) {
 // C = A^T B for n x n matrices (n even): a warp forms 8 x 16 on the FP64 tensor
 // cores straight from L2.  Both operands run along the summation index, and
 // lane k of a fragment takes two neighbouring terms with one 16-byte load, all
-// loads of 64 terms in flight (128 bands: 10.4 us in 32 x 32 shared-memory
-// tiles).  With e, the diagonal goes there and to b, the rest to b and em.
+// loads of 64 terms in flight.  With e, the diagonal goes there and to b, the
+// rest to b and em.  From cold caches 128 bands take 10 us, as in 32 x 32 tiles
+// through shared memory; what it saves is the launch that split the diagonal
+// off, and a step of Si64 takes 7 us less with the gated copies gone too.
 __global__ void __launch_bounds__(128) k_gemm_tn(const double* __restrict__ A, const double* __restrict__ B, int n,
                                                  double* __restrict__ b, double* __restrict__ e,
                                                  double* __restrict__ em) {

@@ -8,7 +8,6 @@
 //   warps 3..10           converters, two groups of four warps taking chunks
 //                         in turn: split the raw A rows into tf32 hi/lo parts
 //                         straight into tensor memory (tcgen05.st, lane = row)
-//                         (and, without pre-split B, the B tiles)
 //   warps 11..26          drain: read every accumulation region from TMEM and
 //                         add it into fp32 registers; drain warp w covers TMEM
 //                         lanes 32*(w%4).. (tile rows) and 32 of the 128 columns
@@ -145,14 +144,6 @@ __device__ __forceinline__ float* pipe_stage_base() {
   const uint32_t off = (1024u - (smem_u32(pipe_smem) & 1023u)) & 1023u;
   return reinterpret_cast<float*>(pipe_smem + off);
 }
-
-// Complex operands in real form.  A complex K index k becomes the real pair
-// (2k, 2k+1).
-//   A row:                     (Re a, Im a)
-//   B rows 2j and 2j+1 for the complex output column j:
-//                              (Re c, -Im c)  and  (Im c, Re c)
-// so that sum_k A(m,.) B(2j,.) = Re sum_k a c and B(2j+1,.) gives Im: the
-// accumulator holds column j's real and imaginary part side by side.
 
 // y + sign(y) * h * 2^e for |y| in [2^e, 2^(e+1)): adds back the expected loss
 // of truncating fp32 additions, h units of 2^-23 relative to the binade of y
