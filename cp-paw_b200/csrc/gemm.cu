@@ -1,6 +1,8 @@
 // Complex FP64 contractions of the WAVES path on the FP64 tensor cores
-// (mma.sync m8n8k4 f64), with the projector functions generated in the tile
-// loaders instead of being stored.
+// (mma.sync m8n8k4 f64) for G sets whose tables do not have the +-G parity that
+// the real products of fold.cu and tc.cu rest on (both precisions then run
+// these), with the projector functions generated in the tile loaders; and the
+// small one-centre kernels of every path.
 //
 // Reference routines and the contraction each kernel replaces:
 //   k_proj      WAVES_PROJECTIONS (src/paw_waves1.f90:5746-5905):
@@ -10,11 +12,6 @@
 //               with the epilogues of WAVES$HPSI (:4793-4916), WAVES_OPSI
 //               (:5043-5096), the mass scaling of WAVES$ORTHOGONALIZE
 //               (src/paw_waves2.f90:140-162) and WAVES$PROPAGATE (:6575-6583)
-//   k_gram      PLANEWAVE$SCALARPRODUCT ' '/'='/'-' (src/paw_fft.f90:2344-2422)
-//               as used by WAVES_OVERLAP (src/paw_waves2.f90:761-853) and the
-//               projector sums of WAVES_1COVERLAP (:856-1022)         [split-K]
-//   k_addx      WAVES_ADDOPSI (src/paw_waves2.f90:547-615), WAVES_ADDOPROJ
-//               (:687-758) and the PSI update of WAVES_GRAMSCHMIDT (:2131-2136)
 //   k_force     WAVES_DEDPRO + WAVES_PROFORCE (src/paw_waves1.f90:5694-5743,
 //               6112-6234) fused: the (NGL,NPRO) array DEDPRO is never stored.
 //
