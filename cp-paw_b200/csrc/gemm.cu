@@ -71,7 +71,6 @@ struct Acc {
   }
 };
 
-template <bool CONJA>
 __device__ __forceinline__ void mma_slice(Acc& acc, const double* Ar, const double* Ai, const double* Br,
                                           const double* Bi, int wm, int wn, int lane) {
   const int r8 = lane >> 2, c4 = lane & 3;
@@ -82,8 +81,7 @@ __device__ __forceinline__ void mma_slice(Acc& acc, const double* Ar, const doub
     for (int mi = 0; mi < 4; ++mi) {
       const int o = (wm * 32 + mi * 8 + r8) * LDS + ks * 4 + c4;
       ar[mi] = Ar[o];
-      double t = Ai[o];
-      ai[mi] = CONJA ? -t : t;
+      ai[mi] = Ai[o];
       as[mi] = ar[mi] + ai[mi];
     }
 #pragma unroll
@@ -124,7 +122,7 @@ __device__ __forceinline__ void tile_rc(int e, int& row, int& kk) {
 }
 
 // Products of the main loop: A0*B0 (+ A1*B0 | + A0*B1 | gram: conj(A0)*B0 and A0*B1)
-enum { MP11 = 0, MP21 = 1, MP12 = 2, MPGRAM = 3 };
+enum { MP11 = 0, MP21 = 1, MP12 = 2 };
 
 // Double-buffered main loop over k in [kbeg, kend): the next slice is read from
 // global memory into registers while the DMMAs run on the current slice, then
@@ -134,7 +132,7 @@ template <int MODE, bool AKF, bool BKF, class FA0, class FA1, class FB0, class F
 __device__ __forceinline__ void mainloop(double* sm, int kbeg, int kend, FA0 fa0, FA1 fa1, FB0 fb0, FB1 fb1,
                                          Acc& acc0, Acc& acc1) {
   constexpr int NA = (MODE == MP21) ? 2 : 1;
-  constexpr int NBO = (MODE == MP12 || MODE == MPGRAM) ? 2 : 1;
+  constexpr int NBO = (MODE == MP12) ? 2 : 1;
   constexpr int STAGE = 2 * TILE * (NA + NBO);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wm = warp >> 2, wn = warp & 3;
   double2 ra[NA][EPT], rb[NBO][EPT];
@@ -183,16 +181,13 @@ __device__ __forceinline__ void mainloop(double* sm, int kbeg, int kend, FA0 fa0
     const double* B0r = base + 2 * NA * TILE;
     const double* B0i = B0r + TILE;
     if (MODE == MP11) {
-      mma_slice<false>(acc0, A0r, A0i, B0r, B0i, wm, wn, lane);
+      mma_slice(acc0, A0r, A0i, B0r, B0i, wm, wn, lane);
     } else if (MODE == MP21) {
-      mma_slice<false>(acc0, A0r, A0i, B0r, B0i, wm, wn, lane);
-      mma_slice<false>(acc1, A0r + 2 * TILE, A0i + 2 * TILE, B0r, B0i, wm, wn, lane);
-    } else if (MODE == MP12) {
-      mma_slice<false>(acc0, A0r, A0i, B0r, B0i, wm, wn, lane);
-      mma_slice<false>(acc1, A0r, A0i, B0r + 2 * TILE, B0i + 2 * TILE, wm, wn, lane);
+      mma_slice(acc0, A0r, A0i, B0r, B0i, wm, wn, lane);
+      mma_slice(acc1, A0r + 2 * TILE, A0i + 2 * TILE, B0r, B0i, wm, wn, lane);
     } else {
-      mma_slice<true>(acc0, A0r, A0i, B0r, B0i, wm, wn, lane);
-      mma_slice<false>(acc1, A0r, A0i, B0r + 2 * TILE, B0i + 2 * TILE, wm, wn, lane);
+      mma_slice(acc0, A0r, A0i, B0r, B0i, wm, wn, lane);
+      mma_slice(acc1, A0r, A0i, B0r + 2 * TILE, B0i + 2 * TILE, wm, wn, lane);
     }
     if (more) store(st ^ 1);
     __syncthreads();
@@ -287,7 +282,7 @@ template <int MODE, bool AKF, bool BKF, bool CB0, bool CB1, class PA0, class PA1
 __device__ __forceinline__ void mainloop2(double2* sm, int kbeg, int kend, PA0 pa0, PA1 pa1, PB0 pb0, PB1 pb1,
                                           CA0 ca0, CA1 ca1, Acc& acc0, Acc& acc1) {
   constexpr int NA = (MODE == MP21) ? 2 : 1;
-  constexpr int NBO = (MODE == MP12 || MODE == MPGRAM) ? 2 : 1;
+  constexpr int NBO = (MODE == MP12) ? 2 : 1;
   constexpr int STAGE = TILE2 * (NA + NBO);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wm = warp >> 2, wn = warp & 3;
   if (kbeg >= kend) return;
@@ -339,12 +334,12 @@ __device__ __forceinline__ void mainloop2(double2* sm, int kbeg, int kend, PA0 p
 template <int MODE>
 constexpr size_t smem2_bytes() {
   return sizeof(double2) * (size_t)NS2 * TILE2 *
-         (((MODE == MP21) ? 2 : 1) + ((MODE == MP12 || MODE == MPGRAM) ? 2 : 1));
+         (((MODE == MP21) ? 2 : 1) + ((MODE == MP12) ? 2 : 1));
 }
 
 template <int MODE>
 constexpr size_t smem_bytes() {
-  return sizeof(double) * 2 * 2 * TILE * (((MODE == MP21) ? 2 : 1) + ((MODE == MP12 || MODE == MPGRAM) ? 2 : 1));
+  return sizeof(double) * 2 * 2 * TILE * (((MODE == MP21) ? 2 : 1) + ((MODE == MP12) ? 2 : 1));
 }
 
 __device__ __forceinline__ double2 gen_pro(int g, int ngl, const ProDesc& d, const double* __restrict__ ylm,
