@@ -380,10 +380,21 @@ struct StepCoef {
 // FP64 tensor-core MMA, m8n8k4, A row-major / B column-major fragments:
 //   a = A[lane>>2][lane&3], b = B[lane&3][lane>>2],
 //   c[0..1] = C[lane>>2][2*(lane&3)+0..1]
+// The instruction needs the whole warp, converged.  `volatile` keeps the compiler
+// from sinking it into code that only some lanes run (its result is often used
+// there alone), and every block of products starts with a __syncwarp, because
+// lanes that took different ways through the loads before need not have met again.
 __device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
-  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
                : "+d"(c[0]), "+d"(c[1])
                : "d"(a), "d"(b));
+}
+// Elements i and i + 1 of a row at p (16-byte aligned, at least two elements), or
+// zeros where !in: the load is unconditional, from the row's start if need be, so
+// that no branch depends on the lane.
+__device__ __forceinline__ double2 row2(const double* p, int i, bool in) {
+  const double2 v = *reinterpret_cast<const double2*>(p + (in ? i : 0));
+  return make_double2(in ? v.x : 0.0, in ? v.y : 0.0);
 }
 
 // host helpers implemented in the .cu files

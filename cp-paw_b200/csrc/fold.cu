@@ -651,7 +651,6 @@ __global__ void __launch_bounds__(128) k_raddoproj(double* __restrict__ out, con
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, fr = lane >> 2, fk = lane & 3;
   const int n0 = (blockIdx.y * 4 + warp) * 8, p0 = blockIdx.x * 16;
   if (n0 >= nb) return;  // the whole warp
-  const double2 zero = make_double2(0.0, 0.0);
   const bool an = n0 + fr < nb, b0 = p0 + fr < npro, b1 = p0 + 8 + fr < npro;
   const double* la = lam + (size_t)nb * (an ? n0 + fr : 0);
   const double* x0 = x + (size_t)nb * (b0 ? p0 + fr : 0);
@@ -664,10 +663,11 @@ __global__ void __launch_bounds__(128) k_raddoproj(double* __restrict__ out, con
     for (int u = 0; u < U; ++u) {
       const int m = m0 + 8 * u + 2 * fk;
       const bool in = m < nb;
-      a[u] = in && an ? *reinterpret_cast<const double2*>(la + m) : zero;
-      v0[u] = in && b0 ? *reinterpret_cast<const double2*>(x0 + m) : zero;
-      v1[u] = in && b1 ? *reinterpret_cast<const double2*>(x1 + m) : zero;
+      a[u] = row2(la, m, in && an);
+      v0[u] = row2(x0, m, in && b0);
+      v1[u] = row2(x1, m, in && b1);
     }
+    __syncwarp();
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       dmma(c0, a[u].x, v0[u].x);

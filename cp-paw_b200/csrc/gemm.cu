@@ -74,6 +74,7 @@ struct Acc {
 __device__ __forceinline__ void mma_slice(Acc& acc, const double* Ar, const double* Ai, const double* Br,
                                           const double* Bi, int wm, int wn, int lane) {
   const int r8 = lane >> 2, c4 = lane & 3;
+  __syncwarp();
 #pragma unroll
   for (int ks = 0; ks < BK / 4; ++ks) {
     double ar[4], ai[4], as[4], br[2], bi[2], bs[2];
@@ -241,6 +242,7 @@ template <bool AKF, bool BKF, bool CB, class CA>
 __device__ __forceinline__ void mma_slice2(Acc& acc, const double2* A, const double2* B, int wm, int wn, int lane,
                                            int k0, CA ca) {
   const int r8 = lane >> 2, c4 = lane & 3;
+  __syncwarp();
 #pragma unroll
   for (int ks = 0; ks < BK / 4; ++ks) {
     const bool cj = ca(k0 + ks * 4 + c4);

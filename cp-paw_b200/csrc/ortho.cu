@@ -479,6 +479,7 @@ __device__ void gemm_acc(const double* A, bool tA, const double* B, bool tB, int
         const int r0 = (t % TR) * 8, c0 = (t / TR) * 8;
         // two independent MMA chains (even and odd k steps) to hide the MMA latency
         double a2[2] = {0.0, 0.0};
+        __syncwarp();
         for (int k = 0; k < kk4; k += 8) {
           dmma(acc[q], smA[(k + fk) * LDA + r0 + fr], smB[(k + fk) * LDB + c0 + fr]);
           if (k + 4 < kk4) dmma(a2, smA[(k + 4 + fk) * LDA + r0 + fr], smB[(k + 4 + fk) * LDB + c0 + fr]);
@@ -687,6 +688,7 @@ __device__ double* lyap_fast(const OrthoArgs& a, int cs, int rank, int i0, int i
       // four independent accumulation chains (two per product, even and odd
       // k steps) to hide the MMA latency
       double ex[2] = {0.0, 0.0}, xe[2] = {0.0, 0.0}, ex1[2] = {0.0, 0.0}, xe1[2] = {0.0, 0.0};
+      __syncwarp();
       for (int k = 0; k < n4; k += 8) {
         dmma(ex, Er[(k + fk) * LDA + r0 + fr], Xc[(c0 + fr) * LDK + k + fk]);
         dmma(xe, Xr[(k + fk) * LDA + r0 + fr], Ec[(c0 + fr) * LDK + k + fk]);
@@ -986,6 +988,7 @@ __global__ void __launch_bounds__(32 * NB * NB) k_ortho_x_small(OrthoArgs a, Sma
   // v += op(A) op(B) of this warp's block
   auto product = [&](const double* A, bool tA, const double* B, bool tB, double (&v)[2]) {
     double w[2] = {0.0, 0.0};
+    __syncwarp();
 #pragma unroll
     for (int k = 0; k < NP; k += 8) {
       const int k0 = k + fk, k1 = k + 4 + fk;
@@ -1289,6 +1292,7 @@ __device__ __forceinline__ void pnl_mma(const PnlTerm& t, int nk4, const double*
   const int as = t.ta ? 4 : 4 * PR;
   const double* pb = t.tb ? sb + fk * PR + c0 + fr : sb + (c0 + fr) * PC + fk;
   const int bs = t.tb ? 4 * PR : 4;
+  __syncwarp();
 #pragma unroll 4
   for (int s = 0; s < nk4; s += 2) {
     dmma(acc, pa[s * as], pb[s * bs]);
@@ -1554,7 +1558,6 @@ __global__ void __launch_bounds__(128) k_gemm_tn(const double* __restrict__ A, c
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, fr = lane >> 2, fk = lane & 3;
   const int i0 = (blockIdx.x * 4 + warp) * 8, j0 = blockIdx.y * 16;
   if (i0 >= n) return;  // the whole warp
-  const double2 zero = make_double2(0.0, 0.0);
   const bool ai = i0 + fr < n, b0 = j0 + fr < n, b1 = j0 + 8 + fr < n;
   const double* pa = A + (size_t)n * (ai ? i0 + fr : 0);
   const double* p0 = B + (size_t)n * (b0 ? j0 + fr : 0);
@@ -1567,10 +1570,11 @@ __global__ void __launch_bounds__(128) k_gemm_tn(const double* __restrict__ A, c
     for (int u = 0; u < U; ++u) {
       const int m = m0 + 8 * u + 2 * fk;
       const bool in = m < n;
-      a[u] = in && ai ? *reinterpret_cast<const double2*>(pa + m) : zero;
-      v0[u] = in && b0 ? *reinterpret_cast<const double2*>(p0 + m) : zero;
-      v1[u] = in && b1 ? *reinterpret_cast<const double2*>(p1 + m) : zero;
+      a[u] = row2(pa, m, in && ai);
+      v0[u] = row2(p0, m, in && b0);
+      v1[u] = row2(p1, m, in && b1);
     }
+    __syncwarp();
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       dmma(c0, a[u].x, v0[u].x);
