@@ -105,6 +105,7 @@ struct Device {
   float *u32 = nullptr;
   float *bpre = nullptr;
   float *bsmall = nullptr;
+  double *diag = nullptr;        // FP64 diagonals of the two slots' overlaps (mixed path)
   double *jac_a = nullptr;                   // packed matrix of the eigensolver when NB is too large for shared memory
   double2 *dh = nullptr;         // (LMNXX, LMNXX, NAT)
   double *dover = nullptr;       // (LNXX, LNXX, NSP)
@@ -320,7 +321,7 @@ __device__ __forceinline__ float2 cmulc(float2 a, float2 b) {
 __device__ __forceinline__ float2 cscale(float2 a, float s) { return make_float2(a.x * s, a.y * s); }
 
 // Sum over split-K partials for output i: scale * part[z][i] (z < nz) + oc[z][i]
-// (z < kc), every array n wide.  A block of 32 x kSumZ threads has kSumZ threads
+// (z < kc) + add of the threads on the output, every array n wide.  A block of 32 x kSumZ threads has kSumZ threads
 // on each of 32 outputs, each with every kSumZ-th split (the outputs of small
 // sets are too few to hide the latency of 140 splits one after another: the
 // overlaps of 32 bands took 27 us and take 12); the result is valid in the threads with threadIdx.y == 0.
@@ -328,14 +329,14 @@ constexpr int kSumZ = 8;
 __device__ __forceinline__ double2 split_get(const double2* p) { return *p; }
 __device__ __forceinline__ double2 split_get(const float2* p) { return make_double2((double)p->x, (double)p->y); }
 template <class P>
-__device__ __forceinline__ double2 split_sum(const P* __restrict__ part, int nz, size_t n, size_t i, double scale,
-                                             const double2* __restrict__ oc, int kc) {
+__device__ __forceinline__ double2 split_sum(const P* __restrict__ part, int nz, size_t n, size_t i, double2 scale,
+                                             const double2* __restrict__ oc, int kc, double2 add) {
   __shared__ double2 sh[kSumZ][32];
   double2 s = make_double2(0.0, 0.0);
   if (i < n) {
 #pragma unroll 4
     for (int z = threadIdx.y; z < nz; z += kSumZ) s = cadd(s, split_get(part + (size_t)z * n + i));
-    s = cscale(s, scale);
+    s = cadd(make_double2(s.x * scale.x, s.y * scale.y), add);
 #pragma unroll 4
     for (int z = threadIdx.y; z < kc; z += kSumZ) s = cadd(s, oc[(size_t)z * n + i]);
   }
@@ -346,6 +347,11 @@ __device__ __forceinline__ double2 split_sum(const P* __restrict__ part, int nz,
     for (int y = 1; y < kSumZ; ++y) s = cadd(s, sh[y][threadIdx.x]);
   }
   return s;
+}
+template <class P>
+__device__ __forceinline__ double2 split_sum(const P* __restrict__ part, int nz, size_t n, size_t i, double scale,
+                                             const double2* __restrict__ oc, int kc) {
+  return split_sum(part, nz, n, i, make_double2(scale, scale), oc, kc, make_double2(0.0, 0.0));
 }
 
 // (-i)^l

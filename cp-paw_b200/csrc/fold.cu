@@ -752,6 +752,7 @@ int fold_setup(Handle* h, const std::vector<int>& mg) {
     drop(g.u32);
     drop(g.bpre);
     drop(g.bsmall);
+    drop(g.diag);
     h->nh = nh;
     h->ldu = ldu;
     CUW_TRY(cudaMalloc(&g.half, sizeof(int2) * nh));

@@ -160,16 +160,26 @@ __global__ void __launch_bounds__(32 * kSumZ)
 }
 
 // out_pair(i + NB j) = scale * sum_z part[z][pair][i][j] + one-centre sum
-// oc[z][pair][i][j] (FP64, kc splits)
+// oc[z][pair][i][j] (FP64, kc splits); on the diagonal the plane-wave sum is that
+// of the nd ranges of dg (diag_sums; which[pair]: 0, 1 or 2 there)
 __global__ void __launch_bounds__(32 * kSumZ)
-    k_tc_gram_sum(const float2* __restrict__ part, int nz, const double2* __restrict__ oc, int kc, int nb, int npair,
-                  double scale, double* __restrict__ o0, double* __restrict__ o1, double* __restrict__ o2) {
+    k_tc_gram_sum(const float2* __restrict__ part, int nz, const double2* __restrict__ oc, int kc,
+                  const double* __restrict__ dg, int nd, int3 which, int nb, int npair, double scale,
+                  double* __restrict__ o0, double* __restrict__ o1, double* __restrict__ o2) {
   const size_t per = (size_t)nb * nb / 2, n = per * npair, t = blockIdx.x * (size_t)32 + threadIdx.x;
-  const double2 s = split_sum(part, nz, n, t, scale, oc, kc);
-  if (threadIdx.y || t >= n) return;
   const int pair = (int)(t / per);
   const size_t e = 2 * (t % per);
   const int i = (int)(e / nb), j = (int)(e % nb);
+  double2 sc = make_double2(scale, scale), add = make_double2(0.0, 0.0);
+  if (t < n && (i & ~1) == j) {
+    const int q = pair == 0 ? which.x : (pair == 1 ? which.y : which.z);
+    double d = 0.0;
+    for (int z = threadIdx.y; z < nd; z += kSumZ) d += dg[((size_t)z * 3 + q) * nb + i];
+    (i == j ? add.x : add.y) = scale * d;
+    (i == j ? sc.x : sc.y) = 0.0;
+  }
+  const double2 s = split_sum(part, nz, n, t, sc, oc, kc, add);
+  if (threadIdx.y || t >= n) return;
   double* o = pair == 0 ? o0 : (pair == 1 ? o1 : o2);
   o[i + (size_t)nb * j] = s.x;
   o[i + (size_t)nb * (j + 1)] = s.y;
@@ -808,12 +818,57 @@ struct BSplitSrc {
   long long set_stride; // follow, its values set_stride further
 };
 
+// dg[z][q][n] = sum_{r in range z} of U_0 U_0, U_1 U_0, U_1 U_1 (q = 0, 1, 2) at
+// (r,n) in FP64, one warp per (range, n): the diagonals of the plane-wave
+// overlaps.  What the tensor-core product leaves in an overlap is the rounding
+// of its fp32 running sums (one addition per K = 8), which scales with the sum
+// itself: about 1e-7 of the diagonals, the norms of 192 bands of 50000 plane
+// waves, and next to nothing of the other overlaps, which are small.  A step's
+// norm error enters the next step's wave-function velocities, and the forces of
+// Si96 at 36 Ry were 8e-6 off after four steps; with these sums they are 2e-6 off.
+// The sums ride in the launch that splits the operands (a launch of their own
+// cost a step of Si8 13 us of 190).
+constexpr int kDiagK = 1024;
+struct DiagSums {
+  const float *u0, *u1;
+  int nk, ldu, nb, nd;  // nd ranges; 0: none
+  double* dg;
+};
+__device__ __forceinline__ void diag_sums(const DiagSums& a, int item) {
+  const int z = item % a.nd, b = item / a.nd * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (b >= a.nb) return;  // the whole warp
+  const float *x = a.u0 + (size_t)a.ldu * b, *y = a.u1 + (size_t)a.ldu * b;
+  const int k1 = min(a.nk, (z + 1) * kDiagK);  // rows are padded with zeros to 32 values
+  double q[3] = {0.0, 0.0, 0.0};
+#pragma unroll 4
+  for (int k = z * kDiagK + 4 * lane; k < k1; k += 128) {
+    const float4 u = *reinterpret_cast<const float4*>(x + k), v = *reinterpret_cast<const float4*>(y + k);
+    const float uv[4] = {u.x, u.y, u.z, u.w}, vv[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const double ud = uv[e], vd = vv[e];
+      q[0] = fma(ud, ud, q[0]);
+      q[1] = fma(ud, vd, q[1]);
+      q[2] = fma(vd, vd, q[2]);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) q[i] += __shfl_xor_sync(0xffffffffu, q[i], o);
+  if (lane < 3) a.dg[((size_t)z * 3 + lane) * a.nb + b] = lane == 0 ? q[0] : (lane == 1 ? q[1] : q[2]);
+}
+
 // B operand split into tf32 hi/lo tiles in the shared-memory layout of the
 // pipeline (tc_pipe.cuh): block (tile, chunk) of 4096 floats = hi then lo,
 // element (row, k) of 128 rows x 16 K at (k/4)*512 + row*4 + k%4.  Zero outside
-// the source.
-__global__ void k_bsplit(BSplitSrc b, int nchk, float* __restrict__ out) {
-  const int tile = blockIdx.y, c = blockIdx.x;
+// the source.  The first ndiag columns of blocks take the items of diag_sums.
+__global__ void __launch_bounds__(256) k_bsplit(BSplitSrc b, int nchk, float* __restrict__ out, DiagSums d, int ndiag) {
+  if ((int)blockIdx.x < ndiag) {
+    diag_sums(d, blockIdx.x * gridDim.y + blockIdx.y);
+    return;
+  }
+  const int tile = blockIdx.y, c = blockIdx.x - ndiag;
   float* o = out + ((size_t)tile * nchk + c) * kBTile;
   for (int it = threadIdx.x; it < 512; it += blockDim.x) {
     const int R = it & 127, kg = it >> 7, k0 = c * kCK + 4 * kg;
@@ -903,6 +958,8 @@ static int map_mfast(Handle* h, CUtensorMap* m, const float* base, int rows) {
   return make_map(h, m, base, 2 * h->nh, rows, h->ldu, 128, 16, CU_TENSOR_MAP_SWIZZLE_NONE);
 }
 static float* u32_slot(const Handle* h, int slot) { return h->g.u32 + (size_t)slot * h->d.nb * h->ldu; }
+// ranges of diag_sums
+static int diag_ranges(const Handle* h) { return ceil_div(2 * h->nh, kDiagK); }
 static int tiles_per_array(const Handle* h) { return ceil_div(h->d.nb, 128); }
 
 int tc_setup(Handle* h) {
@@ -946,6 +1003,7 @@ int tc_rooms(Handle* h) {
   slot = std::max(slot, (size_t)ceil_div(np, 128) * ceil_div(nb, kCK));
   slot = std::max(slot, (size_t)ceil_div(nb, 128) * ceil_div(nb, kCK));
   CUW_RET(alloc(reinterpret_cast<void**>(&g.bsmall), sizeof(float) * slot * kBTile));
+  CUW_RET(alloc(reinterpret_cast<void**>(&g.diag), sizeof(double) * 3 * (size_t)diag_ranges(h) * nb));
   return CUW_OK;
 }
 
@@ -966,13 +1024,15 @@ int tc_fold(Handle* h, const double2* psi, int slot) {
   return CUW_OK;
 }
 
-static int tc_bsplit(Handle* h, const BSplitSrc& b, int ntile, int nchk, float* out) {
-  k_bsplit<<<dim3(nchk, ntile), 256, 0, h->stream>>>(b, nchk, out);
+static int tc_bsplit(Handle* h, const BSplitSrc& b, int ntile, int nchk, float* out, const DiagSums& d = {}) {
+  const int ndiag = ceil_div(d.nd * ceil_div(d.nb, 8), ntile);
+  k_bsplit<<<dim3(ndiag + nchk, ntile), 256, 0, h->stream>>>(b, nchk, out, d, ndiag);
   CUW_LAUNCH_CHECK("k_bsplit");
   return CUW_OK;
 }
 
-// split forms of folded slots 0 .. nset-1 (B operands of tc_proj and tc_gram)
+// split forms of folded slots 0 .. nset-1 (B operands of tc_proj and tc_gram);
+// of both, the diagonals of their overlaps too
 int tc_split(Handle* h, int nset) {
   BSplitSrc b{};
   b.xf = h->g.u32;
@@ -981,7 +1041,9 @@ int tc_split(Handle* h, int nset) {
   b.nk = 2 * h->nh;
   b.tps = tiles_per_array(h);
   b.set_stride = (long long)h->d.nb * h->ldu;
-  return tc_bsplit(h, b, nset * b.tps, ceil_div(2 * h->nh, kCK), h->g.bpre);
+  DiagSums d{};
+  if (nset == 2) d = {u32_slot(h, 0), u32_slot(h, 1), b.nk, h->ldu, b.nrow, diag_ranges(h), h->g.diag};
+  return tc_bsplit(h, b, nset * b.tps, ceil_div(2 * h->nh, kCK), h->g.bpre, d);
 }
 
 // PROJ of slot 0 (and slot 1 when proj1 is given), from the split forms
@@ -1038,6 +1100,7 @@ int tc_addpro(Handle* h, int mode, const double2* hpc, const double2* opc, const
   return CUW_OK;
 }
 
+// overlaps of the slots that tc_split(h, 2) has split
 int tc_gram(Handle* h, const FoldPair* pairs, int npair, double* o0, double* o1, double* o2) {
   if (npair < 1 || npair > 3) return h->fail(CUW_ERR_ARG, "overlaps: one to three pairs");
   const int nb = h->d.nb, tps = tiles_per_array(h);
@@ -1066,9 +1129,10 @@ int tc_gram(Handle* h, const FoldPair* pairs, int npair, double* o0, double* o1,
   k_tc_tn<GramPipe><<<dim3(tps, tps, ks * npair), kThreads, GramPipe::kSmem, h->stream>>>(
       a, tm, reinterpret_cast<float*>(h->g.part), tc_err(h));
   CUW_LAUNCH_CHECK("k_tc_tn");
+  auto which = [&](int i) { return i < npair ? pairs[i].x + pairs[i].y : 0; };
   k_tc_gram_sum<<<(unsigned)((n / 2 + 31) / 32), dim3(32, kSumZ), 0, h->stream>>>(
-      reinterpret_cast<const float2*>(h->g.part), ks, reinterpret_cast<const double2*>(oc), kc, nb, npair,
-      0.5 * h->gweight, o0, o1, o2);
+      reinterpret_cast<const float2*>(h->g.part), ks, reinterpret_cast<const double2*>(oc), kc, h->g.diag,
+      diag_ranges(h), make_int3(which(0), which(1), which(2)), nb, npair, 0.5 * h->gweight, o0, o1, o2);
   CUW_LAUNCH_CHECK("k_tc_gram_sum");
   return CUW_OK;
 }

@@ -86,3 +86,25 @@ def test_mixed_cp_steps(name, nsteps):
     e = rel(mix.download_psi(CUW_PSI0), ref.download_psi(CUW_PSI0))
     print(f"{name}: psi after {nsteps} steps, mixed vs FP64 {e:.2e}")
     assert e < 1e-4
+
+
+@pytest.mark.parametrize("size,ry", [("2x2x3", 36.0), ("1x3x3", 30.0)])
+@pytest.mark.parametrize("seed", [2, 4])
+def test_large_steps_keep_a_quarter_of_the_tolerance(size, ry, seed):
+    """Four CP steps of the largest mixed sets of the performance cases: their
+    tolerance is stated as four times what the path differs from 64 bits by, so
+    energies, forces and wave functions stay within a quarter of it."""
+    from perf import cases
+
+    case = cases._case(None, "step", "Si", size, "mixed", ry=ry, steps=4)
+    state = cases.prepare(case, seed)
+    got, ref = cases.run(state), cases.exact(case, seed)
+    bound = cases.tolerance(case)["rel"] / 4
+    pairs = {"energies": (got["energies"], ref["energies"]), "force": (got["force"], ref["force"].numpy()),
+             "psi": (got["psi"][0].numpy(), ref["psi"][0].numpy())}
+    for name, (a, b) in pairs.items():
+        e = float(np.linalg.norm(a - b) / np.linalg.norm(b))
+        print(f"{size} {name}: {e:.2e}")
+        assert e < bound, f"{name}: {e:.2e}"
+    for w in state["sets"]:
+        w.close()
