@@ -144,7 +144,8 @@ __global__ void __launch_bounds__(RB)
   }
   if (!fin.count) return;
   __shared__ bool last;
-  __threadfence();  // this block's partials before its count
+  __threadfence();  // each thread's partials before the block's count ...
+  __syncwarp();     // ... which thread 0 makes for the four threads of its warp that wrote them
   if (threadIdx.x == 0) last = atomicAdd(fin.count, 1u) == gridDim.x * gridDim.y - 1;
   __syncthreads();
   if (!last) return;

@@ -35,3 +35,22 @@ def test_products_start_with_a_converged_warp(name):
             assert not re.search(r"^}|__ldcg|\? \*reinterpret_cast", lines[back]), f"{name}:{at + 1}: no __syncwarp"
             if "__syncwarp();" in lines[back]:
                 break
+
+
+@pytest.mark.parametrize("name", SOURCES)
+def test_blocks_are_counted_after_every_threads_stores(name):
+    """A block that counts itself as done for the launch's last block: every storing
+    thread fences its stores, and a barrier stands between those fences and the
+    count, which one thread makes for all of them."""
+    lines = code(name)
+    for at, line in enumerate(lines):
+        if "atomicAdd(" not in line:
+            continue
+        barrier = fence = None
+        for back in range(at - 1, -1, -1):
+            if re.search(r"__sync(warp|threads)\(\)", lines[back]):
+                barrier = back
+            if "__threadfence();" in lines[back]:
+                fence = back
+                break
+        assert fence is not None and barrier is not None and fence < barrier, f"{name}:{at + 1}"
