@@ -744,6 +744,7 @@ extern "C" int cuwaves_set_gset(cuw_handle* hp, const int* igvec, const int* min
     NEED(mg[i] >= 0 && mg[i] < ngl, CUW_ERR_ARG, "minusg out of range");
     NEED(minusg[mg[i]] - 1 == i, CUW_ERR_ARG, "minusg is not an involution");
   }
+  h->have_gset = false;  // until every table and buffer of the new set is there
   std::vector<double> x(ngl), y(ngl), z(ngl);
   for (int i = 0; i < ngl; ++i) {
     x[i] = gvec[3 * i];

@@ -23,6 +23,7 @@ struct Status {
   do {                                                             \
     cudaError_t e__ = (expr);                                      \
     if (e__ != cudaSuccess) {                                      \
+      cudaGetLastError(); /* not the next launch's error */        \
       return h->fail(CUW_ERR_CUDA, std::string(#expr) + ": " +     \
                                        cudaGetErrorString(e__));   \
     }                                                              \
@@ -401,6 +402,12 @@ __device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
 __device__ __forceinline__ double2 row2(const double* p, int i, bool in) {
   const double2 v = *reinterpret_cast<const double2*>(p + (in ? i : 0));
   return make_double2(in ? v.x : 0.0, in ? v.y : 0.0);
+}
+
+// frees device buffers; what is not allocated again at once stays null
+template <class... T>
+inline void drop(T*&... p) {
+  ((p ? (void)cudaFree(p) : (void)0, p = nullptr), ...);
 }
 
 // host helpers implemented in the .cu files

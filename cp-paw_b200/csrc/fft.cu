@@ -1402,11 +1402,7 @@ int fft_setup(Handle* h, const int* igvec) {
   batch = std::min(batch, h->d.nbh);
   h->batch = batch;
   Device& g = h->g;
-  if (g.plane_off) {
-    cudaFree(g.plane_off); cudaFree(g.plane_g); cudaFree(g.plane_pos); cudaFree(g.zslot); cudaFree(g.plane_iz);
-    cudaFree(g.plane_rows);
-    cudaFree(g.grid); cudaFree(g.tw1); cudaFree(g.tw2); cudaFree(g.tw3);
-  }
+  drop(g.plane_off, g.plane_g, g.plane_pos, g.zslot, g.plane_iz, g.plane_rows, g.grid, g.tw1, g.tw2, g.tw3);
   CUW_TRY(cudaMalloc(&g.plane_off, sizeof(int) * (nzp + 1)));
   CUW_TRY(cudaMalloc(&g.plane_g, sizeof(int) * ngl));
   CUW_TRY(cudaMalloc(&g.plane_pos, sizeof(int) * ngl));

@@ -741,21 +741,11 @@ int fold_setup(Handle* h, const std::vector<int>& mg) {
     if (i <= mg[i]) half.push_back(make_int2(i, mg[i]));
   const int nh = (int)half.size(), ldu = ceil_div(2 * nh, 32) * 32;
   if (nh != h->nh) {
-    auto drop = [](auto*& p) {
-      if (p) cudaFree(p);
-      p = nullptr;
-    };
-    drop(g.half);
-    drop(g.uf);
-    drop(g.prox);
-    drop(g.pf);
-    drop(g.u32);
-    drop(g.bpre);
-    drop(g.bsmall);
-    drop(g.diag);
+    drop(g.half, g.uf, g.prox, g.pf, g.u32, g.bpre, g.bsmall, g.diag);
+    h->nh = 0;  // an allocation that fails is made again by the next set-up
+    CUW_TRY(cudaMalloc(&g.half, sizeof(int2) * nh));
     h->nh = nh;
     h->ldu = ldu;
-    CUW_TRY(cudaMalloc(&g.half, sizeof(int2) * nh));
   }
   CUW_TRY(cudaMemcpy(g.half, half.data(), sizeof(int2) * nh, cudaMemcpyHostToDevice));
   int bad = 0;

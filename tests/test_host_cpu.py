@@ -1,0 +1,58 @@
+"""The engine's host side on a runtime without a device (fake_cuda.cpp): what it
+allocates, launches and refuses.  No kernel runs, so no result is looked at."""
+import numpy as np
+import pytest
+
+from cuwaves import CUW_PREC_FP64, CUW_PREC_MIXED, WavesError, systems
+
+PRECISIONS = [CUW_PREC_FP64, CUW_PREC_MIXED]
+
+
+def inputs(sy):
+    return systems.build_inputs(sy, psi_init="zero")
+
+
+def every_routine(w):
+    w.projections()
+    w.force()
+    w.hpsi()
+    w.density()
+    w.cp_step(move_atoms=True)
+
+
+@pytest.mark.parametrize("prec", PRECISIONS)
+def test_failed_gset_leaves_no_set(fake_engine, prec):
+    """A set_gset that runs out of memory leaves the handle without a G set: later
+    calls are refused, nothing is launched with the buffers that are gone, and the
+    handle takes a G set again."""
+    inp = inputs(systems.si_small(2, epw_psi_ry=12.0))
+    other = dict(inp, minusg=np.arange(1, inp["ngl"] + 1, dtype=np.int32))  # every G its own partner
+    before = fake_engine.lib.fake_in_use()
+    w = fake_engine.open(inp, prec).setup()
+    every_routine(w)
+    gsets = (other, inp)
+    refused = 0
+    for n in range(1, 100):
+        w.inp = gsets[n % 2]
+        fake_engine.lib.fake_fail_malloc(n)
+        try:
+            w.setup()
+            break
+        except WavesError:
+            refused += 1
+        finally:
+            fake_engine.lib.fake_fail_malloc(-1)
+        fake_engine.launches()
+        for call in (w.projections, w.force, w.hpsi, w.density, w.cp_step, w.ekin):
+            with pytest.raises(WavesError, match="(?i)not loaded"):
+                call()
+        assert fake_engine.launches() == []
+        assert fake_engine.lib.fake_misuse() == 0
+        if n % 3 == 0:  # the same set again, and a change between two good ones
+            w.setup()
+            every_routine(w)
+    assert refused > 8  # the buffers of a G set, one after the other
+    every_routine(w)
+    w.close()
+    assert fake_engine.lib.fake_misuse() == 0
+    assert fake_engine.lib.fake_in_use() == before
