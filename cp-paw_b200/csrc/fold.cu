@@ -182,6 +182,15 @@ __device__ __forceinline__ void rmain(double* sm, const Op& a, int m0, const Op&
   rloop<MI, NI, AKF, BKF>(sm, la, lb, kend - kbeg, acc);
 }
 
+// Tile of block blockIdx.x of a product over the sphere's rows: the column tiles of
+// one row tile are neighbours (they share its rows of the table in L2).  One grid
+// dimension for both, because only x takes more than 65535 row tiles (2.1 million
+// plane waves in tiles of 32 rows).
+__device__ __forceinline__ void tile_of_block(int ncol, int& row, int& col) {
+  row = blockIdx.x / ncol;
+  col = blockIdx.x - row * ncol;
+}
+
 template <int MI, int NI>
 __device__ __forceinline__ void azero(double (&acc)[MI][NI][2]) {
 #pragma unroll
@@ -392,7 +401,9 @@ template <int MI, int NI>
 __global__ void __launch_bounds__(RT, 2) k_raddpro(Op p, Op c, int npro, const double2* base, double2* out,
                                                    const int2* __restrict__ half, int nh, int ldg, int nbh) {
   extern __shared__ __align__(16) double rsm[];
-  const int m0 = blockIdx.y * 16 * MI, n0 = blockIdx.x * 16 * NI;
+  int tm, tn;
+  tile_of_block((c.n + 16 * NI - 1) / (16 * NI), tm, tn);
+  const int m0 = tm * 16 * MI, n0 = tn * 16 * NI;
   double acc[MI][NI][2];
   azero(acc);
   rmain<MI, NI, false, false>(rsm, p, m0, c, n0, 0, npro, acc);
@@ -433,7 +444,9 @@ struct RStepArgs {
 template <int MI, int NI>
 __global__ void __launch_bounds__(RT, 2) k_raddpro_step(RStepArgs a, Op p, Op c1, Op c2, int npro) {
   extern __shared__ __align__(16) double rsm[];
-  const int m0 = blockIdx.y * 16 * MI, n0 = blockIdx.x * 8 * NI;
+  int tm, tn;
+  tile_of_block((c1.n + 8 * NI - 1) / (8 * NI), tm, tn);
+  const int m0 = tm * 16 * MI, n0 = tn * 8 * NI;
   double acc[MI][NI][2];
   azero(acc);
   const Loader<false, 16 * MI> la(p.p, p.ld, p.n, m0, 0);
@@ -508,7 +521,9 @@ template <int MI, int NI>
 __global__ void __launch_bounds__(RT, 2) k_raddx(Op u, Op lam, double2* __restrict__ out,
                                                  const int2* __restrict__ half, int nh, int ldg, int nbh) {
   extern __shared__ __align__(16) double rsm[];
-  const int m0 = blockIdx.y * 16 * MI, n0 = blockIdx.x * 16 * NI;
+  int tm, tn;
+  tile_of_block((lam.n + 16 * NI - 1) / (16 * NI), tm, tn);
+  const int m0 = tm * 16 * MI, n0 = tn * 16 * NI;
   double acc[MI][NI][2];
   azero(acc);
   rmain<MI, NI, false, true>(rsm, u, m0, lam, n0, 0, 2 * nbh, acc);
@@ -907,7 +922,7 @@ int fold_addpro(Handle* h, int mode, const double2* hpc, const double2* opc, con
                       h->ldg, h->ldu, h->nh, h->d.nbh, sc};
     const Op c1{reinterpret_cast<const double*>(hpc), nb, nb}, c2{reinterpret_cast<const double*>(opc), nb, nb};
     const RTile t = pick_tile(h, 2 * h->nh, 2 * nb);
-    const dim3 grid(ceil_div(2 * nb, 16 * t.ni), ceil_div(2 * h->nh, 16 * t.mi));
+    const int grid = ceil_div(2 * nb, 16 * t.ni) * ceil_div(2 * h->nh, 16 * t.mi);
 #define L(MI, NI) k_raddpro_step<MI, NI><<<grid, RT, rsmem<MI, NI>(), h->stream>>>(a, p, c1, c2, npro)
     RTILE_SWITCH(t, L);
 #undef L
@@ -917,7 +932,7 @@ int fold_addpro(Handle* h, int mode, const double2* hpc, const double2* opc, con
   const bool o = mode == ADDPRO_OPSI;
   const Op c{reinterpret_cast<const double*>(o ? opc : hpc), nb, nb};
   const RTile t = pick_tile(h, 2 * h->nh, nb);
-  const dim3 grid(ceil_div(nb, 16 * t.ni), ceil_div(2 * h->nh, 16 * t.mi));
+  const int grid = ceil_div(nb, 16 * t.ni) * ceil_div(2 * h->nh, 16 * t.mi);
 #define L(MI, NI)                                                                                              \
   k_raddpro<MI, NI><<<grid, RT, rsmem<MI, NI>(), h->stream>>>(p, c, npro, o ? g.psi0 : g.hpsi, o ? g.opsi : g.hpsi, \
                                                               g.half, h->nh, h->ldg, h->d.nbh)
@@ -931,7 +946,7 @@ int fold_addx(Handle* h, int slot, const double* lam, double2* out) {
   const int nb = h->d.nb;
   const Op u{slot_ptr(h, slot), h->ldu, 2 * h->nh}, l{lam, nb, nb};
   const RTile t = pick_tile(h, 2 * h->nh, nb);
-  const dim3 grid(ceil_div(nb, 16 * t.ni), ceil_div(2 * h->nh, 16 * t.mi));
+  const int grid = ceil_div(nb, 16 * t.ni) * ceil_div(2 * h->nh, 16 * t.mi);
 #define L(MI, NI)                                                                                             \
   k_raddx<MI, NI><<<grid, RT, rsmem<MI, NI>(), h->stream>>>(u, l, out, h->g.half, h->nh, h->ldg, h->d.nbh)
   RTILE_SWITCH(t, L);

@@ -56,3 +56,26 @@ def test_failed_gset_leaves_no_set(fake_engine, prec):
     w.close()
     assert fake_engine.lib.fake_misuse() == 0
     assert fake_engine.lib.fake_in_use() == before
+
+
+@pytest.mark.parametrize("nb", [2, 34])
+def test_launches_of_long_cells(fake_engine, nb):
+    """More plane waves than 65535 row tiles of the folded products hold (32 rows
+    each, two rows a pair): every launch stays within the grid limits."""
+    n = 2_200_000
+    base = inputs(systems.si_small(2, epw_psi_ry=12.0))
+    g = np.arange(n, dtype=np.int32)
+    igvec = np.stack([g % 100, g // 100 % 100, g // 10000], axis=1).astype(np.int32)
+    inp = dict(base, ngl=n, nb=nb, nbh=nb // 2, grid=(100, 100, 720), igvec=igvec, minusg=(g ^ 1) + 1, gvec=np.zeros((n, 3)),
+               g2=np.ones(n), pro=np.ones((len(base["pro"]), n)), ylm=np.ones((len(base["ylm"]), n)), mpsi=np.ones(n),
+               v=np.zeros(100 * 100 * 720), occ=np.full(nb, 2.0), psi=np.zeros((nb // 2, n), dtype=np.complex128))
+    w = fake_engine.open(inp).setup()
+    w.gramschmidt(0, inp["r0"])
+    w.projections()
+    w.force()
+    w.hpsi()
+    w.propagate()
+    w.orthogonalize()
+    w.cp_step(move_atoms=True)
+    w.close()
+    assert fake_engine.lib.fake_misuse() == 0
