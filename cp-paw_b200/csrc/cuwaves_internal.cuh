@@ -100,11 +100,13 @@ struct Device {
   int2 *half = nullptr;
   double *prox = nullptr;
   double *uf = nullptr;
-  // the same in fp32 (mixed path), and the operands split into tf32 B tiles: the
-  // two slots of U, and the small matrix of the product under way
-  float *pf = nullptr;
+  // mixed path: the two slots of U in fp32, and the operands split into tf32 B
+  // tiles: the two slots of U, and the small matrix of the product under way.
+  // P(r,p) in fp32 lies in prox, and the split slots in uf: a product takes the
+  // FP64 or the split form, and each is formed anew for the products that read it
+  float *pf() const { return reinterpret_cast<float*>(prox); }
+  float *bpre() const { return reinterpret_cast<float*>(uf); }
   float *u32 = nullptr;
-  float *bpre = nullptr;
   float *bsmall = nullptr;
   double *diag = nullptr;        // FP64 diagonals of the two slots' overlaps (mixed path)
   double *jac_a = nullptr;                   // packed matrix of the eigensolver when NB is too large for shared memory
@@ -249,7 +251,7 @@ struct Handle {
   int lyap_max_sweeps = 64;  // sweeps per Lyapunov solve before the fixed point counts as failed
   bool ortho_panel = true;   // ORTHO_X by the panel-staged cluster kernel where it applies (64 < NB <= 128)
   // position buffer (r0, rp or rm) that the projector tables were built from,
-  // and which of them (TAB_*) are current for it
+  // and which of them (TAB_*, 0: none) is current for it
   const double* eigr_src = nullptr;
   int tabs = 0;
   // potential: density G set size, LMRXX, index of G = 0 (-1: none), and
@@ -442,6 +444,13 @@ struct FoldPair {
 };
 int fold_setup(Handle* h, const std::vector<int>& minusg);
 int fold_kernels_setup(Handle* h);
+struct TcRooms {
+  size_t split, u32, small, diag;  // bytes
+};
+struct FoldRooms {
+  size_t uf, prox, eigr;  // prox for tables with parity, else eigr
+  TcRooms tc;             // mixed path
+};
 int fold_rooms(Handle* h);
 int fold_table(Handle* h, const double* r_dev);
 int fold_psi(Handle* h, const double2* psi, int slot);
@@ -465,7 +474,8 @@ cudaError_t smem_allow(const void* fn, int bytes);
 // puts a wave-function array into a slot of U in fp32, tc_split forms the split
 // B operands of slots 0 .. nset-1
 int tc_setup(Handle* h);
-int tc_rooms(Handle* h);
+TcRooms tc_room_sizes(const Handle* h);
+int tc_clear_padding(Handle* h);
 int tc_pro_table(Handle* h, const double* r_dev);
 int tc_fold(Handle* h, const double2* psi, int slot);
 int tc_split(Handle* h, int nset);

@@ -756,7 +756,7 @@ int fold_setup(Handle* h, const std::vector<int>& mg) {
     if (i <= mg[i]) half.push_back(make_int2(i, mg[i]));
   const int nh = (int)half.size(), ldu = ceil_div(2 * nh, 32) * 32;
   if (nh != h->nh) {
-    drop(g.half, g.uf, g.prox, g.pf, g.u32, g.bpre, g.bsmall, g.diag);
+    drop(g.half, g.uf, g.prox, g.u32, g.bsmall, g.diag);
     h->nh = 0;  // an allocation that fails is made again by the next set-up
     CUW_TRY(cudaMalloc(&g.half, sizeof(int2) * nh));
     h->nh = nh;
@@ -776,14 +776,26 @@ int fold_setup(Handle* h, const std::vector<int>& mg) {
 }
 
 // Buffers whose sizes follow from the folded sphere: two folded wave-function
-// arrays (rows of slot 1 follow slot 0's), the projector table or, for tables
-// without parity, EIGR, and the fp32 forms of the mixed path (whose start-up
-// orthonormalisation is FP64).  No later call allocates them, so that no step
-// captured into a graph does.
+// arrays (rows of slot 1 follow slot 0's; on the mixed path the split forms lie in
+// the same buffer), the projector table (FP64 or fp32) or, for tables without
+// parity, EIGR, and what else the tensor-core products need.  No later call
+// allocates them, so that no step captured into a graph does.
+static FoldRooms room_sizes(const Handle* h) {
+  FoldRooms r{};
+  r.uf = sizeof(double) * (size_t)h->ldu * h->d.nb * 2;
+  r.prox = sizeof(double) * (size_t)h->ldu * h->npro;
+  r.eigr = sizeof(double2) * (size_t)h->d.ngl * std::max(1, h->d.nat);
+  if (h->mixed()) {
+    r.tc = tc_room_sizes(h);
+    r.uf = std::max(r.uf, r.tc.split);  // whatever the parity: a later G set of the same size keeps the buffer
+  }
+  return r;
+}
+
 int fold_rooms(Handle* h) {
-  auto room = [&](auto*& p, size_t n, const char* what) -> int {
-    if (p || n == 0) return CUW_OK;
-    if (cudaMalloc(&p, n * sizeof(*p)) != cudaSuccess) {
+  auto room = [&](auto*& p, size_t bytes, const char* what) -> int {
+    if (p || bytes == 0) return CUW_OK;
+    if (cudaMalloc(&p, bytes) != cudaSuccess) {
       cudaGetLastError();
       p = nullptr;
       return h->fail(CUW_ERR_NOMEM, std::string("cudaMalloc of the ") + what + " failed");
@@ -791,10 +803,16 @@ int fold_rooms(Handle* h) {
     return CUW_OK;
   };
   Device& g = h->g;
-  CUW_RET(room(g.uf, (size_t)h->ldu * h->d.nb * 2, "folded wave functions"));
-  if (h->sym) CUW_RET(room(g.prox, (size_t)h->ldu * h->npro, "projector table"));
-  else CUW_RET(room(g.eigr, (size_t)h->d.ngl * std::max(1, h->d.nat), "structure factors"));
-  return h->mixed() && h->sym ? tc_rooms(h) : CUW_OK;
+  const FoldRooms r = room_sizes(h);
+  CUW_RET(room(g.uf, r.uf, "folded wave functions"));
+  if (!h->sym) return room(g.eigr, r.eigr, "structure factors");
+  CUW_RET(room(g.prox, r.prox, "projector table"));
+  if (!h->mixed()) return CUW_OK;
+  const bool fresh = !g.u32;
+  CUW_RET(room(g.u32, r.tc.u32, "fp32 folded wave functions"));
+  CUW_RET(room(g.bsmall, r.tc.small, "split matrices"));
+  CUW_RET(room(g.diag, r.tc.diag, "overlap diagonals"));
+  return fresh ? tc_clear_padding(h) : CUW_OK;
 }
 
 static double* slot_ptr(const Handle* h, int slot) { return h->g.uf + (size_t)slot * h->d.nb * h->ldu; }

@@ -745,26 +745,22 @@ static int choose_split(Handle* h, int tiles, int nk, int minchunk, double mul) 
 }
 
 // Tables of the projectors at r_dev that the present path reads: the folded
-// table in FP64 or, for the tensor-core products of the mixed path, in fp32, or
-// EIGR for a G set without parity.  Those
-// of a position buffer stay current until that buffer is written: R(+) of one
-// step is R(0) of the next.
+// table in FP64 or, for the tensor-core products of the mixed path, in fp32 (in
+// the same buffer), or EIGR for a G set without parity.  That of a position buffer
+// stays current until the buffer is written: R(+) of one step is R(0) of the next.
 int eigr_compute(Handle* h, const double* r_dev) {
   const bool pos = r_dev == h->g.r0 || r_dev == h->g.rp || r_dev == h->g.rm;
   const int need = h->tc_on() ? TAB_F32 : (h->sym ? TAB_F64 : TAB_EIGR);
-  const bool same = pos && r_dev == h->eigr_src;
-  if (same && (h->tabs & need) == need) return CUW_OK;
-  if (!same) h->tabs = 0;
+  if (pos && r_dev == h->eigr_src && h->tabs == need) return CUW_OK;
   h->eigr_src = nullptr;
-  const int todo = need & ~h->tabs;
-  if (todo & TAB_F64) CUW_RET(fold_table(h, r_dev));
-  if (todo & TAB_EIGR) {
+  if (need == TAB_F64) CUW_RET(fold_table(h, r_dev));
+  if (need == TAB_EIGR) {
     dim3 grid(std::min(ceil_div(h->d.ngl, 256), 64), h->d.nat);
     k_eigr<<<grid, 256, 0, h->stream>>>(h->g.gx, h->g.gy, h->g.gz, r_dev, h->d.ngl, h->d.nat, h->g.eigr);
     CUW_LAUNCH_CHECK("k_eigr");
   }
-  if (todo & TAB_F32) CUW_RET(tc_pro_table(h, r_dev));
-  h->tabs = pos ? (h->tabs | todo) : 0;
+  if (need == TAB_F32) CUW_RET(tc_pro_table(h, r_dev));
+  h->tabs = pos ? need : 0;
   if (pos) h->eigr_src = r_dev;
   return CUW_OK;
 }

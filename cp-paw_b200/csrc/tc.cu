@@ -975,35 +975,25 @@ int tc_setup(Handle* h) {
   return CUW_OK;
 }
 
-// buffers whose sizes follow from the folded sphere (called with a new G set)
-int tc_rooms(Handle* h) {
-  Device& g = h->g;
-  auto alloc = [&](void** p, size_t bytes) -> int {
-    if (*p) return CUW_OK;
-    if (cudaMalloc(p, bytes) != cudaSuccess) {
-      cudaGetLastError();
-      *p = nullptr;
-      return h->fail(CUW_ERR_NOMEM, "cudaMalloc of mixed-path scratch failed");
-    }
-    return CUW_OK;
-  };
+// bytes of the buffers of the tensor-core products
+TcRooms tc_room_sizes(const Handle* h) {
   const int np = std::max(1, h->npro), nb = h->d.nb;
-  CUW_RET(alloc(reinterpret_cast<void**>(&g.pf), sizeof(float) * (size_t)h->ldu * np));
-  if (!g.u32) {
-    CUW_RET(alloc(reinterpret_cast<void**>(&g.u32), sizeof(float) * (size_t)h->ldu * nb * 2));
-    // the padding of the rows is read as K values past the sphere (k_bsplit)
-    if (h->ldu > 2 * h->nh)
-      CUW_TRY(cudaMemset2DAsync(g.u32 + 2 * h->nh, sizeof(float) * h->ldu, 0, sizeof(float) * (h->ldu - 2 * h->nh),
-                                (size_t)2 * nb, h->stream));
-  }
-  CUW_RET(alloc(reinterpret_cast<void**>(&g.bpre),
-                sizeof(float) * kBTile * 2 * (size_t)tiles_per_array(h) * ceil_div(2 * h->nh, kCK)));
   // largest small-matrix operand: [C1 | C2] of ADDPRO, DEDPRO or Lambda
   size_t slot = (size_t)ceil_div(nb, 64) * ceil_div(np, kCK);
   slot = std::max(slot, (size_t)ceil_div(np, 128) * ceil_div(nb, kCK));
   slot = std::max(slot, (size_t)ceil_div(nb, 128) * ceil_div(nb, kCK));
-  CUW_RET(alloc(reinterpret_cast<void**>(&g.bsmall), sizeof(float) * slot * kBTile));
-  CUW_RET(alloc(reinterpret_cast<void**>(&g.diag), sizeof(double) * 3 * (size_t)diag_ranges(h) * nb));
+  TcRooms r;
+  r.split = sizeof(float) * kBTile * 2 * (size_t)tiles_per_array(h) * ceil_div(2 * h->nh, kCK);
+  r.u32 = sizeof(float) * (size_t)h->ldu * nb * 2;
+  r.small = sizeof(float) * slot * kBTile;
+  r.diag = sizeof(double) * 3 * (size_t)diag_ranges(h) * nb;
+  return r;
+}
+// the padding of the rows of U is read as K values past the sphere (k_bsplit)
+int tc_clear_padding(Handle* h) {
+  if (h->ldu > 2 * h->nh)
+    CUW_TRY(cudaMemset2DAsync(h->g.u32 + 2 * h->nh, sizeof(float) * h->ldu, 0, sizeof(float) * (h->ldu - 2 * h->nh),
+                              (size_t)2 * h->d.nb, h->stream));
   return CUW_OK;
 }
 
@@ -1012,7 +1002,7 @@ int tc_pro_table(Handle* h, const double* r_dev) {
   const Device& g = h->g;
   k_pro_f32<<<dim3(ceil_div(h->nh, 256), h->d.nat), 256, 0, h->stream>>>(h->nh, h->d.ngl, h->ldu, g.half, g.gx, g.gy,
                                                                          g.gz, r_dev, g.t_ipro0, g.t_nlmn, g.pdesc,
-                                                                         g.ylm, g.pro, g.pf);
+                                                                         g.ylm, g.pro, g.pf());
   CUW_LAUNCH_CHECK("k_pro_f32");
   return CUW_OK;
 }
@@ -1043,7 +1033,7 @@ int tc_split(Handle* h, int nset) {
   b.set_stride = (long long)h->d.nb * h->ldu;
   DiagSums d{};
   if (nset == 2) d = {u32_slot(h, 0), u32_slot(h, 1), b.nk, h->ldu, b.nrow, diag_ranges(h), h->g.diag};
-  return tc_bsplit(h, b, nset * b.tps, ceil_div(2 * h->nh, kCK), h->g.bpre, d);
+  return tc_bsplit(h, b, nset * b.tps, ceil_div(2 * h->nh, kCK), h->g.bpre(), d);
 }
 
 // PROJ of slot 0 (and slot 1 when proj1 is given), from the split forms
@@ -1057,9 +1047,9 @@ int tc_proj(Handle* h, double2* proj0, double2* proj1) {
   a.tps = tiles_per_array(h);
   a.ldp = nset * nb;
   a.nchk = ceil_div(a.nk, kCK);
-  a.bs[0] = h->g.bpre;
+  a.bs[0] = h->g.bpre();
   TcTnMaps tm;
-  CUW_RET(map_kfast(h, &tm.a[0], h->g.pf, npro));
+  CUW_RET(map_kfast(h, &tm.a[0], h->g.pf(), npro));
   tm.a[1] = tm.a[2] = tm.a[0];
   const int tn = ceil_div(npro, 128), tb = nset * a.tps;
   int ks = tc_splits(h, tn * tb, a.nk, h->split_proj);
@@ -1080,7 +1070,7 @@ int tc_addpro(Handle* h, int mode, const double2* hpc, const double2* opc, const
   Device& g = h->g;
   const int nb = h->d.nb, npro = h->npro;
   CUtensorMap tpf;
-  CUW_RET(map_mfast(h, &tpf, g.pf, npro));
+  CUW_RET(map_mfast(h, &tpf, g.pf(), npro));
   const int nchk = ceil_div(npro, kCK);
   BSplitSrc b{};
   b.kind = 2;
@@ -1114,7 +1104,7 @@ int tc_gram(Handle* h, const FoldPair* pairs, int npair, double* o0, double* o1,
   for (int i = 0; i < 3; ++i) {
     const FoldPair& q = pairs[std::min(i, npair - 1)];
     CUW_RET(map_kfast(h, &tm.a[i], u32_slot(h, q.x), nb));
-    a.bs[i] = h->g.bpre + (size_t)q.y * tps * a.nchk * kBTile;
+    a.bs[i] = h->g.bpre() + (size_t)q.y * tps * a.nchk * kBTile;
   }
   int ks = tc_splits(h, tps * tps * npair, a.nk, h->split_gram);
   a.kchunk = ceil_div(ceil_div(a.nk, ks), kCK) * kCK;
@@ -1175,11 +1165,11 @@ int tc_force(Handle* h, const double2* ded, double* fpart, int* ntile) {
     // persistent form: the U tile stays in tensor memory across projector tiles
     const int nitems = tm * tn;
     k_tc_force_p<<<std::min(nitems, h->nsm), kThreads, kForcePSmem, h->stream>>>(
-        tu, g.bsmall, nchk, h->nh, npro, h->ldu, tn, nitems, g.pf, g.half, g.gx, g.gy, g.gz, fpart, tc_err(h));
+        tu, g.bsmall, nchk, h->nh, npro, h->ldu, tn, nitems, g.pf(), g.half, g.gx, g.gy, g.gz, fpart, tc_err(h));
     CUW_LAUNCH_CHECK("k_tc_force_p");
     return CUW_OK;
   }
-  k_tc_force<<<dim3(tm, tn), kThreads, ForcePipe::kSmem, h->stream>>>(tu, g.bsmall, nchk, h->nh, npro, h->ldu, g.pf,
+  k_tc_force<<<dim3(tm, tn), kThreads, ForcePipe::kSmem, h->stream>>>(tu, g.bsmall, nchk, h->nh, npro, h->ldu, g.pf(),
                                                                      g.half, g.gx, g.gy, g.gz, fpart, tc_err(h));
   CUW_LAUNCH_CHECK("k_tc_force");
   return CUW_OK;

@@ -108,3 +108,26 @@ def test_large_steps_keep_a_quarter_of_the_tolerance(size, ry, seed):
         assert e < bound, f"{name}: {e:.2e}"
     for w in state["sets"]:
         w.close()
+
+
+@pytest.mark.parametrize("name", ["Si8-20Ry", "H2O2"])
+def test_mixed_steps_between_fp64_routines(name):
+    """The FP64 routines of a mixed handle share the projector table's buffer and
+    that of the split wave functions: steps between them give the same bits."""
+    inp = systems.build_inputs(CASES[name]())
+    res = []
+    for between in (False, True):
+        w = cuwaves.open_waves(inp, precision=CUW_PREC_MIXED).setup().initialize()
+        out = []
+        for _ in range(4):
+            out.append(w.cp_step(move_atoms=True))
+            if between:
+                assert w.overlap_check()[1] < 1e-4
+                w.set_option(cuwaves.CUW_OPT_CONTRACTION_TILES, 1)
+                w.force()
+                w.set_option(cuwaves.CUW_OPT_CONTRACTION_TILES, 0)
+        out.append((w.download_psi(CUW_PSI0), w.get_proj()))
+        res.append(out)
+        w.close()
+    for (a0, a1), (b0, b1) in zip(*res):
+        assert np.array_equal(a0, b0) and np.array_equal(a1, b1)
