@@ -464,6 +464,9 @@ int fold_addx(Handle* h, int slot, const double* lam, double2* out);
 int fold_oc_splits(const Handle* h, int npair);
 int fold_oc(Handle* h, const FoldPair* pairs, int npair, int kc, double* oc);
 int fold_force(Handle* h, const double2* ded, double* fpart, int* nt);
+size_t part_bytes(const Handle* h);
+size_t fold_part_bytes(const Handle* h);
+size_t tc_part_bytes(const Handle* h);
 int ensure_part(Handle* h, size_t bytes);  // split-K scratch h->g.part of at least `bytes`
 // Raises (never lowers) the dynamic shared-memory limit of kernel fn on the
 // current device.  The limit belongs to the function, so it is shared by all

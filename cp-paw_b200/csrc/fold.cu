@@ -772,7 +772,8 @@ int fold_setup(Handle* h, const std::vector<int>& mg) {
   CUW_TRY(cudaMemcpyAsync(&bad, flag, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
   CUW_TRY(cudaStreamSynchronize(h->stream));
   h->sym = bad == 0;
-  return fold_rooms(h);
+  CUW_RET(fold_rooms(h));
+  return ensure_part(h, part_bytes(h));
 }
 
 // Buffers whose sizes follow from the folded sphere: two folded wave-function
@@ -833,17 +834,32 @@ int fold_table(Handle* h, const double* r_dev) {
   return CUW_OK;
 }
 
+// tile and K splits of the projections of nset arrays, and the bytes of their sums
+struct ProjSplit {
+  RTile t;
+  int ks, kchunk;
+  size_t bytes;
+};
+static ProjSplit proj_split(const Handle* h, int nset) {
+  const int nt = h->d.nb * nset, npro = h->npro, nr = 2 * h->nh;
+  ProjSplit s;
+  s.t = pick_tile(h, npro, nt);
+  s.t.mi = s.t.ni == 8 ? 4 : 2;
+  const int tiles = ceil_div(nt, 16 * s.t.ni) * ceil_div(npro, 16 * s.t.mi);
+  s.kchunk = ceil_div(ceil_div(nr, rsplit(h, tiles, nr, h->split_proj)), RK) * RK;
+  s.ks = ceil_div(nr, s.kchunk);
+  s.bytes = sizeof(double) * (size_t)s.ks * nt * npro;
+  return s;
+}
+
 // PROJ of slot 0 (and slot 1 when proj1 is given)
 int fold_proj(Handle* h, double2* proj0, double2* proj1) {
-  const int nb = h->d.nb, nset = proj1 ? 2 : 1, nt = nb * nset, npro = h->npro, nr = 2 * h->nh;
+  const int nset = proj1 ? 2 : 1, nt = h->d.nb * nset, npro = h->npro, nr = 2 * h->nh;
   if (npro == 0) return CUW_OK;
-  RTile t = pick_tile(h, npro, nt);
-  t.mi = t.ni == 8 ? 4 : 2;
-  const int tiles = ceil_div(nt, 16 * t.ni) * ceil_div(npro, 16 * t.mi);
-  int ks = rsplit(h, tiles, nr, h->split_proj);
-  const int kchunk = ceil_div(ceil_div(nr, ks), RK) * RK;
-  ks = ceil_div(nr, kchunk);
-  CUW_RET(ensure_part(h, sizeof(double) * (size_t)ks * nt * npro));
+  const ProjSplit s = proj_split(h, nset);
+  const RTile t = s.t;
+  const int ks = s.ks, kchunk = s.kchunk;
+  CUW_RET(ensure_part(h, s.bytes));
   double* part = reinterpret_cast<double*>(h->g.part);
   const Op p{h->g.prox, h->ldu, npro}, u{h->g.uf, h->ldu, nt};
   const dim3 grid(ceil_div(nt, 16 * t.ni), ceil_div(npro, 16 * t.mi), ks);
@@ -888,18 +904,36 @@ static int gram_launch(Handle* h, const RGramArgs& a, RTile t, int nz, double* p
   return CUW_OK;
 }
 
+// splits of the overlaps of npair pairs, and the bytes of their sums
+struct GramSplit {
+  int ks, kchunk, kc, pchunk;
+  size_t bytes;
+};
+static GramSplit gram_split(const Handle* h, int npair) {
+  const RTile t = gram_tile(h);
+  const int nb = h->d.nb, npro = h->npro, nr = 2 * h->nh;
+  const int tiles = ceil_div(nb, 16 * t.ni) * ceil_div(nb, 16 * t.mi) * npair;
+  // the one-centre sums take splits of about the same length
+  const int ks0 = rsplit(h, tiles, nr, h->split_gram);
+  GramSplit s;
+  s.pchunk = std::max(RK, ceil_div(std::min(npro, ceil_div(nr, ks0)), RK) * RK);
+  s.kc = ceil_div(npro, s.pchunk);
+  s.kchunk = ceil_div(ceil_div(nr, std::max(1, ks0 - s.kc)), RK) * RK;
+  s.ks = ceil_div(nr, s.kchunk);
+  s.bytes = sizeof(double) * (size_t)(s.ks + s.kc) * npair * nb * nb;
+  return s;
+}
+
 int fold_gram(Handle* h, const FoldPair* pairs, int npair, double* o0, double* o1, double* o2) {
   RGramArgs a;
   CUW_RET(gram_args(h, pairs, npair, &a));
   const RTile t = gram_tile(h);
-  const int tiles = ceil_div(a.nb, 16 * t.ni) * ceil_div(a.nb, 16 * t.mi) * npair;
-  // the one-centre sums take splits of about the same length
-  const int ks0 = rsplit(h, tiles, a.nr, h->split_gram);
-  a.pchunk = std::max(RK, ceil_div(std::min(a.npro, ceil_div(a.nr, ks0)), RK) * RK);
-  const int kc = ceil_div(a.npro, a.pchunk), ks1 = std::max(1, ks0 - kc);
-  a.kchunk = ceil_div(ceil_div(a.nr, ks1), RK) * RK;
-  const int ks = a.ks = ceil_div(a.nr, a.kchunk), nb = a.nb;
-  CUW_RET(ensure_part(h, sizeof(double) * (size_t)(ks + kc) * npair * nb * nb));
+  const GramSplit s = gram_split(h, npair);
+  a.pchunk = s.pchunk;
+  a.kchunk = s.kchunk;
+  a.ks = s.ks;
+  const int ks = s.ks, kc = s.kc, nb = a.nb;
+  CUW_RET(ensure_part(h, s.bytes));
   CUW_RET(gram_launch(h, a, t, ks + kc, reinterpret_cast<double*>(h->g.part)));
   const size_t n = (size_t)nb * nb / 2 * npair;
   k_rgram_sum<<<(unsigned)((n + 31) / 32), dim3(32, kSumZ), 0, h->stream>>>(h->g.part, ks, kc, nb, npair,
@@ -999,6 +1033,13 @@ int fold_force(Handle* h, const double2* ded, double* fpart, int* nt) {
   CUW_LAUNCH_CHECK("k_rforce");
   *nt = gx;
   return CUW_OK;
+}
+
+// bytes of the split sums that the folded products of this set need at most
+size_t fold_part_bytes(const Handle* h) {
+  size_t n = std::max(gram_split(h, 1).bytes, gram_split(h, 3).bytes);
+  if (h->sym && h->npro) n = std::max({n, proj_split(h, 1).bytes, proj_split(h, 2).bytes});
+  return n;
 }
 
 int fold_kernels_setup(Handle* h) {

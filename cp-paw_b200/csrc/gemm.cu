@@ -736,12 +736,36 @@ int ensure_part(Handle* h, size_t bytes) {
   return CUW_OK;
 }
 
-static int choose_split(Handle* h, int tiles, int nk, int minchunk, double mul) {
+static int choose_split(const Handle* h, int tiles, int nk, int minchunk, double mul) {
   // at most 2 mul waves of one CTA per SM (rounded down: a CTA past a whole
   // wave would cost a wave of its own)
   int want = std::max(1, (int)std::floor(2.0 * h->nsm * mul / std::max(1, tiles)));
   int maxs = std::max(1, ceil_div(nk, minchunk));
   return std::min(want, maxs);
+}
+
+// K splits of the complex projections
+static int complex_proj_splits(const Handle* h, int* kchunk) {
+  const int ngl = h->d.ngl, tiles = ceil_div(h->npro, BN) * ceil_div(h->d.nbh, BM);
+  *kchunk = ceil_div(ceil_div(ngl, choose_split(h, tiles, ngl, 256, h->split_proj)), BK) * BK;
+  return ceil_div(ngl, *kchunk);
+}
+// row groups of the force sums: tiles of 64 or 128 G, or CTAs of the folded form
+static size_t force_bytes(const Handle* h) {
+  return sizeof(double) * 3 * (size_t)std::max(ceil_div(h->d.ngl, BM), 2 * h->nsm) * h->npro;
+}
+// Bytes of g.part for every routine of this set: allocated with the G set, so that
+// no first call has to free and allocate it again (which took 0.3 to 0.7 ms of a
+// new set's first single point).  A share of the SMs needs less; only a tuned split
+// factor or more SMs than at set-up need more.
+size_t part_bytes(const Handle* h) {
+  size_t n = std::max(force_bytes(h), fold_part_bytes(h));
+  if (h->mixed() && h->sym) n = std::max(n, tc_part_bytes(h));
+  if (!h->sym) {
+    int kchunk;
+    n = std::max(n, 2 * sizeof(double2) * (size_t)complex_proj_splits(h, &kchunk) * h->d.nbh * h->npro);
+  }
+  return n;
 }
 
 // Tables of the projectors at r_dev that the present path reads: the folded
@@ -785,9 +809,8 @@ int proj_compute(Handle* h, const double2* psiA, double2* projA, const double2* 
   }
   const int nbh = h->d.nbh, npro = h->npro, ngl = h->d.ngl;
   const int tn = ceil_div(npro, BN), tm = ceil_div(nbh, BM);
-  int ks = choose_split(h, tn * tm, ngl, 256, h->split_proj);
-  int kchunk = ceil_div(ceil_div(ngl, ks), BK) * BK;
-  ks = ceil_div(ngl, kchunk);
+  int kchunk;
+  const int ks = complex_proj_splits(h, &kchunk);
   const size_t one = (size_t)ks * nbh * npro;
   const bool dual = (psiB != nullptr);
   CUW_RET(ensure_part(h, sizeof(double2) * one * (dual ? 2 : 1)));
@@ -956,8 +979,7 @@ int oproj_compute(Handle* h, const double2* proj, double2* out, const double2* p
 int force_gemm(Handle* h, const double2* ded, double* force_dev) {
   const int ngl = h->d.ngl, nbh = h->d.nbh, npro = h->npro;
   int tm = ceil_div(ngl, BM);
-  // row groups of the partial sums: tiles of 64 or 128 G, or CTAs of the folded form
-  CUW_RET(ensure_part(h, sizeof(double) * 3 * (size_t)std::max(tm, 2 * h->nsm) * npro));
+  CUW_RET(ensure_part(h, force_bytes(h)));
   double* fpart = reinterpret_cast<double*>(h->g.part);
   if (h->tc_on()) {
     CUW_RET(tc_fold(h, h->g.psi0, 0));

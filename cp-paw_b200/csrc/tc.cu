@@ -907,11 +907,44 @@ __global__ void __launch_bounds__(256) k_bsplit(BSplitSrc b, int nchk, float* __
 static int* tc_err(Handle* h) { return h->g.ostatus + 12; }
 
 // number of K splits so that tiles * splits fills the GPU once (one CTA per SM)
-static int tc_splits(Handle* h, int tiles, int nk, double mul) {
+static int tc_splits(const Handle* h, int tiles, int nk, double mul) {
   // at most mul waves of one CTA per SM (rounded down: a CTA past a whole
   // wave would cost a wave of its own)
   const int want = std::max(1, (int)std::floor(h->nsm * mul / std::max(1, tiles)));
   return std::max(1, std::min(want, ceil_div(nk, 4 * kCK)));
+}
+
+static int tiles_per_array(const Handle* h) { return ceil_div(h->d.nb, 128); }
+// K splits of the projections of nset arrays and of the overlaps of npair pairs,
+// and the bytes of their sums
+struct TcSplit {
+  int ks, kchunk, kc;  // kc: splits of the one-centre sums
+  size_t oc, bytes;    // oc: offset of the one-centre sums
+};
+static TcSplit tc_split_k(const Handle* h, int tiles, double mul) {
+  const int nk = 2 * h->nh;
+  TcSplit s{};
+  s.kchunk = ceil_div(ceil_div(nk, tc_splits(h, tiles, nk, mul)), kCK) * kCK;
+  s.ks = ceil_div(nk, s.kchunk);
+  return s;
+}
+static TcSplit tc_proj_split(const Handle* h, int nset) {
+  TcSplit s = tc_split_k(h, ceil_div(h->npro, 128) * nset * tiles_per_array(h), h->split_proj);
+  s.bytes = sizeof(float2) * (size_t)nset * h->d.nbh * h->npro * s.ks;
+  return s;
+}
+static TcSplit tc_gram_split(const Handle* h, int npair) {
+  TcSplit s = tc_split_k(h, tiles_per_array(h) * tiles_per_array(h) * npair, h->split_gram);
+  // the one-centre sums stay in FP64, behind the fp32 partials
+  const size_t n = (size_t)h->d.nb * h->d.nb * npair;
+  s.kc = fold_oc_splits(h, npair);
+  s.oc = (sizeof(float) * n * s.ks + 255) / 256 * 256;
+  s.bytes = s.oc + sizeof(double) * n * s.kc;
+  return s;
+}
+// bytes of the split sums that the tensor-core products of this set need at most
+size_t tc_part_bytes(const Handle* h) {
+  return std::max({tc_proj_split(h, 1).bytes, tc_proj_split(h, 2).bytes, tc_gram_split(h, 3).bytes});
 }
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (the
@@ -960,7 +993,6 @@ static int map_mfast(Handle* h, CUtensorMap* m, const float* base, int rows) {
 static float* u32_slot(const Handle* h, int slot) { return h->g.u32 + (size_t)slot * h->d.nb * h->ldu; }
 // ranges of diag_sums
 static int diag_ranges(const Handle* h) { return ceil_div(2 * h->nh, kDiagK); }
-static int tiles_per_array(const Handle* h) { return ceil_div(h->d.nb, 128); }
 
 int tc_setup(Handle* h) {
   CUW_TRY(smem_allow((const void*)k_tc_tn<ProjPipe>, (int)ProjPipe::kSmem));
@@ -1052,11 +1084,11 @@ int tc_proj(Handle* h, double2* proj0, double2* proj1) {
   CUW_RET(map_kfast(h, &tm.a[0], h->g.pf(), npro));
   tm.a[1] = tm.a[2] = tm.a[0];
   const int tn = ceil_div(npro, 128), tb = nset * a.tps;
-  int ks = tc_splits(h, tn * tb, a.nk, h->split_proj);
-  a.kchunk = ceil_div(ceil_div(a.nk, ks), kCK) * kCK;
-  ks = ceil_div(a.nk, a.kchunk);
+  const TcSplit s = tc_proj_split(h, nset);
+  const int ks = s.ks;
+  a.kchunk = s.kchunk;
   const size_t n = (size_t)nset * h->d.nbh * npro;
-  CUW_RET(ensure_part(h, sizeof(float2) * n * ks));
+  CUW_RET(ensure_part(h, s.bytes));
   k_tc_tn<ProjPipe><<<dim3(tn, tb, ks), kThreads, ProjPipe::kSmem, h->stream>>>(a, tm, reinterpret_cast<float*>(h->g.part),
                                                                       tc_err(h));
   CUW_LAUNCH_CHECK("k_tc_tn");
@@ -1106,15 +1138,12 @@ int tc_gram(Handle* h, const FoldPair* pairs, int npair, double* o0, double* o1,
     CUW_RET(map_kfast(h, &tm.a[i], u32_slot(h, q.x), nb));
     a.bs[i] = h->g.bpre() + (size_t)q.y * tps * a.nchk * kBTile;
   }
-  int ks = tc_splits(h, tps * tps * npair, a.nk, h->split_gram);
-  a.kchunk = ceil_div(ceil_div(a.nk, ks), kCK) * kCK;
-  ks = ceil_div(a.nk, a.kchunk);
-  // the one-centre sums stay in FP64, behind the fp32 partials
+  const TcSplit s = tc_gram_split(h, npair);
+  const int ks = s.ks, kc = s.kc;
+  a.kchunk = s.kchunk;
   const size_t n = (size_t)nb * nb * npair;
-  const int kc = fold_oc_splits(h, npair);
-  const size_t off = (sizeof(float) * n * ks + 255) / 256 * 256;
-  CUW_RET(ensure_part(h, off + sizeof(double) * n * kc));
-  double* oc = reinterpret_cast<double*>(reinterpret_cast<char*>(h->g.part) + off);
+  CUW_RET(ensure_part(h, s.bytes));
+  double* oc = reinterpret_cast<double*>(reinterpret_cast<char*>(h->g.part) + s.oc);
   CUW_RET(fold_oc(h, pairs, npair, kc, oc));
   k_tc_tn<GramPipe><<<dim3(tps, tps, ks * npair), kThreads, GramPipe::kSmem, h->stream>>>(
       a, tm, reinterpret_cast<float*>(h->g.part), tc_err(h));

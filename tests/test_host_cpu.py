@@ -79,3 +79,29 @@ def test_launches_of_long_cells(fake_engine, nb):
     w.cp_step(move_atoms=True)
     w.close()
     assert fake_engine.lib.fake_misuse() == 0
+
+
+SETS = {
+    "Si2": lambda: systems.si_small(2, epw_psi_ry=12.0),
+    "Si8": lambda: systems.si_supercell(1, 1, 1),
+    "H2O8": lambda: systems.water_cluster(8),  # many plane waves for few bands
+    "Si64": lambda: systems.si_supercell(2, 2, 2),
+}
+
+
+@pytest.mark.parametrize("prec", PRECISIONS)
+@pytest.mark.parametrize("name", SETS)
+def test_set_up_allocates_for_every_routine(fake_engine, prec, name):
+    """The first calls of a new set allocate nothing: what the contractions need is
+    known with the G set."""
+    w = fake_engine.open(inputs(SETS[name]()), prec).setup()
+    before = fake_engine.lib.fake_mallocs()
+    w.gramschmidt(0, w.inp["r0"])
+    w.projections()
+    w.hpsi()
+    w.etot()
+    w.overlap_check()
+    for _ in range(2):
+        w.cp_step(move_atoms=True)
+    assert fake_engine.lib.fake_mallocs() == before
+    w.close()
