@@ -451,6 +451,7 @@ struct FoldRooms {
   size_t uf, prox, eigr;  // prox for tables with parity, else eigr
   TcRooms tc;             // mixed path
 };
+size_t fold_bytes(Handle* h);
 int fold_rooms(Handle* h);
 int fold_table(Handle* h, const double* r_dev);
 int fold_psi(Handle* h, const double2* psi, int slot);

@@ -793,6 +793,20 @@ static FoldRooms room_sizes(const Handle* h) {
   return r;
 }
 
+// bytes of all of them and of the split-sum scratch, whatever the tables' parity;
+// of the handle only the sizes are read
+size_t fold_bytes(Handle* h) {
+  const FoldRooms r = room_sizes(h);
+  const bool sym = h->sym;
+  size_t n = 0;
+  for (bool s : {false, true}) {
+    h->sym = s;
+    n = std::max(n, part_bytes(h) + (s ? r.prox + r.tc.u32 + r.tc.small + r.tc.diag : r.eigr));
+  }
+  h->sym = sym;
+  return sizeof(int2) * h->nh + r.uf + n;
+}
+
 int fold_rooms(Handle* h) {
   auto room = [&](auto*& p, size_t bytes, const char* what) -> int {
     if (p || bytes == 0) return CUW_OK;

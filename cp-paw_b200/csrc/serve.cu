@@ -26,7 +26,7 @@
 #include <thread>
 #include <vector>
 
-#include "../../include/cuwaves.h"
+#include "cuwaves_internal.cuh"
 
 namespace cuw {
 int handle_recycle(cuw_handle* h);  // capi.cu
@@ -99,24 +99,32 @@ int count_projectors(const cuw_dims& d, const int* isp) {
   return n;
 }
 
-// Upper estimate of the device memory of one handle (the allocations of
-// cuwaves_create and the FFT set-up, plus the split-K scratch).
-size_t estimate_bytes(const cuw_dims& d, const int* isp) {
+// Upper estimate of the device memory of one handle: the allocations of
+// cuwaves_create and the FFT set-up, the buffers of the contractions (the sizes
+// that set_gset allocates, for tables with or without parity), and 20 MB for small
+// tables and what the driver rounds up.
+size_t estimate_bytes(const cuw_dims& d, const int* isp, const int* minusg) {
+  cuw::Handle h;  // sizes only
+  h.d = d;
+  h.npro = count_projectors(d, isp);
+  for (int i = 0; i < d.ngl; ++i) h.nh += i + 1 <= minusg[i];
+  h.ldu = cuw::ceil_div(2 * h.nh, 32) * 32;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&h.nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    cudaGetLastError();  // no device: admission still works, by the default count
   const size_t ldg = (size_t)((d.ngl + 31) / 32) * 32, nbh = d.nbh, nb = d.nb, ngl = d.ngl;
-  const size_t npro = count_projectors(d, isp);
   size_t nbare = 0;
   for (int s = 0; s < d.nsp; ++s) nbare += d.lnx[s];
   const size_t nr = (size_t)d.nr1 * d.nr2 * d.nr3;
+  const size_t point = h.mixed() ? sizeof(float2) : sizeof(double2);
   size_t b = 4 * ldg * nbh * 16;                       // psi0, psim, hpsi, opsi
-  b += 4 * nbh * npro * 16;                            // proj, oproj, hproj, pbuf
+  b += 4 * nbh * (size_t)h.npro * 16;                  // proj, oproj, hproj, pbuf
   b += 2 * nb * nb * 16 + 24 * nb * nb * 8;            // Lagrange and solve matrices
-  b += ngl * (3 * 4 + 7 * 8) + ngl * (nbare + d.lmx) * 8;  // G set and tables
+  b += ngl * (7 * 4 + 8 * 8) + ngl * (nbare + d.lmx) * 8;  // G set and tables
   b += nr * 8;                                         // V(r)
-  b += std::min(nbh * nr * 16, ((size_t)48 << 20) + nr * 16);  // FFT work grid
-  b += (size_t)20 << 20;                               // split-K partials and small tables
-  if (d.precision == CUW_PREC_MIXED) b += ldg * npro * 8 + ngl * (size_t)d.nat * 16;  // projector tables (fp32, start-up fp64)
-  else b += ldg * npro * 8 + 2 * ldg * nbh * 16;  // folded fp64 projector table and wave functions
-  return b;
+  b += std::min(nbh * nr * point, std::max((size_t)48 << 20, nr * point));  // FFT work grid
+  return b + cuw::fold_bytes(&h) + ((size_t)20 << 20);
 }
 
 }  // namespace
@@ -428,7 +436,7 @@ extern "C" int cuwaves_server_submit(cuw_server* s, const cuw_request* r, long l
   j->lmnxx = r->lmnxx;
   j->lnxx = r->lnxx;
   j->nsteps = r->nsteps;
-  j->bytes = estimate_bytes(d, in.isp);
+  j->bytes = estimate_bytes(d, in.isp, in.minusg);
   if (j->bytes > s->budget) return CUW_ERR_NOMEM;  // could never be admitted
   {
     // sizes and G set: a pooled handle with the same key serves this request

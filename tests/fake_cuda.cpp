@@ -76,6 +76,7 @@ long long fake_peak() { return (long long)peak; }
 long long fake_mallocs() { return mallocs; }
 long long fake_waits() { return waits; }
 int fake_misuse() { return misuse; }
+void fake_reset_peak() { peak = in_use; }
 // the n-th cudaMalloc from now on fails (1 = the next; -1: none)
 void fake_fail_malloc(long long n) { fail_at = n < 0 ? -1 : mallocs + n; }
 // names of the kernels launched since the last call, one per line; their length

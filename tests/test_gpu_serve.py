@@ -128,6 +128,21 @@ def test_estimate_bounds_the_allocation(inputs):
     assert free0 - free1 <= est, (free0 - free1, est)
 
 
+def test_estimate_bounds_the_mixed_allocation():
+    """The same for a mixed set, whose buffers differ."""
+    import torch
+
+    inp = systems.build_inputs(systems.serving_system("W", 8, 1))
+    est = run_alone(inp, 1, False, CUW_PREC_MIXED)[2]["peak_bytes"]
+    torch.cuda.synchronize()
+    free0 = torch.cuda.mem_get_info()[0]
+    w = cuwaves.open_waves(inp, precision=CUW_PREC_MIXED).setup().initialize()
+    w.cp_step()
+    free1 = torch.cuda.mem_get_info()[0]
+    w.close()
+    assert free0 - free1 <= est, (free0 - free1, est)
+
+
 def test_handles_of_different_grids_interleave():
     """Kernel launch limits are per function and shared by every handle: a set
     created after a larger one must not break the larger one's next step."""

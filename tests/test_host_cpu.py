@@ -105,3 +105,26 @@ def test_set_up_allocates_for_every_routine(fake_engine, prec, name):
         w.cp_step(move_atoms=True)
     assert fake_engine.lib.fake_mallocs() == before
     w.close()
+
+
+@pytest.mark.parametrize("prec", PRECISIONS)
+@pytest.mark.parametrize("name", SETS)
+def test_admission_estimate_bounds_the_memory(fake_engine, prec, name, monkeypatch):
+    """The serving runtime admits a set by an estimate of its device memory: never
+    below what the set allocates, and not far above it."""
+    from cuwaves import serve
+
+    monkeypatch.setattr(serve, "load_library", lambda: fake_engine.lib)
+    monkeypatch.setattr(serve, "_fns", None)
+    inp = inputs(SETS[name]())
+    srv = serve.Server(hbm_budget=1 << 40, workers=1)
+    before = fake_engine.lib.fake_in_use()
+    fake_engine.lib.fake_reset_peak()
+    for nsteps in (0, 2):
+        srv.submit(inp, nsteps=nsteps, precision=prec)
+        srv.wait_all()
+    held = fake_engine.lib.fake_peak() - before
+    est = srv.stats()["peak_bytes"]
+    srv.close()
+    print(f"{name}: {held / 1e6:.1f} MB held, {est / 1e6:.1f} MB estimated")
+    assert held <= est <= 1.1 * held + (24 << 20)
