@@ -24,8 +24,8 @@
 //
 // The projectors satisfy p(-G) = conj p(G) whenever the tables of the G set do
 // (Y_lm(-G) = (-1)^l Y_lm(G), P(|G|) even, G(-G) = -G(G)); fold_setup checks
-// that bit for bit and, where a caller's tables do not, leaves the projector
-// contractions to the complex kernels of gemm.cu.  The overlaps and the
+// that to the last few bits and, where a caller's tables do not, leaves the
+// projector contractions to the complex kernels of gemm.cu.  The overlaps and the
 // rotation by Lambda need only MINUSG and are folded always.
 //
 // One CTA of 128 threads (2 x 2 warps) forms a tile of 16 MI x 16 NI outputs,
@@ -202,18 +202,33 @@ __device__ __forceinline__ void azero(double (&acc)[MI][NI][2]) {
 // ---------------------------------------------------------------------------
 // tables: symmetry of the G set, folded wave functions, folded projectors
 // ---------------------------------------------------------------------------
+// Parity to within kParityUlp units in the last place (of |G|, of the radial
+// value, and of 1 for the spherical harmonics, which cancel near their nodal
+// planes): a host's vectorised or fused arithmetic need not give both signs of G
+// the same bits.  The folded table then takes the values at one of the two, which
+// changes the projectors by less than the phase exp(-iG.R) is rounded.  With bit
+// equality asked for, one such value sent the whole set to the complex kernels (a
+// CP step of Si64 takes 2.57 ms there against 1.59 in FP64, and 2.38 against 1.02
+// on the mixed path).
+constexpr double kParityUlp = 8 * 2.220446049250313e-16;
+__device__ __forceinline__ bool near(double a, double b, double scale) { return fabs(a - b) <= kParityUlp * scale; }
+
 __global__ void k_sym_check(int ngl, int nbare, int lmx, const int* __restrict__ minusg, const double* __restrict__ gx,
                             const double* __restrict__ gy, const double* __restrict__ gz,
                             const double* __restrict__ ylm, const double* __restrict__ pro, int* __restrict__ bad) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= ngl) return;
   const int m = minusg[g];
-  bool ok = gx[m] == -gx[g] && gy[m] == -gy[g] && gz[m] == -gz[g];
-  for (int i = 0; i < nbare; ++i) ok = ok && pro[(size_t)m + (size_t)ngl * i] == pro[(size_t)g + (size_t)ngl * i];
+  const double len = fabs(gx[g]) + fabs(gy[g]) + fabs(gz[g]);
+  bool ok = near(gx[m], -gx[g], len) && near(gy[m], -gy[g], len) && near(gz[m], -gz[g], len);
+  for (int i = 0; i < nbare; ++i) {
+    const double p = pro[(size_t)g + (size_t)ngl * i];
+    ok = ok && near(pro[(size_t)m + (size_t)ngl * i], p, fabs(p));
+  }
   for (int l = 0; l * l < lmx; ++l)
     for (int i = l * l; i < min(lmx, (l + 1) * (l + 1)); ++i) {
       const double y = ylm[(size_t)g + (size_t)ngl * i];
-      ok = ok && ylm[(size_t)m + (size_t)ngl * i] == ((l & 1) ? -y : y);
+      ok = ok && near(ylm[(size_t)m + (size_t)ngl * i], (l & 1) ? -y : y, 1.0);
     }
   if (!ok) *bad = 1;
 }
