@@ -413,7 +413,7 @@ int propagate_run(Handle* h) {
   return CUW_OK;
 }
 
-// DEDPROJ in h->g.hproj, then forces into force_dev (uses eigr of R(0))
+// DEDPROJ in h->g.hproj, then forces into force_dev (from the projector tables of R(0))
 static int force_dev_run(Handle* h, double* force_dev) {
   Device& g = h->g;
   const int nbh = h->d.nbh, npro = h->npro, nb = h->d.nb;
@@ -1126,7 +1126,7 @@ extern "C" int cuwaves_gramschmidt(cuw_handle* hp, int which, const double* r) {
 }
 
 // One CP step (see the header).  Kernel order:
-//   EKIN, WAVEKINETIC(1) | EIGR(R0) | forces | FFT V.psi | DH.PROJ, DO.PROJ |
+//   EKIN, WAVEKINETIC(1) | projector tables of R(0) | forces | FFT V.psi | DH.PROJ, DO.PROJ |
 //   fused ADDPRO (HPSI, OPSI, PROPAGATE) | <psi|H|psi> | atoms |
 //   ORTHOGONALIZE at R(+) | WAVEKINETIC(2) | SWITCH
 // Single-point evaluation at the current wave functions and positions, the
@@ -1135,7 +1135,7 @@ extern "C" int cuwaves_gramschmidt(cuw_handle* hp, int which, const double* r) {
 // (WAVES_OVERLAP) plus one-centre part (WAVES_1COVERLAP) of projections formed
 // afresh at R(0), as the real NB x NB matrix of the Gamma point.  Always FP64,
 // whatever the handle's precision, so that it measures the state itself.
-// Uses only scratch of the step (PBUF, HPROJ, TMAT, WK2); PROJ is untouched.
+// Uses only scratch of the step (PBUF, HPROJ, WK2, the folded arrays); PROJ is untouched.
 extern "C" int cuwaves_overlap_check(cuw_handle* hp, double* mat, double* maxdev) {
   H(hp);
   NEED(h->have_gset && h->have_do, CUW_ERR_STATE, "inputs not loaded");

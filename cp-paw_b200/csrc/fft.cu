@@ -304,10 +304,10 @@ __host__ __device__ constexpr Split2 split2(int N) {
 
 // One Stockham stage on lines [line0, line0+nl) of length n held in shared
 // memory: element e of line L lives at buf[L*ls + e*es].  tw[k] = exp(sgn*2 pi i k/n).
-// jfast selects the thread mapping (consecutive threads -> consecutive j).
+// Consecutive threads take consecutive lines.
 // The caller guarantees nl*n/R <= blockDim.x * BPT.
 template <int R, class C>
-__device__ __noinline__ void stage(C* buf, int n, int ns, int line0, int nl, int ls, int es, bool jfast,
+__device__ __noinline__ void stage(C* buf, int n, int ns, int line0, int nl, int ls, int es,
                                       const C* tw, typename CT<C>::R sgn) {
   constexpr int BPT = (kMaxV / R) > 0 ? (kMaxV / R) : 1;
   const int nq = n / R;
@@ -319,10 +319,7 @@ __device__ __noinline__ void stage(C* buf, int n, int ns, int line0, int nl, int
     int bf = threadIdx.x + t * blockDim.x;
     line_[t] = -1;
     if (bf < total) {
-      int line, j;
-      if (jfast) { j = bf % nq; line = bf / nq; }
-      else { line = bf % nl; j = bf / nl; }
-      line += line0;
+      const int j = bf / nl, line = line0 + bf % nl;
       line_[t] = line;
       j_[t] = j;
       const int k = j % ns;
@@ -391,24 +388,20 @@ __host__ __device__ constexpr int chunk_lines(int N) {
 }
 
 template <int N, int R, int NS, int LC, class C>
-__device__ __forceinline__ void stage_fixed(C* buf, int line0, int nl, int ls, int es, bool jfast, const C* tw,
+__device__ __forceinline__ void stage_fixed(C* buf, int line0, int nl, int ls, int es, const C* tw,
                                             typename CT<C>::R sgn) {
   constexpr int BPT = bpt_of(R);
   constexpr int NQ = N / R;
   constexpr int TSTEP = N / (NS * R);
-  // jfast: index space nl*NQ (line = bf / NQ); otherwise the full chunk LC*NQ
-  // decoded modulo LC, with the lines beyond nl masked
-  const int total = jfast ? nl * NQ : LC * NQ;
+  // the full chunk LC*NQ decoded modulo LC, with the lines beyond nl masked
   C v[BPT][R];
   int off_[BPT];
   bool act[BPT];
 #pragma unroll
   for (int t = 0; t < BPT; ++t) {
     const int bf = threadIdx.x + t * kPlaneThreads;
-    int line, j;
-    if (jfast) { j = bf % NQ; line = bf / NQ; }
-    else { line = bf % LC; j = bf / LC; }
-    act[t] = (bf < total) && (line < nl) && (j < NQ);
+    const int line = bf % LC, j = bf / LC;
+    act[t] = line < nl && j < NQ;
     const int k = j % NS;
     off_[t] = line * N + ((j / NS) * NS * R + k);  // (line, destination index) packed
     if (act[t]) {
@@ -436,22 +429,22 @@ __device__ __forceinline__ void stage_fixed(C* buf, int line0, int nl, int ls, i
 }
 
 template <int N, int S, int NS, int LC, class C>
-__device__ __forceinline__ void stages_fixed(C* buf, int line0, int nl, int ls, int es, bool jfast, const C* tw,
+__device__ __forceinline__ void stages_fixed(C* buf, int line0, int nl, int ls, int es, const C* tw,
                                              typename CT<C>::R sgn) {
   constexpr RadixList L = radices_of(N);
   if constexpr (S < L.n) {
     constexpr int R = L.r[S];
-    stage_fixed<N, R, NS, LC>(buf, line0, nl, ls, es, jfast, tw, sgn);
-    stages_fixed<N, S + 1, NS * R, LC>(buf, line0, nl, ls, es, jfast, tw, sgn);
+    stage_fixed<N, R, NS, LC>(buf, line0, nl, ls, es, tw, sgn);
+    stages_fixed<N, S + 1, NS * R, LC>(buf, line0, nl, ls, es, tw, sgn);
   }
 }
 
 template <int N, class C>
-__device__ void transform_fixed(C* buf, int nlines, int ls, int es, bool jfast, const C* tw, typename CT<C>::R sgn) {
+__device__ void transform_fixed(C* buf, int nlines, int ls, int es, const C* tw, typename CT<C>::R sgn) {
   constexpr int LC = chunk_lines(N);
   for (int l0 = 0; l0 < nlines; l0 += LC) {
     const int nl = min(LC, nlines - l0);
-    stages_fixed<N, 0, 1, LC>(buf, l0, nl, ls, es, jfast, tw, sgn);
+    stages_fixed<N, 0, 1, LC>(buf, l0, nl, ls, es, tw, sgn);
   }
 }
 
@@ -468,22 +461,22 @@ __device__ __forceinline__ int lines_per_chunk(const AxisArg& ax, int nlines) {
 }
 
 template <class C>
-__device__ void transform(C* buf, const AxisArg& ax, int nlines, int ls, int es, bool jfast, const C* tw,
+__device__ void transform(C* buf, const AxisArg& ax, int nlines, int ls, int es, const C* tw,
                           typename CT<C>::R sgn) {
   switch (ax.n) {
-    case 16: transform_fixed<16>(buf, nlines, ls, es, jfast, tw, sgn); return;
-    case 20: transform_fixed<20>(buf, nlines, ls, es, jfast, tw, sgn); return;
-    case 24: transform_fixed<24>(buf, nlines, ls, es, jfast, tw, sgn); return;
-    case 28: transform_fixed<28>(buf, nlines, ls, es, jfast, tw, sgn); return;
-    case 32: transform_fixed<32>(buf, nlines, ls, es, jfast, tw, sgn); return;
-    case 36: transform_fixed<36>(buf, nlines, ls, es, jfast, tw, sgn); return;
-    case 40: transform_fixed<40>(buf, nlines, ls, es, jfast, tw, sgn); return;
-    case 48: transform_fixed<48>(buf, nlines, ls, es, jfast, tw, sgn); return;
-    case 56: transform_fixed<56>(buf, nlines, ls, es, jfast, tw, sgn); return;
-    case 64: transform_fixed<64>(buf, nlines, ls, es, jfast, tw, sgn); return;
-    case 72: transform_fixed<72>(buf, nlines, ls, es, jfast, tw, sgn); return;
-    case 80: transform_fixed<80>(buf, nlines, ls, es, jfast, tw, sgn); return;
-    case 96: transform_fixed<96>(buf, nlines, ls, es, jfast, tw, sgn); return;
+    case 16: transform_fixed<16>(buf, nlines, ls, es, tw, sgn); return;
+    case 20: transform_fixed<20>(buf, nlines, ls, es, tw, sgn); return;
+    case 24: transform_fixed<24>(buf, nlines, ls, es, tw, sgn); return;
+    case 28: transform_fixed<28>(buf, nlines, ls, es, tw, sgn); return;
+    case 32: transform_fixed<32>(buf, nlines, ls, es, tw, sgn); return;
+    case 36: transform_fixed<36>(buf, nlines, ls, es, tw, sgn); return;
+    case 40: transform_fixed<40>(buf, nlines, ls, es, tw, sgn); return;
+    case 48: transform_fixed<48>(buf, nlines, ls, es, tw, sgn); return;
+    case 56: transform_fixed<56>(buf, nlines, ls, es, tw, sgn); return;
+    case 64: transform_fixed<64>(buf, nlines, ls, es, tw, sgn); return;
+    case 72: transform_fixed<72>(buf, nlines, ls, es, tw, sgn); return;
+    case 80: transform_fixed<80>(buf, nlines, ls, es, tw, sgn); return;
+    case 96: transform_fixed<96>(buf, nlines, ls, es, tw, sgn); return;
     default: break;
   }
   const int lc = lines_per_chunk(ax, nlines);
@@ -492,13 +485,13 @@ __device__ void transform(C* buf, const AxisArg& ax, int nlines, int ls, int es,
     int ns = 1;
     for (int s = 0; s < ax.nstage; ++s) {
       switch (ax.radix[s]) {
-        case 2: stage<2>(buf, ax.n, ns, l0, nl, ls, es, jfast, tw, sgn); break;
-        case 3: stage<3>(buf, ax.n, ns, l0, nl, ls, es, jfast, tw, sgn); break;
-        case 4: stage<4>(buf, ax.n, ns, l0, nl, ls, es, jfast, tw, sgn); break;
-        case 5: stage<5>(buf, ax.n, ns, l0, nl, ls, es, jfast, tw, sgn); break;
-        case 7: stage<7>(buf, ax.n, ns, l0, nl, ls, es, jfast, tw, sgn); break;
-        case 8: stage<8>(buf, ax.n, ns, l0, nl, ls, es, jfast, tw, sgn); break;
-        case 11: stage<11>(buf, ax.n, ns, l0, nl, ls, es, jfast, tw, sgn); break;
+        case 2: stage<2>(buf, ax.n, ns, l0, nl, ls, es, tw, sgn); break;
+        case 3: stage<3>(buf, ax.n, ns, l0, nl, ls, es, tw, sgn); break;
+        case 4: stage<4>(buf, ax.n, ns, l0, nl, ls, es, tw, sgn); break;
+        case 5: stage<5>(buf, ax.n, ns, l0, nl, ls, es, tw, sgn); break;
+        case 7: stage<7>(buf, ax.n, ns, l0, nl, ls, es, tw, sgn); break;
+        case 8: stage<8>(buf, ax.n, ns, l0, nl, ls, es, tw, sgn); break;
+        case 11: stage<11>(buf, ax.n, ns, l0, nl, ls, es, tw, sgn); break;
       }
       ns *= ax.radix[s];
     }
@@ -555,8 +548,8 @@ __global__ void __launch_bounds__(kPlaneThreads, 2)
   for (int k = plane_off[p] + threadIdx.x; k < plane_off[p + 1]; k += blockDim.x)
     plane[plane_pos[k]] = from_d2<C>(src[plane_g[k]]);
   __syncthreads();
-  transform(plane, a1, nr2, ps, 1, false, tw1, (typename CT<C>::R)1);   // x lines
-  transform(plane, a2, nr1, 1, ps, false, tw2, (typename CT<C>::R)1);   // y lines
+  transform(plane, a1, nr2, ps, 1, tw1, (typename CT<C>::R)1);   // x lines
+  transform(plane, a2, nr1, 1, ps, tw2, (typename CT<C>::R)1);   // y lines
   C* dst = grid + ((size_t)bl * nzp + p) * npl;
   for (int i = threadIdx.x; i < npl; i += blockDim.x) dst[i] = plane[i + i / nr1];
 }
@@ -588,7 +581,7 @@ __global__ void __launch_bounds__(kPlaneThreads, 2)
     tile[i] = val;
   }
   __syncthreads();
-  transform(tile, a3, TX, 1, TX, false, tw, (T)1);
+  transform(tile, a3, TX, 1, TX, tw, (T)1);
   for (int i = threadIdx.x; i < nr3 * TX; i += blockDim.x) {
     int iz = i / TX, x = i % TX;
     double vv = 0.0;
@@ -599,7 +592,7 @@ __global__ void __launch_bounds__(kPlaneThreads, 2)
   // forward transform: conjugated twiddles
   for (int k = threadIdx.x; k < nr3; k += blockDim.x) tw[k].y = -tw[k].y;
   __syncthreads();
-  transform(tile, a3, TX, 1, TX, false, tw, (T)-1);
+  transform(tile, a3, TX, 1, TX, tw, (T)-1);
   for (int i = threadIdx.x; i < nr3 * TX; i += blockDim.x) {
     int iz = i / TX, x = i % TX;
     int s = zslot[iz];
@@ -819,7 +812,7 @@ __global__ void __launch_bounds__(kPlaneThreads, 2)
       tile[i] = val;
     }
     __syncthreads();
-    transform(tile, a3, TX, 1, TX, false, tw, (T)1);
+    transform(tile, a3, TX, 1, TX, tw, (T)1);
 #pragma unroll
     for (int e = 0; e < EPT; ++e) {
       const int i = threadIdx.x + e * blockDim.x;
@@ -1056,8 +1049,8 @@ __global__ void __launch_bounds__(kPlaneThreads, 2)
   load_tw(tw1, tw1g, nr1, -1.0);
   load_tw(tw2, tw2g, nr2, -1.0);
   __syncthreads();
-  transform(plane, a2, nr1, 1, pst, false, tw2, (typename CT<C>::R)-1);  // y lines
-  transform(plane, a1, nr2, pst, 1, false, tw1, (typename CT<C>::R)-1);  // x lines
+  transform(plane, a2, nr1, 1, pst, tw2, (typename CT<C>::R)-1);  // y lines
+  transform(plane, a1, nr2, pst, 1, tw1, (typename CT<C>::R)-1);  // x lines
   double2* dst = out + (size_t)ldg * b;
   const double2* ps = psi + (size_t)ldg * b;
   for (int k = plane_off[p] + threadIdx.x; k < plane_off[p + 1]; k += blockDim.x) {
@@ -1096,7 +1089,7 @@ __global__ void __launch_bounds__(kPlaneThreads)
       tile[r * (n + 1) + x] = grid[(size_t)(row0 + r) * nr1 + x];
     }
     __syncthreads();
-    transform(tile, ax, nl, n + 1, 1, false, tw, sgn);
+    transform(tile, ax, nl, n + 1, 1, tw, sgn);
     for (int i = threadIdx.x; i < nl * n; i += blockDim.x) {
       const int r = i / n, x = i % n;
       grid[(size_t)(row0 + r) * nr1 + x] = tile[r * (n + 1) + x];
@@ -1114,7 +1107,7 @@ __global__ void __launch_bounds__(kPlaneThreads)
     tile[i] = x < nl ? grid[base + (size_t)e * es + x0 + x] : make_double2(0.0, 0.0);
   }
   __syncthreads();
-  transform(tile, ax, TX, 1, TX, false, tw, sgn);
+  transform(tile, ax, TX, 1, TX, tw, sgn);
   for (int i = threadIdx.x; i < n * TX; i += blockDim.x) {
     const int e = i / TX, x = i % TX;
     if (x < nl) grid[base + (size_t)e * es + x0 + x] = tile[i];
@@ -1318,9 +1311,9 @@ static int fft_select(Handle* h) {
   return fft_select_v<C, N1, N2, 0>(h);
 }
 
-// Kernels of the handle's grid and plan variant: grids of the table get
-// kernels compiled for their lengths (every index divisor and Stockham stage a
-// constant); any other grid takes the kernels with run-time lengths.
+// Kernels of the handle's grid and plan variant: grids of the table get xy planes
+// compiled for their lengths (two register steps an axis); any other grid takes
+// the Stockham stages of run-time lengths.  The z kernels go by NR3 alone.
 static int fft_choose(Handle* h) {
   const int nr1 = h->d.nr1, nr2 = h->d.nr2, nr3 = h->d.nr3;
   int rc = CUW_OK;

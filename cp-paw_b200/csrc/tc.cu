@@ -3,12 +3,13 @@
 // Every product is a real GEMM C = A * B^T whose operands are split into tf32
 // pairs (hi + lo) and multiplied as lo*hi + hi*lo + hi*hi with fp32
 // accumulation in tensor memory (three-term split precision), drained after
-// every K = 8 step into register sums (tc_pipe.cuh).  Complex products use the
-// real form of tc_pipe.cuh.  Operand data is staged raw (FP64 wave functions
-// and matrices, the fp32 projector table) with cp.async several chunks ahead,
-// then split in shared memory by the converter warps.  Every wait is bounded;
-// a wait that runs out sets an error flag and the kernel leaves through its
-// cleanup path (TMEM released) instead of hanging.
+// every K = 8 step into register sums (tc_pipe.cuh).  The A operands are the
+// folded fp32 arrays (projector table, wave functions), fetched by TMA several
+// chunks ahead and split by the converter warps on their way into tensor memory;
+// the B operands (folded wave functions, small FP64 matrices) are split by
+// k_bsplit beforehand and arrive by bulk copies.  Every wait is bounded; a wait
+// that runs out sets an error flag and the kernel leaves through its cleanup path
+// (TMEM released) instead of hanging.
 #include <cuda_runtime.h>
 
 #include <algorithm>
