@@ -323,23 +323,23 @@ __device__ __forceinline__ float2 cmulc(float2 a, float2 b) {
 }
 __device__ __forceinline__ float2 cscale(float2 a, float s) { return make_float2(a.x * s, a.y * s); }
 
-// Sum over split-K partials for output i: scale * part[z][i] (z < nz) + oc[z][i]
-// (z < kc) + add of the threads on the output, every array n wide.  A block of 32 x kSumZ threads has kSumZ threads
+// Sum over split-K partials for output i: scaled(sum of part[z][i], z < nz) + oc[z][i]
+// (z < kc), every array n wide; scaled acts on each thread's share.  A block of 32 x kSumZ threads has kSumZ threads
 // on each of 32 outputs, each with every kSumZ-th split (the outputs of small
 // sets are too few to hide the latency of 140 splits one after another: the
 // overlaps of 32 bands took 27 us and take 12); the result is valid in the threads with threadIdx.y == 0.
 constexpr int kSumZ = 8;
 __device__ __forceinline__ double2 split_get(const double2* p) { return *p; }
 __device__ __forceinline__ double2 split_get(const float2* p) { return make_double2((double)p->x, (double)p->y); }
-template <class P>
-__device__ __forceinline__ double2 split_sum(const P* __restrict__ part, int nz, size_t n, size_t i, double2 scale,
-                                             const double2* __restrict__ oc, int kc, double2 add) {
+template <class P, class F>
+__device__ __forceinline__ double2 split_sum(const P* __restrict__ part, int nz, size_t n, size_t i, F scaled,
+                                             const double2* __restrict__ oc, int kc) {
   __shared__ double2 sh[kSumZ][32];
   double2 s = make_double2(0.0, 0.0);
   if (i < n) {
 #pragma unroll 4
     for (int z = threadIdx.y; z < nz; z += kSumZ) s = cadd(s, split_get(part + (size_t)z * n + i));
-    s = cadd(make_double2(s.x * scale.x, s.y * scale.y), add);
+    s = scaled(s);
 #pragma unroll 4
     for (int z = threadIdx.y; z < kc; z += kSumZ) s = cadd(s, oc[(size_t)z * n + i]);
   }
@@ -351,11 +351,10 @@ __device__ __forceinline__ double2 split_sum(const P* __restrict__ part, int nz,
   }
   return s;
 }
-template <class P>
-__device__ __forceinline__ double2 split_sum(const P* __restrict__ part, int nz, size_t n, size_t i, double scale,
-                                             const double2* __restrict__ oc, int kc) {
-  return split_sum(part, nz, n, i, make_double2(scale, scale), oc, kc, make_double2(0.0, 0.0));
-}
+struct Scaled {
+  double f;
+  __device__ __forceinline__ double2 operator()(double2 s) const { return cscale(s, f); }
+};
 
 // (-i)^l
 __device__ __forceinline__ double2 mipow(int l) {
@@ -404,6 +403,48 @@ __device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
 __device__ __forceinline__ double2 row2(const double* p, int i, bool in) {
   const double2 v = *reinterpret_cast<const double2*>(p + (in ? i : 0));
   return make_double2(in ? v.x : 0.0, in ? v.y : 0.0);
+}
+// A warp's 8 x 16 block of A B^T over n values of k (n even), straight from global
+// memory (L2): c0 and c1 are its two 8 x 8 halves; a, b0, b1 the lane's rows
+// (lane / 4) of the operands, k contiguous, and whether they are within them.  Lane
+// k of a fragment takes two neighbouring values of k with one 16-byte load, which
+// fills the fragments of two MMAs.  The sums are short, so what counts is loads in
+// flight: those of the next 64 values are issued before the MMAs of the present
+// ones (the __syncwarp, which no load may pass, would else put them behind the
+// MMAs: 128 bands by 512 projectors take 10.7 us from cold caches, and took 12.4 so).
+__device__ __forceinline__ void rows_8x16(const double* __restrict__ a, bool ain, const double* __restrict__ b0,
+                                          bool in0, const double* __restrict__ b1, bool in1, int n, double (&c0)[2],
+                                          double (&c1)[2]) {
+  constexpr int U = 8, K = 8 * U;
+  const int fk = threadIdx.x & 3;
+  double2 av[2][U], v0[2][U], v1[2][U];
+  auto load = [&](int s, int k0) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int k = k0 + 8 * u + 2 * fk;
+      av[s][u] = row2(a, k, ain && k < n);
+      v0[s][u] = row2(b0, k, in0 && k < n);
+      v1[s][u] = row2(b1, k, in1 && k < n);
+    }
+  };
+  auto products = [&](int s) {
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      dmma(c0, av[s][u].x, v0[s][u].x);
+      dmma(c1, av[s][u].x, v1[s][u].x);
+      dmma(c0, av[s][u].y, v0[s][u].y);
+      dmma(c1, av[s][u].y, v1[s][u].y);
+    }
+  };
+  load(0, 0);
+  for (int k0 = 0; k0 < n; k0 += 2 * K) {  // n is the same for the whole warp
+    const bool second = k0 + K < n;
+    if (second) load(1, k0 + K);
+    products(0);
+    if (k0 + 2 * K < n) load(0, k0 + 2 * K);
+    if (second) products(1);
+  }
 }
 
 // frees device buffers; what is not allocated again at once stays null

@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(32 * kSumZ)
                 double2* __restrict__ out0, double2* __restrict__ out1) {
   const int nw = nset * nbh;
   const size_t n = (size_t)nw * npro, i = blockIdx.x * (size_t)32 + threadIdx.x;
-  const double2 s = split_sum(part, nz, n, i, scale, (const double2*)nullptr, 0);
+  const double2 s = split_sum(part, nz, n, i, Scaled{scale}, (const double2*)nullptr, 0);
   if (threadIdx.y || i >= n) return;
   const int b = (int)(i % nw);
   const size_t p = i / nw;
@@ -373,7 +373,7 @@ __global__ void __launch_bounds__(32 * kSumZ)
     k_rgram_sum(const double2* __restrict__ part, int ks, int kc, int nb, int npair, double scale,
                 double* __restrict__ o0, double* __restrict__ o1, double* __restrict__ o2) {
   const size_t per = (size_t)nb * nb / 2, n = per * npair, t = blockIdx.x * (size_t)32 + threadIdx.x;
-  const double2 s = split_sum(part, ks, n, t, scale, part + (size_t)ks * n, kc);
+  const double2 s = split_sum(part, ks, n, t, Scaled{scale}, part + (size_t)ks * n, kc);
   if (threadIdx.y || t >= n) return;
   const int pair = (int)(t / per);
   const size_t e = 2 * (t % per);
@@ -669,13 +669,9 @@ __global__ void __launch_bounds__(RT, 2) k_rforce(Op u, Op ded, const double* __
 }
 
 // PROJ(n, p) += sum_m O(m, p) Lambda(m, n) on the real views (n + NB p) of the
-// projection arrays (WAVES_ADDOPROJ, src/paw_waves2.f90:687-758).  A warp forms
-// 8 n x 16 p on the FP64 tensor cores straight from global memory (L2): both
-// operands run along m, and lane k of a fragment takes m = 8 s + 2 k and the
-// next one with one 16-byte load (NB is even), so a load fills the fragments
-// of two MMAs.  The sum is short (NB terms), so what counts is that all of its
-// loads are in flight at once: 128 bands and 512 projectors take 9.1 us, and
-// took 19.5 us through shared memory, 32 values of m at a time.
+// projection arrays (WAVES_ADDOPROJ, src/paw_waves2.f90:687-758), 8 n x 16 p a
+// warp: 128 bands and 512 projectors take 10.7 us (19.5 through shared memory, 32
+// values of m at a time).
 __global__ void __launch_bounds__(128) k_raddoproj(double* __restrict__ out, const double* __restrict__ x,
                                                    const double* __restrict__ lam, int npro, int nb) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, fr = lane >> 2, fk = lane & 3;
@@ -685,35 +681,15 @@ __global__ void __launch_bounds__(128) k_raddoproj(double* __restrict__ out, con
   const double* la = lam + (size_t)nb * (an ? n0 + fr : 0);
   const double* x0 = x + (size_t)nb * (b0 ? p0 + fr : 0);
   const double* x1 = x + (size_t)nb * (b1 ? p0 + 8 + fr : 0);
-  double c0[2] = {0.0, 0.0}, c1[2] = {0.0, 0.0};
-  constexpr int U = 8;
-  for (int m0 = 0; m0 < nb; m0 += 8 * U) {
-    double2 a[U], v0[U], v1[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int m = m0 + 8 * u + 2 * fk;
-      const bool in = m < nb;
-      a[u] = row2(la, m, in && an);
-      v0[u] = row2(x0, m, in && b0);
-      v1[u] = row2(x1, m, in && b1);
-    }
-    __syncwarp();
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      dmma(c0, a[u].x, v0[u].x);
-      dmma(c1, a[u].x, v1[u].x);
-      dmma(c0, a[u].y, v0[u].y);
-      dmma(c1, a[u].y, v1[u].y);
-    }
-  }
+  double old[4], c0[2] = {0.0, 0.0}, c1[2] = {0.0, 0.0};
   const int n = n0 + fr;
-  if (n >= nb) return;
+  auto col = [&](int k) { return p0 + 8 * (k >> 1) + 2 * fk + (k & 1); };
 #pragma unroll
-  for (int e = 0; e < 2; ++e) {
-    const int p = p0 + 2 * fk + e;
-    if (p < npro) out[n + (size_t)nb * p] += c0[e];
-    if (p + 8 < npro) out[n + (size_t)nb * (p + 8)] += c1[e];
-  }
+  for (int k = 0; k < 4; ++k) old[k] = an && col(k) < npro ? out[n + (size_t)nb * col(k)] : 0.0;  // under the products
+  rows_8x16(la, an, x0, b0, x1, b1, nb, c0, c1);
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (an && col(k) < npro) out[n + (size_t)nb * col(k)] = old[k] + (k < 2 ? c0[k] : c1[k - 2]);
 }
 
 }  // namespace

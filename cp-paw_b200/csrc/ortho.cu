@@ -1545,13 +1545,10 @@ __global__ void __launch_bounds__(512, 1) k_ortho_x_pnl(OrthoArgs a) {
   cl.sync();
 }
 
-// C = A^T B for n x n matrices (n even): a warp forms 8 x 16 on the FP64 tensor
-// cores straight from L2.  Both operands run along the summation index, and
-// lane k of a fragment takes two neighbouring terms with one 16-byte load, all
-// loads of 64 terms in flight.  With e, the diagonal goes there and to b, the
-// rest to b and em.  From cold caches 128 bands take 10 us, as in 32 x 32 tiles
-// through shared memory; what it saves is the launch that split the diagonal
-// off, and a step of Si64 takes 7 us less with the gated copies gone too.
+// C = A^T B for n x n matrices (n even), 8 x 16 a warp.  With e, the diagonal goes
+// there and to b, the rest to b and em: what this saves against 32 x 32 tiles
+// through shared memory, which take 10 us for 128 bands against 11, is the launch
+// that split the diagonal off.
 __global__ void __launch_bounds__(128) k_gemm_tn(const double* __restrict__ A, const double* __restrict__ B, int n,
                                                  double* __restrict__ b, double* __restrict__ e,
                                                  double* __restrict__ em) {
@@ -1563,26 +1560,7 @@ __global__ void __launch_bounds__(128) k_gemm_tn(const double* __restrict__ A, c
   const double* p0 = B + (size_t)n * (b0 ? j0 + fr : 0);
   const double* p1 = B + (size_t)n * (b1 ? j0 + 8 + fr : 0);
   double c0[2] = {0.0, 0.0}, c1[2] = {0.0, 0.0};
-  constexpr int U = 8;
-  for (int m0 = 0; m0 < n; m0 += 8 * U) {
-    double2 a[U], v0[U], v1[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int m = m0 + 8 * u + 2 * fk;
-      const bool in = m < n;
-      a[u] = row2(pa, m, in && ai);
-      v0[u] = row2(p0, m, in && b0);
-      v1[u] = row2(p1, m, in && b1);
-    }
-    __syncwarp();
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      dmma(c0, a[u].x, v0[u].x);
-      dmma(c1, a[u].x, v1[u].x);
-      dmma(c0, a[u].y, v0[u].y);
-      dmma(c1, a[u].y, v1[u].y);
-    }
-  }
+  rows_8x16(pa, ai, p0, b0, p1, b1, n, c0, c1);
   const int i = i0 + fr;
 #pragma unroll
   for (int k = 0; k < 4; ++k) {

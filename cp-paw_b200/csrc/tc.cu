@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(32 * kSumZ)
                   double2* __restrict__ out0, double2* __restrict__ out1) {
   const int nw = nset * nbh;
   const size_t n = (size_t)nw * npro, i = blockIdx.x * (size_t)32 + threadIdx.x;
-  const double2 s = split_sum(part, nz, n, i, scale, (const double2*)nullptr, 0);
+  const double2 s = split_sum(part, nz, n, i, Scaled{scale}, (const double2*)nullptr, 0);
   if (threadIdx.y || i >= n) return;
   const int b = (int)(i % nw);
   const size_t p = i / nw;
@@ -167,19 +167,22 @@ __global__ void __launch_bounds__(32 * kSumZ)
     k_tc_gram_sum(const float2* __restrict__ part, int nz, const double2* __restrict__ oc, int kc,
                   const double* __restrict__ dg, int nd, int3 which, int nb, int npair, double scale,
                   double* __restrict__ o0, double* __restrict__ o1, double* __restrict__ o2) {
-  const size_t per = (size_t)nb * nb / 2, n = per * npair, t = blockIdx.x * (size_t)32 + threadIdx.x;
-  const int pair = (int)(t / per);
-  const size_t e = 2 * (t % per);
-  const int i = (int)(e / nb), j = (int)(e % nb);
-  double2 sc = make_double2(scale, scale), add = make_double2(0.0, 0.0);
-  if (t < n && (i & ~1) == j) {
-    const int q = pair == 0 ? which.x : (pair == 1 ? which.y : which.z);
-    double d = 0.0;
-    for (int z = threadIdx.y; z < nd; z += kSumZ) d += dg[((size_t)z * 3 + q) * nb + i];
-    (i == j ? add.x : add.y) = scale * d;
-    (i == j ? sc.x : sc.y) = 0.0;
-  }
-  const double2 s = split_sum(part, nz, n, t, sc, oc, kc, add);
+  // one row of one pair and 32 pairs of columns a block (index divisions in front of
+  // the loads took 3 us of 10)
+  const int pair = blockIdx.z, i = blockIdx.y, c = blockIdx.x * 32 + threadIdx.x, j = 2 * c, w = nb / 2;
+  const size_t n = (size_t)npair * nb * w, t = c < w ? ((size_t)pair * nb + i) * w + c : n;
+  const int q = pair == 0 ? which.x : (pair == 1 ? which.y : which.z);
+  auto scaled = [&](double2 v) {
+    v = cscale(v, scale);
+    if (c == i >> 1) {
+      double d = 0.0;
+#pragma unroll 4
+      for (int z = threadIdx.y; z < nd; z += kSumZ) d += dg[((size_t)z * 3 + q) * nb + i];
+      (i & 1 ? v.y : v.x) = scale * d;
+    }
+    return v;
+  };
+  const double2 s = split_sum(part, nz, n, t, scaled, oc, kc);
   if (threadIdx.y || t >= n) return;
   double* o = pair == 0 ? o0 : (pair == 1 ? o1 : o2);
   o[i + (size_t)nb * j] = s.x;
@@ -1150,7 +1153,7 @@ int tc_gram(Handle* h, const FoldPair* pairs, int npair, double* o0, double* o1,
       a, tm, reinterpret_cast<float*>(h->g.part), tc_err(h));
   CUW_LAUNCH_CHECK("k_tc_tn");
   auto which = [&](int i) { return i < npair ? pairs[i].x + pairs[i].y : 0; };
-  k_tc_gram_sum<<<(unsigned)((n / 2 + 31) / 32), dim3(32, kSumZ), 0, h->stream>>>(
+  k_tc_gram_sum<<<dim3(ceil_div(nb / 2, 32), nb, npair), dim3(32, kSumZ), 0, h->stream>>>(
       reinterpret_cast<const float2*>(h->g.part), ks, reinterpret_cast<const double2*>(oc), kc, h->g.diag,
       diag_ranges(h), make_int3(which(0), which(1), which(2)), nb, npair, 0.5 * h->gweight, o0, o1, o2);
   CUW_LAUNCH_CHECK("k_tc_gram_sum");
