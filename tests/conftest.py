@@ -64,12 +64,14 @@ class FakeEngine:
 @pytest.fixture(scope="session")
 def fake_engine(engine_lib, tmp_path_factory):
     import glob
+    import shutil
     import subprocess
 
     import build as b
 
     out = str(tmp_path_factory.mktemp("fake") / "libfake.so")
-    cuda = os.path.join(os.path.dirname(os.path.dirname(b.nvcc())), "include")
+    nvcc = shutil.which(b.nvcc()) or b.nvcc()
+    cuda = os.path.join(os.path.dirname(os.path.dirname(nvcc)), "include")
     subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-Wl,--no-undefined,-Bsymbolic", f"-I{cuda}", "-o", out,
                     os.path.join(ROOT, "tests", "fake_cuda.cpp"), *sorted(glob.glob(os.path.join(b.OBJ, "*.o"))),
                     "-lpthread"], check=True)
