@@ -31,6 +31,18 @@ def test_plane_variants(grid, prec, oracle):
         check(grid, prec, oracle, 60.0, (0,))
 
 
+# every length with Stockham stages of its own, and run-time lengths beside them, on
+# planes that are not in the table; the last three differ from table grids in NR3 only
+OTHER = ((16, 20, 24), (24, 28, 24), (32, 36, 24), (40, 48, 24), (56, 64, 24), (72, 80, 24), (96, 16, 24), (42, 84, 24),
+         (24, 24, 48), (28, 28, 84), (28, 56, 80))
+
+
+@pytest.mark.parametrize("prec", [CUW_PREC_FP64, CUW_PREC_MIXED])
+@pytest.mark.parametrize("grid", OTHER)
+def test_planes_off_the_table(grid, prec, oracle):
+    check(grid, prec, oracle, 9.0)
+
+
 def check(grid, prec, oracle, ry, variants=(0,)):
     """H|psi> and the density against the oracle.  Both are sums of a few
     transforms' outputs: each step of a transform rounds by half an ulp of its
